@@ -1,7 +1,8 @@
 """ctypes binding of csrc/libmetile_b200.so (C ABI declared in include/metile_b200.h).
 
-The shared object is built in-tree by `python -m metile_b200.build`.  If it is missing the
-import of any operator fails loudly: there is no CPU or PyTorch fallback on this path.
+The shared object is built in-tree by `python -m metile_b200.build`, and with it `_native.so`, the
+module through which torch tensors reach the same entry points (csrc/binding.cpp).  If one is missing
+the first call of any operator fails loudly: there is no CPU or PyTorch fallback on this path.
 """
 
 from __future__ import annotations
@@ -57,6 +58,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 
 
 def load():
@@ -76,6 +78,20 @@ def load():
         function.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def native():
+    """The torch binding; raise if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as error:
+            raise ImportError(f"metile_b200/_native.so cannot be loaded ({error}). Build it with `python -m "
+                              "metile_b200.build`; this package has no fallback path.") from error
+        _native = module
+    return _native
 
 
 def status_string(code):

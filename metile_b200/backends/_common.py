@@ -105,3 +105,17 @@ def check_affine_triple(name, values, weight, scales, biases, group_size, bits):
 
 def library():
     return _lib.load()
+
+
+def native():
+    """The torch binding (csrc/binding.cpp).  Its functions serve the plain case of an operator -- contiguous
+    tensors of the documented types on one device -- and answer None for anything else, which the
+    operators below then check, copy or refuse in Python."""
+    return _lib.native()
+
+
+def native_result(result, what):
+    """The tensor(s) a native call returned, or the exception its status code stands for."""
+    if type(result) is int:
+        _lib.check(result, what)
+    return result

@@ -15,12 +15,24 @@ import ctypes
 import torch
 
 from .. import _lib
-from ._common import launch, library, pointer, require_cuda_bf16, require_on_device, rows_of
+from ._common import (
+    launch,
+    library,
+    native,
+    native_result,
+    pointer,
+    require_cuda_bf16,
+    require_on_device,
+    rows_of,
+)
 
 
 def mlx_rms_norm(values, weight, eps, *, autotune=True):
     """RMSNorm over the last axis: bf16(x * rsqrt(mean(x^2) + eps) * w)."""
     del autotune
+    out = native().norm(values, None, weight, eps)
+    if out is not None:
+        return native_result(out, "mlx_rms_norm")
     if values.ndim < 1 or weight.ndim != 1 or values.shape[-1] != weight.shape[0]:
         raise ValueError("meTile RMSNorm requires a matching one-dimensional weight")
     if values.dtype != weight.dtype:
@@ -41,6 +53,9 @@ def mlx_rms_norm(values, weight, eps, *, autotune=True):
 def mlx_add_rms_norm(values, residual, weight, eps, *, autotune=True):
     """Fused residual add + RMSNorm; returns (summed, normalized)."""
     del autotune
+    pair = native().norm(values, residual, weight, eps)
+    if pair is not None:
+        return native_result(pair, "mlx_add_rms_norm")
     if values.shape != residual.shape or values.dtype != residual.dtype:
         raise ValueError("meTile fused add/RMSNorm requires matching residual inputs")
     if values.ndim < 1 or weight.ndim != 1 or values.shape[-1] != weight.shape[0]:
@@ -108,6 +123,9 @@ def mlx_attention_decode(query, key, value, *, scale, autotune=True, lengths=Non
     larger in-place cache [B, Hkv, capacity, D] (no copy is made either way).  `lengths` (int32 [B] on
     the device) limits sequence b to its first lengths[b] tokens.  Returns [B, Hq, 1, D]."""
     del autotune
+    out = native().attention(query, key, value, scale, lengths)
+    if out is not None:
+        return native_result(out, "mlx_attention_decode")
     if query.ndim != 4 or key.ndim != 4 or value.ndim != 4:
         raise ValueError("meTile attention expects rank-four query, key, and value arrays")
     if query.shape[2] != 1:
@@ -149,6 +167,9 @@ def rope_kv_append(query, key, value, positions, key_cache, value_cache, *, thet
     q|k|v projection [B, (Hq + 2 Hkv) D] (no copy is made); positions int32 [B] (device): the row of
     each sequence's cache [B, Hkv, capacity, D] that receives the new token.  Returns the rotated
     query as a dense [B, Hq, D] tensor."""
+    out = native().rope_kv_append(query, key, value, positions, key_cache, value_cache, theta)
+    if out is not None:
+        return native_result(out, "rope_kv_append")
     require_cuda_bf16(query, "rope_kv_append")
     batch, q_heads, dim = query.shape
     kv_heads, capacity = key_cache.shape[1], key_cache.shape[2]

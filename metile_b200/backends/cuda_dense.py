@@ -10,7 +10,16 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from ._common import contiguous_2d, launch, library, pointer, require_cuda_bf16, require_on_device
+from ._common import (
+    contiguous_2d,
+    launch,
+    library,
+    native,
+    native_result,
+    pointer,
+    require_cuda_bf16,
+    require_on_device,
+)
 
 
 def _check_dense(name, values, weight):
@@ -28,6 +37,9 @@ def _check_dense(name, values, weight):
 def mlx_dense_residual_qmv(values, weight, residual=None):
     """bf16(bf16(values @ weight^T) + residual); residual may be None."""
     name = "dense residual projection"
+    out = native().dense(values, weight, None, residual)
+    if out is not None:
+        return native_result(out, name)
     _check_dense(name, values, weight)
     expected = (*values.shape[:-1], weight.shape[0])
     if residual is not None and (tuple(residual.shape) != expected or residual.dtype != values.dtype):
@@ -45,6 +57,9 @@ def mlx_dense_residual_qmv(values, weight, residual=None):
 def mlx_dense_swiglu(values, gate_weight, up_weight):
     """Typed SwiGLU of two dense projections (each rounded to bf16 before the activation)."""
     name = "dense SwiGLU"
+    out = native().dense(values, gate_weight, up_weight, None)
+    if out is not None:
+        return native_result(out, name)
     _check_dense(name, values, gate_weight)
     _check_dense(name, values, up_weight)
     if gate_weight.shape != up_weight.shape:

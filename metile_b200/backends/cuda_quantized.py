@@ -34,6 +34,8 @@ from ._common import (
     contiguous_2d,
     launch,
     library,
+    native,
+    native_result,
     pointer,
     require_cuda_bf16,
     require_on_device,
@@ -89,11 +91,17 @@ def _algorithm(rows, flags):
 
 def _record(table, rows, input_features, output_features, dtype, group_size, bits, flags):
     key = (rows, input_features, output_features, str(dtype), group_size, bits)
-    with _dispatch_lock:
-        table[key] = _algorithm(rows, flags)
+    algorithm = _algorithm(rows, flags)
+    if table.get(key) != algorithm:
+        with _dispatch_lock:
+            table[key] = algorithm
 
 
 def _project(name, values, weight, scales, biases, residual, group_size, bits):
+    flags = _flags()
+    out = native().project(values, weight, scales, biases, residual, group_size, bits, flags)
+    if out is not None:
+        return native_result(out, name), flags
     require_cuda_bf16(values, name)
     output_features = check_affine_triple(name, values, weight, scales, biases, group_size, bits)
     expected_shape = (*values.shape[:-1], output_features)
@@ -104,7 +112,6 @@ def _project(name, values, weight, scales, biases, residual, group_size, bits):
     x = contiguous_2d(values)
     res = None if residual is None else contiguous_2d(residual)
     out = torch.empty((x.shape[0], output_features), dtype=values.dtype, device=values.device)
-    flags = _flags()
     code = launch(library().mt_affine_qmv, values.device, pointer(x), pointer(weight), pointer(scales),
                   pointer(biases), pointer(res), pointer(out), x.shape[0], x.shape[1], output_features,
                   group_size, bits, flags)
@@ -135,6 +142,14 @@ def mlx_affine_residual_qmv(values, weight, scales, biases, residual, *, group_s
 
 def _swiglu(name, values, gate_weight, gate_scales, gate_biases, up_weight, up_scales, up_biases,
             group_size, bits):
+    flags = _flags()
+    if bits == 4 and group_size == 64:
+        out = native().swiglu(values, gate_weight, gate_scales, gate_biases, up_weight, up_scales, up_biases, flags)
+        if out is not None:
+            native_result(out, name)
+            _record(_swiglu_dispatches, rows_of(values), values.shape[-1], gate_weight.shape[0], values.dtype,
+                    group_size, bits, flags)
+            return out
     if not (bits == 4 and group_size == 64):
         raise ValueError(f"{name} requires 4-bit group-64 weights")
     if gate_biases is None or up_biases is None:
@@ -153,7 +168,6 @@ def _swiglu(name, values, gate_weight, gate_scales, gate_biases, up_weight, up_s
     check_affine_triple(name, values, up_weight, up_scales, up_biases, group_size, bits)
     x = contiguous_2d(values)
     out = torch.empty((x.shape[0], output_features), dtype=values.dtype, device=values.device)
-    flags = _flags()
     code = launch(library().mt_affine_swiglu, values.device, pointer(x), pointer(gate_weight),
                   pointer(gate_scales), pointer(gate_biases), pointer(up_weight), pointer(up_scales),
                   pointer(up_biases), pointer(out), x.shape[0], x.shape[1], output_features, group_size,
@@ -227,8 +241,12 @@ def mlx_affine_mlp_executor(sample_values, gate_weight, gate_scales, gate_biases
     pointers = [pointer(t) for t in bound]
 
     workspace = {"hidden": None}  # grow-only scratch for the bf16 hidden activations, owned by the callable
+    plan, call = native().mlp_plan(*bound), native().mlp
 
     def execute(values, residual=None):
+        out = call(plan, values, residual, workspace["hidden"], _flags())
+        if out is not None:
+            return native_result(out, name)
         if not isinstance(values, torch.Tensor) or values.dtype != torch.bfloat16 \
                 or values.shape[-1] != hidden_features:
             raise ValueError("affine MLP executor received activations of a different layout")
