@@ -62,8 +62,10 @@ class GraphedDecoder:
         if min(lengths) < 1:
             raise ValueError("prefill before the first decode step")
         real, token = self.cache, self.token.clone()
+        # Inside the `with` the current stream IS self.stream: what the caller queued before must be waited
+        # for here, outside it.
+        self.stream.wait_stream(torch.cuda.current_stream(self.device))
         with torch.no_grad(), torch.cuda.stream(self.stream):
-            self.stream.wait_stream(torch.cuda.current_stream(self.device))
             scratch = self.model.make_cache(self.batch, self.capacity)
             for cache, length in zip(scratch, lengths):
                 cache.reset(length)
@@ -89,10 +91,11 @@ class GraphedDecoder:
             self._capture()
         if self.cache[0].length + 1 > self.capacity:
             raise ValueError("KV cache capacity exceeded")
+        caller = torch.cuda.current_stream(self.device)
+        self.stream.wait_stream(caller)       # the token and the caches as the caller's stream leaves them
         with torch.cuda.stream(self.stream):
-            self.stream.wait_stream(torch.cuda.current_stream(self.device))
             self.graph.replay()
-        torch.cuda.current_stream(self.device).wait_stream(self.stream)
+        caller.wait_stream(self.stream)
         for cache in self.cache:
             cache.length += 1                 # the device-side count was advanced by the graph
         return self.logits
