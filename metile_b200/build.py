@@ -66,7 +66,7 @@ def build(force=False, verbose=False):
     if force or is_stale():
         command = [
             _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
-            "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xlinker", "-soname=libmetile_b200.so",
+            "-shared", "-Xcompiler", "-fPIC,-fno-gnu-unique", "--expt-relaxed-constexpr", "-Xlinker", "-soname=libmetile_b200.so",
         ]
         if verbose:
             command += ["-Xptxas", "-v"]

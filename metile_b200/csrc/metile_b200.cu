@@ -71,16 +71,7 @@ static int run_projection(const void* x, const AffineWeights& first, const Affin
         return second ? launch_gemv<true>(x, a, b, residual, out, M, K, N, sms, stream)
                       : launch_gemv<false>(x, a, b, residual, out, M, K, N, sms, stream);
     }
-    const uint16_t* xp = static_cast<const uint16_t*>(x);
-    const uint16_t* rp = static_cast<const uint16_t*>(residual);
-    uint16_t* op = static_cast<uint16_t*>(out);
-    for (int m0 = 0; m0 < M; m0 += 128) {
-        const int rows = M - m0 < 128 ? M - m0 : 128;
-        const int rc = launch_umma(xp + (size_t)m0 * K, &first, second, rp ? rp + (size_t)m0 * N : nullptr,
-                                   op + (size_t)m0 * N, rows, K, N, stream);
-        if (rc != MT_OK) return rc;
-    }
-    return MT_OK;
+    return launch_umma(x, &first, second, residual, out, M, K, N, stream);
 }
 
 // C[M,N] = act(A[M,K] @ B[K,N]); a thread owns two adjacent output columns of kRows rows.
