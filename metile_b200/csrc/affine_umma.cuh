@@ -109,6 +109,7 @@ struct UmmaParams {
     int unit_shift;        // log2 of the accumulator units in tensor memory
     int sum_bytes;         // shared memory of the running sum over a CTA's slices, or of the slices a cluster's CTA adds
     bool wide_out;         // rows of the output and the residual are 16-byte aligned
+    bool paired;           // the output and the residual have the same alignment within a 4-byte word
     bool windows;          // the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables)
 };
 
@@ -560,22 +561,45 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 const int m0 = (tile - row_tile * p.act_tiles) * npad;
                 const int rows = min(npad, p.M - m0);
                 const int n_tile = row_tile * kOut;
-                // Residual vectors of sixteen activation rows, requested one step ahead (two steps took eight registers
-                // that are not there); the first ones leave while the tile is still being multiplied.
-                const bool staged_residual = !kSwiglu && p.residual && p.wide_out;
-                uint4 extra[kOut / 64];
-                auto request_residual = [&](int c0, uint4 (&into)[kOut / 64]) {
+                // Residuals of sixteen activation rows, requested one step ahead (two steps took eight registers that
+                // are not there); the first ones leave while the tile is still being multiplied.  Vectors of eight
+                // where rows are 16-byte aligned; else words: warp q has rows 4 q .. 4 q + 3 of a step, a lane the
+                // aligned pairs `lane` and `lane + 32` of each, counted from the row's first element less `row_odd`.
+                const bool staged_residual = !kSwiglu && p.residual != nullptr;
+                uint32_t extra[8];
+                auto row_odd = [&](int m) { return (int)((reinterpret_cast<uintptr_t>(p.out) >> 1) + (uint32_t)(m0 + m) * (uint32_t)p.N) & 1; };
+                auto request_residual = [&](int c0) {
                     if constexpr (!kSwiglu) {
                         if (!staged_residual || c0 >= rows) return;
+                        if (p.wide_out) {
 #pragma unroll
-                        for (int i = 0; i < kOut / 64; ++i) {
-                            const int at = thread + 128 * i, m = c0 + at / kVectors, n = n_tile + at % kVectors * 8;
-                            into[i] = m < rows && n < p.N ? ptx::ld_global_dependent_u4(p.residual + (size_t)(m0 + m) * p.N + n)
-                                                           : make_uint4(0u, 0u, 0u, 0u);
+                            for (int i = 0; i < 2; ++i) {
+                                const int at = thread + 128 * i, m = c0 + at / kVectors, n = n_tile + at % kVectors * 8;
+                                if (m < rows && n < p.N) {
+                                    const uint4 v = ptx::ld_global_dependent_u4(p.residual + (size_t)(m0 + m) * p.N + n);
+                                    extra[4 * i] = v.x; extra[4 * i + 1] = v.y; extra[4 * i + 2] = v.z; extra[4 * i + 3] = v.w;
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const int m = c0 + quadrant * 4 + (i >> 1), n = n_tile + 2 * (lane + 32 * (i & 1)) - row_odd(m);
+                                const uint16_t* from = p.residual + (size_t)(m0 + m) * p.N + n;
+                                uint32_t lo = 0, hi = 0;
+                                if (m < rows) {
+                                    if (n >= n_tile && n + 1 < p.N && p.paired) {
+                                        extra[i] = ptx::ld_global_dependent_u32(from);
+                                        continue;
+                                    }
+                                    if (n >= n_tile && n < p.N) lo = ptx::ld_global_dependent_u16(from);
+                                    if (n + 1 < p.N) hi = ptx::ld_global_dependent_u16(from + 1);
+                                }
+                                extra[i] = lo | (hi << 16);
+                            }
                         }
                     }
                 };
-                request_residual(0, extra);
+                request_residual(0);
 
                 // Slices that the final pass does not read itself go to the running sum, which holds all padded rows.
                 const int direct = kSwiglu && my_slices == 2 ? 2 : 1;
@@ -621,27 +645,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
 #pragma unroll
                         for (int j = 0; j < 16; ++j) v[j] = sums[(c0 + j) * kUmmaTileRows] + v[j];
                     }
-                    if constexpr (!kSwiglu) {
-                        if (!p.wide_out) {
-                            // Rows that cannot be stored as vectors (N not a multiple of eight): two bytes at a time.
-                            const int n = n_tile + thread;
-                            const size_t at = (size_t)(m0 + c0) * p.N + n;
-#pragma unroll
-                            for (int part = 0; part < 2; ++part) {
-                                uint32_t narrow[8];
-#pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    narrow[j] = p.residual && n < p.N && c0 + 8 * part + j < rows
-                                                    ? ptx::ld_global_dependent_u16(p.residual + at + (size_t)(8 * part + j) * p.N) : 0u;
-#pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    if (n < p.N && c0 + 8 * part + j < rows)
-                                        p.out[at + (size_t)(8 * part + j) * p.N] =
-                                            f32_to_bf16_bits(fmaf(v[8 * part + j], kDequantUndo, bf16_bits_to_f32(narrow[j])));
-                            }
-                            continue;
-                        }
-                    }
                     if constexpr (kSwiglu) {
                         float gate[8], up[8], value[8];
 #pragma unroll
@@ -670,11 +673,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                                 const float4 hi = *reinterpret_cast<const float4*>(out_tile + j * kPitch + at % kVectors * 8 + 4);
                                 uint4 packed;
                                 if (staged_residual) {
-                                    const uint4 r = extra[i];
-                                    packed.x = pack_bf16x2(lo.x + bf16_lo(r.x), lo.y + bf16_hi(r.x));
-                                    packed.y = pack_bf16x2(lo.z + bf16_lo(r.y), lo.w + bf16_hi(r.y));
-                                    packed.z = pack_bf16x2(hi.x + bf16_lo(r.z), hi.y + bf16_hi(r.z));
-                                    packed.w = pack_bf16x2(hi.z + bf16_lo(r.w), hi.w + bf16_hi(r.w));
+                                    const uint32_t* r = &extra[4 * i];
+                                    packed.x = pack_bf16x2(lo.x + bf16_lo(r[0]), lo.y + bf16_hi(r[0]));
+                                    packed.y = pack_bf16x2(lo.z + bf16_lo(r[1]), lo.w + bf16_hi(r[1]));
+                                    packed.z = pack_bf16x2(hi.x + bf16_lo(r[2]), hi.y + bf16_hi(r[2]));
+                                    packed.w = pack_bf16x2(hi.z + bf16_lo(r[3]), hi.w + bf16_hi(r[3]));
                                 } else {
                                     packed = make_uint4(pack_bf16x2(lo.x, lo.y), pack_bf16x2(lo.z, lo.w), pack_bf16x2(hi.x, hi.y),
                                                         pack_bf16x2(hi.z, hi.w));
@@ -682,9 +685,33 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                                 *reinterpret_cast<uint4*>(p.out + (size_t)(m0 + c0 + j) * p.N + n) = packed;
                             }
                         }
-                        request_residual(c0 + 16, extra);
+                        request_residual(c0 + 16);
+                    } else if constexpr (!kSwiglu) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int j = quadrant * 4 + (i >> 1), m = c0 + j;
+                            if (m >= rows) continue;
+                            const int e = 2 * (lane + 32 * (i & 1)) - row_odd(m), n = n_tile + e;
+                            const float* from = out_tile + j * kPitch + e;
+                            const uint32_t r = staged_residual ? extra[i] : 0u;
+                            uint16_t* to = p.out + (size_t)(m0 + m) * p.N + n;
+                            if (e >= 0 && n + 1 < p.N) {
+                                *reinterpret_cast<uint32_t*>(to) = pack_bf16x2(from[0] + bf16_lo(r), from[1] + bf16_hi(r));
+                            } else {
+                                if (e >= 0 && n < p.N) to[0] = f32_to_bf16_bits(from[0] + bf16_lo(r));
+                                if (e < 0) to[1] = f32_to_bf16_bits(from[1] + bf16_hi(r));
+                            }
+                        }
+                        // The last element of a row that starts in the middle of a word.
+                        const int j = quadrant * 4 + (lane & 3), m = c0 + j, n = n_tile + 127;
+                        if (lane < 4 && m < rows && n < p.N && row_odd(m)) {
+                            const size_t at = (size_t)(m0 + m) * p.N + n;
+                            const float r = staged_residual ? bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + at)) : 0.0f;
+                            p.out[at] = f32_to_bf16_bits(out_tile[j * kPitch + 127] + r);
+                        }
+                        request_residual(c0 + 16);
                     } else {
-                        const int o = thread % kOut, n = n_tile + o;  // gate|up only
+                        const int o = thread % kOut, n = n_tile + o;
                         for (int j = thread / kOut; j < 16 && c0 + j < rows; j += 128 / kOut)
                             if (n < p.N) p.out[(size_t)(m0 + c0 + j) * p.N + n] = f32_to_bf16_bits(out_tile[j * kPitch + o]);
                     }
@@ -1090,6 +1117,7 @@ inline int launch_umma(const void* x, const AffineWeights* first, const AffineWe
     params.N = N;
     params.row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128;
     params.wide_out = N % 8 == 0 && aligned_to(out, 16) && (!residual || aligned_to(residual, 16));
+    params.paired = residual && (reinterpret_cast<uintptr_t>(out) - reinterpret_cast<uintptr_t>(residual)) % 4 == 0;
     params.windows = (K / kUmmaBlockK) % 4 != 0;
     for (int t = 0; t < 2; ++t)
         params.windows = params.windows || !aligned_to(params.scales[t], 8) || !aligned_to(params.biases[t], 8);

@@ -303,6 +303,12 @@ __device__ __forceinline__ uint32_t ld_global_dependent_u16(const uint16_t* p) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t ld_global_dependent_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // 128-bit load served from L2, for data other CTAs of the SAME grid wrote before a grid-wide barrier.
 __device__ __forceinline__ uint4 ld_global_l2_u4(const void* p) {
     uint4 v;
