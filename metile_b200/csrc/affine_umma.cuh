@@ -70,24 +70,28 @@ constexpr int kUmmaMaxXSlots = 8;
 constexpr int kUmmaStages = 2;                       // operand stages of four k-blocks, one per dequant group
 constexpr int kUmmaBarrierBytes = 512;
 constexpr int kUmmaOutBytes = 16 * 128 * 4;          // epilogue: sixteen activation rows of the tile, fp32
+constexpr int kUmmaResidualPitch = 272;              // bytes of a residual row: 128 elements and the words at both ends
+constexpr int kUmmaResidualSteps = 4;                // steps of sixteen rows whose residuals are in flight
+constexpr int kUmmaResidualBytes = kUmmaResidualSteps * 16 * kUmmaResidualPitch;
 constexpr int kUmmaSmemBytes = 227 * 1024;           // one CTA per SM, whatever the row count
 constexpr int kUmmaTmemCols = 512;                   // 256 accumulator columns, 2 x 128 operand columns
 constexpr int kUmmaAColumn = 256;
 
 // Activation slots of two k-blocks.
-__host__ __device__ constexpr int umma_x_slots(int npad, bool windows, int sum_bytes) {
-    return npad > 64 ? (windows ? 4 : 5) : sum_bytes ? 6 : 8;
+__host__ __device__ constexpr int umma_x_slots(int npad, bool windows, int side_bytes) {
+    return npad > 64 ? (windows || side_bytes ? 4 : 5) : side_bytes ? 6 : 8;
 }
 // Ring depth: what the activation slots and the sums leave of shared memory.  With unaligned tables there are
 // three more table entries than slots (see UmmaTables).
-__host__ __device__ constexpr int umma_ring_slots(int npad, bool windows, int sum_bytes) {
-    const int x_bytes = umma_x_slots(npad, windows, sum_bytes) * 2 * npad * 128;
-    const int left = kUmmaSmemBytes - 1024 - kUmmaBarrierBytes - kUmmaOutBytes - sum_bytes - x_bytes - (windows ? 3 * kUmmaTableBytes : 0);
+__host__ __device__ constexpr int umma_ring_slots(int npad, bool windows, int side_bytes) {
+    const int x_bytes = umma_x_slots(npad, windows, side_bytes) * 2 * npad * 128;
+    const int left = kUmmaSmemBytes - 1024 - kUmmaBarrierBytes - kUmmaOutBytes - side_bytes - x_bytes - (windows ? 3 * kUmmaTableBytes : 0);
     const int slots = left / (kUmmaSlotBytes + kUmmaTableBytes);
     return slots > kUmmaMaxSlots ? kUmmaMaxSlots : slots > 3 ? slots & ~1 : slots;  // even where there is a choice: see the dequant warps
 }
 static_assert(umma_ring_slots(128, false, 0) >= 3 && umma_ring_slots(128, true, 0) >= 3 && umma_ring_slots(64, true, 0) >= 4 &&
-              umma_ring_slots(64, true, 64 * 512) >= 4 && umma_ring_slots(64, true, 8 * 16 * 512) >= 2, "the ring is too short");
+              umma_ring_slots(64, true, 64 * 512) >= 4 && umma_ring_slots(64, true, 8 * 16 * 512) >= 2 &&
+              umma_ring_slots(64, true, 64 * 512 + kUmmaResidualBytes) >= 3 && umma_ring_slots(128, true, kUmmaResidualBytes) >= 3, "the ring is too short");
 static_assert(8 * 32 * kUmmaTileRows * 4 <= umma_ring_slots(128, true, 0) * kUmmaSlotBytes + umma_x_slots(128, true, 0) * 2 * 128 * 128 &&
               8 * 24 * kUmmaTileRows * 4 <= umma_ring_slots(96, true, 0) * kUmmaSlotBytes + umma_x_slots(96, true, 0) * 2 * 96 * 128 &&
               8 * 20 * kUmmaTileRows * 4 <= umma_ring_slots(80, true, 0) * kUmmaSlotBytes + umma_x_slots(80, true, 0) * 2 * 80 * 128,
@@ -108,8 +112,8 @@ struct UmmaParams {
     int row_tiles, act_tiles, npad;
     int unit_shift;        // log2 of the accumulator units in tensor memory
     int sum_bytes;         // shared memory of the running sum over a CTA's slices, or of the slices a cluster's CTA adds
+    int side_bytes;        // that and the residuals in flight
     bool wide_out;         // rows of the output and the residual are 16-byte aligned
-    bool paired;           // the output and the residual have the same alignment within a 4-byte word
     bool windows;          // the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables)
 };
 
@@ -349,16 +353,17 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int npad = p.npad;
     const UmmaShare w = umma_share<kCluster>(p);
-    const int ring_space = umma_ring_slots(npad, p.windows, p.sum_bytes);
+    const int ring_space = umma_ring_slots(npad, p.windows, p.side_bytes);
     const int ring_slots = umma_ring_in_use(p, w, ring_space);
     const int table_slots = p.windows ? ring_slots + 3 : ring_slots;
-    const int x_slots = umma_x_slots(npad, p.windows, p.sum_bytes), x_slot_bytes = 2 * npad * 128;
+    const int x_slots = umma_x_slots(npad, p.windows, p.side_bytes), x_slot_bytes = 2 * npad * 128;
     uint8_t* ring = smem;
     uint8_t* x_tiles = ring + ring_space * kUmmaSlotBytes;
     uint8_t* tables = x_tiles + x_slots * x_slot_bytes;
     float* out_tile = reinterpret_cast<float*>(tables + (p.windows ? ring_space + 3 : ring_space) * kUmmaTableBytes);
     float* sum_tile = out_tile + kUmmaOutBytes / 4;
-    uint64_t* ring_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sum_tile) + p.sum_bytes);
+    uint8_t* residual_ring = reinterpret_cast<uint8_t*>(sum_tile) + p.sum_bytes;
+    uint64_t* ring_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sum_tile) + p.side_bytes);
     uint64_t* ring_empty = ring_full + kUmmaMaxSlots;
     uint64_t* a_full = ring_empty + kUmmaMaxSlots;
     uint64_t* stage_empty = a_full + kUmmaStages;
@@ -561,45 +566,41 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 const int m0 = (tile - row_tile * p.act_tiles) * npad;
                 const int rows = min(npad, p.M - m0);
                 const int n_tile = row_tile * kOut;
-                // Residuals of sixteen activation rows, requested one step ahead (two steps took eight registers that
-                // are not there); the first ones leave while the tile is still being multiplied.  Vectors of eight
-                // where rows are 16-byte aligned; else words: warp q has rows 4 q .. 4 q + 3 of a step, a lane the
-                // aligned pairs `lane` and `lane + 32` of each, counted from the row's first element less `row_odd`.
-                const bool staged_residual = !kSwiglu && p.residual != nullptr;
-                uint32_t extra[8];
-                auto row_odd = [&](int m) { return (int)((reinterpret_cast<uintptr_t>(p.out) >> 1) + (uint32_t)(m0 + m) * (uint32_t)p.N) & 1; };
+                // The residuals of four steps of sixteen activation rows are on their way by asynchronous copies, the first
+                // ones while the tile is still being multiplied; held in registers one step ahead they cost a memory
+                // round trip per step (445 rows 1024 -> 50240: 115 us against 86, and 67 without a residual).  Where
+                // rows are 16-byte aligned, 16 bytes per copy; else the words that hold the row's elements: warp q has
+                // rows 4 q .. 4 q + 3 of a step, a lane words `lane` and `lane + 32`, one lane per row a 65th.
+                const bool has_residual = !kSwiglu && p.residual != nullptr;
+                auto odd_start = [&](const uint16_t* base, int m) {  // whether the tile's row m starts in the middle of a word
+                    return (int)((reinterpret_cast<uintptr_t>(base) >> 1) + (uint32_t)(m0 + m) * (uint32_t)p.N) & 1;
+                };
                 auto request_residual = [&](int c0) {
                     if constexpr (!kSwiglu) {
-                        if (!staged_residual || c0 >= rows) return;
-                        if (p.wide_out) {
+                        if (!has_residual) return;
+                        uint8_t* step = residual_ring + (c0 / 16 % kUmmaResidualSteps) * (16 * kUmmaResidualPitch);
+                        if (c0 < rows && p.wide_out) {
 #pragma unroll
                             for (int i = 0; i < 2; ++i) {
-                                const int at = thread + 128 * i, m = c0 + at / kVectors, n = n_tile + at % kVectors * 8;
-                                if (m < rows && n < p.N) {
-                                    const uint4 v = ptx::ld_global_dependent_u4(p.residual + (size_t)(m0 + m) * p.N + n);
-                                    extra[4 * i] = v.x; extra[4 * i + 1] = v.y; extra[4 * i + 2] = v.z; extra[4 * i + 3] = v.w;
-                                }
+                                const int at = thread + 128 * i, j = at / kVectors, n = n_tile + at % kVectors * 8;
+                                if (c0 + j < rows && n < p.N)
+                                    ptx::cp_async_16(step + j * kUmmaResidualPitch + at % kVectors * 16, p.residual + (size_t)(m0 + c0 + j) * p.N + n);
                             }
-                        } else {
+                        } else if (c0 < rows) {
+                            auto copy_word = [&](int j, int word) {
+                                const int n = n_tile + 2 * word - odd_start(p.residual, c0 + j);  // n, n + 1: at least one is in the row
+                                if (c0 + j < rows && n < p.N)
+                                    ptx::cp_async_4(step + j * kUmmaResidualPitch + 4 * word, p.residual + (size_t)(m0 + c0 + j) * p.N + n);
+                            };
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const int m = c0 + quadrant * 4 + (i >> 1), n = n_tile + 2 * (lane + 32 * (i & 1)) - row_odd(m);
-                                const uint16_t* from = p.residual + (size_t)(m0 + m) * p.N + n;
-                                uint32_t lo = 0, hi = 0;
-                                if (m < rows) {
-                                    if (n >= n_tile && n + 1 < p.N && p.paired) {
-                                        extra[i] = ptx::ld_global_dependent_u32(from);
-                                        continue;
-                                    }
-                                    if (n >= n_tile && n < p.N) lo = ptx::ld_global_dependent_u16(from);
-                                    if (n + 1 < p.N) hi = ptx::ld_global_dependent_u16(from + 1);
-                                }
-                                extra[i] = lo | (hi << 16);
-                            }
+                            for (int i = 0; i < 8; ++i) copy_word(quadrant * 4 + (i >> 1), lane + 32 * (i & 1));
+                            if (lane < 4 && odd_start(p.residual, c0 + quadrant * 4 + lane)) copy_word(quadrant * 4 + lane, 64);
                         }
+                        ptx::cp_async_commit();
                     }
                 };
-                request_residual(0);
+#pragma unroll
+                for (int i = 0; i < kUmmaResidualSteps; ++i) request_residual(16 * i);
 
                 // Slices that the final pass does not read itself go to the running sum, which holds all padded rows.
                 const int direct = kSwiglu && my_slices == 2 ? 2 : 1;
@@ -662,7 +663,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                         if (c0 > 0) ptx::named_barrier_sync(1, 128);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) out_tile[j * kPitch + thread] = v[j] * kDequantUndo;
+                        ptx::cp_async_wait_group<kUmmaResidualSteps - 1>();  // this step's residuals
                     }
+                    const uint8_t* residual_step = residual_ring + (c0 / 16 % kUmmaResidualSteps) * (16 * kUmmaResidualPitch);
                     ptx::named_barrier_sync(1, 128);
                     if (p.wide_out) {
 #pragma unroll
@@ -672,12 +675,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                                 const float4 lo = *reinterpret_cast<const float4*>(out_tile + j * kPitch + at % kVectors * 8);
                                 const float4 hi = *reinterpret_cast<const float4*>(out_tile + j * kPitch + at % kVectors * 8 + 4);
                                 uint4 packed;
-                                if (staged_residual) {
-                                    const uint32_t* r = &extra[4 * i];
-                                    packed.x = pack_bf16x2(lo.x + bf16_lo(r[0]), lo.y + bf16_hi(r[0]));
-                                    packed.y = pack_bf16x2(lo.z + bf16_lo(r[1]), lo.w + bf16_hi(r[1]));
-                                    packed.z = pack_bf16x2(hi.x + bf16_lo(r[2]), hi.y + bf16_hi(r[2]));
-                                    packed.w = pack_bf16x2(hi.z + bf16_lo(r[3]), hi.w + bf16_hi(r[3]));
+                                if (has_residual) {
+                                    const uint4 r = *reinterpret_cast<const uint4*>(residual_step + j * kUmmaResidualPitch + at % kVectors * 16);
+                                    packed.x = pack_bf16x2(lo.x + bf16_lo(r.x), lo.y + bf16_hi(r.x));
+                                    packed.y = pack_bf16x2(lo.z + bf16_lo(r.y), lo.w + bf16_hi(r.y));
+                                    packed.z = pack_bf16x2(hi.x + bf16_lo(r.z), hi.y + bf16_hi(r.z));
+                                    packed.w = pack_bf16x2(hi.z + bf16_lo(r.w), hi.w + bf16_hi(r.w));
                                 } else {
                                     packed = make_uint4(pack_bf16x2(lo.x, lo.y), pack_bf16x2(lo.z, lo.w), pack_bf16x2(hi.x, hi.y),
                                                         pack_bf16x2(hi.z, hi.w));
@@ -685,31 +688,40 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                                 *reinterpret_cast<uint4*>(p.out + (size_t)(m0 + c0 + j) * p.N + n) = packed;
                             }
                         }
-                        request_residual(c0 + 16);
+                        request_residual(c0 + 16 * kUmmaResidualSteps);
                     } else if constexpr (!kSwiglu) {
+                        // All reads before the first store, with no branch among them: a step is bounded by shared
+                        // memory's latency (445 rows 1024 -> 50243: 84 us, 132 as one branching loop over the words).
+                        uint32_t packed[8];
+                        auto element_pair = [&](int j, int e, int residual_odd) {  // elements e, e + 1 of a row; one may lie outside the tile
+                            float a = out_tile[j * kPitch + e], b = out_tile[j * kPitch + e + 1];
+                            if (has_residual) {
+                                const uint16_t* r = reinterpret_cast<const uint16_t*>(residual_step + j * kUmmaResidualPitch) + e + residual_odd;
+                                a += bf16_bits_to_f32(r[0]);
+                                b += bf16_bits_to_f32(r[1]);
+                            }
+                            return pack_bf16x2(a, b);
+                        };
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            const int j = quadrant * 4 + (i >> 1), m = c0 + j;
-                            if (m >= rows) continue;
-                            const int e = 2 * (lane + 32 * (i & 1)) - row_odd(m), n = n_tile + e;
-                            const float* from = out_tile + j * kPitch + e;
-                            const uint32_t r = staged_residual ? extra[i] : 0u;
+                            const int j = quadrant * 4 + (i >> 1);
+                            packed[i] = element_pair(j, 2 * (lane + 32 * (i & 1)) - odd_start(p.out, c0 + j), odd_start(p.residual, c0 + j));
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int m = c0 + quadrant * 4 + (i >> 1), e = 2 * (lane + 32 * (i & 1)) - odd_start(p.out, m), n = n_tile + e;
                             uint16_t* to = p.out + (size_t)(m0 + m) * p.N + n;
-                            if (e >= 0 && n + 1 < p.N) {
-                                *reinterpret_cast<uint32_t*>(to) = pack_bf16x2(from[0] + bf16_lo(r), from[1] + bf16_hi(r));
-                            } else {
-                                if (e >= 0 && n < p.N) to[0] = f32_to_bf16_bits(from[0] + bf16_lo(r));
-                                if (e < 0) to[1] = f32_to_bf16_bits(from[1] + bf16_hi(r));
-                            }
+                            const bool low = m < rows && e >= 0 && n < p.N, high = m < rows && n + 1 < p.N;
+                            if (low && high) *reinterpret_cast<uint32_t*>(to) = packed[i];
+                            if (low && !high) to[0] = (uint16_t)packed[i];
+                            if (high && !low) to[1] = (uint16_t)(packed[i] >> 16);
                         }
                         // The last element of a row that starts in the middle of a word.
-                        const int j = quadrant * 4 + (lane & 3), m = c0 + j, n = n_tile + 127;
-                        if (lane < 4 && m < rows && n < p.N && row_odd(m)) {
-                            const size_t at = (size_t)(m0 + m) * p.N + n;
-                            const float r = staged_residual ? bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + at)) : 0.0f;
-                            p.out[at] = f32_to_bf16_bits(out_tile[j * kPitch + 127] + r);
-                        }
-                        request_residual(c0 + 16);
+                        const int last_row = quadrant * 4 + (lane & 3);
+                        if (lane < 4 && c0 + last_row < rows && n_tile + 127 < p.N && odd_start(p.out, c0 + last_row))
+                            p.out[(size_t)(m0 + c0 + last_row) * p.N + n_tile + 127] = (uint16_t)element_pair(last_row, 127, odd_start(p.residual, c0 + last_row));
+                        __syncwarp();  // the copies below overwrite what other lanes read
+                        request_residual(c0 + 16 * kUmmaResidualSteps);
                     } else {
                         const int o = thread % kOut, n = n_tile + o;
                         for (int j = thread / kOut; j < 16 && c0 + j < rows; j += 128 / kOut)
@@ -1085,6 +1097,7 @@ inline int launch_umma_family(UmmaParams& params, cudaStream_t stream) {
     params.npad = 0;
     umma_plan<kSwiglu>(params, slots_total, device);
     if (params.npad == 0) return MT_ERR_LAUNCH;  // not even one CTA fits the device
+    params.side_bytes = params.sum_bytes + (params.residual && params.ksplit == 1 ? kUmmaResidualBytes : 0);
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
     const int tiles = params.row_tiles * params.act_tiles;
     if (params.ksplit > 1) return launch_umma_instance<kSwiglu, true>(params, tiles * params.ksplit, device, stream);
@@ -1117,7 +1130,6 @@ inline int launch_umma(const void* x, const AffineWeights* first, const AffineWe
     params.N = N;
     params.row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128;
     params.wide_out = N % 8 == 0 && aligned_to(out, 16) && (!residual || aligned_to(residual, 16));
-    params.paired = residual && (reinterpret_cast<uintptr_t>(out) - reinterpret_cast<uintptr_t>(residual)) % 4 == 0;
     params.windows = (K / kUmmaBlockK) % 4 != 0;
     for (int t = 0; t < 2; ++t)
         params.windows = params.windows || !aligned_to(params.scales[t], 8) || !aligned_to(params.biases[t], 8);

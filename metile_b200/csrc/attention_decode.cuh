@@ -43,15 +43,6 @@ struct AttentionParams {
     float scale;
 };
 
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* global_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(smem_dst)), "l"(global_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
-}
-
 constexpr int kAttnThreads = 256;
 constexpr int kAttnRowPad = 8;  // bf16 elements: a tile row in shared memory is 16 bytes longer than in the cache
 
@@ -125,14 +116,14 @@ __global__ void __launch_bounds__(kAttnThreads) attention_decode_split_kernel(co
     constexpr int kChunks = kD / 8;
     for (int c = threadIdx.x; c < rows * kChunks; c += kAttnThreads) {
         const int row = c / kChunks, chunk = c - row * kChunks;
-        cp_async_16(key_tile + row * kRow + chunk * 8, p.k + cache_row0 + (size_t)(split_first + row) * kD + chunk * 8);
+        ptx::cp_async_16(key_tile + row * kRow + chunk * 8, p.k + cache_row0 + (size_t)(split_first + row) * kD + chunk * 8);
     }
-    cp_async_commit();
+    ptx::cp_async_commit();
     for (int c = threadIdx.x; c < rows * kChunks; c += kAttnThreads) {
         const int row = c / kChunks, chunk = c - row * kChunks;
-        cp_async_16(value_tile + row * kRow + chunk * 8, p.v + cache_row0 + (size_t)(split_first + row) * kD + chunk * 8);
+        ptx::cp_async_16(value_tile + row * kRow + chunk * 8, p.v + cache_row0 + (size_t)(split_first + row) * kD + chunk * 8);
     }
-    cp_async_commit();
+    ptx::cp_async_commit();
     // Rows past the sequence's end enter the value product with probability zero; their bytes must
     // still be numbers (0 x NaN is NaN).  Key rows past the end only produce scores that are masked.
     const int first_unused = max(rows, 0);
@@ -155,7 +146,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_decode_split_kernel(co
             qf[s][1] = g < kG ? hi : 0u;
         }
     }
-    cp_async_wait<1>();
+    ptx::cp_async_wait_group<1>();
     __syncthreads();
 
     // ---------------------------------------------------------------- scores: 16 tokens per warp
@@ -224,7 +215,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_decode_split_kernel(co
             prob_lo[head][token] = f32_to_bf16_bits(value - bf16_bits_to_f32(hi));
         }
     }
-    cp_async_wait<0>();
+    ptx::cp_async_wait_group<0>();
     __syncthreads();  // values have landed and every probability is written
     // ---------------------------------------------------------------- values: D / 8 columns per warp
     float acc[kNTiles][4];

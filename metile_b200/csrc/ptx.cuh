@@ -145,6 +145,17 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tensor_m
 __device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait_group() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -300,12 +311,6 @@ __device__ __forceinline__ uint4 ld_global_dependent_u4(const void* p) {
 __device__ __forceinline__ uint32_t ld_global_dependent_u16(const uint16_t* p) {
     uint16_t v;
     asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-    return v;
-}
-
-__device__ __forceinline__ uint32_t ld_global_dependent_u32(const void* p) {
-    uint32_t v;
-    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 
