@@ -1,0 +1,62 @@
+"""The edges of the kernels' tiles, chunks and rings, against the CPU oracle or rows run alone."""
+import pytest
+import torch
+
+from metile_b200 import backends as B, synth
+from oracle import affine as A
+from tests.helpers import assert_bit_equal, assert_within, f32, triple_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,k,n", [
+    (1, 128, 1),          # fewer outputs than a warp takes, one block
+    (3, 384, 5),          # a chunk with an odd row
+    (12, 1024, 130),      # ring shorter than the row, a last task that overlaps its neighbour
+    (13, 2304, 1001),     # rows past the chunk's
+    (16, 16384, 40),      # activations of sixteen rows do not fit
+    (17, 512, 300),       # two chunks
+    (620, 256, 96),       # two launches
+])
+def test_dense_rows_edges(cuda_device, rows, k, n):
+    x = synth.activations(1, rows, k, cuda_device)
+    w, g = (synth.dense_weight(seed, n, k, cuda_device) for seed in (2, 3))
+    r = synth.activations(4, rows, n, cuda_device)
+    some = sorted({0, rows // 2, rows - 1})
+    y = B.mlx_dense_residual_qmv(x, w, r)
+    assert (f32(y[some]) == A.dense_rows(f32(x[some]), f32(w), f32(r[some]))).all()
+    swi = B.mlx_dense_swiglu(x, g, w)
+    alone = torch.cat([B.mlx_dense_swiglu(x[i:i + 1], g, w) for i in some])
+    assert_bit_equal(swi[some], alone, "dense swiglu rows alone")
+    # Weights that are 8-byte aligned only.
+    shifted = torch.empty(n * k + 4, dtype=w.dtype, device=w.device)[4:].view(n, k).copy_(w)
+    assert_bit_equal(B.mlx_dense_residual_qmv(x, shifted, r), y, "dense weights off a 16-byte boundary")
+
+
+@pytest.mark.parametrize("rows,k,n", [
+    (2, 64, 5),           # one k-block, narrow rows, unaligned tables
+    (17, 8192, 128),      # slices over a thread-block cluster
+    (65, 320, 131),       # the first size with one accumulator unit, odd rows
+    (128, 6080, 1000),    # unaligned tables over a long range
+    (129, 448, 257),      # two activation tiles
+    (300, 1024, 1111),    # several tiles per CTA, odd rows that start on either half of a word
+    (445, 4096, 2048),    # the running sum over several slices
+])
+def test_tcgen05_projection_edges(cuda_device, rows, k, n):
+    x = synth.activations(1, rows, k, cuda_device)
+    triple = synth.affine_weight(2, n, k, cuda_device)
+    r = synth.activations(3, rows, n, cuda_device)
+    some = sorted({0, 1, rows // 2, rows - 1})
+    with B.force_kernel("umma"):
+        plain, added = B.mlx_affine_qmv(x, *triple), B.mlx_affine_residual_qmv(x, *triple, r)
+        alone = torch.cat([B.mlx_affine_residual_qmv(x[i:i + 1], *triple, r[i:i + 1]) for i in some])
+        assert_bit_equal(added[some], alone, "rows alone")
+        # The residual and the output apart by half a word.
+        shifted = torch.empty(r.numel() + 1, dtype=r.dtype, device=r.device)[1:].view_as(r).copy_(r)
+        assert_bit_equal(B.mlx_affine_residual_qmv(x, *triple, shifted), added, "shifted residual")
+        swi = B.mlx_affine_swiglu(x, *triple, *triple)
+        alone = torch.cat([B.mlx_affine_swiglu(x[i:i + 1], *triple, *triple) for i in some])
+        assert_bit_equal(swi[some], alone, "swiglu rows alone")
+    weights = triple_np(triple)
+    assert_within(plain[some], A.qmm(f32(x[some]), *weights, weights="bf16"))
+    assert_within(added[some], A.qmm(f32(x[some]), *weights, residual=f32(r[some]), weights="bf16"))
