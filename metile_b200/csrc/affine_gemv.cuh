@@ -27,6 +27,8 @@
 // for a row run alone or inside a batch of up to 8.
 #pragma once
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -297,6 +299,200 @@ affine_gemv_kernel(const uint16_t* x, GemvWeights first, GemvWeights second, con
     }
 }
 
+// ---- one activation row, weights through per-warp rings --------------------------------------------
+// The same sums in the same order as affine_gemv_kernel<1, ...>; what differs is how the operands get there.
+// Weights requested into registers one iteration ahead kept about 70 KB in flight per SM at best.  Here every lane
+// copies its own 16 bytes of packed words, and a warp the words that hold its scales and biases, into a ring of the
+// warp's, two iterations ahead, by asynchronous copies (96 KB in flight per SM, no registers, and no synchronisation
+// beyond the warp's).  The fp32 activations and the slot sums are made by one thread per slot with one barrier; the
+// lanes' totals of all rows are folded together (5 exchanges instead of 16); the warps' rows are dealt out SM by SM.
+constexpr int kGemvRingSlots = 3;
+constexpr int kGemvRingRows = 4;  // weight rows of a half-warp: four outputs, or two of gate and two of up
+constexpr int kGemvTableWords = 5;  // nine groups of a row and step, wherever they start within a word
+constexpr int kGemvRingBytes = 8 * kGemvRingSlots * kGemvRingRows * (32 * 16 + 2 * 2 * kGemvTableWords * 4);  // of a CTA of eight warps
+
+template <bool kDual>
+__global__ void __launch_bounds__(256, 2)
+affine_gemv_ring_kernel(const uint16_t* x, GemvWeights first, GemvWeights second, const uint16_t* residual, uint16_t* out,
+                        int K, int N, int ksplit) {
+    constexpr int kStreams = kDual ? 2 : 1, kRows = kGemvRingRows / kStreams, kWarps = 8;
+    constexpr int kTableSlot = kGemvRingRows * 4 * kGemvTableWords;  // words
+    extern __shared__ uint4 gemv_smem[];
+    __shared__ float partial[kWarps][2][kGemvRingRows];
+    const int lane = threadIdx.x & 31, half = lane >> 4, l16 = lane & 15, warp = threadIdx.x >> 5;
+    const int part = warp % ksplit, team = warp / ksplit, teams = kWarps / ksplit;
+    const int slots_per_row = K >> 5, groups_per_row = K >> 6;
+    const int slots_per_part = (slots_per_row + ksplit - 1) / ksplit;
+    const int slot_begin = part * slots_per_part, slot_end = min(slot_begin + slots_per_part, slots_per_row);
+    const int steps = (slots_per_part + 15) >> 4;
+    const int tasks = (N + 2 * kRows - 1) / (2 * kRows);  // a task is the 2 kRows outputs of one warp pass
+    const int stride = teams * gridDim.x;
+    const int first_task = team * gridDim.x + blockIdx.x;
+
+    // [slot][row][lane] 16 bytes, then [slot][row][scales, biases][half][kGemvTableWords] words.
+    uint4* ring = gemv_smem + warp * (kGemvRingSlots * kGemvRingRows * 32) + lane;
+    uint32_t* table_ring = reinterpret_cast<uint32_t*>(gemv_smem + kWarps * kGemvRingSlots * kGemvRingRows * 32) +
+                           warp * (kGemvRingSlots * kTableSlot) + half * kGemvTableWords;
+    float4* xq = reinterpret_cast<float4*>(gemv_smem) + kGemvRingBytes / 16;
+    float* slot_sum = reinterpret_cast<float*>(xq + ((slots_per_row + 15) >> 4) * 128);
+
+    // The first row of this half-warp in a task; the last task repeats some of its neighbour's rows.
+    auto task_row = [&](int task) { return min(task * 2 * kRows + half * kRows, N - kRows); };
+    // Byte offsets of the next packed words of each row, and of the first table word that this lane copies: lane 4 r + i of
+    // a half-warp has word i of row r, for 4 bytes per lane would be sixteen times the bytes and as many accesses to
+    // shared memory as all else together (131072 rows of 1024: 23.5 us).
+    uint32_t word_at[kRows], table_at = 0;
+    const int table_row = l16 >> 2, table_word = l16 & 3;
+    const int group_begin = slot_begin >> 1, group_end = (slot_end + 1) >> 1;
+    int table_left = 0;         // groups from the word's first one to the end of the part
+    bool table_fifth = false;
+    int copy_task = first_task, copy_step = 0;
+    auto start_copies = [&] {
+        const int n = task_row(copy_task);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) word_at[r] = (uint32_t)(n + r) * (uint32_t)(K >> 1) + (slot_begin + l16) * 16;
+        const uint32_t entry = (uint32_t)(n + table_row % kRows) * groups_per_row + group_begin;
+        table_at = ((entry >> 1) + table_word) * 4;
+        table_left = group_end - group_begin + (int)(entry & 1u) - 2 * table_word;
+        table_fifth = table_word == 0 && ((entry | slot_begin) & 1u);
+    };
+    start_copies();
+    auto copy_next = [&](int ring_slot) {
+        if (copy_task < tasks) {
+            uint8_t* to = reinterpret_cast<uint8_t*>(ring) + ring_slot * (kGemvRingRows * 512);
+            uint32_t* table_to = table_ring + ring_slot * kTableSlot + table_row * (4 * kGemvTableWords) + table_word;
+            if (slot_begin + l16 + (copy_step << 4) < slot_end) {
+#pragma unroll
+                for (int r = 0; r < kGemvRingRows; ++r)
+                    ptx::cp_async_16(to + r * 512, reinterpret_cast<const uint8_t*>((r < kRows ? first : second).w) + word_at[r % kRows]);
+            }
+            const GemvWeights& wt = kDual && table_row >= kRows ? second : first;
+            const uint8_t* scales = reinterpret_cast<const uint8_t*>(wt.scales) + table_at;
+            const uint8_t* biases = reinterpret_cast<const uint8_t*>(wt.biases) + table_at;
+            if (table_left > 0) {
+                ptx::cp_async_4(table_to, scales);
+                ptx::cp_async_4(table_to + 2 * kGemvTableWords, biases);
+            }
+            if (table_fifth && table_left > 8) {
+                ptx::cp_async_4(table_to + 4, scales + 16);
+                ptx::cp_async_4(table_to + 2 * kGemvTableWords + 4, biases + 16);
+            }
+        }
+        ptx::cp_async_commit();
+        if (++copy_step == steps) {
+            copy_step = 0;
+            copy_task += stride;
+            start_copies();
+        } else {
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) word_at[r] += 256;
+            table_at += 16;
+            table_left -= 8;
+        }
+    };
+
+    ptx::griddep_launch_dependents();
+#pragma unroll
+    for (int i = 0; i < kGemvRingSlots - 1; ++i) copy_next(i);
+    ptx::griddep_wait();  // activations and residual are the preceding kernel's output
+    for (int slot = threadIdx.x; slot < slots_per_row; slot += blockDim.x) {
+        uint4 raw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) raw[i] = ptx::ld_global_dependent_u4(x + (size_t)slot * 32 + i * 8);
+        float4* dst = xq + (slot >> 4) * 128 + (slot & 15);  // chunk i of slot j lies at ((j / 16) * 8 + i) * 16 + j % 16
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 a = make_float4(bf16_lo(raw[i].x), bf16_hi(raw[i].x), bf16_lo(raw[i].y), bf16_hi(raw[i].y));
+            const float4 b = make_float4(bf16_lo(raw[i].z), bf16_hi(raw[i].z), bf16_lo(raw[i].w), bf16_hi(raw[i].w));
+            dst[32 * i] = a;
+            dst[32 * i + 16] = b;
+            sum += a.x; sum += a.y; sum += a.z; sum += a.w;
+            sum += b.x; sum += b.y; sum += b.z; sum += b.w;
+        }
+        slot_sum[slot] = sum;
+    }
+    __syncthreads();
+
+    int ring_slot = 0;
+    // Every warp of a CTA makes the same number of passes: the barriers below are reached by all of them.
+    for (int task0 = blockIdx.x; task0 < tasks; task0 += stride) {
+        const int task = task0 + team * gridDim.x;
+        const int row = task_row(task);
+        // Where this lane's scale lies among the table words of even and odd rows, the same in every step.
+        const int offset = ((slot_begin + l16) >> 1) - group_begin;
+        const uint32_t entry = (uint32_t)row * groups_per_row + group_begin;
+        const uint32_t half_at[2] = {offset + (entry & 1u), offset + ((entry ^ groups_per_row) & 1u)};
+        float acc[kGemvRingRows] = {};
+        for (int step = 0; step < steps; ++step) {
+            ptx::cp_async_wait_group<kGemvRingSlots - 2>();
+            __syncwarp();
+            copy_next(ring_slot == 0 ? kGemvRingSlots - 1 : ring_slot - 1);  // the slot that was read before this one
+            const uint4* words = ring + ring_slot * (kGemvRingRows * 32);
+            const uint16_t* tables = reinterpret_cast<const uint16_t*>(table_ring + ring_slot * kTableSlot);
+            if (++ring_slot == kGemvRingSlots) ring_slot = 0;
+            const int slot = slot_begin + l16 + (step << 4);
+            if (task >= tasks || slot >= slot_end) continue;
+            const float4* xs = xq + (slot >> 4) * 128 + (slot & 15);
+            uint4 packed[kGemvRingRows];
+            float dot[kGemvRingRows];
+#pragma unroll
+            for (int r = 0; r < kGemvRingRows; ++r) {
+                packed[r] = words[r * 32];
+                dot[r] = 0.0f;
+            }
+#pragma unroll
+            for (int wi = 0; wi < 4; ++wi) {
+                const float4 a = xs[32 * wi], b = xs[32 * wi + 16];
+                const float xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int r = 0; r < kGemvRingRows; ++r) {
+                    float q[8];
+                    unpack_word_f32_offset128(wi == 0 ? packed[r].x : wi == 1 ? packed[r].y : wi == 2 ? packed[r].z : packed[r].w, q);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) dot[r] = fmaf(q[e], xv[e], dot[r]);
+                }
+            }
+            const float xsum = slot_sum[slot];
+#pragma unroll
+            for (int r = 0; r < kGemvRingRows; ++r) {
+                const float scale = bf16_bits_to_f32(tables[r * (8 * kGemvTableWords) + half_at[r % kRows & 1]]);
+                const float bias = bf16_bits_to_f32(tables[r * (8 * kGemvTableWords) + 4 * kGemvTableWords + half_at[r % kRows & 1]]);
+                acc[r] = fmaf(scale, dot[r], fmaf(fmaf(-128.0f, scale, bias), xsum, acc[r]));
+            }
+        }
+
+        // The 16-lane butterfly of the four rows: after two halvings a lane has the sums of row l16 / 4.
+        {
+            const bool upper8 = l16 & 8, upper4 = l16 & 4;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float keep = upper8 ? acc[i + 2] : acc[i], send = upper8 ? acc[i] : acc[i + 2];
+                acc[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 8);
+            }
+            const float keep = upper4 ? acc[1] : acc[0], send = upper4 ? acc[0] : acc[1];
+            acc[0] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 4);
+            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], 2);
+            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1);
+        }
+        float total = acc[0];
+        if (ksplit > 1) {  // the K parts in order
+            if ((l16 & 3) == 0) partial[warp][half][l16 >> 2] = total;
+            __syncthreads();
+            if (part == 0)
+                for (int q = 1; q < ksplit; ++q) total += partial[warp + q][half][l16 >> 2];
+            __syncthreads();
+        }
+        const float other = kDual ? __shfl_down_sync(0xFFFFFFFFu, total, 8) : 0.0f;  // up, whose rows are two further on
+        const int n = row + (l16 >> 2);
+        if (part == 0 && task < tasks && (l16 & 3) == 0 && (l16 >> 2) < kRows && n >= task * 2 * kRows + half * kRows) {
+            float v = kDual ? swiglu_f32(total, other) : total;
+            if (residual) v += bf16_bits_to_f32(ptx::ld_global_dependent_u16(residual + n));
+            out[n] = f32_to_bf16_bits(v);
+        }
+    }
+}
+
 constexpr int kGemvStageLimit = 104 * 1024;
 
 // K parts per row: enough warps to keep the memory system busy when N is small.  Depends on
@@ -347,6 +543,43 @@ inline int launch_gemv_instance(const uint16_t* x, GemvWeights a, GemvWeights b,
                                                                                                      : MT_ERR_LAUNCH;
 }
 
+constexpr int kGemvRingLimit = 112 * 1024;  // two CTAs per SM
+
+template <bool kDual>
+inline bool gemv_ring_applicable(const GemvWeights& a, const GemvWeights& b, int K, int N) {
+    for (const GemvWeights* w : {&a, &b})
+        if (!aligned_to(w->scales, 4) || !aligned_to(w->biases, 4)) return false;
+    return N >= kGemvRingRows && (long)N * (K >> 1) < (1l << 32) && gemv_f32_stage_bytes(K) + kGemvRingBytes <= kGemvRingLimit;
+}
+
+template <bool kDual>
+inline int launch_gemv_ring(const uint16_t* x, GemvWeights a, GemvWeights b, const uint16_t* residual, uint16_t* out, int K,
+                            int N, int sm_count, cudaStream_t stream) {
+    static bool configured[64] = {};
+    int device = 0;
+    cudaGetDevice(&device);
+    if (device >= 64 || !configured[device]) {
+        if (cudaFuncSetAttribute(affine_gemv_ring_kernel<kDual>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvRingLimit) != cudaSuccess)
+            return MT_ERR_LAUNCH;
+        if (device < 64) configured[device] = true;
+    }
+    const int ksplit = gemv_ksplit(K, N);
+    const int rows_per_cta = 8 / ksplit * 2 * (kGemvRingRows / (kDual ? 2 : 1));
+    const int grid = std::min((N + rows_per_cta - 1) / rows_per_cta, 2 * sm_count);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid, 1, 1);
+    config.blockDim = dim3(256, 1, 1);
+    config.dynamicSmemBytes = gemv_f32_stage_bytes(K) + kGemvRingBytes;
+    config.stream = stream;
+    cudaLaunchAttribute attrs[1];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attrs;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, affine_gemv_ring_kernel<kDual>, x, a, b, residual, out, K, N, ksplit) == cudaSuccess
+               ? MT_OK : MT_ERR_LAUNCH;
+}
+
 // Activations are staged in shared memory when they fit kGemvStageLimit, which leaves room for two
 // CTAs per SM (one row as fp32: K up to 24576; more rows as bf16); larger problems read them from
 // global memory.
@@ -354,6 +587,8 @@ template <int kM, bool kDual>
 inline int launch_gemv_m(const uint16_t* x, GemvWeights a, GemvWeights b, const uint16_t* residual, uint16_t* out,
                          int K, int N, int sm_count, cudaStream_t stream) {
     if constexpr (kM == 1) {
+        if (gemv_ring_applicable<kDual>(a, b, K, N))
+            return launch_gemv_ring<kDual>(x, a, b, residual, out, K, N, sm_count, stream);
         if (gemv_f32_stage_bytes(K) <= kGemvStageLimit)
             return launch_gemv_instance<kM, kDual, kStageF32>(x, a, b, residual, out, K, N, sm_count, stream);
     }
