@@ -202,6 +202,15 @@ int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row
                       const int* positions, void* q_out, void* k_cache, void* v_cache, int batch,
                       int q_heads, int kv_heads, int capacity, int head_dim, float theta, void* stream);
 
+/* The same for the `steps` tokens of a prompt, which go to rows first, first + 1, ... of every cache.
+ * q: dense bf16 [batch, steps, q_heads, head_dim], k, v: [batch, steps, kv_heads, head_dim]; q_out like q;
+ * inverse: fp32 [head_dim / 2] on the device, the angle of pair i is position * inverse[i] in fp32; products,
+ * sums and differences are rounded one by one.  positions: int32 [batch] on the device or null, advanced
+ * by `steps`. */
+int mt_rope_kv_prefill(const void* q, const void* k, const void* v, const float* inverse, void* q_out,
+                       void* k_cache, void* v_cache, int* positions, int batch, int steps, int first,
+                       int q_heads, int kv_heads, int capacity, int head_dim, void* stream);
+
 /* Sum of bf16 partial results over the GPUs of one node (one process per GPU), for the
  * tensor-parallel form of the fused MLP: the down projection of a K-sharded MLP leaves a partial
  * [M, H] result on every rank.  NO COUNTERPART IN THE REFERENCE, which is single-device.

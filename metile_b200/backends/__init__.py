@@ -5,6 +5,8 @@ from .cuda import (  # noqa: F401
     mlx_attention_decode,
     mlx_rms_norm,
     rope_kv_append,
+    rope_kv_prefill,
+    supports_rope_kv_prefill,
     supports_attention_decode,
 )
 from .cuda_affine import MLXAffineWeight, mlx_affine_matmul  # noqa: F401
@@ -15,6 +17,7 @@ from .cuda_dense import (  # noqa: F401
 from .cuda_quantized import (  # noqa: F401
     batch_invariant,
     force_kernel,
+    kernel_pinned,
     mlx_affine_mlp_executor,
     mlx_affine_mlp_host_executor,
     mlx_affine_qmv,

@@ -202,3 +202,42 @@ def rope_kv_append(query, key, value, positions, key_cache, value_cache, *, thet
                   pointer(value_cache), batch, q_heads, kv_heads, capacity, dim, ctypes.c_float(float(theta)))
     _lib.check(code, "rope_kv_append")
     return out
+
+
+def supports_rope_kv_prefill(query, key, value, key_cache, value_cache):
+    """Whether rope_kv_prefill serves these tensors: dense bfloat16 on one CUDA device."""
+    tensors = (query, key, value, key_cache, value_cache)
+    return all(type(t) is torch.Tensor and t.is_cuda and t.device == query.device and t.dtype == torch.bfloat16
+               and t.ndim == 4 and t.is_contiguous() and not t.requires_grad for t in tensors) \
+        and query.numel() > 0 and query.shape[-1] % 2 == 0 and query.shape[-1] <= 4096
+
+
+def rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache):
+    """Rotate the query and key rows of a prompt and write key and value to the caches, in place.
+
+    query [B, T, Hq, D], key / value [B, T, Hkv, D]; inverse fp32 [D/2]: pair i of the token at position
+    p is turned by p * inverse[i]; positions int32 [B] (device) is advanced by T; row `first + t` of each
+    cache [B, Hkv, capacity, D] receives token t.  Returns the rotated query, shaped like `query`."""
+    out = native().rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache)
+    if out is not None:
+        return native_result(out, "rope_kv_prefill")
+    require_cuda_bf16(query, "rope_kv_prefill")
+    batch, steps, q_heads, dim = query.shape
+    kv_heads, capacity = key_cache.shape[1], key_cache.shape[2]
+    if key.shape != (batch, steps, kv_heads, dim) or value.shape != key.shape:
+        raise ValueError("rope_kv_prefill expects key and value rows of shape [batch, steps, kv_heads, head_dim]")
+    if key_cache.shape != (batch, kv_heads, capacity, dim) or value_cache.shape != key_cache.shape:
+        raise ValueError("rope_kv_prefill expects caches of shape [batch, kv_heads, capacity, head_dim]")
+    if first < 0 or first + steps > capacity:
+        raise ValueError("rope_kv_prefill: the cache has no room for the prompt")
+    for label, tensor in (("query", query), ("key", key), ("value", value), ("key cache", key_cache),
+                          ("value cache", value_cache)):
+        require_on_device(tensor, query, label, dtype=torch.bfloat16)
+    require_on_device(inverse, query, "inverse", dtype=torch.float32, min_numel=dim // 2)
+    require_on_device(positions, query, "positions", dtype=torch.int32, min_numel=batch)
+    out = torch.empty_like(query)
+    code = launch(library().mt_rope_kv_prefill, query.device, pointer(query), pointer(key), pointer(value),
+                  pointer(inverse), pointer(out), pointer(key_cache), pointer(value_cache), pointer(positions), batch,
+                  steps, int(first), q_heads, kv_heads, capacity, dim)
+    _lib.check(code, "rope_kv_prefill")
+    return out

@@ -64,6 +64,11 @@ def batch_invariant(enabled=True):
         _state.flags = previous
 
 
+def kernel_pinned():
+    """Whether a kernel family is pinned in this thread (batch_invariant, force_kernel)."""
+    return _flags() != 0
+
+
 @contextlib.contextmanager
 def force_kernel(name):
     """Pin the kernel family: "gemv" (CUDA cores, up to 8 rows), "umma" (tcgen05), "mlp_fused" /

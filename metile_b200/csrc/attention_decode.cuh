@@ -434,4 +434,81 @@ __global__ void rope_kv_append_kernel(const RopeAppendParams p) {
     }
 }
 
+// The same for a prompt: `steps` new tokens of each sequence at rows `first`, `first + 1`, ... of its cache.  Every
+// product, sum and difference is rounded by itself, the angle is position * inverse[pair], and cosf / sinf are those
+// of the library: what the framework's op-by-op form computes, to the bit.  One CTA per token; its cosines and
+// sines are computed once for all heads.  Bound by launch latency and bytes (512 tokens of 12 + 2 x 2 heads of 128:
+// PREFILL_US; as some 45 framework launches per layer it took about 180 us of host time).
+struct RopePrefillParams {
+    const uint16_t* q;        // [B, steps, Hq, D]
+    const uint16_t* k;        // [B, steps, Hkv, D]
+    const uint16_t* v;        // [B, steps, Hkv, D]
+    const float* inverse;     // [D / 2]
+    uint16_t* q_out;          // [B, steps, Hq, D]
+    uint16_t* k_cache;        // [B, Hkv, capacity, D]
+    uint16_t* v_cache;
+    int* positions;           // [B] or null: advanced by `steps`
+    int steps, first, q_heads, kv_heads, capacity, head_dim;
+};
+
+template <bool kVector>
+__global__ void __launch_bounds__(256) rope_kv_prefill_kernel(const RopePrefillParams p) {
+    extern __shared__ float rope_angles[];  // cosines, then sines
+    const int b = blockIdx.x / p.steps, step = blockIdx.x - b * p.steps;
+    const int dim = p.head_dim, half = dim >> 1;
+    float *cosines = rope_angles, *sines = rope_angles + half;
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        const float angle = __fmul_rn((float)(p.first + step), p.inverse[i]);
+        cosines[i] = cosf(angle);
+        sines[i] = sinf(angle);
+    }
+    __syncthreads();
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();
+    if (step == 0 && threadIdx.x == 0 && p.positions) p.positions[b] += p.steps;
+    constexpr int kWidth = kVector ? 8 : 1;   // pairs of a thread
+    const int units = half / kWidth;          // threads of a head
+    for (int at = threadIdx.x; at < (p.q_heads + 2 * p.kv_heads) * units; at += blockDim.x) {
+        const int slot = at / units, i = (at - slot * units) * kWidth;
+        const bool is_query = slot < p.q_heads;
+        const int h = is_query ? slot : (slot - p.q_heads) % p.kv_heads;
+        const bool is_value = slot >= p.q_heads + p.kv_heads;
+        const uint16_t* from = is_query ? p.q + ((size_t)blockIdx.x * p.q_heads + h) * dim
+                                        : (is_value ? p.v : p.k) + ((size_t)blockIdx.x * p.kv_heads + h) * dim;
+        uint16_t* to = is_query ? p.q_out + ((size_t)blockIdx.x * p.q_heads + h) * dim
+                                : (is_value ? p.v_cache : p.k_cache) + (((size_t)b * p.kv_heads + h) * p.capacity + p.first + step) * dim;
+        auto rotate = [&](float first, float second, int pair, float& low, float& high) {
+            const float c = cosines[pair], s = sines[pair];
+            low = __fsub_rn(__fmul_rn(first, c), __fmul_rn(second, s));
+            high = __fadd_rn(__fmul_rn(second, c), __fmul_rn(first, s));
+        };
+        if constexpr (kVector) {
+            const uint4 a = ptx::ld_global_dependent_u4(from + i), z = ptx::ld_global_dependent_u4(from + i + half);
+            uint4 low4 = a, high4 = z;
+            if (!is_value) {
+                const uint32_t first[4] = {a.x, a.y, a.z, a.w}, second[4] = {z.x, z.y, z.z, z.w};
+                uint32_t low[4], high[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float l0, h0, l1, h1;
+                    rotate(bf16_lo(first[j]), bf16_lo(second[j]), i + 2 * j, l0, h0);
+                    rotate(bf16_hi(first[j]), bf16_hi(second[j]), i + 2 * j + 1, l1, h1);
+                    low[j] = pack_bf16x2(l0, l1);
+                    high[j] = pack_bf16x2(h0, h1);
+                }
+                low4 = make_uint4(low[0], low[1], low[2], low[3]);
+                high4 = make_uint4(high[0], high[1], high[2], high[3]);
+            }
+            *reinterpret_cast<uint4*>(to + i) = low4;
+            *reinterpret_cast<uint4*>(to + i + half) = high4;
+        } else {
+            const uint16_t a = ptx::ld_global_dependent_u16(from + i), z = ptx::ld_global_dependent_u16(from + i + half);
+            float low, high;
+            rotate(bf16_bits_to_f32(a), bf16_bits_to_f32(z), i, low, high);
+            to[i] = is_value ? a : f32_to_bf16_bits(low);
+            to[i + half] = is_value ? z : f32_to_bf16_bits(high);
+        }
+    }
+}
+
 }  // namespace mt

@@ -364,9 +364,49 @@ PyObject* rope_kv_append(PyObject*, PyObject* const* args, Py_ssize_t count) {
     }
 }
 
+// rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache)
+PyObject* rope_kv_prefill(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    if (count != 8) Py_RETURN_NONE;
+    const Tensor* t[8] = {};
+    for (int i : {0, 1, 2, 3, 4, 6, 7})
+        if (!(t[i] = plain(args[i]))) Py_RETURN_NONE;
+    const long first = PyLong_AsLong(args[5]);
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    const Tensor &q = *t[0], &k = *t[1], &v = *t[2], &inverse = *t[3], &positions = *t[4], &keys = *t[6], &values = *t[7];
+    if (!q.is_cuda() || q.dim() != 4 || k.dim() != 4 || keys.dim() != 4 || q.numel() == 0) Py_RETURN_NONE;
+    const auto device = q.device();
+    const int64_t batch = q.size(0), steps = q.size(1), heads = q.size(2), dim = q.size(3);
+    const int64_t kv_heads = keys.size(1), capacity = keys.size(2);
+    if (k.size(0) != batch || k.size(1) != steps || k.size(2) != kv_heads || k.size(3) != dim || v.sizes() != k.sizes() ||
+        keys.size(0) != batch || keys.size(3) != dim || values.sizes() != keys.sizes() || kv_heads < 1 || dim % 2)
+        Py_RETURN_NONE;
+    for (const Tensor* tensor : {&q, &k, &v, &keys, &values})
+        if (!bf16_on(*tensor, device)) Py_RETURN_NONE;
+    if (inverse.device() != device || inverse.scalar_type() != at::kFloat || !inverse.is_contiguous() || inverse.numel() != dim / 2)
+        Py_RETURN_NONE;
+    if (positions.device() != device || positions.scalar_type() != at::kInt || !positions.is_contiguous() || positions.numel() < batch)
+        Py_RETURN_NONE;
+    if (!fits_int(batch * steps) || !fits_int(capacity) || first < 0 || first + steps > capacity) Py_RETURN_NONE;
+    try {
+        const Launch launch(device);
+        Tensor out = new_like(q);
+        int code;
+        Py_BEGIN_ALLOW_THREADS
+        code = mt_rope_kv_prefill(address(q), address(k), address(v), static_cast<const float*>(address(inverse)), address(out),
+                                  address(keys), address(values), static_cast<int*>(address(positions)), (int)batch, (int)steps,
+                                  (int)first, (int)heads, (int)kv_heads, (int)capacity, (int)dim, launch.stream());
+        Py_END_ALLOW_THREADS
+        return code_or(code, std::move(out));
+    } catch (const std::exception& error) {
+        PyErr_SetString(PyExc_RuntimeError, error.what());
+        return nullptr;
+    }
+}
+
 #define MT_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MT_METHOD(project), MT_METHOD(swiglu),    MT_METHOD(mlp_plan),       MT_METHOD(mlp), MT_METHOD(norm),
-                         MT_METHOD(dense),   MT_METHOD(attention), MT_METHOD(rope_kv_append), {nullptr, nullptr, 0, nullptr}};
+                         MT_METHOD(dense),   MT_METHOD(attention), MT_METHOD(rope_kv_append),
+                         MT_METHOD(rope_kv_prefill), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -555,6 +555,48 @@ int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row
     return cudaLaunchKernelEx(&config, rope_kv_append_kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
+int mt_rope_kv_prefill(const void* q, const void* k, const void* v, const float* inverse, void* q_out, void* k_cache,
+                       void* v_cache, int* positions, int batch, int steps, int first, int q_heads, int kv_heads,
+                       int capacity, int head_dim, void* stream) {
+    if (batch < 0 || steps < 0 || first < 0 || q_heads < 1 || kv_heads < 1 || head_dim < 2 || head_dim % 2 || head_dim > 4096)
+        return MT_ERR_SHAPE;
+    if (first > capacity - steps || (long long)batch * steps > 0x7FFFFFFF) return MT_ERR_SHAPE;
+    if (batch == 0 || steps == 0) return MT_OK;
+    if (!q || !k || !v || !inverse || !q_out || !k_cache || !v_cache) return MT_ERR_NULL;
+    if (!device_is_sm100()) return MT_ERR_DEVICE;
+    RopePrefillParams params;
+    params.q = static_cast<const uint16_t*>(q);
+    params.k = static_cast<const uint16_t*>(k);
+    params.v = static_cast<const uint16_t*>(v);
+    params.inverse = inverse;
+    params.q_out = static_cast<uint16_t*>(q_out);
+    params.k_cache = static_cast<uint16_t*>(k_cache);
+    params.v_cache = static_cast<uint16_t*>(v_cache);
+    params.positions = positions;
+    params.steps = steps;
+    params.first = first;
+    params.q_heads = q_heads;
+    params.kv_heads = kv_heads;
+    params.capacity = capacity;
+    params.head_dim = head_dim;
+    bool vector = head_dim % 16 == 0;
+    for (const void* pointer : {q, k, v, (const void*)q_out, (const void*)k_cache, (const void*)v_cache})
+        vector = vector && aligned_to(pointer, 16);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(batch * steps, 1, 1);
+    config.blockDim = dim3(128, 1, 1);
+    config.dynamicSmemBytes = head_dim * sizeof(float);
+    config.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attrs[1];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attrs;
+    config.numAttrs = 1;
+    const cudaError_t rc = vector ? cudaLaunchKernelEx(&config, rope_kv_prefill_kernel<true>, params)
+                                  : cudaLaunchKernelEx(&config, rope_kv_prefill_kernel<false>, params);
+    return rc == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+}
+
 int mt_dense_rows(const void* x, const void* w, const void* residual, void* out, int M, int K, int N, void* stream) {
     if (!x || !w || !out) return MT_ERR_NULL;
     if (M == 0) return MT_OK;

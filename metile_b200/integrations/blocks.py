@@ -106,11 +106,16 @@ class GatedMLP(nn.Module):
         return self.down_proj(nn.functional.silu(self.gate_proj(values)) * self.up_proj(values))
 
 
+def _rope_frequencies(theta, dim, device):
+    """theta^(-2i/D) for the pairs i of a head: a constant of the model, kept like a weight."""
+    return 1.0 / (theta ** (torch.arange(0, dim, 2, device=device, dtype=torch.float32) / dim))
+
+
 def _rope(values, positions, theta):
     """Rotary embedding over the last axis (half-split form); values [B, heads, T, D], positions [T]
     or [B, T]."""
     dim = values.shape[-1]
-    inverse = 1.0 / (theta ** (torch.arange(0, dim, 2, device=values.device, dtype=torch.float32) / dim))
+    inverse = _rope_frequencies(theta, dim, values.device)
     angles = positions.float()[..., None] * inverse
     if angles.ndim == 2:
         angles = angles[None]
@@ -146,6 +151,17 @@ class KVCache:
         self.advance(steps)
         return self.keys[:, :, :self.length], self.values[:, :, :self.length]
 
+    def rotate_and_fetch(self, queries, keys, values, frequencies):
+        """update_and_fetch with the rotary embedding in front of it, in one kernel: queries [B, T, Hq, D], keys /
+        values [B, T, Hkv, D] as the projections leave them.  Returns the rotated queries and the views."""
+        steps = keys.shape[1]
+        if self.length + steps > self.capacity:
+            raise ValueError("KV cache capacity exceeded")
+        queries = backends.rope_kv_prefill(queries, keys, values, frequencies, self.positions, self.length, self.keys,
+                                           self.values)
+        self.length += steps  # the kernel advanced the device-side count
+        return queries, self.keys[:, :, :self.length], self.values[:, :, :self.length]
+
     def advance(self, steps=1):
         # The device-side count is incremented, not overwritten with the host's number, so that a
         # captured CUDA graph of a decode step advances it on every replay.
@@ -176,19 +192,33 @@ class Attention(nn.Module):
         self.q_proj, self.k_proj, self.v_proj, self.o_proj = q_proj, k_proj, v_proj, o_proj
         self.heads, self.kv_heads, self.head_dim, self.rope_theta = heads, kv_heads, head_dim, rope_theta
         self.scale = head_dim ** -0.5
+        self._frequencies = None
+
+    def _frequencies_on(self, device):
+        if self._frequencies is None or self._frequencies[0] != (self.rope_theta, device):
+            table = _rope_frequencies(self.rope_theta, self.head_dim, device)
+            if torch.cuda.is_current_stream_capturing():
+                return table  # belongs to the graph that is being captured
+            self._frequencies = ((self.rope_theta, device), table)
+        return self._frequencies[1]
 
     def forward(self, values, cache=None):
         batch, steps, _ = values.shape
-        q = self.q_proj(values).view(batch, steps, self.heads, self.head_dim).transpose(1, 2)
-        k = self.k_proj(values).view(batch, steps, self.kv_heads, self.head_dim).transpose(1, 2)
-        v = self.v_proj(values).view(batch, steps, self.kv_heads, self.head_dim).transpose(1, 2)
+        q = self.q_proj(values).view(batch, steps, self.heads, self.head_dim)
+        k = self.k_proj(values).view(batch, steps, self.kv_heads, self.head_dim)
+        v = self.v_proj(values).view(batch, steps, self.kv_heads, self.head_dim)
         offset = 0 if cache is None else cache.length
         if steps > 1 and offset > 0:
             raise ValueError("multi-token continuation is not supported by this harness")
-        positions = torch.arange(offset, offset + steps, device=values.device)
-        q, k = _rope(q, positions, self.rope_theta), _rope(k, positions, self.rope_theta)
-        if cache is not None:
-            k, v = cache.update_and_fetch(k, v)
+        if steps > 1 and type(cache) is KVCache and backends.supports_rope_kv_prefill(q, k, v, cache.keys, cache.values):
+            q, k, v = cache.rotate_and_fetch(q, k, v, self._frequencies_on(values.device))
+            q = q.transpose(1, 2)
+        else:
+            q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
+            positions = torch.arange(offset, offset + steps, device=values.device)
+            q, k = _rope(q, positions, self.rope_theta), _rope(k, positions, self.rope_theta)
+            if cache is not None:
+                k, v = cache.update_and_fetch(k, v)
         out = scaled_dot_product_attention(q, k, v, cache, self.scale, "causal" if steps > 1 else None)
         return self.o_proj(out.transpose(1, 2).reshape(batch, steps, self.heads * self.head_dim))
 
@@ -225,10 +255,17 @@ class TinyCausalLM(nn.Module):
                                   attention.q_proj.weight.device))
         return caches
 
-    def forward(self, tokens, cache=None):
+    def forward(self, tokens, cache=None, logits_to_keep=0):
+        """Logits [batch, tokens, vocabulary]; with `logits_to_keep`, of that many last positions only."""
         hidden = self.embed_tokens(tokens)
         for index, layer in enumerate(self.layers):
             hidden = layer(hidden, None if cache is None else cache[index])
+        if 0 < logits_to_keep < hidden.shape[1]:
+            hidden = hidden[:, -logits_to_keep:].contiguous()
+            # The logits that all positions together would give: one row alone is else another kernel's.
+            if not backends.kernel_pinned():
+                with backends.batch_invariant():
+                    return self.lm_head(self.norm(hidden))
         return self.lm_head(self.norm(hidden))
 
 

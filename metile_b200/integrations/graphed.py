@@ -18,6 +18,8 @@ falls back to its own forward slices the cache at the host's count, which a grap
 
 from __future__ import annotations
 
+import inspect
+
 import torch
 
 
@@ -32,6 +34,7 @@ class GraphedDecoder:
         self.cache = model.make_cache(self.batch, self.capacity)
         device = self.cache[0].keys.device
         self.device = device
+        self._keeps_logits = "logits_to_keep" in inspect.signature(model.forward).parameters
         self.token = torch.zeros((self.batch, 1), dtype=torch.long, device=device)   # input of the next step
         self.logits = None                                                          # output of the last step
         self.graph = None
@@ -45,8 +48,10 @@ class GraphedDecoder:
             raise ValueError("prompt does not fit the decoder's batch or capacity")
         for cache in self.cache:
             cache.reset(0)
+        # Only the last position's logits are asked for: a head over the whole prompt is most of a small model.
+        last_only = {"logits_to_keep": 1} if self._keeps_logits else {}
         with torch.no_grad():
-            out = _logits_of(self.model(tokens, cache=self.cache))
+            out = _logits_of(self.model(tokens, cache=self.cache, **last_only))
         return out[:, -1, :].float()
 
     def _step(self):

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from metile_b200 import backends as B, synth
+from metile_b200.integrations import blocks
 from oracle import affine as A
 from tests.helpers import assert_bit_equal, assert_within, f32, triple_np
 
@@ -60,3 +61,28 @@ def test_tcgen05_projection_edges(cuda_device, rows, k, n):
     weights = triple_np(triple)
     assert_within(plain[some], A.qmm(f32(x[some]), *weights, weights="bf16"))
     assert_within(added[some], A.qmm(f32(x[some]), *weights, residual=f32(r[some]), weights="bf16"))
+
+
+@pytest.mark.parametrize("batch,steps,first,heads,kv_heads,dim", [
+    (1, 1, 0, 1, 1, 2), (2, 7, 3, 3, 1, 20), (1, 130, 0, 6, 2, 64), (3, 33, 40, 4, 4, 128), (1, 2, 30000, 2, 1, 48),
+])
+def test_rope_kv_prefill_is_the_op_by_op_form(cuda_device, batch, steps, first, heads, kv_heads, dim):
+    q, k, v = (synth.activations(seed, batch * steps, width * dim, cuda_device).view(batch, steps, width, dim)
+               for seed, width in ((1, heads), (2, kv_heads), (3, kv_heads)))
+    theta, positions = 1e6, torch.arange(first, first + steps, device=cuda_device)
+    cache = blocks.KVCache(batch, kv_heads, first + steps + 1, dim, cuda_device)
+    cache.reset(first)
+    rotated, keys, values = cache.rotate_and_fetch(q, k, v, blocks._rope_frequencies(theta, dim, q.device))
+    assert_bit_equal(rotated.transpose(1, 2), blocks._rope(q.transpose(1, 2), positions, theta), "queries")
+    assert_bit_equal(keys[:, :, first:], blocks._rope(k.transpose(1, 2), positions, theta), "keys")
+    assert_bit_equal(values[:, :, first:], v.transpose(1, 2), "values")
+    assert not cache.keys[:, :, :first].any() and not cache.keys[:, :, first + steps:].any()
+    assert cache.length == first + steps and (cache.positions == first + steps).all()
+
+
+def test_last_positions_logits_are_those_of_all_positions(cuda_device):
+    model = blocks.random_model(3, device=cuda_device)
+    tokens = torch.arange(23, device=cuda_device).view(1, 23)
+    with torch.no_grad():
+        every, last = model(tokens), model(tokens, logits_to_keep=1)
+    assert_bit_equal(last, every[:, -1:], "logits of the last position")
