@@ -438,7 +438,7 @@ __global__ void rope_kv_append_kernel(const RopeAppendParams p) {
 // product, sum and difference is rounded by itself, the angle is position * inverse[pair], and cosf / sinf are those
 // of the library: what the framework's op-by-op form computes, to the bit.  One CTA per token; its cosines and
 // sines are computed once for all heads.  Bound by launch latency and bytes (512 tokens of 12 + 2 x 2 heads of 128:
-// PREFILL_US; as some 45 framework launches per layer it took about 180 us of host time).
+// 4.4 us; as some 45 framework launches per layer, together with the head over all positions, 540 us per block).
 struct RopePrefillParams {
     const uint16_t* q;        // [B, steps, Hq, D]
     const uint16_t* k;        // [B, steps, Hkv, D]
