@@ -202,6 +202,15 @@ int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row
                       const int* positions, void* q_out, void* k_cache, void* v_cache, int batch,
                       int q_heads, int kv_heads, int capacity, int head_dim, float theta, void* stream);
 
+/* The same, and every position is advanced by one. */
+int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long long row_stride,
+                              int* positions, void* q_out, void* k_cache, void* v_cache, int batch,
+                              int q_heads, int kv_heads, int capacity, int head_dim, float theta, void* stream);
+
+/* The end of a greedy decode step: out[r][i] = fp32 of the bf16 logits[r][i], tokens[r] = the index of the
+ * row's largest value, the first of equals; a NaN counts as larger than any number. */
+int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream);
+
 /* The same for the `steps` tokens of a prompt, which go to rows first, first + 1, ... of every cache.
  * q: dense bf16 [batch, steps, q_heads, head_dim], k, v: [batch, steps, kv_heads, head_dim]; q_out like q;
  * inverse: fp32 [head_dim / 2] on the device, the angle of pair i is position * inverse[i] in fp32; products,

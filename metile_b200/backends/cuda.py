@@ -160,14 +160,14 @@ def mlx_attention_decode(query, key, value, *, scale, autotune=True, lengths=Non
     return out.reshape(batch, q_heads, 1, dim)
 
 
-def rope_kv_append(query, key, value, positions, key_cache, value_cache, *, theta):
+def rope_kv_append(query, key, value, positions, key_cache, value_cache, *, theta, advance=False):
     """Rotate the new query and key rows and append key and value to the caches, in place.
 
     query [B, Hq, D], key / value [B, Hkv, D] -- dense, or three views into the rows of one fused
     q|k|v projection [B, (Hq + 2 Hkv) D] (no copy is made); positions int32 [B] (device): the row of
     each sequence's cache [B, Hkv, capacity, D] that receives the new token.  Returns the rotated
-    query as a dense [B, Hq, D] tensor."""
-    out = native().rope_kv_append(query, key, value, positions, key_cache, value_cache, theta)
+    query as a dense [B, Hq, D] tensor.  With `advance` every position is one higher afterwards."""
+    out = native().rope_kv_append(query, key, value, positions, key_cache, value_cache, theta, bool(advance))
     if out is not None:
         return native_result(out, "rope_kv_append")
     require_cuda_bf16(query, "rope_kv_append")
@@ -197,10 +197,22 @@ def rope_kv_append(query, key, value, positions, key_cache, value_cache, *, thet
         value = fused[:, (q_heads + kv_heads) * dim:].view(batch, kv_heads, dim)
     row_stride = query.stride(0) if batch > 1 else (q_heads + 2 * kv_heads) * dim
     out = torch.empty((batch, q_heads, dim), dtype=torch.bfloat16, device=query.device)
-    code = launch(library().mt_rope_kv_append, query.device, pointer(query), pointer(key), pointer(value),
+    entry = library().mt_rope_kv_append_advance if advance else library().mt_rope_kv_append
+    code = launch(entry, query.device, pointer(query), pointer(key), pointer(value),
                   ctypes.c_longlong(int(row_stride)), pointer(positions), pointer(out), pointer(key_cache),
                   pointer(value_cache), batch, q_heads, kv_heads, capacity, dim, ctypes.c_float(float(theta)))
     _lib.check(code, "rope_kv_append")
+    return out
+
+
+def greedy_token(logits, tokens):
+    """The end of a greedy step: logits [rows, vocabulary] bfloat16 as float32, and in `tokens` (int64, one per row,
+    in place) the index of each row's largest value, as torch.argmax of the result gives it."""
+    out = native().greedy_token(logits, tokens)
+    if out is not None:
+        return native_result(out, "greedy_token")
+    out = logits.float()
+    tokens.copy_(out.argmax(dim=-1).reshape(tokens.shape))
     return out
 
 

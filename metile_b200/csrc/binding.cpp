@@ -321,14 +321,21 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t count) {
     }
 }
 
+int append(const void* q, const void* k, const void* v, long long row_stride, int* positions, void* q_out, void* k_cache,
+           void* v_cache, int batch, int q_heads, int kv_heads, int capacity, int head_dim, float theta, void* stream) {
+    return mt_rope_kv_append(q, k, v, row_stride, positions, q_out, k_cache, v_cache, batch, q_heads, kv_heads, capacity,
+                             head_dim, theta, stream);
+}
+
 inline bool head_major(const Tensor& t, int64_t dim) { return t.stride(2) == 1 && t.stride(1) == dim; }
 
-// rope_kv_append(query, key, value, positions, key_cache, value_cache, theta)
+// rope_kv_append(query, key, value, positions, key_cache, value_cache, theta, advance)
 PyObject* rope_kv_append(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 7) Py_RETURN_NONE;
+    if (count != 8) Py_RETURN_NONE;
     const Tensor* t[6];
     for (int i = 0; i < 6; ++i)
         if (!(t[i] = plain(args[i]))) Py_RETURN_NONE;
+    const bool advance = args[7] == Py_True;
     const double theta = PyFloat_AsDouble(args[6]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
     const Tensor &q = *t[0], &k = *t[1], &v = *t[2], &positions = *t[3], &keys = *t[4], &values = *t[5];
@@ -353,9 +360,9 @@ PyObject* rope_kv_append(PyObject*, PyObject* const* args, Py_ssize_t count) {
         Tensor out = new_bf16({batch, heads, dim}, device);
         int code;
         Py_BEGIN_ALLOW_THREADS
-        code = mt_rope_kv_append(address(q), address(k), address(v), row_stride, static_cast<const int*>(address(positions)),
-                                 address(out), address(keys), address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity,
-                                 (int)dim, (float)theta, launch.stream());
+        code = (advance ? mt_rope_kv_append_advance : append)(
+            address(q), address(k), address(v), row_stride, static_cast<int*>(address(positions)), address(out), address(keys),
+            address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity, (int)dim, (float)theta, launch.stream());
         Py_END_ALLOW_THREADS
         return code_or(code, std::move(out));
     } catch (const std::exception& error) {
@@ -403,10 +410,35 @@ PyObject* rope_kv_prefill(PyObject*, PyObject* const* args, Py_ssize_t count) {
     }
 }
 
+// greedy_token(logits [rows, vocabulary] bf16, tokens [rows] or [rows, 1] int64) -> logits as float32
+PyObject* greedy_token(PyObject*, PyObject* const* args, Py_ssize_t count) {
+    if (count != 2) Py_RETURN_NONE;
+    const Tensor *logits = plain(args[0]), *tokens = plain(args[1]);
+    if (!logits || !tokens || !logits->is_cuda() || logits->dim() != 2 || logits->numel() == 0) Py_RETURN_NONE;
+    const auto device = logits->device();
+    const int64_t rows = logits->size(0), vocabulary = logits->size(1);
+    if (!bf16_on(*logits, device) || tokens->device() != device || tokens->scalar_type() != at::kLong || !tokens->is_contiguous() ||
+        tokens->numel() != rows || !fits_int(rows) || !fits_int(vocabulary))
+        Py_RETURN_NONE;
+    try {
+        const Launch launch(device);
+        Tensor out = at::detail::empty_cuda({rows, vocabulary}, at::kFloat, device, std::nullopt);
+        int code;
+        Py_BEGIN_ALLOW_THREADS
+        code = mt_greedy_token(address(*logits), static_cast<float*>(address(out)), static_cast<long long*>(address(*tokens)), (int)rows,
+                               (int)vocabulary, launch.stream());
+        Py_END_ALLOW_THREADS
+        return code_or(code, std::move(out));
+    } catch (const std::exception& error) {
+        PyErr_SetString(PyExc_RuntimeError, error.what());
+        return nullptr;
+    }
+}
+
 #define MT_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MT_METHOD(project), MT_METHOD(swiglu),    MT_METHOD(mlp_plan),       MT_METHOD(mlp), MT_METHOD(norm),
                          MT_METHOD(dense),   MT_METHOD(attention), MT_METHOD(rope_kv_append),
-                         MT_METHOD(rope_kv_prefill), {nullptr, nullptr, 0, nullptr}};
+                         MT_METHOD(rope_kv_prefill), MT_METHOD(greedy_token), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

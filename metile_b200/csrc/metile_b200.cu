@@ -520,12 +520,14 @@ int mt_attention_decode(const void* q, const void* k_cache, const void* v_cache,
                            : launch_attention_dim<64>(params, batch, q_heads / kv_heads, s);
 }
 
-int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row_stride, const int* positions,
-                      void* q_out, void* k_cache, void* v_cache, int batch, int q_heads, int kv_heads, int capacity,
-                      int head_dim, float theta, void* stream) {
+static int run_rope_kv_append(const void* q, const void* k, const void* v, long long row_stride, int* positions, bool advance,
+                              void* q_out, void* k_cache, void* v_cache, int batch, int q_heads, int kv_heads, int capacity,
+                              int head_dim, float theta, void* stream) {
     if (batch < 0 || q_heads < 1 || kv_heads < 1 || capacity < 1 || head_dim < 2 || head_dim % 2 || theta <= 0.0f)
         return MT_ERR_SHAPE;
     if (row_stride < (long long)kv_heads * head_dim) return MT_ERR_SHAPE;
+    const int smem = head_dim * (int)sizeof(float);
+    if (head_dim > 56 * 1024) return MT_ERR_SHAPE;
     if (batch == 0) return MT_OK;
     if (!q || !k || !v || !positions || !q_out || !k_cache || !v_cache) return MT_ERR_NULL;
     if (!device_is_sm100()) return MT_ERR_DEVICE;
@@ -542,10 +544,16 @@ int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row
     params.capacity = capacity;
     params.head_dim = head_dim;
     params.row_stride = row_stride;
+    params.advance = advance;
     params.log2_theta = log2f(theta);
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(batch * (q_heads + 2 * kv_heads), 1, 1);
-    config.blockDim = dim3(64, 1, 1);
+    const long long pairs = (long long)(q_heads + 2 * kv_heads) * (head_dim / 2);
+    config.gridDim = dim3(batch, 1, 1);
+    config.blockDim = dim3(pairs < kRopeThreads ? (int)((pairs + 31) / 32 * 32) : kRopeThreads, 1, 1);
+    config.dynamicSmemBytes = smem;
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(rope_kv_append_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return MT_ERR_LAUNCH;
     config.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attrs[1];
     attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -553,6 +561,45 @@ int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row
     config.attrs = attrs;
     config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, rope_kv_append_kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+}
+
+int mt_rope_kv_append(const void* q, const void* k, const void* v, long long row_stride, const int* positions,
+                      void* q_out, void* k_cache, void* v_cache, int batch, int q_heads, int kv_heads, int capacity,
+                      int head_dim, float theta, void* stream) {
+    return run_rope_kv_append(q, k, v, row_stride, const_cast<int*>(positions), false, q_out, k_cache, v_cache, batch,
+                              q_heads, kv_heads, capacity, head_dim, theta, stream);
+}
+
+int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long long row_stride, int* positions,
+                              void* q_out, void* k_cache, void* v_cache, int batch, int q_heads, int kv_heads,
+                              int capacity, int head_dim, float theta, void* stream) {
+    return run_rope_kv_append(q, k, v, row_stride, positions, true, q_out, k_cache, v_cache, batch, q_heads, kv_heads,
+                              capacity, head_dim, theta, stream);
+}
+
+int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream) {
+    if (rows < 0 || vocabulary < 1 || rows > 0x7FFFFFFF / kGreedyCluster) return MT_ERR_SHAPE;
+    if (rows == 0) return MT_OK;
+    if (!logits || !out || !tokens) return MT_ERR_NULL;
+    if (!device_is_sm100()) return MT_ERR_DEVICE;
+    GreedyParams params{static_cast<const uint16_t*>(logits), out, tokens, vocabulary};
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(rows * kGreedyCluster, 1, 1);
+    config.blockDim = dim3(kGreedyThreads, 1, 1);
+    config.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = kGreedyCluster;
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    config.attrs = attrs;
+    config.numAttrs = 2;
+    const bool vector = vocabulary % 8 == 0 && aligned_to(logits, 16) && aligned_to(out, 16);
+    const cudaError_t rc = vector ? cudaLaunchKernelEx(&config, greedy_token_kernel<true>, params)
+                                  : cudaLaunchKernelEx(&config, greedy_token_kernel<false>, params);
+    return rc == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
 int mt_rope_kv_prefill(const void* q, const void* k, const void* v, const float* inverse, void* q_out, void* k_cache,

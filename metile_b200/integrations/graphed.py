@@ -22,6 +22,8 @@ import inspect
 
 import torch
 
+from .. import backends
+
 
 def _logits_of(output):
     return getattr(output, "logits", output)
@@ -56,10 +58,8 @@ class GraphedDecoder:
 
     def _step(self):
         out = _logits_of(self.model(self.token, cache=self.cache))
-        logits = out[:, -1, :].float()
         # The next step's input is chosen on the device: replays need no host in between.
-        self.token.copy_(logits.argmax(dim=-1, keepdim=True))
-        return logits
+        return backends.greedy_token(out[:, -1, :], self.token)
 
     def _capture(self):
         """Warm every lazily built piece on scratch caches, then capture one step on the real ones."""

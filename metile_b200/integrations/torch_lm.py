@@ -28,6 +28,7 @@ from dataclasses import dataclass, field
 import torch
 
 from .. import backends
+from .blocks import KVCache
 
 FEATURES = ("attention", "rms_norm", "graph_fusion", "quantized_mlp")
 _GATED_MLP_ATTRIBUTES = ("gate_proj", "up_proj", "down_proj")
@@ -218,8 +219,13 @@ def execute_attention_decode(module, values, cache, residual=None):
     q = qkv[:, :heads * dim].view(batch, heads, dim)
     k = qkv[:, heads * dim:(heads + kv_heads) * dim].view(batch, kv_heads, dim)
     v = qkv[:, (heads + kv_heads) * dim:].view(batch, kv_heads, dim)
-    rotated = backends.rope_kv_append(q, k, v, cache.positions, cache.keys, cache.values, theta=module.rope_theta)
-    cache.advance(1)
+    own_cache = type(cache) is KVCache  # of which we know that advancing is counting, on the host and on the device
+    rotated = backends.rope_kv_append(q, k, v, cache.positions, cache.keys, cache.values, theta=module.rope_theta,
+                                      advance=own_cache)
+    if own_cache:
+        cache.length += 1
+    else:
+        cache.advance(1)
     scale = getattr(module, "scale", dim ** -0.5)
     # The whole cache with the per-sequence lengths on the device (not a slice cut at the host's count):
     # the same 128-token splits are merged either way, and nothing of the step depends on a host number,

@@ -86,3 +86,31 @@ def test_last_positions_logits_are_those_of_all_positions(cuda_device):
     with torch.no_grad():
         every, last = model(tokens), model(tokens, logits_to_keep=1)
     assert_bit_equal(last, every[:, -1:], "logits of the last position")
+
+
+@pytest.mark.parametrize("rows,vocabulary", [(1, 1), (3, 7), (16, 32768), (2, 2047), (5, 40000)])
+def test_greedy_token_is_float_and_argmax(cuda_device, rows, vocabulary):
+    logits = synth.activations(1, rows, vocabulary, cuda_device).round()   # many equal values
+    tokens = torch.full((rows, 1), -1, dtype=torch.long, device=cuda_device)
+    for special in (None, float("inf"), float("nan")):
+        if special is not None:
+            logits[rows // 2, vocabulary // 3:] = special
+        assert_bit_equal(B.greedy_token(logits, tokens), logits.float(), "logits")
+        assert (tokens == logits.float().argmax(-1, keepdim=True)).all()
+    logits[:] = float("-inf")
+    B.greedy_token(logits, tokens)
+    assert (tokens == logits.float().argmax(-1, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,dim", [(1, 1, 1, 2), (3, 5, 5, 128), (2, 40, 8, 128)])
+def test_rope_append_advances_every_position_once(cuda_device, batch, heads, kv_heads, dim):
+    q, k, v = (synth.activations(seed, batch * width, dim, cuda_device).view(batch, width, dim)
+               for seed, width in ((1, heads), (2, kv_heads), (3, kv_heads)))
+    positions = torch.arange(batch, dtype=torch.int32, device=cuda_device)
+    caches = [torch.zeros(batch, kv_heads, batch + 1, dim, dtype=torch.bfloat16, device=cuda_device) for _ in range(4)]
+    kept = B.rope_kv_append(q, k, v, positions, *caches[:2], theta=1e4)
+    assert (positions.cpu() == torch.arange(batch)).all()
+    assert_bit_equal(B.rope_kv_append(q, k, v, positions, *caches[2:], theta=1e4, advance=True), kept, "queries")
+    assert (positions.cpu() == torch.arange(batch) + 1).all()
+    assert_bit_equal(caches[2], caches[0], "keys")
+    assert_bit_equal(caches[3], caches[1], "values")
