@@ -46,6 +46,7 @@ _state = threading.local()
 _dispatch_lock = threading.RLock()
 _swiglu_dispatches = {}
 _residual_dispatches = {}
+_recorded = set()  # calls that would record what the tables hold already
 
 
 def _flags():
@@ -100,6 +101,15 @@ def _record(table, rows, input_features, output_features, dtype, group_size, bit
     if table.get(key) != algorithm:
         with _dispatch_lock:
             table[key] = algorithm
+            _recorded.clear()
+
+
+def _record_call(table, values, weight, group_size, bits, flags):
+    """_record for a call's tensors; the usual call, one like an earlier one, costs one look-up."""
+    call = (table is _swiglu_dispatches, values.shape, weight.shape, values.dtype, group_size, bits, flags)
+    if call not in _recorded:
+        _record(table, rows_of(values), values.shape[-1], weight.shape[0], values.dtype, group_size, bits, flags)
+        _recorded.add(call)
 
 
 def _project(name, values, weight, scales, biases, residual, group_size, bits):
@@ -140,8 +150,7 @@ def mlx_affine_residual_qmv(values, weight, scales, biases, residual, *, group_s
     del autotune
     out, flags = _project("affine residual QMV", values, weight, scales, biases, residual,
                           group_size, bits)
-    _record(_residual_dispatches, rows_of(values), values.shape[-1], weight.shape[0], values.dtype,
-            group_size, bits, flags)
+    _record_call(_residual_dispatches, values, weight, group_size, bits, flags)
     return out
 
 
@@ -152,8 +161,7 @@ def _swiglu(name, values, gate_weight, gate_scales, gate_biases, up_weight, up_s
         out = native().swiglu(values, gate_weight, gate_scales, gate_biases, up_weight, up_scales, up_biases, flags)
         if out is not None:
             native_result(out, name)
-            _record(_swiglu_dispatches, rows_of(values), values.shape[-1], gate_weight.shape[0], values.dtype,
-                    group_size, bits, flags)
+            _record_call(_swiglu_dispatches, values, gate_weight, group_size, bits, flags)
             return out
     if not (bits == 4 and group_size == 64):
         raise ValueError(f"{name} requires 4-bit group-64 weights")
