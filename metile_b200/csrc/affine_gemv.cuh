@@ -306,6 +306,10 @@ affine_gemv_kernel(const uint16_t* x, GemvWeights first, GemvWeights second, con
 // warp's, two iterations ahead, by asynchronous copies (96 KB in flight per SM, no registers, and no synchronisation
 // beyond the warp's).  The fp32 activations and the slot sums are made by one thread per slot with one barrier; the
 // lanes' totals of all rows are folded together (5 exchanges instead of 16); the warps' rows are dealt out SM by SM.
+// Times in a replayed graph, with registers and with rings: 1536 -> 8960 6.8 and 4.7 us, 4096 -> 4096 7.6 and 5.0, 2048 ->
+// 16384 10.3 and 7.1, 2048 -> 128256 42.2 and 37.6.  The largest are bound by the logic pipe: 44 instructions per 32
+// weights for the unpack and 12 more beside it, at half rate, in a warp that issues 117.  Three CTAs of 80 registers
+// per SM instead of two of 125: 38.5 us.
 constexpr int kGemvRingSlots = 3;
 constexpr int kGemvRingRows = 4;  // weight rows of a half-warp: four outputs, or two of gate and two of up
 constexpr int kGemvTableWords = 5;  // nine groups of a row and step, wherever they start within a word
@@ -545,6 +549,9 @@ inline int launch_gemv_instance(const uint16_t* x, GemvWeights a, GemvWeights b,
 
 constexpr int kGemvRingLimit = 112 * 1024;  // two CTAs per SM
 
+// Where the rings serve: table words are copied whole, so tables start on one; byte offsets are 32 bits wide; the fp32
+// activations of a row have the room that two CTAs' rings leave (K up to 13824), and a half-warp's rows exist.
+// Everything else takes the register form below.
 template <bool kDual>
 inline bool gemv_ring_applicable(const GemvWeights& a, const GemvWeights& b, int K, int N) {
     for (const GemvWeights* w : {&a, &b})
