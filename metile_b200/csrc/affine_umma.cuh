@@ -500,11 +500,18 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                     const RingCursor second = x_at;
                     if (valid > 2) x_at.advance(x_slots);
                     if ((int)(count & 1u) != mine) continue;
-                    alive = (st > begin || ptx::mbar_wait_spin(&acc_empty[unit], ((q >> p.unit_shift) & 1u) ^ 1u, abort_flag, kWaitAccEmpty)) &&
+                    // A parity wait is only right when the phase before the awaited one is known to be over.  For the
+                    // accumulators that is the previous slice's own wait: with two units and more it lies at least two slots
+                    // back, and this warp has had the turn since; with one unit and a slice of one slot it is the other
+                    // warp's for the slot just before, so there the turn comes first.
+                    const uint32_t acc_parity = ((q >> p.unit_shift) & 1u) ^ 1u;
+                    const bool acc_first = st == begin && unit_mask != 0, acc_last = st == begin && unit_mask == 0;
+                    alive = (!acc_first || ptx::mbar_wait_spin(&acc_empty[unit], acc_parity, abort_flag, kWaitAccEmpty)) &&
                             ptx::mbar_wait_spin(&x_full[first.slot], first.phase, abort_flag, kWaitXFull) &&
                             (valid <= 2 || ptx::mbar_wait_spin(&x_full[second.slot], second.phase, abort_flag, kWaitXFull)) &&
                             ptx::mbar_wait_spin(&a_full[mine], (count >> 1) & 1u, abort_flag, kWaitAbFull) &&
-                            (count == 0 || ptx::mbar_wait_spin(&turn[mine], ((count - 1) >> 1) & 1u, abort_flag, kWaitTurn));
+                            (count == 0 || ptx::mbar_wait_spin(&turn[mine], ((count - 1) >> 1) & 1u, abort_flag, kWaitTurn)) &&
+                            (!acc_last || ptx::mbar_wait_spin(&acc_empty[unit], acc_parity, abort_flag, kWaitAccEmpty));
                     if (!alive) break;
                     __syncwarp();
                     ptx::tc_fence_after_sync();

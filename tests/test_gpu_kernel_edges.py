@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from metile_b200 import backends as B, synth
+from metile_b200 import _lib, backends as B, synth
 from metile_b200.integrations import blocks
 from oracle import affine as A
 from tests.helpers import assert_bit_equal, assert_within, f32, triple_np
@@ -61,6 +61,26 @@ def test_tcgen05_projection_edges(cuda_device, rows, k, n):
     weights = triple_np(triple)
     assert_within(plain[some], A.qmm(f32(x[some]), *weights, weights="bf16"))
     assert_within(added[some], A.qmm(f32(x[some]), *weights, residual=f32(r[some]), weights="bf16"))
+
+
+@pytest.mark.parametrize("rows,k,n", [
+    (300, 64, 20480),     # one ring slot per tile, one accumulator unit, four tiles per CTA
+    (300, 256, 20480),
+    (2000, 192, 3333),    # the same with unaligned tables, narrow rows
+    (2000, 512, 5000),    # two slots per tile
+])
+def test_tcgen05_projection_of_short_rows_over_many_tiles(cuda_device, rows, k, n):
+    x = synth.activations(1, rows, k, cuda_device)
+    triple = synth.affine_weight(2, n, k, cuda_device)
+    r = synth.activations(3, rows, n, cuda_device)
+    y, added = B.mlx_affine_qmv(x, *triple), B.mlx_affine_residual_qmv(x, *triple, r)
+    few = [(B.mlx_affine_qmv(x[i:i + 48], *triple), B.mlx_affine_residual_qmv(x[i:i + 48], *triple, r[i:i + 48]))
+           for i in range(0, rows, 48)]
+    assert_bit_equal(y, torch.cat([plain for plain, _ in few]), "rows in batches of 48")
+    assert_bit_equal(added, torch.cat([sums for _, sums in few]), "with a residual")
+    some = [0, rows // 2, rows - 1]
+    assert_within(y[some], A.qmm(f32(x[some]), *triple_np(triple), weights="bf16"))
+    assert _lib.device_status()[0]
 
 
 @pytest.mark.parametrize("batch,steps,first,heads,kv_heads,dim", [
