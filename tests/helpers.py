@@ -1,9 +1,12 @@
 """Shared helpers for the parity tests: torch tensors <-> the numpy oracle."""
 
+import os
+import subprocess
+
 import numpy as np
 import torch
 
-from metile_b200 import synth
+from metile_b200 import build, synth
 from oracle import affine as oracle
 
 
@@ -34,3 +37,16 @@ def assert_bit_equal(a, b, what=""):
     b16 = b.detach().cpu().contiguous().view(torch.uint16)
     mismatches = int((a16 != b16).sum())
     assert mismatches == 0, f"{what}: {mismatches} of {a16.numel()} outputs differ bitwise"
+
+
+def host_program(folder, source):
+    """Compile a program over the kernels' headers and run it HERE, without a GPU: the rows of integers it prints.
+    For rules that the host and the device share, taken from where they stand."""
+    path = os.path.join(folder, "program.cu")
+    with open(path, "w") as file:
+        file.write(source)
+    binary = os.path.join(folder, "program")
+    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "--expt-relaxed-constexpr",
+                    "-I", build.CSRC, path, "-o", binary], check=True)
+    lines = subprocess.run([binary], check=True, capture_output=True, text=True).stdout.split("\n")
+    return [tuple(int(word) for word in line.split()) for line in lines if line]
