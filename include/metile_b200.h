@@ -17,6 +17,11 @@
  *   biases   bf16  [N, K/64]     w[n,k] = scales[n,k/64] * q[n,k] + biases[n,k/64]
  *   out      bf16  [M, N]        y = x @ w^T, fp32 accumulation, one rounding at the store
  *
+ * Packed weights, scales and biases are read ahead of the stream order: a kernel may start on them while
+ * the one in front of it still runs.  What writes them must be complete when the call is made, or be followed
+ * on the stream by a kernel that starts after its end; activations, residuals, caches, dense and norm weights and
+ * tables may be the output of the kernel directly in front.
+ *
  * Return value: 0 (MT_OK) or a negative code; mt_status_string() names it.  Codes:
  *   -1 shape, -2 alignment, -3 quantisation format, -4 CUDA launch error, -5 wrong device,
  *   -6 null pointer, -7 workspace, -8 a bounded device-side wait gave up.

@@ -483,14 +483,14 @@ __global__ void __launch_bounds__(256) rope_kv_prefill_kernel(const RopePrefillP
     const int b = blockIdx.x / p.steps, step = blockIdx.x - b * p.steps;
     const int dim = p.head_dim, half = dim >> 1;
     float *cosines = rope_angles, *sines = rope_angles + half;
+    ptx::griddep_launch_dependents();
+    ptx::griddep_wait();  // the table too may be the preceding kernel's output
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         const float angle = __fmul_rn((float)(p.first + step), p.inverse[i]);
         cosines[i] = cosf(angle);
         sines[i] = sinf(angle);
     }
     __syncthreads();
-    ptx::griddep_launch_dependents();
-    ptx::griddep_wait();
     if (step == 0 && threadIdx.x == 0 && p.positions) p.positions[b] += p.steps;
     constexpr int kWidth = kVector ? 8 : 1;   // pairs of a thread
     const int units = half / kWidth;          // threads of a head
