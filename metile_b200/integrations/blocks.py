@@ -203,24 +203,28 @@ class Attention(nn.Module):
         return self._frequencies[1]
 
     def forward(self, values, cache=None):
-        batch, steps, _ = values.shape
-        q = self.q_proj(values).view(batch, steps, self.heads, self.head_dim)
-        k = self.k_proj(values).view(batch, steps, self.kv_heads, self.head_dim)
-        v = self.v_proj(values).view(batch, steps, self.kv_heads, self.head_dim)
+        return self.o_proj(self.attend(self.q_proj(values), self.k_proj(values), self.v_proj(values), cache))
+
+    def attend(self, q, k, v, cache=None):
+        """Rotary embedding, cache and attention of projected rows [B, T, heads D]; returns [B, T, Hq D]."""
+        batch, steps, _ = q.shape
+        q = q.view(batch, steps, self.heads, self.head_dim)
+        k = k.view(batch, steps, self.kv_heads, self.head_dim)
+        v = v.view(batch, steps, self.kv_heads, self.head_dim)
         offset = 0 if cache is None else cache.length
         if steps > 1 and offset > 0:
             raise ValueError("multi-token continuation is not supported by this harness")
         if steps > 1 and type(cache) is KVCache and backends.supports_rope_kv_prefill(q, k, v, cache.keys, cache.values):
-            q, k, v = cache.rotate_and_fetch(q, k, v, self._frequencies_on(values.device))
+            q, k, v = cache.rotate_and_fetch(q, k, v, self._frequencies_on(q.device))
             q = q.transpose(1, 2)
         else:
             q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
-            positions = torch.arange(offset, offset + steps, device=values.device)
+            positions = torch.arange(offset, offset + steps, device=q.device)
             q, k = _rope(q, positions, self.rope_theta), _rope(k, positions, self.rope_theta)
             if cache is not None:
                 k, v = cache.update_and_fetch(k, v)
         out = scaled_dot_product_attention(q, k, v, cache, self.scale, "causal" if steps > 1 else None)
-        return self.o_proj(out.transpose(1, 2).reshape(batch, steps, self.heads * self.head_dim))
+        return out.transpose(1, 2).reshape(batch, steps, self.heads * self.head_dim)
 
 
 class DecoderBlock(nn.Module):

@@ -26,6 +26,7 @@ import weakref
 from dataclasses import dataclass, field
 
 import torch
+from torch.nn.modules import module as torch_module
 
 from .. import backends
 from . import blocks
@@ -244,95 +245,70 @@ def execute_attention_decode(module, values, cache, residual=None):
 
 
 _ATTENTION_FORWARD, _LINEAR_FORWARD = blocks.Attention.forward, blocks.QuantizedLinear.forward
+_MODULE_CALL = torch.nn.Module.__call__
+_norm_replacements, _attention_replacements = weakref.WeakSet(), weakref.WeakSet()  # forwards made by the patcher
 
 
-class _PrefillPlan:
-    """What a decoder block's prefill calls, looked up once: a module of torch costs a few microseconds per call
-    and attribute, and a short prompt is bound by them (64 tokens, four blocks of 1024: 557 us per call, 452 with plans).  The same operators in the same order as the modules' own forwards; `current()` tells
-    whether those would still do that."""
-
-    def __init__(self, block, eps):
-        attention, mlp = block.self_attn, block.mlp
-        self.attention = attention
-        self.norms = block.input_layernorm, block.post_attention_layernorm
-        self.eps = _norm_eps(self.norms[0]), eps
-        linears = [getattr(attention, name) for name in _ATTENTION_ATTRIBUTES]
-        self.triples = [(linear.weight, linear.scales, linear.biases) for linear in linears]
-        self.weights = [norm.weight for norm in self.norms]
-        linears += [getattr(mlp, name) for name in _GATED_MLP_ATTRIBUTES]
-        self.modules = [attention, mlp, *self.norms, *linears]
-        self.mlp = mlp
-        self.parts = [(block._modules, name, block._modules[name])
-                      for name in ("self_attn", "mlp", "input_layernorm", "post_attention_layernorm")]
-        for owner, names in ((attention, _ATTENTION_ATTRIBUTES), (mlp, _GATED_MLP_ATTRIBUTES)):
-            self.parts += [(owner._modules, name, owner._modules[name]) for name in names]
-        for module in (*linears, *self.norms):
-            self.parts += [(module._buffers, name, tensor) for name, tensor in module._buffers.items()]
-        self.forwards = [(type(module), type(module).forward) for module in self.modules[:4]]
-
-    @classmethod
-    def of(cls, block, eps):
-        """The plan of a block whose parts are this package's own, or None."""
-        attention, mlp = block.self_attn, block.mlp
-        norms = block.input_layernorm, block.post_attention_layernorm
-        if type(attention) is not blocks.Attention or type(mlp) is not blocks.GatedMLP \
-                or any(type(norm) is not blocks.RMSNorm for norm in norms):
-            return None
-        patched = getattr(blocks.Attention.forward, "_metile_original", blocks.Attention.forward)
-        if patched is not _ATTENTION_FORWARD or blocks.QuantizedLinear.forward is not _LINEAR_FORWARD \
-                or getattr(blocks.RMSNorm.forward, "_metile_original", None) is None or _norm_eps(norms[0]) is None:
-            return None
-        linears = [getattr(attention, name, None) for name in _ATTENTION_ATTRIBUTES]
-        linears += [getattr(mlp, name, None) for name in _GATED_MLP_ATTRIBUTES]
-        if any(type(linear) is not blocks.QuantizedLinear or not _is_affine_int4(linear) or linear.bias is not None
-               for linear in linears):
-            return None
-        return cls(block, eps)
-
-    def current(self):
-        return all(owner.get(name) is part for owner, name, part in self.parts) \
-            and all(kind.forward is forward for kind, forward in self.forwards) \
-            and blocks.QuantizedLinear.forward is _LINEAR_FORWARD \
-            and not any(module._forward_hooks or module._forward_pre_hooks for module in self.modules)
-
-    def run(self, values, cache):
-        attention = self.attention
-        heads, kv_heads, dim = attention.heads, attention.kv_heads, attention.head_dim
-        batch, steps, _ = values.shape
-        normed = backends.mlx_rms_norm(values, self.weights[0], self.eps[0])
-        q, k, v = (backends.mlx_affine_qmv(normed, *triple).view(batch, steps, count, dim)
-                   for triple, count in zip(self.triples, (heads, kv_heads, kv_heads)))
-        q, k, v = cache.rotate_and_fetch(q, k, v, attention._frequencies_on(values.device))
-        out = blocks.scaled_dot_product_attention(q.transpose(1, 2), k, v, cache, attention.scale, "causal")
-        attended = backends.mlx_affine_qmv(out.transpose(1, 2).reshape(batch, steps, heads * dim), *self.triples[3])
-        hidden, normalized = backends.mlx_add_rms_norm(values, attended, self.weights[1], self.eps[1])
-        return execute_quantized_mlp(self.mlp, normalized, hidden)
+def _is_plain_call(module, kind):
+    """Whether calling `module` is kind.forward and nothing else: no hook, no forward of its own, not compiled."""
+    state = module.__dict__
+    return type(module) is kind and kind.__call__ is _MODULE_CALL and "forward" not in state \
+        and state.get("_compiled_call_impl") is None \
+        and not (state["_forward_hooks"] or state["_forward_pre_hooks"] or state["_backward_hooks"]
+                 or state["_backward_pre_hooks"])
 
 
-_prefill_plans = weakref.WeakKeyDictionary()
-
-
-def _prefill_plan(block, values, cache, eps):
-    """The plan for this call, or None: a prompt into an empty in-place cache of this package, dense bfloat16."""
-    if type(cache) is not KVCache or cache.length or values.ndim != 3 or not 1 < values.shape[1] <= cache.keys.shape[2] \
-            or values.shape[0] != cache.keys.shape[0] or type(values) is not torch.Tensor or values.requires_grad \
-            or not values.is_contiguous() or cache.keys.dtype != torch.bfloat16 or cache.keys.device != values.device:
+def _plain_triple(linear):
+    """The buffers of a projection whose call is mlx_affine_qmv of them and nothing else, or None."""
+    if not _is_plain_call(linear, blocks.QuantizedLinear) or linear.bias is not None \
+            or linear.group_size != 64 or linear.bits != 4:
         return None
-    plan = _prefill_plans.get(block)
-    if plan is None or not plan.current() or plan.eps[1] != eps:
-        plan = _PrefillPlan.of(block, eps)
-        if plan is None or not plan.current() or quantized_mlp_refusal(block.mlp, values) is not None:
+    buffers = linear._buffers
+    triple = buffers.get("weight"), buffers.get("scales"), buffers.get("biases")
+    return None if any(tensor is None for tensor in triple) else triple
+
+
+def prompt_attention(norm, attention, values, cache):
+    """attention(norm(values), cache) for a prompt, by the operators that the two modules' own forwards call; None when
+    they, or one of the four projections, would do anything else.
+
+    A module of torch costs a few microseconds per call and attribute, and a short prompt is bound by them.
+    Nothing is kept from one call for the next: every part, tensor and setting is looked at where the
+    modules themselves would read it."""
+    if type(cache) is not KVCache or values.ndim != 3 or values.shape[1] < 2 or torch._C._get_tracing_state() \
+            or torch_module._has_any_global_hook():
+        return None
+    forward = blocks.Attention.forward
+    if forward is not _ATTENTION_FORWARD and (forward not in _attention_replacements
+                                              or forward._metile_original is not _ATTENTION_FORWARD):
+        return None
+    if blocks.QuantizedLinear.forward is not _LINEAR_FORWARD or blocks.RMSNorm.forward not in _norm_replacements \
+            or not _is_plain_call(norm, blocks.RMSNorm) or not _is_plain_call(attention, blocks.Attention):
+        return None
+    weight, eps = norm._buffers.get("weight"), _norm_eps(norm)
+    if weight is None or eps is None or weight.dtype != values.dtype:
+        return None
+    parts = attention._modules
+    triples = []
+    for name in _ATTENTION_ATTRIBUTES:
+        linear = parts.get(name)
+        triple = None if linear is None else _plain_triple(linear)
+        if triple is None:
             return None
-        _prefill_plans[block] = plan
-    return plan
+        triples.append(triple)
+    normed = backends.mlx_rms_norm(values, weight, eps)
+    attended = attention.attend(*(backends.mlx_affine_qmv(normed, *triple) for triple in triples[:3]), cache)
+    return backends.mlx_affine_qmv(attended, *triples[3])
 
 
-def _replace_forward(patch, cls, make_replacement):
+def _replace_forward(patch, cls, make_replacement, known=None):
     original = cls.forward
     if getattr(original, "_metile_original", None) is not None:
         return False
     replacement = make_replacement(original)
     replacement._metile_original = original
+    if known is not None:
+        known.add(replacement)
     patch.replacements.append((cls, "forward", original))
     cls.forward = replacement
     return True
@@ -398,7 +374,7 @@ def _patch_rms_norm(model, patch):
 
             return replacement
 
-        _replace_forward(patch, norm_class, make)
+        _replace_forward(patch, norm_class, make, _norm_replacements)
 
 
 def _patch_attention(model, patch):
@@ -443,7 +419,7 @@ def _patch_attention(model, patch):
 
             return replacement
 
-        _replace_forward(patch, attention_class, make)
+        _replace_forward(patch, attention_class, make, _attention_replacements)
     if len(patch.replacements) == before:
         patch.refuse("attention", "the model exposes no attention surface that can be replaced")
 
@@ -466,14 +442,12 @@ def _patch_graph_fusion(model, patch, quantized_mlp):
                     patch.refuse("graph_fusion", "activations are not bfloat16 on a CUDA device")
                     return original(self, values, *args, **kwargs)
                 cache = args[0] if args else kwargs.get("cache")
-                if quantized_mlp and len(args) <= 1 and set(kwargs) <= {"cache"}:
-                    plan = _prefill_plan(self, values, cache, eps)
-                    if plan is not None:
-                        return plan.run(values, cache)
-                normed_input = self.input_layernorm(values)
+                only_cache = len(args) <= 1 and set(kwargs) <= {"cache"}
+                attended = prompt_attention(self.input_layernorm, attention, values, cache) if only_cache else None
+                normed_input = self.input_layernorm(values) if attended is None else None
                 fused_attention = (
-                    getattr(type(attention).forward, "_metile_original", None) is not None
-                    and len(args) <= 1 and set(kwargs) <= {"cache"}
+                    attended is None and only_cache
+                    and getattr(type(attention).forward, "_metile_original", None) is not None
                     and _has_parts(attention, _ATTENTION_ATTRIBUTES)
                     and attention_decode_refusal(attention, normed_input, cache) is None)
                 if fused_attention:
@@ -482,7 +456,8 @@ def _patch_graph_fusion(model, patch, quantized_mlp):
                     hidden = execute_attention_decode(attention, normed_input, cache, residual=values)
                     normalized = backends.mlx_rms_norm(hidden, post.weight, eps)
                 else:
-                    attended = attention(normed_input, *args, **kwargs)
+                    if attended is None:
+                        attended = attention(normed_input, *args, **kwargs)
                     hidden, normalized = backends.mlx_add_rms_norm(values, attended, post.weight, eps)
                 if quantized_mlp:
                     reason = quantized_mlp_refusal(self.mlp, normalized)

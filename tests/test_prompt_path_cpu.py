@@ -1,0 +1,104 @@
+"""A prompt through a patched block calls operators in place of torch modules: only where the modules would do
+nothing else, whatever a program has changed about them since the last call."""
+
+import pytest
+import torch
+
+from metile_b200 import backends
+from metile_b200.integrations import blocks
+from metile_b200.integrations.torch_lm import apply_metile_to_torch_lm, prompt_attention
+
+
+def stand_in_projection(values, weight, scales, biases, *, group_size=64, bits=4):
+    dense = (scales.float() * (1 + weight[:, ::8].view(torch.int32).float().abs() / 2**31)).repeat_interleave(64, dim=1)
+    return torch.nn.functional.linear(values.float(), dense + biases.float().mean()).to(values.dtype) * (bits / 4)
+
+
+def stand_in_norm(values, weight, eps):
+    return (torch.nn.functional.rms_norm(values.float(), weight.shape, eps=eps) * weight.float()).to(values.dtype)
+
+
+@pytest.fixture
+def block(monkeypatch):
+    monkeypatch.setattr(backends, "mlx_affine_qmv", stand_in_projection)
+    monkeypatch.setattr(backends, "mlx_rms_norm", stand_in_norm)
+    model = blocks.random_model(1, hidden=128, intermediate=128, heads=2, kv_heads=1, layers=1, vocab=64, device="cpu")
+    # The patched norm asks for a CUDA device; here its own replacement is what a GPU would run.
+    with apply_metile_to_torch_lm(model, attention=True):
+        replacement = blocks.RMSNorm.forward
+        norm_forward = lambda self, values: backends.mlx_rms_norm(values, self.weight, self.eps)  # noqa: E731
+        norm_forward._metile_original = replacement._metile_original
+        monkeypatch.setattr("metile_b200.integrations.torch_lm._norm_replacements", {norm_forward})
+        blocks.RMSNorm.forward = norm_forward
+        yield model.layers[0]
+
+
+def both_ways(block):
+    values = torch.randn(1, 5, 128, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16)
+
+    def cache():
+        return blocks.KVCache(1, 1, 8, 64, "cpu")
+    short = prompt_attention(block.input_layernorm, block.self_attn, values, cache())
+    return short, block.self_attn(block.input_layernorm(values), cache())
+
+
+def doubled(forward):
+    return lambda *args, **kwargs: 2 * forward(*args, **kwargs)
+
+
+def test_the_modules_as_they_were_made(block):
+    short, modules = both_ways(block)
+    assert short is not None and torch.equal(short, modules)
+
+
+@pytest.mark.parametrize("change", [
+    lambda b: setattr(b.input_layernorm, "eps", 0.5),
+    lambda b: setattr(b.self_attn, "scale", 0.01),
+    lambda b: setattr(b.self_attn, "rope_theta", 1e2),
+    lambda b: setattr(b.self_attn.q_proj, "scales", b.self_attn.q_proj.scales * 2),
+    lambda b: setattr(b.self_attn, "o_proj", blocks.QuantizedLinear.from_seed(9, 128, 128)),
+    lambda b: b.input_layernorm.weight.mul_(3),
+])
+def test_changed_tensors_and_settings_count(block, change):
+    before, _ = both_ways(block)
+    change(block)
+    short, modules = both_ways(block)
+    assert short is not None and torch.equal(short, modules) and not torch.equal(short, before)
+
+
+@pytest.mark.parametrize("change", [
+    lambda b: setattr(b.self_attn, "forward", doubled(b.self_attn.forward)),
+    lambda b: setattr(b.self_attn.v_proj, "forward", doubled(b.self_attn.v_proj.forward)),
+    lambda b: setattr(b.input_layernorm, "forward", doubled(b.input_layernorm.forward)),
+    lambda b: setattr(b.self_attn.o_proj, "bias", torch.ones(128, dtype=torch.bfloat16)),
+    lambda b: setattr(b.self_attn.o_proj, "bias", torch.nn.Parameter(torch.ones(128, dtype=torch.bfloat16))),
+    lambda b: setattr(b.self_attn.v_proj, "bits", 8),
+    lambda b: setattr(b.self_attn, "v_proj", torch.nn.Linear(128, 64, dtype=torch.bfloat16)),
+    lambda b: setattr(b.input_layernorm, "weight", b.input_layernorm.weight.float()),
+    lambda b: b.self_attn.v_proj.register_forward_hook(lambda module, args, out: 2 * out),
+    lambda b: b.self_attn.register_forward_pre_hook(lambda module, args: (2 * args[0], args[1])),
+    lambda b: b.self_attn.o_proj.register_full_backward_hook(lambda *args: None),
+    lambda b: b.self_attn.o_proj.register_full_backward_pre_hook(lambda *args: None),
+    lambda b: setattr(b.self_attn.k_proj, "_compiled_call_impl", b.self_attn.k_proj._call_impl),
+])
+def test_what_a_call_of_the_module_adds_is_not_left_out(block, change):
+    assert both_ways(block)[0] is not None
+    change(block)
+    assert both_ways(block)[0] is None
+
+
+def test_global_hooks_and_classes_changed_under_it(block, monkeypatch):
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda module, args, out: None)
+    assert both_ways(block)[0] is None
+    handle.remove()
+    assert both_ways(block)[0] is not None
+    for kind in (blocks.QuantizedLinear, blocks.Attention, blocks.RMSNorm):
+        with monkeypatch.context() as patch:
+            forward = doubled(kind.forward)
+            forward._metile_original = getattr(kind.forward, "_metile_original", None)  # as functools.wraps would copy it
+            patch.setattr(kind, "forward", forward)
+            assert both_ways(block)[0] is None
+        with monkeypatch.context() as patch:
+            patch.setattr(kind, "__call__", doubled(kind.__call__))
+            assert both_ways(block)[0] is None
+    assert both_ways(block)[0] is not None
