@@ -14,6 +14,7 @@ fused path keeps fp32 intermediates and can differ from the op-by-op path by rou
 from __future__ import annotations
 
 import math
+import weakref
 
 import torch
 from torch import nn
@@ -107,8 +108,16 @@ class GatedMLP(nn.Module):
 
 
 def _rope_frequencies(theta, dim, device):
-    """theta^(-2i/D) for the pairs i of a head: a constant of the model, kept like a weight."""
+    """theta^(-2i/D) for the pairs i of a head."""
     return 1.0 / (theta ** (torch.arange(0, dim, 2, device=device, dtype=torch.float32) / dim))
+
+
+_frequency_tables = weakref.WeakKeyDictionary()  # attention module -> {(theta, dim, device, stream): table}
+_MOST_FREQUENCY_TABLES = 4  # of a module; none of them is part of its state
+
+
+def _current_stream(device):
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def _rope(values, positions, theta):
@@ -192,15 +201,21 @@ class Attention(nn.Module):
         self.q_proj, self.k_proj, self.v_proj, self.o_proj = q_proj, k_proj, v_proj, o_proj
         self.heads, self.kv_heads, self.head_dim, self.rope_theta = heads, kv_heads, head_dim, rope_theta
         self.scale = head_dim ** -0.5
-        self._frequencies = None
 
     def _frequencies_on(self, device):
-        if self._frequencies is None or self._frequencies[0] != (self.rope_theta, device):
+        # A table serves the stream it was made on, in whose order it is also given back.  A graph that is being
+        # captured makes its own, which lives as long as the graph does.
+        if torch.cuda.is_current_stream_capturing():
+            return _rope_frequencies(self.rope_theta, self.head_dim, device)
+        tables = _frequency_tables.setdefault(self, {})
+        key = self.rope_theta, self.head_dim, device, _current_stream(device)
+        table = tables.get(key)
+        if table is None:
             table = _rope_frequencies(self.rope_theta, self.head_dim, device)
-            if torch.cuda.is_current_stream_capturing():
-                return table  # belongs to the graph that is being captured
-            self._frequencies = ((self.rope_theta, device), table)
-        return self._frequencies[1]
+            if len(tables) >= _MOST_FREQUENCY_TABLES:
+                tables.clear()
+            tables[key] = table
+        return table
 
     def forward(self, values, cache=None):
         return self.o_proj(self.attend(self.q_proj(values), self.k_proj(values), self.v_proj(values), cache))

@@ -1,6 +1,8 @@
 """A prompt through a patched block calls operators in place of torch modules: only where the modules would do
 nothing else, whatever a program has changed about them since the last call."""
 
+import copy
+
 import pytest
 import torch
 
@@ -102,3 +104,30 @@ def test_global_hooks_and_classes_changed_under_it(block, monkeypatch):
             patch.setattr(kind, "__call__", doubled(kind.__call__))
             assert both_ways(block)[0] is None
     assert both_ways(block)[0] is not None
+
+
+def test_frequency_tables_belong_to_a_stream_and_not_to_the_module(block, monkeypatch):
+    attention, cpu = block.self_attn, torch.device("cpu")
+    stream, capturing = [1], [False]
+    monkeypatch.setattr(blocks, "_current_stream", lambda device: stream[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    table = attention._frequencies_on(cpu)
+    assert torch.equal(table, blocks._rope_frequencies(1e6, 64, cpu)) and attention._frequencies_on(cpu) is table
+    stream[0] = 2
+    assert attention._frequencies_on(cpu) is not table      # made in another stream's order
+    stream[0] = 1
+    assert attention._frequencies_on(cpu) is table
+    capturing[0] = True
+    assert attention._frequencies_on(cpu) is not table      # a graph may outlive what is kept
+    capturing[0] = False
+    attention.head_dim = 32
+    assert attention._frequencies_on(cpu).shape == (16,)
+    attention.head_dim = 64
+    attention.rope_theta = 1e2
+    assert torch.equal(attention._frequencies_on(cpu), blocks._rope_frequencies(1e2, 64, cpu))
+    for stream[0] in range(3, 40):
+        attention._frequencies_on(cpu)
+        assert len(blocks._frequency_tables[attention]) <= 4
+    # Nothing of it is saved or copied with the module.
+    assert not any(isinstance(value, (torch.Tensor, tuple)) for value in vars(attention).values())
+    assert copy.deepcopy(attention) not in blocks._frequency_tables
