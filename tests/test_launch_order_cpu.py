@@ -29,7 +29,7 @@ def kernels():
                 yield pytest.param(match.group(2), body.split("griddep_wait")[0], id=match.group(1))
 
 
-@pytest.mark.parametrize("parameters,before", kernels())
+@pytest.mark.parametrize("parameters,before", list(kernels()))
 def test_only_weights_are_read_before_the_wait(parameters, before):
     pointers = set(re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)", parameters))
     touched = {name for name in re.findall(r"(\bp\.\w+|\b\w+)\s*\[", before) if name in pointers or name.startswith("p.")}
