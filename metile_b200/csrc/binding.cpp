@@ -10,7 +10,8 @@
 // the arguments is not the plain case (another type, dtype, device, layout or shape) -- the caller then
 // runs its Python form, which copies what must be copied and raises the operator's own exceptions; or the
 // library's negative status code as an int.  Nothing is queued unless a tensor is returned or the code
-// says so.
+// says so.  A C++ exception -- a tensor without strides or storage, no memory for the result -- becomes the
+// Python exception torch raises for it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -19,6 +20,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/metile_b200.h"
@@ -82,8 +84,7 @@ inline int64_t triple_rows(const Tensor* w, const Tensor* s, const Tensor* b, in
 inline bool fits_int(int64_t v) { return v <= 0x7FFFFFFF; }
 
 // project(values, weight, scales, biases, residual | None, group_size, bits, flags)
-PyObject* project(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 8) Py_RETURN_NONE;
+PyObject* project(PyObject* const* args) {
     const Tensor* x = plain(args[0]);
     const Tensor* residual = args[4] == Py_None ? nullptr : plain(args[4]);
     const long group = PyLong_AsLong(args[5]), bits = PyLong_AsLong(args[6]), flags = PyLong_AsLong(args[7]);
@@ -97,25 +98,19 @@ PyObject* project(PyObject*, PyObject* const* args, Py_ssize_t count) {
     c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = n;
     if (residual && (residual->sizes() != at::IntArrayRef(sizes) || !bf16_on(*residual, device))) Py_RETURN_NONE;
-    try {
-        const Launch launch(device);
-        Tensor out = new_bf16(sizes, device);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_affine_qmv(address(*x), static_cast<const uint32_t*>(address(*w)), address(*s), address(*b),
-                             residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k, (int)n, (int)group,
-                             (int)bits, (unsigned int)flags, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_bf16(sizes, device);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_affine_qmv(address(*x), static_cast<const uint32_t*>(address(*w)), address(*s), address(*b),
+                         residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k, (int)n, (int)group,
+                         (int)bits, (unsigned int)flags, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // swiglu(values, gate_weight, gate_scales, gate_biases, up_weight, up_scales, up_biases, flags)
-PyObject* swiglu(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 8) Py_RETURN_NONE;
+PyObject* swiglu(PyObject* const* args) {
     const Tensor* x = plain(args[0]);
     const long flags = PyLong_AsLong(args[7]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
@@ -129,20 +124,15 @@ PyObject* swiglu(PyObject*, PyObject* const* args, Py_ssize_t count) {
         Py_RETURN_NONE;
     c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = n;
-    try {
-        const Launch launch(device);
-        Tensor out = new_bf16(sizes, device);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_affine_swiglu(address(*x), static_cast<const uint32_t*>(address(*t[0])), address(*t[1]), address(*t[2]),
-                                static_cast<const uint32_t*>(address(*t[3])), address(*t[4]), address(*t[5]), address(out),
-                                (int)rows, (int)k, (int)n, 64, 4, (unsigned int)flags, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_bf16(sizes, device);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_affine_swiglu(address(*x), static_cast<const uint32_t*>(address(*t[0])), address(*t[1]), address(*t[2]),
+                            static_cast<const uint32_t*>(address(*t[3])), address(*t[4]), address(*t[5]), address(out),
+                            (int)rows, (int)k, (int)n, 64, 4, (unsigned int)flags, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // The nine weight addresses of a bound MLP and its shape; the Python executor owns the tensors.
@@ -156,8 +146,7 @@ constexpr const char* kMlpPlanName = "metile_b200.mlp_plan";
 void free_mlp_plan(PyObject* capsule) { delete static_cast<MlpPlan*>(PyCapsule_GetPointer(capsule, kMlpPlanName)); }
 
 // mlp_plan(nine weight tensors as for mlx_affine_mlp_executor, already checked) -> capsule, or None
-PyObject* mlp_plan(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 9) Py_RETURN_NONE;
+PyObject* mlp_plan(PyObject* const* args) {
     MlpPlan plan;
     for (int i = 0; i < 9; ++i) {
         const Tensor* t = plain(args[i]);
@@ -174,8 +163,8 @@ PyObject* mlp_plan(PyObject*, PyObject* const* args, Py_ssize_t count) {
 }
 
 // mlp(plan, values, residual | None, workspace | None, flags): None also when the workspace is too small.
-PyObject* mlp(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 5 || !PyCapsule_IsValid(args[0], kMlpPlanName)) Py_RETURN_NONE;
+PyObject* mlp(PyObject* const* args) {
+    if (!PyCapsule_IsValid(args[0], kMlpPlanName)) Py_RETURN_NONE;
     const MlpPlan& plan = *static_cast<const MlpPlan*>(PyCapsule_GetPointer(args[0], kMlpPlanName));
     const Tensor* x = plain(args[1]);
     const Tensor* residual = args[2] == Py_None ? nullptr : plain(args[2]);
@@ -186,28 +175,22 @@ PyObject* mlp(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (args[2] != Py_None && (!residual || residual->sizes() != x->sizes() || !bf16_on(*residual, plan.device))) Py_RETURN_NONE;
     const int64_t rows = x->numel() / plan.hidden;
     if (!fits_int(rows) || workspace->numel() < rows * plan.inter) Py_RETURN_NONE;
-    try {
-        const Launch launch(plan.device);
-        Tensor out = new_like(*x);
-        void* const* w = plan.weights;
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_affine_mlp(address(*x), static_cast<const uint32_t*>(w[0]), w[1], w[2], static_cast<const uint32_t*>(w[3]),
-                             w[4], w[5], static_cast<const uint32_t*>(w[6]), w[7], w[8],
-                             residual ? address(*residual) : nullptr, address(*workspace), (size_t)workspace->numel() * 2,
-                             address(out), (int)rows, (int)plan.hidden, (int)plan.inter, 64, 4, (unsigned int)flags,
-                             launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(plan.device);
+    Tensor out = new_like(*x);
+    void* const* w = plan.weights;
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_affine_mlp(address(*x), static_cast<const uint32_t*>(w[0]), w[1], w[2], static_cast<const uint32_t*>(w[3]),
+                         w[4], w[5], static_cast<const uint32_t*>(w[6]), w[7], w[8],
+                         residual ? address(*residual) : nullptr, address(*workspace), (size_t)workspace->numel() * 2,
+                         address(out), (int)rows, (int)plan.hidden, (int)plan.inter, 64, 4, (unsigned int)flags,
+                         launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // norm(values, residual | None, weight, eps): the normalised rows, or (summed, normalised) with a residual.
-PyObject* norm(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 4) Py_RETURN_NONE;
+PyObject* norm(PyObject* const* args) {
     const Tensor *x = plain(args[0]), *weight = plain(args[2]);
     const Tensor* residual = args[1] == Py_None ? nullptr : plain(args[1]);
     const double eps = PyFloat_AsDouble(args[3]);
@@ -217,32 +200,26 @@ PyObject* norm(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (args[1] != Py_None && (!residual || residual->sizes() != x->sizes() || !bf16_on(*residual, x->device()))) Py_RETURN_NONE;
     const int64_t width = x->size(-1), rows = x->numel() / width;
     if (!fits_int(rows) || !fits_int(width)) Py_RETURN_NONE;
-    try {
-        const Launch launch(x->device());
-        Tensor normalized = new_like(*x), summed;
-        int code;
-        if (residual) summed = new_like(*x);
-        Py_BEGIN_ALLOW_THREADS
-        code = residual ? mt_add_rmsnorm(address(*x), address(*residual), address(*weight), address(summed), address(normalized),
-                                         (int)rows, (int)width, (float)eps, launch.stream())
-                        : mt_rmsnorm(address(*x), address(*weight), address(normalized), (int)rows, (int)width, (float)eps,
-                                     launch.stream());
-        Py_END_ALLOW_THREADS
-        if (!residual || code != 0) return code_or(code, std::move(normalized));
-        PyObject* pair = PyTuple_New(2);
-        if (!pair) return nullptr;
-        PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(summed)));
-        PyTuple_SET_ITEM(pair, 1, THPVariable_Wrap(std::move(normalized)));
-        return pair;
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(x->device());
+    Tensor normalized = new_like(*x), summed;
+    int code;
+    if (residual) summed = new_like(*x);
+    Py_BEGIN_ALLOW_THREADS
+    code = residual ? mt_add_rmsnorm(address(*x), address(*residual), address(*weight), address(summed), address(normalized),
+                                     (int)rows, (int)width, (float)eps, launch.stream())
+                    : mt_rmsnorm(address(*x), address(*weight), address(normalized), (int)rows, (int)width, (float)eps,
+                                 launch.stream());
+    Py_END_ALLOW_THREADS
+    if (!residual || code != 0) return code_or(code, std::move(normalized));
+    PyObject* pair = PyTuple_New(2);
+    if (!pair) return nullptr;
+    PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(summed)));
+    PyTuple_SET_ITEM(pair, 1, THPVariable_Wrap(std::move(normalized)));
+    return pair;
 }
 
 // dense(values, weight, up_weight | None, residual | None): with an up weight the SwiGLU of both.
-PyObject* dense(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 4) Py_RETURN_NONE;
+PyObject* dense(PyObject* const* args) {
     const Tensor *x = plain(args[0]), *w = plain(args[1]);
     const Tensor* up = args[2] == Py_None ? nullptr : plain(args[2]);
     const Tensor* residual = args[3] == Py_None ? nullptr : plain(args[3]);
@@ -255,20 +232,15 @@ PyObject* dense(PyObject*, PyObject* const* args, Py_ssize_t count) {
     sizes.back() = n;
     if (args[3] != Py_None && (!residual || residual->sizes() != at::IntArrayRef(sizes) || !bf16_on(*residual, device)))
         Py_RETURN_NONE;
-    try {
-        const Launch launch(device);
-        Tensor out = new_bf16(sizes, device);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = up ? mt_dense_swiglu(address(*x), address(*w), address(*up), address(out), (int)rows, (int)k, (int)n, launch.stream())
-                  : mt_dense_rows(address(*x), address(*w), residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k,
-                                  (int)n, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_bf16(sizes, device);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = up ? mt_dense_swiglu(address(*x), address(*w), address(*up), address(out), (int)rows, (int)k, (int)n, launch.stream())
+              : mt_dense_rows(address(*x), address(*w), residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k,
+                              (int)n, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // Tokens per head a [B, H, N, D] cache (or a view of its first N tokens) has room for; -1: another layout.
@@ -280,8 +252,7 @@ inline int64_t cache_capacity(const Tensor& t) {
 }
 
 // attention(query, key, value, scale, lengths | None)
-PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 5) Py_RETURN_NONE;
+PyObject* attention(PyObject* const* args) {
     const Tensor *q = plain(args[0]), *k = plain(args[1]), *v = plain(args[2]);
     const Tensor* lengths = args[4] == Py_None ? nullptr : plain(args[4]);
     const double scale = PyFloat_AsDouble(args[3]);
@@ -301,24 +272,19 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (lengths && (lengths->device() != device || lengths->scalar_type() != at::kInt || !lengths->is_contiguous() ||
                     lengths->numel() < batch))
         Py_RETURN_NONE;
-    try {
-        const Launch launch(device);
-        Tensor out = new_like(*q);
-        const size_t needed = mt_attention_decode_workspace_bytes((int)batch, (int)heads, (int)tokens, (int)dim);
-        // Scratch of this call only: the caching allocator hands it to later work of the same stream.
-        c10::DataPtr scratch;
-        if (needed) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(needed);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_attention_decode(address(*q), address(*k), address(*v), lengths ? static_cast<const int*>(address(*lengths)) : nullptr,
-                                   address(out), scratch.get(), needed, (int)batch, (int)heads, (int)kv_heads, (int)tokens,
-                                   (int)capacity, (int)dim, (float)scale, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_like(*q);
+    const size_t needed = mt_attention_decode_workspace_bytes((int)batch, (int)heads, (int)tokens, (int)dim);
+    // Scratch of this call only: the caching allocator hands it to later work of the same stream.
+    c10::DataPtr scratch;
+    if (needed) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(needed);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_attention_decode(address(*q), address(*k), address(*v), lengths ? static_cast<const int*>(address(*lengths)) : nullptr,
+                               address(out), scratch.get(), needed, (int)batch, (int)heads, (int)kv_heads, (int)tokens,
+                               (int)capacity, (int)dim, (float)scale, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 int append(const void* q, const void* k, const void* v, long long row_stride, int* positions, void* q_out, void* k_cache,
@@ -330,8 +296,7 @@ int append(const void* q, const void* k, const void* v, long long row_stride, in
 inline bool head_major(const Tensor& t, int64_t dim) { return t.stride(2) == 1 && t.stride(1) == dim; }
 
 // rope_kv_append(query, key, value, positions, key_cache, value_cache, theta, advance)
-PyObject* rope_kv_append(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 8) Py_RETURN_NONE;
+PyObject* rope_kv_append(PyObject* const* args) {
     const Tensor* t[6];
     for (int i = 0; i < 6; ++i)
         if (!(t[i] = plain(args[i]))) Py_RETURN_NONE;
@@ -355,25 +320,19 @@ PyObject* rope_kv_append(PyObject*, PyObject* const* args, Py_ssize_t count) {
         Py_RETURN_NONE;
     if (!fits_int(batch * (heads + 2 * kv_heads)) || !fits_int(capacity)) Py_RETURN_NONE;
     const int64_t row_stride = batch > 1 ? q.stride(0) : (heads + 2 * kv_heads) * dim;
-    try {
-        const Launch launch(device);
-        Tensor out = new_bf16({batch, heads, dim}, device);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = (advance ? mt_rope_kv_append_advance : append)(
-            address(q), address(k), address(v), row_stride, static_cast<int*>(address(positions)), address(out), address(keys),
-            address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity, (int)dim, (float)theta, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_bf16({batch, heads, dim}, device);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = (advance ? mt_rope_kv_append_advance : append)(
+        address(q), address(k), address(v), row_stride, static_cast<int*>(address(positions)), address(out), address(keys),
+        address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity, (int)dim, (float)theta, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache)
-PyObject* rope_kv_prefill(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 8) Py_RETURN_NONE;
+PyObject* rope_kv_prefill(PyObject* const* args) {
     const Tensor* t[8] = {};
     for (int i : {0, 1, 2, 3, 4, 6, 7})
         if (!(t[i] = plain(args[i]))) Py_RETURN_NONE;
@@ -394,25 +353,19 @@ PyObject* rope_kv_prefill(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (positions.device() != device || positions.scalar_type() != at::kInt || !positions.is_contiguous() || positions.numel() < batch)
         Py_RETURN_NONE;
     if (!fits_int(batch * steps) || !fits_int(capacity) || first < 0 || first + steps > capacity) Py_RETURN_NONE;
-    try {
-        const Launch launch(device);
-        Tensor out = new_like(q);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_rope_kv_prefill(address(q), address(k), address(v), static_cast<const float*>(address(inverse)), address(out),
-                                  address(keys), address(values), static_cast<int*>(address(positions)), (int)batch, (int)steps,
-                                  (int)first, (int)heads, (int)kv_heads, (int)capacity, (int)dim, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
-        return nullptr;
-    }
+    const Launch launch(device);
+    Tensor out = new_like(q);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_rope_kv_prefill(address(q), address(k), address(v), static_cast<const float*>(address(inverse)), address(out),
+                              address(keys), address(values), static_cast<int*>(address(positions)), (int)batch, (int)steps,
+                              (int)first, (int)heads, (int)kv_heads, (int)capacity, (int)dim, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
 }
 
 // greedy_token(logits [rows, vocabulary] bf16, tokens [rows] or [rows, 1] int64) -> logits as float32
-PyObject* greedy_token(PyObject*, PyObject* const* args, Py_ssize_t count) {
-    if (count != 2) Py_RETURN_NONE;
+PyObject* greedy_token(PyObject* const* args) {
     const Tensor *logits = plain(args[0]), *tokens = plain(args[1]);
     if (!logits || !tokens || !logits->is_cuda() || logits->dim() != 2 || logits->numel() == 0) Py_RETURN_NONE;
     const auto device = logits->device();
@@ -420,25 +373,32 @@ PyObject* greedy_token(PyObject*, PyObject* const* args, Py_ssize_t count) {
     if (!bf16_on(*logits, device) || tokens->device() != device || tokens->scalar_type() != at::kLong || !tokens->is_contiguous() ||
         tokens->numel() != rows || !fits_int(rows) || !fits_int(vocabulary))
         Py_RETURN_NONE;
+    const Launch launch(device);
+    Tensor out = at::detail::empty_cuda({rows, vocabulary}, at::kFloat, device, std::nullopt);
+    int code;
+    Py_BEGIN_ALLOW_THREADS
+    code = mt_greedy_token(address(*logits), static_cast<float*>(address(out)), static_cast<long long*>(address(*tokens)), (int)rows,
+                           (int)vocabulary, launch.stream());
+    Py_END_ALLOW_THREADS
+    return code_or(code, std::move(out));
+}
+
+template <PyObject* (*kBody)(PyObject* const*), Py_ssize_t kCount>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t count) {
     try {
-        const Launch launch(device);
-        Tensor out = at::detail::empty_cuda({rows, vocabulary}, at::kFloat, device, std::nullopt);
-        int code;
-        Py_BEGIN_ALLOW_THREADS
-        code = mt_greedy_token(address(*logits), static_cast<float*>(address(out)), static_cast<long long*>(address(*tokens)), (int)rows,
-                               (int)vocabulary, launch.stream());
-        Py_END_ALLOW_THREADS
-        return code_or(code, std::move(out));
-    } catch (const std::exception& error) {
-        PyErr_SetString(PyExc_RuntimeError, error.what());
+        if (count != kCount) Py_RETURN_NONE;
+        return kBody(args);
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
 }
 
-#define MT_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {MT_METHOD(project), MT_METHOD(swiglu),    MT_METHOD(mlp_plan),       MT_METHOD(mlp), MT_METHOD(norm),
-                         MT_METHOD(dense),   MT_METHOD(attention), MT_METHOD(rope_kv_append),
-                         MT_METHOD(rope_kv_prefill), MT_METHOD(greedy_token), {nullptr, nullptr, 0, nullptr}};
+#define MT_METHOD(name, count) \
+    {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<name, count>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {MT_METHOD(project, 8), MT_METHOD(swiglu, 8), MT_METHOD(mlp_plan, 9), MT_METHOD(mlp, 5), MT_METHOD(norm, 4),
+                         MT_METHOD(dense, 4), MT_METHOD(attention, 5), MT_METHOD(rope_kv_append, 8), MT_METHOD(rope_kv_prefill, 8),
+                         MT_METHOD(greedy_token, 2), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -127,3 +127,31 @@ def test_a_call_on_a_device_that_is_not_current(cuda_device):
     y1 = B.mlx_affine_mlp_executor(x1, *gate, *up, *down, x1)(x1, x1)
     assert_within(y1, A.mlp(f32(x1), triple_np(gate), triple_np(up), triple_np(down), f32(x1)), rel=4e-3)
     assert torch.cuda.current_device() == 0
+
+
+def test_tensors_without_strides_or_sizes_raise(cuda_device):
+    x = synth.activations(1, 4, 64, cuda_device)
+    weight, triple = synth.norm_weight(2, 64, cuda_device), synth.affine_weight(3, 64, 64, cuda_device)
+    dense = synth.dense_weight(4, 64, 64, cuda_device)
+    query = x.view(1, 4, 1, 64)
+    expected = B.mlx_add_rms_norm(x, x, weight, 1e-6)
+    for strange in (x.to_sparse(), x.to_sparse_csr(), torch.nested.nested_tensor([x[:1], x[1:]])):
+        for call in (lambda: B.mlx_rms_norm(strange, weight, 1e-6), lambda: B.mlx_add_rms_norm(x, strange, weight, 1e-6),
+                     lambda: B.mlx_affine_qmv(strange, *triple), lambda: B.mlx_affine_residual_qmv(x, *triple, strange),
+                     lambda: B.mlx_affine_swiglu(strange, *triple, *triple), lambda: B.mlx_dense_swiglu(strange, dense, dense),
+                     lambda: B.mlx_dense_residual_qmv(x.view(2, 128), dense.view(32, 128), strange),
+                     lambda: B.mlx_attention_decode(query, query, query, scale=1.0, lengths=strange)):
+            with pytest.raises((RuntimeError, ValueError, TypeError)):
+                call()
+    for found, wanted in zip(B.mlx_add_rms_norm(x, x, weight, 1e-6), expected):
+        assert_bit_equal(found, wanted, "after the refusals")
+
+
+def test_no_memory_for_the_result_is_torchs_own_error(cuda_device):
+    rows, n = 1 << 17, 1 << 21  # 512 GiB of results for 16 MiB of activations and 64 MiB of weights
+    triple = (torch.zeros((n, 8), dtype=torch.int32, device=cuda_device),
+              *(torch.zeros((n, 1), dtype=torch.bfloat16, device=cuda_device) for _ in range(2)))
+    x = torch.zeros((rows, 64), dtype=torch.bfloat16, device=cuda_device)
+    with pytest.raises(torch.OutOfMemoryError):
+        B.mlx_affine_qmv(x, *triple)
+    assert not B.mlx_affine_qmv(x[:2], *triple).any()
