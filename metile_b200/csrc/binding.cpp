@@ -54,6 +54,19 @@ private:
     cudaStream_t stream_;
 };
 
+// Other Python threads may run while this lives.  An exception that leaves its block -- a tensor under vmap has no
+// address -- meets the interpreter with its lock held again.
+class Unlocked {
+public:
+    Unlocked() : thread_(PyEval_SaveThread()) {}
+    ~Unlocked() { PyEval_RestoreThread(thread_); }
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+
+private:
+    PyThreadState* thread_;
+};
+
 inline Tensor new_bf16(at::IntArrayRef sizes, c10::Device device) {
     return at::detail::empty_cuda(sizes, at::kBFloat16, device, std::nullopt);
 }
@@ -101,11 +114,12 @@ PyObject* project(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_bf16(sizes, device);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_affine_qmv(address(*x), static_cast<const uint32_t*>(address(*w)), address(*s), address(*b),
-                         residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k, (int)n, (int)group,
-                         (int)bits, (unsigned int)flags, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_affine_qmv(address(*x), static_cast<const uint32_t*>(address(*w)), address(*s), address(*b),
+                             residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k, (int)n, (int)group,
+                             (int)bits, (unsigned int)flags, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -127,11 +141,12 @@ PyObject* swiglu(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_bf16(sizes, device);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_affine_swiglu(address(*x), static_cast<const uint32_t*>(address(*t[0])), address(*t[1]), address(*t[2]),
-                            static_cast<const uint32_t*>(address(*t[3])), address(*t[4]), address(*t[5]), address(out),
-                            (int)rows, (int)k, (int)n, 64, 4, (unsigned int)flags, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_affine_swiglu(address(*x), static_cast<const uint32_t*>(address(*t[0])), address(*t[1]), address(*t[2]),
+                                static_cast<const uint32_t*>(address(*t[3])), address(*t[4]), address(*t[5]), address(out),
+                                (int)rows, (int)k, (int)n, 64, 4, (unsigned int)flags, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -179,13 +194,14 @@ PyObject* mlp(PyObject* const* args) {
     Tensor out = new_like(*x);
     void* const* w = plan.weights;
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_affine_mlp(address(*x), static_cast<const uint32_t*>(w[0]), w[1], w[2], static_cast<const uint32_t*>(w[3]),
-                         w[4], w[5], static_cast<const uint32_t*>(w[6]), w[7], w[8],
-                         residual ? address(*residual) : nullptr, address(*workspace), (size_t)workspace->numel() * 2,
-                         address(out), (int)rows, (int)plan.hidden, (int)plan.inter, 64, 4, (unsigned int)flags,
-                         launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_affine_mlp(address(*x), static_cast<const uint32_t*>(w[0]), w[1], w[2], static_cast<const uint32_t*>(w[3]),
+                             w[4], w[5], static_cast<const uint32_t*>(w[6]), w[7], w[8],
+                             residual ? address(*residual) : nullptr, address(*workspace), (size_t)workspace->numel() * 2,
+                             address(out), (int)rows, (int)plan.hidden, (int)plan.inter, 64, 4, (unsigned int)flags,
+                             launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -204,12 +220,13 @@ PyObject* norm(PyObject* const* args) {
     Tensor normalized = new_like(*x), summed;
     int code;
     if (residual) summed = new_like(*x);
-    Py_BEGIN_ALLOW_THREADS
-    code = residual ? mt_add_rmsnorm(address(*x), address(*residual), address(*weight), address(summed), address(normalized),
-                                     (int)rows, (int)width, (float)eps, launch.stream())
-                    : mt_rmsnorm(address(*x), address(*weight), address(normalized), (int)rows, (int)width, (float)eps,
-                                 launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = residual ? mt_add_rmsnorm(address(*x), address(*residual), address(*weight), address(summed), address(normalized),
+                                         (int)rows, (int)width, (float)eps, launch.stream())
+                        : mt_rmsnorm(address(*x), address(*weight), address(normalized), (int)rows, (int)width, (float)eps,
+                                     launch.stream());
+    }
     if (!residual || code != 0) return code_or(code, std::move(normalized));
     PyObject* pair = PyTuple_New(2);
     if (!pair) return nullptr;
@@ -235,11 +252,12 @@ PyObject* dense(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_bf16(sizes, device);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = up ? mt_dense_swiglu(address(*x), address(*w), address(*up), address(out), (int)rows, (int)k, (int)n, launch.stream())
-              : mt_dense_rows(address(*x), address(*w), residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k,
-                              (int)n, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = up ? mt_dense_swiglu(address(*x), address(*w), address(*up), address(out), (int)rows, (int)k, (int)n, launch.stream())
+                  : mt_dense_rows(address(*x), address(*w), residual ? address(*residual) : nullptr, address(out), (int)rows, (int)k,
+                                  (int)n, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -279,11 +297,12 @@ PyObject* attention(PyObject* const* args) {
     c10::DataPtr scratch;
     if (needed) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(needed);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_attention_decode(address(*q), address(*k), address(*v), lengths ? static_cast<const int*>(address(*lengths)) : nullptr,
-                               address(out), scratch.get(), needed, (int)batch, (int)heads, (int)kv_heads, (int)tokens,
-                               (int)capacity, (int)dim, (float)scale, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_attention_decode(address(*q), address(*k), address(*v), lengths ? static_cast<const int*>(address(*lengths)) : nullptr,
+                                   address(out), scratch.get(), needed, (int)batch, (int)heads, (int)kv_heads, (int)tokens,
+                                   (int)capacity, (int)dim, (float)scale, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -323,11 +342,12 @@ PyObject* rope_kv_append(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_bf16({batch, heads, dim}, device);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = (advance ? mt_rope_kv_append_advance : append)(
-        address(q), address(k), address(v), row_stride, static_cast<int*>(address(positions)), address(out), address(keys),
-        address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity, (int)dim, (float)theta, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = (advance ? mt_rope_kv_append_advance : append)(
+            address(q), address(k), address(v), row_stride, static_cast<int*>(address(positions)), address(out), address(keys),
+            address(values), (int)batch, (int)heads, (int)kv_heads, (int)capacity, (int)dim, (float)theta, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -356,11 +376,12 @@ PyObject* rope_kv_prefill(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_like(q);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_rope_kv_prefill(address(q), address(k), address(v), static_cast<const float*>(address(inverse)), address(out),
-                              address(keys), address(values), static_cast<int*>(address(positions)), (int)batch, (int)steps,
-                              (int)first, (int)heads, (int)kv_heads, (int)capacity, (int)dim, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_rope_kv_prefill(address(q), address(k), address(v), static_cast<const float*>(address(inverse)), address(out),
+                                  address(keys), address(values), static_cast<int*>(address(positions)), (int)batch, (int)steps,
+                                  (int)first, (int)heads, (int)kv_heads, (int)capacity, (int)dim, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 
@@ -376,10 +397,11 @@ PyObject* greedy_token(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = at::detail::empty_cuda({rows, vocabulary}, at::kFloat, device, std::nullopt);
     int code;
-    Py_BEGIN_ALLOW_THREADS
-    code = mt_greedy_token(address(*logits), static_cast<float*>(address(out)), static_cast<long long*>(address(*tokens)), (int)rows,
-                           (int)vocabulary, launch.stream());
-    Py_END_ALLOW_THREADS
+    {
+        const Unlocked unlocked;
+        code = mt_greedy_token(address(*logits), static_cast<float*>(address(out)), static_cast<long long*>(address(*tokens)), (int)rows,
+                               (int)vocabulary, launch.stream());
+    }
     return code_or(code, std::move(out));
 }
 

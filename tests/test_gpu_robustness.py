@@ -155,3 +155,13 @@ def test_no_memory_for_the_result_is_torchs_own_error(cuda_device):
     with pytest.raises(torch.OutOfMemoryError):
         B.mlx_affine_qmv(x, *triple)
     assert not B.mlx_affine_qmv(x[:2], *triple).any()
+
+
+def test_tensors_without_an_address_raise(cuda_device):
+    x = synth.activations(1, 4, 64, cuda_device)
+    weight, triple = synth.norm_weight(2, 64, cuda_device), synth.affine_weight(3, 64, 64, cuda_device)
+    for call in (lambda row: B.mlx_rms_norm(row, weight, 1e-6), lambda row: B.mlx_affine_qmv(row, *triple),
+                 lambda row: B.mlx_affine_swiglu(row, *triple, *triple)):
+        with pytest.raises(RuntimeError):
+            torch.vmap(call)(x.view(4, 1, 64))
+    assert torch.isfinite(B.mlx_rms_norm(x, weight, 1e-6)).all()
