@@ -46,7 +46,6 @@ _state = threading.local()
 _dispatch_lock = threading.RLock()
 _swiglu_dispatches = {}
 _residual_dispatches = {}
-_recorded = set()  # calls that would record what the tables hold already
 
 
 def _flags():
@@ -95,21 +94,22 @@ def _algorithm(rows, flags):
     return "gemv" if rows <= 1 else "umma"
 
 
-def _record(table, rows, input_features, output_features, dtype, group_size, bits, flags):
-    key = (rows, input_features, output_features, str(dtype), group_size, bits)
-    algorithm = _algorithm(rows, flags)
-    if table.get(key) != algorithm:
-        with _dispatch_lock:
-            table[key] = algorithm
-            _recorded.clear()
+_calls = {}          # (the call's shapes, types and flags) -> its row of the dispatch tables; nothing but a memory
+_MOST_CALLS = 4096   # of that function's values
 
 
 def _record_call(table, values, weight, group_size, bits, flags):
-    """_record for a call's tensors; the usual call, one like an earlier one, costs one look-up."""
-    call = (table is _swiglu_dispatches, values.shape, weight.shape, values.dtype, group_size, bits, flags)
-    if call not in _recorded:
-        _record(table, rows_of(values), values.shape[-1], weight.shape[0], values.dtype, group_size, bits, flags)
-        _recorded.add(call)
+    """Which kernel family served this call: the last call of a shape counts."""
+    call = (values.shape, weight.shape, values.dtype, group_size, bits, flags)
+    row = _calls.get(call)
+    if row is None:
+        rows = rows_of(values)
+        row = (rows, values.shape[-1], weight.shape[0], str(values.dtype), group_size, bits), _algorithm(rows, flags)
+        if len(_calls) >= _MOST_CALLS:
+            _calls.clear()
+        _calls[call] = row
+    with _dispatch_lock:
+        table[row[0]] = row[1]
 
 
 def _project(name, values, weight, scales, biases, residual, group_size, bits):
@@ -186,8 +186,7 @@ def _swiglu(name, values, gate_weight, gate_scales, gate_biases, up_weight, up_s
                   pointer(up_biases), pointer(out), x.shape[0], x.shape[1], output_features, group_size,
                   bits, flags)
     _lib.check(code, name)
-    _record(_swiglu_dispatches, x.shape[0], x.shape[1], output_features, values.dtype, group_size,
-            bits, flags)
+    _record_call(_swiglu_dispatches, values, gate_weight, group_size, bits, flags)
     return out.reshape(*values.shape[:-1], output_features)
 
 

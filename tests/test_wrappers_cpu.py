@@ -87,3 +87,25 @@ def test_every_call_runs_with_the_tensors_device_current(monkeypatch):
     here = torch.device("cuda", 0)
     assert _common.launch(entry_point, here, 4) == 0
     assert events == [("call", (4, ("stream-of", here)))]
+
+
+def test_the_dispatch_record_holds_the_last_call_and_stays_small():
+    from metile_b200 import _lib
+    from metile_b200.backends import cuda_quantized as q
+
+    weight = types.SimpleNamespace(shape=torch.Size((96, 8)))
+    values = torch.zeros((1, 64), dtype=torch.bfloat16)
+    table, other = {}, {}
+    key = (1, 64, 96, "torch.bfloat16", 64, 4)
+    for flags, family in ((0, "gemv"), (_lib.FLAG_FORCE_UMMA, "umma"), (0, "gemv"), (_lib.FLAG_FORCE_UMMA, "umma")):
+        q._record_call(table, values, weight, 64, 4, flags)
+        assert table == {key: family}
+        # Another thread's call between the look-ups of this one: what this one did is still what it records.
+        table[key] = "another thread's"
+        q._record_call(table, values, weight, 64, 4, flags)
+        assert table == {key: family}
+    q._record_call(other, values, weight, 64, 4, 0)
+    assert other == {key: "gemv"} and table == {key: "umma"}
+    for rows in range(1, 6000):
+        q._record_call({}, values.expand(rows, 64), weight, 64, 4, 0)
+    assert len(q._calls) <= 4096
