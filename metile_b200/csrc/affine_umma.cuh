@@ -87,14 +87,13 @@ __host__ __device__ constexpr int umma_ring_slots(int npad, bool windows, int si
     const int x_bytes = umma_x_slots(npad, windows, side_bytes) * 2 * npad * 128;
     const int left = kUmmaSmemBytes - 1024 - kUmmaBarrierBytes - kUmmaOutBytes - side_bytes - x_bytes - (windows ? 3 * kUmmaTableBytes : 0);
     const int slots = left / (kUmmaSlotBytes + kUmmaTableBytes);
-    return slots > kUmmaMaxSlots ? kUmmaMaxSlots : slots > 3 ? slots & ~1 : slots;
+    return slots > kUmmaMaxSlots ? kUmmaMaxSlots : slots > 3 ? slots & ~1 : slots;  // even where there is a choice
 }
-// Barriers that report the ring's fills.  The two dequant groups take the slots in turn, and a group waits for its own
-// fills only, so a barrier has to belong to one group: of a phase that the other group consumes a waiter could see
-// the parity too late, when the next fill has already been over it.  In a ring of even length a slot is always the same
-// group's; in an odd one it changes hands with every fill and has two barriers, used in turn.
-__host__ __device__ constexpr int umma_fill_barriers(int ring_slots) { return ring_slots % 2 ? 2 * ring_slots : ring_slots; }
-static_assert(umma_fill_barriers(3) <= kUmmaMaxSlots, "an odd ring has three slots at most");
+// Warps that report a ring slot as done.  The two dequant groups take the slots in turn.  In a ring of even length a slot
+// always belongs to the same group, which sees every phase of its barriers.  In an odd one it changes hands with
+// every fill; a parity wait cannot tell a fill from the next but one, so there both groups wait for every fill, and the
+// slot is filled again only when both have said that they saw it.
+__host__ __device__ constexpr int umma_slot_reports(int ring_slots) { return ring_slots % 2 ? kUmmaDequantWarps : kUmmaDequantWarps / 2; }
 static_assert(umma_ring_slots(128, false, 0) >= 3 && umma_ring_slots(128, true, 0) >= 3 && umma_ring_slots(64, true, 0) >= 4 &&
               umma_ring_slots(64, true, 64 * 512) >= 4 && umma_ring_slots(64, true, 8 * 16 * 512) >= 2 &&
               umma_ring_slots(64, true, 64 * 512 + kUmmaResidualBytes) >= 3 && umma_ring_slots(128, true, kUmmaResidualBytes) >= 3, "the ring is too short");
@@ -361,7 +360,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
     const UmmaShare w = umma_share<kCluster>(p);
     const int ring_space = umma_ring_slots(npad, p.windows, p.side_bytes);
     const int ring_slots = umma_ring_in_use(p, w, ring_space);
-    const int fill_barriers = umma_fill_barriers(ring_slots);
     const int table_slots = p.windows ? ring_slots + 3 : ring_slots;
     const int x_slots = umma_x_slots(npad, p.windows, p.side_bytes), x_slot_bytes = 2 * npad * 128;
     uint8_t* ring = smem;
@@ -389,8 +387,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
     const uint32_t second_col = unit_cols >> 1;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < fill_barriers; ++i) ptx::mbar_init(&ring_full[i], 1 + 32);  // the weight copy, and every lane's table copies
-        for (int i = 0; i < ring_slots; ++i) ptx::mbar_init(&ring_empty[i], kUmmaDequantWarps / 2);
+        for (int i = 0; i < ring_slots; ++i) {
+            ptx::mbar_init(&ring_full[i], 1 + 32);  // the weight copy, and every lane's table copies
+            ptx::mbar_init(&ring_empty[i], umma_slot_reports(ring_slots));
+        }
         for (int i = 0; i < kUmmaStages; ++i) {
             ptx::mbar_init(&a_full[i], kUmmaDequantWarps / 2);
             ptx::mbar_init(&stage_empty[i], 1);
@@ -431,21 +431,20 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
         }
         __syncwarp();
         UmmaTables copies;
-        RingCursor at, fill_at, table_at;
+        RingCursor at, table_at;
         bool alive = true;
         for (int tile = w.first_tile; tile < w.tiles && alive; tile += w.tile_step) {
             const int n0 = tile / p.act_tiles * kOut;
             copies.start_tile<kSwiglu>(p, w, n0, lane);
-            for (int st = 0; st < w.nslots; ++st, at.advance(ring_slots), fill_at.advance(fill_barriers)) {
-                uint64_t* full = &ring_full[fill_at.slot];
+            for (int st = 0; st < w.nslots; ++st, at.advance(ring_slots)) {
                 if (!ptx::mbar_wait(&ring_empty[at.slot], at.phase ^ 1u, abort_flag, kWaitRingEmpty)) { alive = false; break; }
                 __syncwarp();
                 if (ptx::elect_one()) {
-                    ptx::mbar_expect_tx(full, kUmmaSlotBytes);
+                    ptx::mbar_expect_tx(&ring_full[at.slot], kUmmaSlotBytes);
                     uint8_t* slot = ring + at.slot * kUmmaSlotBytes;
                     const int word = w.kb_begin * 8 + st * 32;
-                    ptx::tma_load_2d(slot, &p.w_map[0], word, n0, full);
-                    if (kSwiglu) ptx::tma_load_2d(slot + kUmmaSlotBytes / 2, &p.w_map[1], word, n0, full);
+                    ptx::tma_load_2d(slot, &p.w_map[0], word, n0, &ring_full[at.slot]);
+                    if (kSwiglu) ptx::tma_load_2d(slot + kUmmaSlotBytes / 2, &p.w_map[1], word, n0, &ring_full[at.slot]);
                 }
                 __syncwarp();
                 if (p.windows && st == 0) {
@@ -454,7 +453,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 }
                 copies.copy(st, w.nkb - st * kUmmaKBlocksPerSlot, tables + table_at.slot * kUmmaTableBytes, lane);
                 table_at.advance(table_slots);
-                ptx::cp_async_arrive(full);
+                ptx::cp_async_arrive(&ring_full[at.slot]);
             }
         }
         ptx::cp_async_wait_all();
@@ -756,7 +755,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
         const int row = kSwiglu ? (lane >> 4) * 64 + quadrant * 16 + (lane & 15) : r;
         const uint32_t a_lane = tmem_base + ((uint32_t)(quadrant * 32) << 16) + kUmmaAColumn + group * 128 + half * 64;
         const uint16_t* table_base[2] = {p.scales[kSwiglu && lane >= 16], p.biases[kSwiglu && lane >= 16]};
-        RingCursor fill_at, table_at;
+        const bool even_ring = (ring_slots & 1) == 0;
+        RingCursor at, table_at;
         uint32_t count = 0, use = 0;  // slots seen, slots handled
         bool alive = true;
         for (int tile = w.first_tile; tile < w.tiles && alive; tile += w.tile_step) {
@@ -772,11 +772,15 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 }
                 table_at.advance(table_slots);  // the first windows
             }
-            for (int st = 0; st < w.nslots; ++st, ++count, fill_at.advance(fill_barriers), table_at.advance(table_slots)) {
-                if ((count & 1u) != (uint32_t)group) continue;
-                if (!ptx::mbar_wait(&ring_full[fill_at.slot], fill_at.phase, abort_flag, kWaitRingFull)) { alive = false; break; }
-                const int ring_slot = fill_at.slot < ring_slots ? fill_at.slot : fill_at.slot - ring_slots;
-                const uint8_t* slot = ring + ring_slot * kUmmaSlotBytes + row * 128;
+            for (int st = 0; st < w.nslots; ++st, ++count, at.advance(ring_slots), table_at.advance(table_slots)) {
+                if ((count & 1u) != (uint32_t)group && even_ring) continue;
+                if (!ptx::mbar_wait(&ring_full[at.slot], at.phase, abort_flag, kWaitRingFull)) { alive = false; break; }
+                if ((count & 1u) != (uint32_t)group) {
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(&ring_empty[at.slot]);
+                    continue;
+                }
+                const uint8_t* slot = ring + at.slot * kUmmaSlotBytes + row * 128;
                 uint32_t pair[2];  // the scales and the biases of this thread's two k-blocks
                 const uint8_t* own = tables + table_at.slot * kUmmaTableBytes + r * 8;
                 if (p.windows) {
@@ -825,7 +829,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 __syncwarp();
                 if (lane == 0) {
                     ptx::mbar_arrive(&a_full[group]);
-                    ptx::mbar_arrive(&ring_empty[ring_slot]);
+                    ptx::mbar_arrive(&ring_empty[at.slot]);
                 }
             }
         }

@@ -39,13 +39,13 @@ def expect(found, wanted, what):
 
 class Pipeline:
     """One CTA.  units: accumulator units; slices of a tile's K range; slots: ring slots of a tile; kblocks: its
-    k-blocks; fills: barriers that report the ring's fills; accumulators_last: with one unit, the wait for it comes
+    k-blocks; reports: groups that report a ring slot as done; accumulators_last: with one unit, the wait for it comes
     after the turn."""
 
-    def __init__(self, *, ring, fills, x_slots, units, slices, slots, kblocks, tiles, accumulators_last=True, warps=2):
+    def __init__(self, *, ring, reports, x_slots, units, slices, slots, kblocks, tiles, accumulators_last=True, warps=2):
         self.__dict__.update(locals())
-        self.ring_full = [Barrier(1) for _ in range(fills)]
-        self.ring_empty = [Barrier(warps) for _ in range(ring)]
+        self.ring_full = [Barrier(1) for _ in range(ring)]
+        self.ring_empty = [Barrier(reports * warps) for _ in range(ring)]
         self.a_full = [Barrier(warps) for _ in range(2)]
         self.stage_empty = [Barrier(1) for _ in range(2)]
         self.x_full = [Barrier(1) for _ in range(x_slots)]
@@ -69,7 +69,7 @@ class Pipeline:
 
             def land(slot=slot, count=count):
                 self.ring_holds[slot] = count
-                self.ring_full[count % self.fills].arrive()
+                self.ring_full[slot].arrive()
             self.ring_holds[slot] = "a copy under way"
             self.copies.append(land)
 
@@ -88,11 +88,12 @@ class Pipeline:
         uses = 0
         for count in range(self.tiles * self.slots):
             slot = count % self.ring
-            every_fill = self.fills % 2 == 1  # barriers that change hands: a group waits for the other one's fills as well
-            if count & 1 != group and not every_fill:
+            if count & 1 != group and self.ring % 2 == 0:
                 continue
-            yield self.ring_full[count % self.fills], (count // self.fills) & 1
+            yield self.ring_full[slot], (count // self.ring) & 1
             if count & 1 != group:
+                if self.reports == 2:
+                    self.ring_empty[slot].arrive()
                 continue
             expect(self.ring_holds[slot], count, "ring slot")
             yield None
@@ -195,7 +196,7 @@ def faults(schedules, **shape):
 
 @pytest.mark.parametrize("units", [1, 2, 4])
 def test_a_slice_waits_until_the_one_before_has_left_its_accumulators(units):
-    shape = dict(ring=4, fills=4, x_slots=5, units=units, slices=1, slots=1, kblocks=4, tiles=9)
+    shape = dict(ring=4, reports=1, x_slots=5, units=units, slices=1, slots=1, kblocks=4, tiles=9)
     assert not faults(200, **shape)
     # Waiting for the accumulators ahead of the turn is what one unit and slices of one slot do not allow.
     assert bool(faults(50, accumulators_last=False, **shape)) == (units == 1)
@@ -213,16 +214,16 @@ int main() {
                     if (sums && npad > 64) continue;
                     const int side = sums * 64 * 512 + residual * kUmmaResidualBytes;
                     const int ring = umma_ring_slots(npad, windows, side);
-                    std::printf("%d %d %d\\n", ring, umma_fill_barriers(ring), umma_x_slots(npad, windows, side));
+                    std::printf("%d %d %d\\n", ring, umma_slot_reports(ring) / (kUmmaDequantWarps / 2), umma_x_slots(npad, windows, side));
                 }
-    std::printf("1 %d %d\\n", umma_fill_barriers(1), umma_x_slots(128, true, 0));  // window tables, one slot per tile
+    std::printf("1 %d %d\\n", umma_slot_reports(1) / (kUmmaDequantWarps / 2), umma_x_slots(128, true, 0));  // window tables, one slot per tile
 }
 """
 
 
 @pytest.fixture(scope="module")
 def geometries(tmp_path_factory):
-    """(ring slots, fill barriers, activation slots) of every launch, from the kernel's own header."""
+    """(ring slots, groups that report a slot, activation slots) of every launch, from the kernel's own header."""
     return sorted(set(host_program(tmp_path_factory.mktemp("geometry"), GEOMETRY)))
 
 
@@ -231,8 +232,8 @@ def test_every_ring_of_the_kernel_under_every_shape(geometries):
     rng = random.Random(1)
     for seed in range(600):
         slots = rng.randint(1, 9)
-        ring, fills, x_slots = rng.choice(geometries)
-        shape = dict(ring=ring, fills=fills, x_slots=x_slots, units=rng.choice((1, 2, 4)),
+        ring, reports, x_slots = rng.choice(geometries)
+        shape = dict(ring=ring, reports=reports, x_slots=x_slots, units=rng.choice((1, 2, 4)),
                      slices=rng.randint(1, min(8, slots)), slots=slots, kblocks=4 * slots - rng.randint(0, 3),
                      tiles=rng.randint(1, 6))
         fault = Pipeline(**shape).run(seed)
@@ -240,7 +241,7 @@ def test_every_ring_of_the_kernel_under_every_shape(geometries):
 
 
 @pytest.mark.parametrize("ring", [1, 3])
-def test_an_odd_ring_needs_two_barriers_per_slot(ring):
+def test_in_an_odd_ring_both_groups_report_a_slot(ring):
     shape = dict(ring=ring, x_slots=5, units=2, slices=1, slots=8 if ring > 1 else 1, kblocks=32 if ring > 1 else 3, tiles=6)
-    assert not faults(200, fills=2 * ring, **shape)
-    assert faults(50, fills=ring, **shape)  # even when both groups wait for every fill
+    assert not faults(200, reports=2, **shape)
+    assert faults(50, reports=1, **shape)  # although both groups wait for every fill
