@@ -373,13 +373,16 @@ affine_gemv_ring_kernel(const uint16_t* x, GemvWeights first, GemvWeights second
             const GemvWeights& wt = kDual && table_row >= kRows ? second : first;
             const uint8_t* scales = reinterpret_cast<const uint8_t*>(wt.scales) + table_at;
             const uint8_t* biases = reinterpret_cast<const uint8_t*>(wt.biases) + table_at;
+            // A word of which the part has only the first group: the rest may lie past the end of the array.
             if (table_left > 0) {
-                ptx::cp_async_4(table_to, scales);
-                ptx::cp_async_4(table_to + 2 * kGemvTableWords, biases);
+                const uint32_t bytes = table_left > 1 ? 4 : 2;
+                ptx::cp_async_4(table_to, scales, bytes);
+                ptx::cp_async_4(table_to + 2 * kGemvTableWords, biases, bytes);
             }
             if (table_fifth && table_left > 8) {
-                ptx::cp_async_4(table_to + 4, scales + 16);
-                ptx::cp_async_4(table_to + 2 * kGemvTableWords + 4, biases + 16);
+                const uint32_t bytes = table_left > 9 ? 4 : 2;
+                ptx::cp_async_4(table_to + 4, scales + 16, bytes);
+                ptx::cp_async_4(table_to + 2 * kGemvTableWords + 4, biases + 16, bytes);
             }
         }
         ptx::cp_async_commit();

@@ -1,6 +1,6 @@
-"""Index arithmetic of the INT4 GEMV launch, restated on the CPU.
+"""Index arithmetic of the INT4 projections, restated on the CPU.
 
-The kernel (metile_b200/csrc/affine_gemv.cuh) hands row blocks blockIdx, blockIdx + grid, ... to a
+The GEMV kernel (metile_b200/csrc/affine_gemv.cuh) hands row blocks blockIdx, blockIdx + grid, ... to a
 CTA and lets it run `(row_blocks - 1 - blockIdx) / grid + 1` passes, in unsigned arithmetic.  That
 is only right while the grid has at most `row_blocks` CTAs, which the launcher guarantees by
 construction; these checks pin both halves for the shapes the library is used with."""
@@ -62,3 +62,68 @@ def test_pass_counts_differ_by_at_most_one():
     assert (rows_per_cta, row_blocks, grid) == (16, 512, 444)
     passes = [(row_blocks - 1 - cta) // grid + 1 for cta in range(grid)]
     assert passes.count(2) == 68 and passes.count(1) == 376
+
+
+# ---- one activation row: the ring form of the GEMV ----------------------------------------------------------
+
+
+def ring_parts(k, n):
+    """(first slot, slots' end) of each K part of a row; a slot is 32 columns."""
+    ksplit, slots = ksplit_of(k, n), k // 32
+    per_part = -(-slots // ksplit)
+    return [(part * per_part, min((part + 1) * per_part, slots)) for part in range(ksplit)]
+
+
+def ring_table_words(entry, slot_begin, slot_end, steps):
+    """(step, table word, first byte, bytes) of a row's copies; `entry` is its first group of the part in the array."""
+    group_begin, group_end = slot_begin // 2, (slot_end + 1) // 2
+    for step in range(steps):
+        for word in range(4):
+            left = group_end - group_begin + entry % 2 - 2 * word - 8 * step
+            at = (entry // 2 + word) * 4 + 16 * step
+            if left > 0:
+                yield step, word, at, 4 if left > 1 else 2
+            if word == 0 and (entry | slot_begin) & 1 and left > 8:
+                yield step, 4, at + 16, 4 if left > 9 else 2
+
+
+RING_SHAPES = [(64, 4), (64, 5), (192, 7), (320, 131), (4160, 1001), (9024, 9), (1536, 8960), (13824, 257), (8192, 130)]
+
+
+@pytest.mark.parametrize("k,n", RING_SHAPES)
+def test_ring_copies_every_scale_and_nothing_outside_the_array(k, n):
+    groups, end = k // 64, 2 * n * (k // 64)
+    for slot_begin, slot_end in ring_parts(k, n):
+        steps = -(-(-(-(k // 32) // len(ring_parts(k, n)))) // 16)
+        for row in sorted({0, 1, n // 2, n - 2, n - 1}):
+            entry = row * groups + slot_begin // 2
+            copied = set()
+            for step, word, at, size in ring_table_words(entry, slot_begin, slot_end, steps):
+                assert at % 4 == 0 and 0 <= at and at + size <= end
+                copied |= {(step, 2 * word + half) for half in range(size // 2)}
+            for slot in range(slot_begin, slot_end):
+                step, lane = (slot - slot_begin) // 16, (slot - slot_begin) % 16
+                half = (slot_begin + lane) // 2 - slot_begin // 2 + entry % 2
+                assert (step, half) in copied
+                # The half-word read there is the slot's own group.
+                assert 2 * (entry // 2) + 8 * step + half == row * groups + slot // 2
+
+
+@pytest.mark.parametrize("k,n", RING_SHAPES)
+@pytest.mark.parametrize("dual", [False, True])
+def test_ring_tasks_store_every_row_once(k, n, dual):
+    rows, ksplit = 2 if dual else 4, ksplit_of(k, n)
+    tasks = -(-n // (2 * rows))
+    teams = WARPS // ksplit
+    grid = min(-(-n // (teams * 2 * rows)), 2 * SM_COUNT)
+    stored = [0] * n
+    for cta in range(grid):
+        for task0 in range(cta, tasks, teams * grid):  # the same passes for all warps of a CTA
+            for team in range(teams):
+                task = task0 + team * grid
+                for half in range(2):
+                    row = min(task * 2 * rows + half * rows, n - rows)
+                    for r in range(rows):
+                        if task < tasks and row + r >= task * 2 * rows + half * rows:
+                            stored[row + r] += 1
+    assert stored == [1] * n
