@@ -220,8 +220,9 @@ __device__ __forceinline__ int umma_row(int n0, int r, int n_rows) {
 // its own window and the one before, which the previous slot brought; the first slot of a tile brings window 0 in
 // an entry of its own.  So the table ring has three entries more than the weight ring: entry E is overwritten
 // ring + 3 entries later, when the slot after E's is known to be done, tile starts included while a tile has at
-// least ring / 2 + 1 slots (umma_ring_in_use).  A window holds at least one entry of the row, so no copy
-// touches memory past the 8 bytes around an array's end.  (Word by word -- up to 24 4-byte copies per lane and
+// least ring / 2 + 1 slots (umma_ring_in_use).  A copy ends with the row's last entry: the rest of its window may lie
+// past the end of the array, and is filled with zeros.  It starts with the window, which for the first row of an array
+// off an 8-byte boundary is up to six bytes in front of it.  (Word by word -- up to 24 4-byte copies per lane and
 // slot, each touching sixteen rows -- a slot took 1150 cycles at 106 rows, 6080 -> 11919.)
 struct UmmaTables {
     const uint8_t* at[2][4];   // [scales, biases][rows 32 q + lane]: first window
@@ -242,13 +243,15 @@ struct UmmaTables {
                 offsets |= offset << (8 * t + 2 * q);
             }
     }
-    // The first windows of a tile, for rows that do not start one.
-    __device__ __forceinline__ void copy_head(uint8_t* entry, int lane) const {
+    // The first windows of a tile, for rows that do not start one; a row has `left` entries.
+    __device__ __forceinline__ void copy_head(uint8_t* entry, int left, int lane) const {
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if ((offsets >> (8 * t + 2 * q)) & 3u) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q]);
+            for (int q = 0; q < 4; ++q) {
+                const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
+                if (offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q], 2 * min(offset + left, 4));
+            }
     }
     // The windows of slot `st`, of whose k-blocks `left` remain in the share.
     __device__ __forceinline__ void copy(int st, int left, uint8_t* entry, int lane) const {
@@ -257,8 +260,9 @@ struct UmmaTables {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
-                if (offset == 0 || left >= 5 - offset)
-                    ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * (st + (offset ? 1 : 0)));
+                const int entries = offset ? left - 4 + offset : left;  // of this row from the window's start on
+                if (entries > 0)
+                    ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * (st + (offset ? 1 : 0)), 2 * min(entries, 4));
             }
     }
 };
@@ -448,7 +452,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 }
                 __syncwarp();
                 if (p.windows && st == 0) {
-                    copies.copy_head(tables + table_at.slot * kUmmaTableBytes, lane);
+                    copies.copy_head(tables + table_at.slot * kUmmaTableBytes, w.nkb, lane);
                     table_at.advance(table_slots);
                 }
                 copies.copy(st, w.nkb - st * kUmmaKBlocksPerSlot, tables + table_at.slot * kUmmaTableBytes, lane);

@@ -127,3 +127,35 @@ def test_ring_tasks_store_every_row_once(k, n, dual):
                         if task < tasks and row + r >= task * 2 * rows + half * rows:
                             stored[row + r] += 1
     assert stored == [1] * n
+
+
+# ---- the tables of the tcgen05 projection --------------------------------------------------------------------
+
+
+def window_copies(start, entries):
+    """(window, first byte, bytes) of a row's table copies; `start` is the byte address of its first entry.  Window 0 is
+    the one the row starts in the middle of; window st + 1 belongs to slot st, as does window st of an aligned row."""
+    offset = start // 2 % 4
+    base = start - 2 * offset
+    if offset:
+        yield 0, base, 2 * min(offset + entries, 4)
+    for st in range(-(-entries // 4)):
+        left = entries - 4 * st
+        there = left - 4 + offset if offset else left
+        if there > 0:
+            yield st + (offset > 0), base + 8 * (st + (offset > 0)), 2 * min(there, 4)
+
+
+@pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 7, 8, 21, 95])
+@pytest.mark.parametrize("rows", [1, 2, 3, 130])
+@pytest.mark.parametrize("shift", [0, 2, 4, 6])
+def test_window_copies_bring_every_entry_and_end_with_the_row(groups, rows, shift):
+    for row in {0, 1, rows - 1} & set(range(rows)):
+        start = 1024 + shift + 2 * row * groups
+        brought = set()
+        for _, at, size in window_copies(start, groups):
+            assert at % 8 == 0 and size in (2, 4, 6, 8)
+            assert at + size <= start + 2 * groups                  # nothing past the row, so nothing past the array
+            assert at >= 1024 + (0 if row * groups >= 3 or shift == 0 else shift - 6)
+            brought |= set(range(at, at + size, 2))
+        assert brought >= {start + 2 * entry for entry in range(groups)}
