@@ -16,6 +16,8 @@
  *   scales   bf16  [N, K/64]     one per group of 64 along K
  *   biases   bf16  [N, K/64]     w[n,k] = scales[n,k/64] * q[n,k] + biases[n,k/64]
  *   out      bf16  [M, N]        y = x @ w^T, fp32 accumulation, one rounding at the store
+ * No array is read past its end.  One that does not start on an 8-byte boundary (scales, biases) or a 4-byte one
+ * (residual) is read from that boundary on, which lies in the same allocation.
  *
  * Packed weights, scales and biases are read ahead of the stream order: a kernel may start on them while
  * the one in front of it still runs.  What writes them must be complete when the call is made, or be followed

@@ -605,8 +605,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                         } else if (c0 < rows) {
                             auto copy_word = [&](int j, int word) {
                                 const int n = n_tile + 2 * word - odd_start(p.residual, c0 + j);  // n, n + 1: at least one is in the row
+                                const bool inside = n + 1 < p.N || m0 + c0 + j + 1 < p.M;  // else the array ends within the word
                                 if (c0 + j < rows && n < p.N)
-                                    ptx::cp_async_4(step + j * kUmmaResidualPitch + 4 * word, p.residual + (size_t)(m0 + c0 + j) * p.N + n);
+                                    ptx::cp_async_4(step + j * kUmmaResidualPitch + 4 * word, p.residual + (size_t)(m0 + c0 + j) * p.N + n, inside ? 4 : 2);
                             };
 #pragma unroll
                             for (int i = 0; i < 8; ++i) copy_word(quadrant * 4 + (i >> 1), lane + 32 * (i & 1));

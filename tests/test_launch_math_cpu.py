@@ -159,3 +159,20 @@ def test_window_copies_bring_every_entry_and_end_with_the_row(groups, rows, shif
             assert at >= 1024 + (0 if row * groups >= 3 or shift == 0 else shift - 6)
             brought |= set(range(at, at + size, 2))
         assert brought >= {start + 2 * entry for entry in range(groups)}
+
+
+@pytest.mark.parametrize("rows,n", [(1, 1), (1, 129), (3, 5), (16, 257), (17, 131), (4, 128)])
+@pytest.mark.parametrize("odd", [0, 1])  # the residual starts in the middle of a word
+def test_residual_words_bring_every_element_and_stay_inside_the_array(rows, n, odd):
+    brought = set()
+    for m in range(rows):
+        start = (odd + m * n) % 2
+        for tile in range(0, n, 128):
+            for word in range(65 if (odd + m * n + tile) % 2 else 64):
+                first = tile + 2 * word - start                     # elements first, first + 1
+                if first < n:
+                    size = 4 if first + 1 < n or m + 1 < rows else 2
+                    at = 2 * (odd + m * n + first)
+                    assert at % 4 == 0 and at + size <= 2 * (odd + rows * n) and at >= 0
+                    brought |= {at, at + size - 2}
+    assert brought >= {2 * (odd + i) for i in range(rows * n)}
