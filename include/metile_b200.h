@@ -215,7 +215,10 @@ int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long 
                               int q_heads, int kv_heads, int capacity, int head_dim, float theta, void* stream);
 
 /* The end of a greedy decode step: out[r][i] = fp32 of the bf16 logits[r][i], tokens[r] = the index of the
- * row's largest value, the first of equals; a NaN counts as larger than any number. */
+ * row's largest value, the first of equals; a NaN counts as larger than any number.  More rows or a larger
+ * vocabulary than the limits: -1. */
+#define MT_GREEDY_MAX_ROWS 0x0FFFFFFF
+#define MT_GREEDY_MAX_VOCABULARY 0x7FFFBFFF
 int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream);
 
 /* The same for the `steps` tokens of a prompt, which go to rows first, first + 1, ... of every cache.

@@ -551,6 +551,8 @@ struct GreedyParams {
 };
 
 constexpr int kGreedyThreads = 256, kGreedyCluster = 8;
+// Beyond the limits a loop's next index or the grid would not fit an int.
+static_assert(MT_GREEDY_MAX_VOCABULARY <= 0x7FFFFFFF - kGreedyThreads * kGreedyCluster * 8 && MT_GREEDY_MAX_ROWS <= 0x7FFFFFFF / kGreedyCluster, "int overflow");
 
 struct GreedyCandidate {
     float value;

@@ -392,7 +392,7 @@ PyObject* greedy_token(PyObject* const* args) {
     const auto device = logits->device();
     const int64_t rows = logits->size(0), vocabulary = logits->size(1);
     if (!bf16_on(*logits, device) || tokens->device() != device || tokens->scalar_type() != at::kLong || !tokens->is_contiguous() ||
-        tokens->numel() != rows || !fits_int(rows) || !fits_int(vocabulary))
+        tokens->numel() != rows || rows > MT_GREEDY_MAX_ROWS || vocabulary > MT_GREEDY_MAX_VOCABULARY)
         Py_RETURN_NONE;
     const Launch launch(device);
     Tensor out = at::detail::empty_cuda({rows, vocabulary}, at::kFloat, device, std::nullopt);

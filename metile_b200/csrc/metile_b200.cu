@@ -578,7 +578,7 @@ int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long 
 }
 
 int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream) {
-    if (rows < 0 || vocabulary < 1 || rows > 0x7FFFFFFF / kGreedyCluster) return MT_ERR_SHAPE;
+    if (rows < 0 || vocabulary < 1 || rows > MT_GREEDY_MAX_ROWS || vocabulary > MT_GREEDY_MAX_VOCABULARY) return MT_ERR_SHAPE;
     if (rows == 0) return MT_OK;
     if (!logits || !out || !tokens) return MT_ERR_NULL;
     if (!device_is_sm100()) return MT_ERR_DEVICE;

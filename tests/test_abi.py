@@ -51,6 +51,9 @@ def test_arguments_are_validated_before_any_gpu_work():
     # Workspace too small for the MLP.
     assert lib.mt_affine_mlp(*([one] * 10), None, one, 16, one, 4, 64, 64, 64, 4, 0, None) == -7
     assert lib.mt_affine_mlp_workspace_bytes(4, 2048, 8192) == 4 * 8192 * 2
+    # Greedy tokens: sizes whose indexes would not fit 32 bits.
+    for rows, vocabulary in ((1, 0x7FFFFFFF), (1, 0x7FFFC000), (0x10000000, 1), (1, 0)):
+        assert lib.mt_greedy_token(one, one, one, rows, vocabulary, None) == -1
     with pytest.raises(ValueError):
         _lib.check(-3, "probe")
     with pytest.raises(RuntimeError):
