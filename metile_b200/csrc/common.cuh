@@ -81,7 +81,8 @@ __device__ __forceinline__ float swiglu_f32(float gate, float up) { return gate 
 // "Computation of elementary functions on the IBM RISC System/6000 processor", 1990): an approximate
 // reciprocal, one Newton step on it, the quotient, its exact remainder by FMA, one correction.  That rounds as the
 // division does while 1 + exp(-g) and its reciprocal are normal numbers; beyond (g below -69) all eight divide.
-// Checked against the division over all 2^32 gates: the only other bits are a gate of -0, whose zero is positive.
+// The remainder is taken with the other sign, which keeps the sign of a zero.  A test compares it with the division
+// over all 2^32 gates.
 __device__ __forceinline__ void swiglu8_f32(const float (&gate)[8], const float (&up)[8], float (&out)[8]) {
     float d[8], largest = 0.0f;
 #pragma unroll
@@ -95,7 +96,7 @@ __device__ __forceinline__ void swiglu8_f32(const float (&gate)[8], const float 
             const float r0 = __fdividef(1.0f, d[i]);
             const float r = fmaf(fmaf(-d[i], r0, 1.0f), r0, r0);
             const float quotient = gate[i] * r;
-            out[i] = fmaf(fmaf(-d[i], quotient, gate[i]), r, quotient) * up[i];
+            out[i] = fmaf(-fmaf(d[i], quotient, -gate[i]), r, quotient) * up[i];
         }
     } else {
 #pragma unroll

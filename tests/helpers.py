@@ -1,5 +1,6 @@
 """Shared helpers for the parity tests: torch tensors <-> the numpy oracle."""
 
+import ctypes
 import os
 import subprocess
 
@@ -37,6 +38,16 @@ def assert_bit_equal(a, b, what=""):
     b16 = b.detach().cpu().contiguous().view(torch.uint16)
     mismatches = int((a16 != b16).sum())
     assert mismatches == 0, f"{what}: {mismatches} of {a16.numel()} outputs differ bitwise"
+
+
+def device_library(folder, source):
+    """A shared library of kernels over the package's headers, compiled for the GPU."""
+    path, library = os.path.join(folder, "kernels.cu"), os.path.join(folder, "kernels.so")
+    with open(path, "w") as file:
+        file.write(source)
+    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
+                    "-shared", "-Xcompiler", "-fPIC", "-I", build.CSRC, path, "-o", library], check=True)
+    return ctypes.CDLL(library)
 
 
 def host_program(folder, source):

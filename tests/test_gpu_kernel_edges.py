@@ -1,11 +1,13 @@
 """The edges of the kernels' tiles, chunks and rings, against the CPU oracle or rows run alone."""
+import ctypes
+
 import pytest
 import torch
 
 from metile_b200 import _lib, backends as B, synth
 from metile_b200.integrations import blocks
 from oracle import affine as A
-from tests.helpers import assert_bit_equal, assert_within, f32, triple_np
+from tests.helpers import assert_bit_equal, assert_within, device_library, f32, triple_np
 
 pytestmark = pytest.mark.gpu
 
@@ -134,3 +136,40 @@ def test_rope_append_advances_every_position_once(cuda_device, batch, heads, kv_
     assert (positions.cpu() == torch.arange(batch) + 1).all()
     assert_bit_equal(caches[2], caches[0], "keys")
     assert_bit_equal(caches[3], caches[1], "values")
+
+
+SWIGLU_SOURCE = """
+#include "common.cuh"
+// Eight gates per thread: neighbours, or (apart) an eighth of all numbers from one another.
+__global__ void compare(unsigned long long* different, unsigned int* example, int apart, float up_value) {
+    const unsigned int thread = blockIdx.x * blockDim.x + threadIdx.x;
+    float gate[8], up[8], out[8];
+    for (int i = 0; i < 8; ++i) {
+        gate[i] = __uint_as_float(apart ? thread + ((unsigned int)i << 29) : 8 * thread + i);
+        up[i] = up_value;
+    }
+    mt::swiglu8_f32(gate, up, out);
+    for (int i = 0; i < 8; ++i) {
+        const float one = mt::swiglu_f32(gate[i], up[i]);
+        if (__float_as_uint(one) != __float_as_uint(out[i]) && !(one != one && out[i] != out[i])) {
+            atomicAdd(different, 1ull);
+            *example = __float_as_uint(gate[i]);
+        }
+    }
+}
+extern "C" int run(void* different, void* example, int apart, float up, void* stream) {
+    compare<<<1 << 21, 256, 0, (cudaStream_t)stream>>>((unsigned long long*)different, (unsigned int*)example, apart, up);
+    return (int)cudaGetLastError();
+}
+"""
+
+
+def test_eight_swiglus_have_the_bits_of_one_for_every_gate(cuda_device, tmp_path):
+    run = device_library(tmp_path, SWIGLU_SOURCE).run
+    counts = torch.zeros(2, dtype=torch.int64, device=cuda_device)
+    stream = ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    for apart in (0, 1):
+        for up in (1.0, -0.37):
+            assert run(ctypes.c_void_p(counts.data_ptr()), ctypes.c_void_p(counts[1:].data_ptr()), apart, ctypes.c_float(up),
+                       stream) == 0
+            assert counts[0].item() == 0, hex(counts[1].item())
