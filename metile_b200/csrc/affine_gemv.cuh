@@ -373,17 +373,19 @@ affine_gemv_ring_kernel(const uint16_t* x, GemvWeights first, GemvWeights second
             const GemvWeights& wt = kDual && table_row >= kRows ? second : first;
             const uint8_t* scales = reinterpret_cast<const uint8_t*>(wt.scales) + table_at;
             const uint8_t* biases = reinterpret_cast<const uint8_t*>(wt.biases) + table_at;
-            // A word of which the part has only the first group: the rest may lie past the end of the array.
-            if (table_left > 0) {
-                const uint32_t bytes = table_left > 1 ? 4 : 2;
-                ptx::cp_async_4(table_to, scales, bytes);
-                ptx::cp_async_4(table_to + 2 * kGemvTableWords, biases, bytes);
-            }
-            if (table_fifth && table_left > 8) {
-                const uint32_t bytes = table_left > 9 ? 4 : 2;
-                ptx::cp_async_4(table_to + 4, scales + 16, bytes);
-                ptx::cp_async_4(table_to + 2 * kGemvTableWords + 4, biases + 16, bytes);
-            }
+            // Of a word that holds one more group of the part, the rest may lie past the end of the array: it is read alone.
+            auto copy_table_word = [&](int word, int left) {
+                uint32_t* to = table_to + word;
+                if (left > 1) {
+                    ptx::cp_async_4(to, scales + 4 * word);
+                    ptx::cp_async_4(to + 2 * kGemvTableWords, biases + 4 * word);
+                } else if (left == 1) {
+                    to[0] = *reinterpret_cast<const uint16_t*>(scales + 4 * word);
+                    to[2 * kGemvTableWords] = *reinterpret_cast<const uint16_t*>(biases + 4 * word);
+                }
+            };
+            copy_table_word(0, table_left);
+            if (table_fifth) copy_table_word(4, table_left - 8);
         }
         ptx::cp_async_commit();
         if (++copy_step == steps) {

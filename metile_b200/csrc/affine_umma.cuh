@@ -255,6 +255,14 @@ struct UmmaTables {
     }
     // The windows of slot `st`, of whose k-blocks `left` remain in the share.
     __device__ __forceinline__ void copy(int st, int left, uint8_t* entry, int lane) const {
+        if (left >= 7 || (left >= 4 && offsets == 0)) {  // full windows, whatever the rows' offsets
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * (st + ((offsets >> (8 * t + 2 * q)) & 3u ? 1 : 0)));
+            return;
+        }
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
