@@ -7,7 +7,6 @@ from .cuda import (  # noqa: F401
     greedy_token,
     rope_kv_append,
     rope_kv_prefill,
-    supports_rope_kv_prefill,
     supports_attention_decode,
 )
 from .cuda_affine import MLXAffineWeight, mlx_affine_matmul  # noqa: F401

@@ -216,23 +216,18 @@ def greedy_token(logits, tokens):
     return out
 
 
-def supports_rope_kv_prefill(query, key, value, key_cache, value_cache):
-    """Whether rope_kv_prefill serves these tensors: dense bfloat16 on one CUDA device."""
-    tensors = (query, key, value, key_cache, value_cache)
-    return all(type(t) is torch.Tensor and t.is_cuda and t.device == query.device and t.dtype == torch.bfloat16
-               and t.ndim == 4 and t.is_contiguous() and not t.requires_grad for t in tensors) \
-        and query.numel() > 0 and query.shape[-1] % 2 == 0 and query.shape[-1] <= 4096
-
-
-def rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache):
+def rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache, *, only_native=False):
     """Rotate the query and key rows of a prompt and write key and value to the caches, in place.
 
     query [B, T, Hq, D], key / value [B, T, Hkv, D]; inverse fp32 [D/2]: pair i of the token at position
     p is turned by p * inverse[i]; positions int32 [B] (device) is advanced by T; row `first + t` of each
-    cache [B, Hkv, capacity, D] receives token t.  Returns the rotated query, shaped like `query`."""
+    cache [B, Hkv, capacity, D] receives token t.  Returns the rotated query, shaped like `query`; with `only_native`
+    None, and nothing done, unless all are dense tensors of these types on one device."""
     out = native().rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache)
     if out is not None:
         return native_result(out, "rope_kv_prefill")
+    if only_native:
+        return None
     require_cuda_bf16(query, "rope_kv_prefill")
     batch, steps, q_heads, dim = query.shape
     kv_heads, capacity = key_cache.shape[1], key_cache.shape[2]

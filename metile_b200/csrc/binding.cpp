@@ -364,7 +364,7 @@ PyObject* rope_kv_prefill(PyObject* const* args) {
     const int64_t batch = q.size(0), steps = q.size(1), heads = q.size(2), dim = q.size(3);
     const int64_t kv_heads = keys.size(1), capacity = keys.size(2);
     if (k.size(0) != batch || k.size(1) != steps || k.size(2) != kv_heads || k.size(3) != dim || v.sizes() != k.sizes() ||
-        keys.size(0) != batch || keys.size(3) != dim || values.sizes() != keys.sizes() || kv_heads < 1 || dim % 2)
+        keys.size(0) != batch || keys.size(3) != dim || values.sizes() != keys.sizes() || kv_heads < 1 || dim % 2 || dim > 4096)
         Py_RETURN_NONE;
     for (const Tensor* tensor : {&q, &k, &v, &keys, &values})
         if (!bf16_on(*tensor, device)) Py_RETURN_NONE;

@@ -20,6 +20,7 @@ import torch
 from torch import nn
 
 from .. import backends
+from ..backends._common import stream_pointer
 
 
 class QuantizedLinear(nn.Module):
@@ -117,7 +118,7 @@ _MOST_FREQUENCY_TABLES = 4  # of a module; none of them is part of its state
 
 
 def _current_stream(device):
-    return torch.cuda.current_stream(device).cuda_stream
+    return stream_pointer(device).value
 
 
 def _rope(values, positions, theta):
@@ -160,14 +161,17 @@ class KVCache:
         self.advance(steps)
         return self.keys[:, :, :self.length], self.values[:, :, :self.length]
 
-    def rotate_and_fetch(self, queries, keys, values, frequencies):
+    def rotate_and_fetch(self, queries, keys, values, frequencies, only_native=False):
         """update_and_fetch with the rotary embedding in front of it, in one kernel: queries [B, T, Hq, D], keys /
-        values [B, T, Hkv, D] as the projections leave them.  Returns the rotated queries and the views."""
+        values [B, T, Hkv, D] as the projections leave them.  Returns the rotated queries and the views; with
+        `only_native` None for tensors that the native call does not take, and nothing has been done."""
         steps = keys.shape[1]
         if self.length + steps > self.capacity:
             raise ValueError("KV cache capacity exceeded")
         queries = backends.rope_kv_prefill(queries, keys, values, frequencies, self.positions, self.length, self.keys,
-                                           self.values)
+                                           self.values, only_native=only_native)
+        if queries is None:
+            return None
         self.length += steps  # the kernel advanced the device-side count
         return queries, self.keys[:, :, :self.length], self.values[:, :, :self.length]
 
@@ -181,6 +185,15 @@ class KVCache:
         """Forget everything after the first `length` tokens (host and device counts together)."""
         self.length = int(length)
         self.positions.fill_(self.length)
+
+
+_UPDATE, _ADVANCE = KVCache.update_and_fetch, KVCache.advance
+
+
+def appends_in_place(cache):
+    """Whether `cache` is a KVCache whose update_and_fetch and advance are the ones above."""
+    return type(cache) is KVCache and KVCache.update_and_fetch is _UPDATE and KVCache.advance is _ADVANCE \
+        and "update_and_fetch" not in cache.__dict__ and "advance" not in cache.__dict__
 
 
 def scaled_dot_product_attention(queries, keys, values, cache, scale, mask=None):
@@ -229,8 +242,11 @@ class Attention(nn.Module):
         offset = 0 if cache is None else cache.length
         if steps > 1 and offset > 0:
             raise ValueError("multi-token continuation is not supported by this harness")
-        if steps > 1 and type(cache) is KVCache and backends.supports_rope_kv_prefill(q, k, v, cache.keys, cache.values):
-            q, k, v = cache.rotate_and_fetch(q, k, v, self._frequencies_on(q.device))
+        served = None
+        if steps > 1 and q.is_cuda and appends_in_place(cache) and not (q.requires_grad or k.requires_grad or v.requires_grad):
+            served = cache.rotate_and_fetch(q, k, v, self._frequencies_on(q.device), only_native=True)
+        if served is not None:
+            q, k, v = served
             q = q.transpose(1, 2)
         else:
             q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)

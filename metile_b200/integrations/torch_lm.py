@@ -109,7 +109,10 @@ def _structurally_matches(cls, required):
 
 
 def _has_parts(module, required):
-    return all(getattr(module, name, None) is not None for name in required)
+    for name in required:
+        if _part(module, name) is None:
+            return False
+    return True
 
 
 def _is_affine_int4(linear):
@@ -123,6 +126,37 @@ def _is_affine_int4(linear):
     )
 
 
+_MODULE_CALL = torch.nn.Module.__call__
+_OWN_CLASSES = blocks.DecoderBlock, blocks.Attention, blocks.GatedMLP
+
+
+def _has_plain_call(state):
+    """Whether a module with this __dict__ runs the forward of its class and nothing else: no hook, no forward of its
+    own, not compiled."""
+    return not (state["_forward_hooks"] or state["_forward_pre_hooks"] or state["_backward_hooks"]
+                or state["_backward_pre_hooks"] or "forward" in state) and state.get("_compiled_call_impl") is None
+
+
+def _plain_triple(linear):
+    """The buffers of a projection whose call is mlx_affine_qmv of them and nothing else, or None."""
+    if type(linear) is not blocks.QuantizedLinear:
+        return None
+    state = linear.__dict__
+    if not _has_plain_call(state) or state.get("bias", linear) is not None \
+            or state.get("group_size") != 64 or state.get("bits") != 4:
+        return None
+    buffers = state["_buffers"]
+    weight, scales, biases = buffers.get("weight"), buffers.get("scales"), buffers.get("biases")
+    return None if weight is None or scales is None or biases is None else (weight, scales, biases)
+
+
+def _part(module, name):
+    """getattr(module, name, None), without torch's search where the parts are this package's own modules'."""
+    if type(module) in _OWN_CLASSES and name not in module.__dict__:
+        return module._modules.get(name)
+    return getattr(module, name, None)
+
+
 def quantized_mlp_refusal(module, values):
     """None when the fused INT4 MLP can serve this call, else the reason it cannot.
 
@@ -131,20 +165,26 @@ def quantized_mlp_refusal(module, values):
     quantisation biases and no additive bias; activations in the kernels' dtype (bfloat16 here,
     float16 there) on a CUDA device.
     """
+    weights = []
     for name in _GATED_MLP_ATTRIBUTES:
-        linear = getattr(module, name, None)
+        linear = _part(module, name)
         if linear is None:
             return f"{name} is missing"
+        triple = _plain_triple(linear)
+        if triple is not None and linear.mode == "affine":
+            weights.append(triple[0])
+            continue
         if not _is_affine_int4(linear):
             return f"{name} is not an affine 4-bit group-64 quantized projection"
         if getattr(linear, "bias", None) is not None:
             return f"{name} has an additive bias"
+        weights.append(linear.weight)
     if values.dtype != torch.bfloat16:
         return f"activations are {values.dtype}, the kernels take bfloat16"
     if not values.is_cuda:
         return "activations are not on a CUDA device"
-    gate, up, down = module.gate_proj, module.up_proj, module.down_proj
-    if gate.weight.shape != up.weight.shape or down.weight.shape[0] != values.shape[-1]:
+    gate, up, down = weights
+    if gate.shape != up.shape or down.shape[0] != values.shape[-1]:
         return "projection shapes do not form gate|up -> down"
     return None
 
@@ -245,27 +285,12 @@ def execute_attention_decode(module, values, cache, residual=None):
 
 
 _ATTENTION_FORWARD, _LINEAR_FORWARD = blocks.Attention.forward, blocks.QuantizedLinear.forward
-_MODULE_CALL = torch.nn.Module.__call__
-_norm_replacements, _attention_replacements = weakref.WeakSet(), weakref.WeakSet()  # forwards made by the patcher
+_PROMPT_CLASSES = blocks.RMSNorm, blocks.Attention, blocks.QuantizedLinear
 
 
-def _is_plain_call(module, kind):
-    """Whether calling `module` is kind.forward and nothing else: no hook, no forward of its own, not compiled."""
-    state = module.__dict__
-    return type(module) is kind and kind.__call__ is _MODULE_CALL and "forward" not in state \
-        and state.get("_compiled_call_impl") is None \
-        and not (state["_forward_hooks"] or state["_forward_pre_hooks"] or state["_backward_hooks"]
-                 or state["_backward_pre_hooks"])
-
-
-def _plain_triple(linear):
-    """The buffers of a projection whose call is mlx_affine_qmv of them and nothing else, or None."""
-    if not _is_plain_call(linear, blocks.QuantizedLinear) or linear.bias is not None \
-            or linear.group_size != 64 or linear.bits != 4:
-        return None
-    buffers = linear._buffers
-    triple = buffers.get("weight"), buffers.get("scales"), buffers.get("biases")
-    return None if any(tensor is None for tensor in triple) else triple
+def _made_by_the_patcher(forward):
+    # The mark names its function: a wrapper that took over the function's attributes is not it.
+    return getattr(forward, "_metile_replacement", None) is forward
 
 
 def prompt_attention(norm, attention, values, cache):
@@ -275,40 +300,43 @@ def prompt_attention(norm, attention, values, cache):
     A module of torch costs a few microseconds per call and attribute, and a short prompt is bound by them.
     Nothing is kept from one call for the next: every part, tensor and setting is looked at where the
     modules themselves would read it."""
-    if type(cache) is not KVCache or values.ndim != 3 or values.shape[1] < 2 or torch._C._get_tracing_state() \
+    if type(attention) is not blocks.Attention or type(norm) is not blocks.RMSNorm or type(cache) is not KVCache \
+            or values.ndim != 3 or values.shape[1] < 2 or torch._C._get_tracing_state() \
             or torch_module._has_any_global_hook():
         return None
+    # The classes: their forwards are this package's own or the patcher's, and a call of a module is torch's.
     forward = blocks.Attention.forward
-    if forward is not _ATTENTION_FORWARD and (forward not in _attention_replacements
+    if forward is not _ATTENTION_FORWARD and (not _made_by_the_patcher(forward)
                                               or forward._metile_original is not _ATTENTION_FORWARD):
         return None
-    if blocks.QuantizedLinear.forward is not _LINEAR_FORWARD or blocks.RMSNorm.forward not in _norm_replacements \
-            or not _is_plain_call(norm, blocks.RMSNorm) or not _is_plain_call(attention, blocks.Attention):
+    if blocks.QuantizedLinear.forward is not _LINEAR_FORWARD or not _made_by_the_patcher(blocks.RMSNorm.forward) \
+            or any(kind.__call__ is not _MODULE_CALL for kind in _PROMPT_CLASSES):
         return None
-    weight, eps = norm._buffers.get("weight"), _norm_eps(norm)
+    # The modules, and what they hold now.
+    if not _has_plain_call(norm.__dict__) or not _has_plain_call(attention.__dict__):
+        return None
+    weight, eps = norm.__dict__["_buffers"].get("weight"), _norm_eps(norm)
     if weight is None or eps is None or weight.dtype != values.dtype:
         return None
-    parts = attention._modules
     triples = []
     for name in _ATTENTION_ATTRIBUTES:
-        linear = parts.get(name)
-        triple = None if linear is None else _plain_triple(linear)
+        triple = _plain_triple(_part(attention, name))
         if triple is None:
             return None
         triples.append(triple)
     normed = backends.mlx_rms_norm(values, weight, eps)
-    attended = attention.attend(*(backends.mlx_affine_qmv(normed, *triple) for triple in triples[:3]), cache)
-    return backends.mlx_affine_qmv(attended, *triples[3])
+    project = backends.mlx_affine_qmv
+    q, k, v = project(normed, *triples[0]), project(normed, *triples[1]), project(normed, *triples[2])
+    return project(attention.attend(q, k, v, cache), *triples[3])
 
 
-def _replace_forward(patch, cls, make_replacement, known=None):
+def _replace_forward(patch, cls, make_replacement):
     original = cls.forward
     if getattr(original, "_metile_original", None) is not None:
         return False
     replacement = make_replacement(original)
     replacement._metile_original = original
-    if known is not None:
-        known.add(replacement)
+    replacement._metile_replacement = replacement
     patch.replacements.append((cls, "forward", original))
     cls.forward = replacement
     return True
@@ -374,7 +402,7 @@ def _patch_rms_norm(model, patch):
 
             return replacement
 
-        _replace_forward(patch, norm_class, make, _norm_replacements)
+        _replace_forward(patch, norm_class, make)
 
 
 def _patch_attention(model, patch):
@@ -419,7 +447,7 @@ def _patch_attention(model, patch):
 
             return replacement
 
-        _replace_forward(patch, attention_class, make, _attention_replacements)
+        _replace_forward(patch, attention_class, make)
     if len(patch.replacements) == before:
         patch.refuse("attention", "the model exposes no attention surface that can be replaced")
 

@@ -30,7 +30,7 @@ def block(monkeypatch):
         replacement = blocks.RMSNorm.forward
         norm_forward = lambda self, values: backends.mlx_rms_norm(values, self.weight, self.eps)  # noqa: E731
         norm_forward._metile_original = replacement._metile_original
-        monkeypatch.setattr("metile_b200.integrations.torch_lm._norm_replacements", {norm_forward})
+        norm_forward._metile_replacement = norm_forward
         blocks.RMSNorm.forward = norm_forward
         yield model.layers[0]
 
@@ -97,7 +97,7 @@ def test_global_hooks_and_classes_changed_under_it(block, monkeypatch):
     for kind in (blocks.QuantizedLinear, blocks.Attention, blocks.RMSNorm):
         with monkeypatch.context() as patch:
             forward = doubled(kind.forward)
-            forward._metile_original = getattr(kind.forward, "_metile_original", None)  # as functools.wraps would copy it
+            forward.__dict__.update(kind.forward.__dict__)  # as functools.wraps would
             patch.setattr(kind, "forward", forward)
             assert both_ways(block)[0] is None
         with monkeypatch.context() as patch:
