@@ -261,7 +261,7 @@ def execute_attention_decode(module, values, cache, residual=None):
     q = qkv[:, :heads * dim].view(batch, heads, dim)
     k = qkv[:, heads * dim:(heads + kv_heads) * dim].view(batch, kv_heads, dim)
     v = qkv[:, (heads + kv_heads) * dim:].view(batch, kv_heads, dim)
-    own_cache = type(cache) is KVCache  # of which we know that advancing is counting, on the host and on the device
+    own_cache = blocks.appends_in_place(cache)  # then advancing is counting, on the host and on the device
     rotated = backends.rope_kv_append(q, k, v, cache.positions, cache.keys, cache.values, theta=module.rope_theta,
                                       advance=own_cache)
     if own_cache:

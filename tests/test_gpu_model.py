@@ -108,3 +108,23 @@ def test_qwen_block_prefill_and_decode_patched_against_unpatched(cuda_device):
         peak = ref.float().abs().max()
         assert (out.float() - ref.float()).abs().max() <= 1e-2 * peak
     assert_bit_equal(again, out_decode, "patched decode step is repeatable")
+
+
+def test_cache_methods_replaced_on_the_instance_are_called(cuda_device):
+    model = blocks.random_model(5, device=cuda_device, layers=1)
+    tokens = torch.arange(9, device=cuda_device).view(1, 9)
+    with torch_lm.apply_metile_to_torch_lm(model, attention=True), torch.no_grad():
+        plain, replaced = model.make_cache(1, 16), model.make_cache(1, 16)
+        called = []
+        for name in ("update_and_fetch", "advance"):
+            def counting(*args, _name=name, _method=getattr(replaced[0], name)):
+                called.append(_name)
+                return _method(*args)
+            setattr(replaced[0], name, counting)
+        replaced[0].positions = replaced[0].positions.long()       # a program's own count: not the kernel's type
+        assert_bit_equal(model(tokens, cache=replaced), model(tokens, cache=plain), "prompt")
+        assert called == ["update_and_fetch", "advance"] and (replaced[0].positions == 9).all()
+        replaced[0].positions = replaced[0].positions.int()
+        assert_bit_equal(model(tokens[:, :1], cache=replaced), model(tokens[:, :1], cache=plain), "decode step")
+        assert called[2:] == ["advance"] and replaced[0].length == 10 and (replaced[0].positions == 10).all()
+        assert_bit_equal(replaced[0].keys, plain[0].keys, "keys")

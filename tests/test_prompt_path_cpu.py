@@ -131,3 +131,19 @@ def test_frequency_tables_belong_to_a_stream_and_not_to_the_module(block, monkey
     # Nothing of it is saved or copied with the module.
     assert not any(isinstance(value, (torch.Tensor, tuple)) for value in vars(attention).values())
     assert copy.deepcopy(attention) not in blocks._frequency_tables
+
+
+def test_a_cache_with_methods_of_its_own_is_not_passed_by(monkeypatch):
+    cache = blocks.KVCache(1, 1, 8, 64, "cpu")
+    assert blocks.appends_in_place(cache)
+    for name in ("update_and_fetch", "advance"):
+        other = blocks.KVCache(1, 1, 8, 64, "cpu")
+        setattr(other, name, getattr(other, name))
+        assert not blocks.appends_in_place(other)
+        with monkeypatch.context() as patch:
+            patch.setattr(blocks.KVCache, name, doubled(getattr(blocks.KVCache, name)))
+            assert not blocks.appends_in_place(cache)
+
+    class Counted(blocks.KVCache):
+        pass
+    assert not blocks.appends_in_place(Counted(1, 1, 8, 64, "cpu"))
