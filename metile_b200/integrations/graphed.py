@@ -29,6 +29,13 @@ def _logits_of(output):
     return getattr(output, "logits", output)
 
 
+def _takes(function, parameter):
+    try:
+        return parameter in inspect.signature(function).parameters
+    except (TypeError, ValueError):  # not every callable tells
+        return False
+
+
 class GraphedDecoder:
     def __init__(self, model, batch=1, capacity=4096):
         self.model = model
@@ -36,7 +43,7 @@ class GraphedDecoder:
         self.cache = model.make_cache(self.batch, self.capacity)
         device = self.cache[0].keys.device
         self.device = device
-        self._keeps_logits = "logits_to_keep" in inspect.signature(model.forward).parameters
+        self._keeps_logits = _takes(model.forward, "logits_to_keep")
         self.token = torch.zeros((self.batch, 1), dtype=torch.long, device=device)   # input of the next step
         self.logits = None                                                          # output of the last step
         self.graph = None

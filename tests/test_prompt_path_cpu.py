@@ -147,3 +147,12 @@ def test_a_cache_with_methods_of_its_own_is_not_passed_by(monkeypatch):
     class Counted(blocks.KVCache):
         pass
     assert not blocks.appends_in_place(Counted(1, 1, 8, 64, "cpu"))
+
+
+def test_a_forward_that_tells_no_parameters_is_asked_for_all_logits():
+    from metile_b200.integrations import graphed
+
+    assert graphed._takes(blocks.TinyCausalLM.forward, "logits_to_keep")
+    assert not graphed._takes(blocks.DecoderBlock.forward, "logits_to_keep")
+    assert not graphed._takes(dict.fromkeys, "logits_to_keep") and not graphed._takes(type("C", (), {}).__new__, "x")
+    assert not graphed._takes(max, "logits_to_keep")  # inspect.signature raises ValueError
