@@ -226,8 +226,8 @@ def mlx_affine_mlp_executor(sample_values, gate_weight, gate_scales, gate_biases
     """Validate once and return `execute(values, residual)` = down(swiglu(values)) + residual.
 
     One C-ABI call (mt_affine_mlp) runs both kernels back to back on the current stream; the
-    bf16 hidden activations live in a workspace the callable owns and grows on demand (calls of one
-    executor on different streams would share it: give each stream its own executor).  Unlike the
+    bf16 hidden activations live in scratch of that call alone, so one executor serves any stream, and a captured graph
+    keeps its own.  Unlike the
     reference (metile/backends/mlx_quantized.py:1806-1820) any row count is accepted and no
     1-row call is needed first.
     """
@@ -252,11 +252,10 @@ def mlx_affine_mlp_executor(sample_values, gate_weight, gate_scales, gate_biases
              down_scales, down_biases)
     pointers = [pointer(t) for t in bound]
 
-    workspace = {"hidden": None}  # grow-only scratch for the bf16 hidden activations, owned by the callable
     plan, call = native().mlp_plan(*bound), native().mlp
 
     def execute(values, residual=None):
-        out = call(plan, values, residual, workspace["hidden"], _flags())
+        out = call(plan, values, residual, _flags())
         if out is not None:
             return native_result(out, name)
         if not isinstance(values, torch.Tensor) or values.dtype != torch.bfloat16 \
@@ -272,9 +271,7 @@ def mlx_affine_mlp_executor(sample_values, gate_weight, gate_scales, gate_biases
             require_on_device(residual, values, "residual", contiguous=False)
             res = contiguous_2d(residual)
         rows = x.shape[0]
-        hidden = workspace["hidden"]
-        if hidden is None or hidden.numel() < rows * intermediate:
-            hidden = workspace["hidden"] = torch.empty(rows * intermediate, dtype=torch.bfloat16, device=device)
+        hidden = torch.empty(rows * intermediate, dtype=torch.bfloat16, device=device)
         out = torch.empty((rows, hidden_features), dtype=torch.bfloat16, device=device)
         code = launch(lib.mt_affine_mlp, device, pointer(x), *pointers, pointer(res), pointer(hidden),
                       hidden.numel() * 2, pointer(out), rows, hidden_features, intermediate, group_size, bits,

@@ -71,6 +71,10 @@ inline Tensor new_bf16(at::IntArrayRef sizes, c10::Device device) {
     return at::detail::empty_cuda(sizes, at::kBFloat16, device, std::nullopt);
 }
 
+// Scratch of one call: the caching allocator hands it to later work of the same stream, and keeps it for the graph when
+// the call is captured.
+inline c10::DataPtr call_scratch(size_t bytes) { return c10::cuda::CUDACachingAllocator::get()->allocate(bytes); }
+
 inline Tensor new_like(const Tensor& t) { return new_bf16(t.sizes(), t.device()); }
 
 inline PyObject* code_or(int code, Tensor&& result) {
@@ -177,28 +181,29 @@ PyObject* mlp_plan(PyObject* const* args) {
     return PyCapsule_New(new MlpPlan(plan), kMlpPlanName, free_mlp_plan);
 }
 
-// mlp(plan, values, residual | None, workspace | None, flags): None also when the workspace is too small.
+// mlp(plan, values, residual | None, flags)
 PyObject* mlp(PyObject* const* args) {
     if (!PyCapsule_IsValid(args[0], kMlpPlanName)) Py_RETURN_NONE;
     const MlpPlan& plan = *static_cast<const MlpPlan*>(PyCapsule_GetPointer(args[0], kMlpPlanName));
     const Tensor* x = plain(args[1]);
     const Tensor* residual = args[2] == Py_None ? nullptr : plain(args[2]);
-    const Tensor* workspace = plain(args[3]);
-    const long flags = PyLong_AsLong(args[4]);
+    const long flags = PyLong_AsLong(args[3]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (!activations_ok(x) || x->device() != plan.device || x->size(-1) != plan.hidden || !workspace) Py_RETURN_NONE;
+    if (!activations_ok(x) || x->device() != plan.device || x->size(-1) != plan.hidden) Py_RETURN_NONE;
     if (args[2] != Py_None && (!residual || residual->sizes() != x->sizes() || !bf16_on(*residual, plan.device))) Py_RETURN_NONE;
     const int64_t rows = x->numel() / plan.hidden;
-    if (!fits_int(rows) || workspace->numel() < rows * plan.inter) Py_RETURN_NONE;
+    if (!fits_int(rows)) Py_RETURN_NONE;
     const Launch launch(plan.device);
     Tensor out = new_like(*x);
+    const size_t needed = mt_affine_mlp_workspace_bytes((int)rows, (int)plan.hidden, (int)plan.inter);
+    const c10::DataPtr scratch = call_scratch(needed);
     void* const* w = plan.weights;
     int code;
     {
         const Unlocked unlocked;
         code = mt_affine_mlp(address(*x), static_cast<const uint32_t*>(w[0]), w[1], w[2], static_cast<const uint32_t*>(w[3]),
                              w[4], w[5], static_cast<const uint32_t*>(w[6]), w[7], w[8],
-                             residual ? address(*residual) : nullptr, address(*workspace), (size_t)workspace->numel() * 2,
+                             residual ? address(*residual) : nullptr, scratch.get(), needed,
                              address(out), (int)rows, (int)plan.hidden, (int)plan.inter, 64, 4, (unsigned int)flags,
                              launch.stream());
     }
@@ -293,9 +298,8 @@ PyObject* attention(PyObject* const* args) {
     const Launch launch(device);
     Tensor out = new_like(*q);
     const size_t needed = mt_attention_decode_workspace_bytes((int)batch, (int)heads, (int)tokens, (int)dim);
-    // Scratch of this call only: the caching allocator hands it to later work of the same stream.
     c10::DataPtr scratch;
-    if (needed) scratch = c10::cuda::CUDACachingAllocator::get()->allocate(needed);
+    if (needed) scratch = call_scratch(needed);
     int code;
     {
         const Unlocked unlocked;
@@ -418,7 +422,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t count) {
 
 #define MT_METHOD(name, count) \
     {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<name, count>)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {MT_METHOD(project, 8), MT_METHOD(swiglu, 8), MT_METHOD(mlp_plan, 9), MT_METHOD(mlp, 5), MT_METHOD(norm, 4),
+PyMethodDef methods[] = {MT_METHOD(project, 8), MT_METHOD(swiglu, 8), MT_METHOD(mlp_plan, 9), MT_METHOD(mlp, 4), MT_METHOD(norm, 4),
                          MT_METHOD(dense, 4), MT_METHOD(attention, 5), MT_METHOD(rope_kv_append, 8), MT_METHOD(rope_kv_prefill, 8),
                          MT_METHOD(greedy_token, 2), {nullptr, nullptr, 0, nullptr}};
 

@@ -82,7 +82,7 @@ class GraphedDecoder:
             for cache, length in zip(scratch, lengths):
                 cache.reset(length)
             self.cache = scratch
-            self._step()                      # builds executors, fused q|k|v triples, workspaces
+            self._step()                      # builds executors and fused q|k|v triples
             self.cache = real
             self.token.copy_(token)
             self.stream.synchronize()

@@ -158,7 +158,7 @@ class TensorParallelMLP:
         self.gate, self.up, self.down = gate, up, down
         self.rank, self.world, self.group = rank, world, group
         # With the CUDA operators, the shard's MLP is ONE C-ABI call on a bound executor (both kernels,
-        # workspace owned by the executor, the residual in rank 0's down epilogue): one Python dispatch
+        # the residual in rank 0's down epilogue): one Python dispatch
         # and one all-reduce per MLP.  Injected stand-ins take the two-step path.
         self._executor = None
         self._swiglu, self._down = swiglu_fn, down_fn

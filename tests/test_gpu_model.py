@@ -6,8 +6,9 @@ import pytest
 import torch
 
 import metile_b200
-from metile_b200 import synth
+from metile_b200 import backends, synth
 from metile_b200.integrations import blocks, torch_lm
+from metile_b200.integrations.graphed import GraphedDecoder
 from tests.helpers import assert_bit_equal
 
 pytestmark = pytest.mark.gpu
@@ -128,3 +129,39 @@ def test_cache_methods_replaced_on_the_instance_are_called(cuda_device):
         assert_bit_equal(model(tokens[:, :1], cache=replaced), model(tokens[:, :1], cache=plain), "decode step")
         assert called[2:] == ["advance"] and replaced[0].length == 10 and (replaced[0].positions == 10).all()
         assert_bit_equal(replaced[0].keys, plain[0].keys, "keys")
+
+
+def test_a_captured_step_keeps_its_scratch_when_a_longer_prompt_follows(cuda_device):
+    model = blocks.random_model(6, device=cuda_device)
+    first, longer = (torch.randint(0, 512, (2, length), device=cuda_device) for length in (3, 150))
+    with torch_lm.apply_metile_to_torch_lm(model, attention=True):
+        decoder = GraphedDecoder(model, batch=2, capacity=200)
+        decoder.generate(decoder.prefill(first).argmax(-1), 2)      # captured with the scratch of two rows
+        fresh = GraphedDecoder(model, batch=2, capacity=200)
+        expected = fresh.generate(fresh.prefill(longer).argmax(-1), 4)
+        start = decoder.prefill(longer).argmax(-1)                  # two times 150 rows
+        # Whatever the longer prompt made free now belongs to these.
+        others = [torch.full((rows, width), 3.0, dtype=torch.bfloat16, device=cuda_device)
+                  for rows in (1, 2, 4, 6, 300) for width in (256, 512) for _ in range(20)]
+        assert (decoder.generate(start, 4) == expected).all()
+        torch.cuda.synchronize()
+        assert all(bool((other == 3.0).all()) for other in others)
+
+
+def test_one_executor_on_two_streams(cuda_device):
+    rows, hidden, inter = 64, 1024, 4096
+    gate, up, down = synth.mlp_weights(7, hidden, inter, cuda_device)
+    inputs = [synth.activations(seed, rows, hidden, cuda_device) for seed in (1, 2)]
+    execute = backends.mlx_affine_mlp_executor(inputs[0], *gate, *up, *down, None)
+    expected = [execute(x) for x in inputs]
+    streams = [torch.cuda.Stream(cuda_device) for _ in inputs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        found = []
+        for stream, x in zip(streams, inputs):
+            with torch.cuda.stream(stream):
+                found.append([execute(x) for _ in range(10)])
+        torch.cuda.synchronize()
+        for results, wanted in zip(found, expected):
+            for result in results:
+                assert_bit_equal(result, wanted, "an executor's result")
