@@ -240,13 +240,18 @@ def attention_decode_refusal(module, values, cache):
 
 def _fused_qkv(module):
     """The q, k and v triples concatenated along the output axis, built once per module: one
-    projection launch reads the activations once and writes one q|k|v row per sequence."""
+    projection launch reads the activations once and writes one q|k|v row per sequence.
+
+    The copies are complete before they are used: a projection reads its weights ahead of the stream order,
+    and later calls may come on other streams.  A graph being captured makes its own."""
     fused = _qkv_cache.get(module)
     if fused is None:
         parts = (module.q_proj, module.k_proj, module.v_proj)
         fused = tuple(torch.cat([getattr(linear, name) for linear in parts], dim=0).contiguous()
                       for name in ("weight", "scales", "biases"))
-        _qkv_cache[module] = fused
+        if not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(fused[0].device).synchronize()
+            _qkv_cache[module] = fused
     return fused
 
 

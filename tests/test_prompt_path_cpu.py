@@ -156,3 +156,23 @@ def test_a_forward_that_tells_no_parameters_is_asked_for_all_logits():
     assert not graphed._takes(blocks.DecoderBlock.forward, "logits_to_keep")
     assert not graphed._takes(dict.fromkeys, "logits_to_keep") and not graphed._takes(type("C", (), {}).__new__, "x")
     assert not graphed._takes(max, "logits_to_keep")  # inspect.signature raises ValueError
+
+
+def test_fused_projections_are_complete_before_they_are_kept(block, monkeypatch):
+    from metile_b200.integrations import torch_lm
+
+    class Stream:
+        waits = 0
+
+        def synchronize(self):
+            assert block.self_attn not in torch_lm._qkv_cache
+            Stream.waits += 1
+
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    torch_lm._fused_qkv(block.self_attn)
+    assert Stream.waits == 0 and block.self_attn not in torch_lm._qkv_cache
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    weight, scales, biases = torch_lm._fused_qkv(block.self_attn)
+    assert Stream.waits == 1 and torch_lm._fused_qkv(block.self_attn)[0] is weight and Stream.waits == 1
+    assert weight.shape[0] == scales.shape[0] == biases.shape[0] == 128 + 64 + 64
