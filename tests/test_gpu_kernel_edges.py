@@ -7,6 +7,7 @@ import torch
 from metile_b200 import _lib, backends as B, synth
 from metile_b200.integrations import blocks
 from oracle import affine as A
+from oracle import attention as OA
 from tests.helpers import assert_bit_equal, assert_within, device_library, f32, triple_np
 
 pytestmark = pytest.mark.gpu
@@ -173,3 +174,109 @@ def test_eight_swiglus_have_the_bits_of_one_for_every_gate(cuda_device, tmp_path
             assert run(ctypes.c_void_p(counts.data_ptr()), ctypes.c_void_p(counts[1:].data_ptr()), apart, ctypes.c_float(up),
                        stream) == 0
             assert counts[0].item() == 0, hex(counts[1].item())
+
+
+def at_offset(tensor, elements):
+    """The same values `elements` elements into an allocation."""
+    return torch.empty(tensor.numel() + elements, dtype=tensor.dtype, device=tensor.device)[elements:].view(tensor.shape).copy_(tensor)
+
+
+@pytest.mark.parametrize("k,n", [
+    (64, 3),          # fewer outputs than a half-warp has rows: the register form
+    (64, 4), (64, 5),  # one group per row, rows that share a table word, a last word with one group
+    (192, 7),         # three groups, a last task that overlaps its neighbour
+    (320, 131),       # five groups
+    (4160, 1001),     # K parts that begin in the middle of a group
+    (9024, 9),        # 141 groups in eight parts
+    (13824, 257),     # the longest row whose activations fit beside the rings
+    (13888, 257),     # the first that does not
+])
+def test_one_row_gemv_edges(cuda_device, k, n):
+    x = synth.activations(1, 2, k, cuda_device)
+    gate, up = synth.affine_weight(2, n, k, cuda_device), synth.affine_weight(3, n, k, cuda_device)
+    r = synth.activations(4, 2, n, cuda_device)
+    with B.force_kernel("gemv"):
+        # Two rows take the register form: the same sums in the same order.
+        two = B.mlx_affine_qmv(x, *gate), B.mlx_affine_residual_qmv(x, *gate, r), B.mlx_affine_swiglu(x, *gate, *up)
+    one = B.mlx_affine_qmv(x[:1], *gate), B.mlx_affine_residual_qmv(x[:1], *gate, r[:1]), B.mlx_affine_swiglu(x[:1], *gate, *up)
+    for found, wanted, what in zip(one, two, ("plain", "residual", "swiglu")):
+        assert_bit_equal(found, wanted[:1], what)
+    weights = triple_np(gate)
+    assert_within(one[0], A.qmm(f32(x[:1]), *weights))
+    assert_within(one[1], A.qmm(f32(x[:1]), *weights, residual=f32(r[:1])))
+    assert_within(one[2], A.swiglu_fused(f32(x[:1]), weights, triple_np(up)))
+    # Tables off a 4-byte boundary (the register form) and off an 8-byte one.
+    for offset in (1, 2):
+        moved = gate[0], at_offset(gate[1], offset), at_offset(gate[2], offset)
+        assert_bit_equal(B.mlx_affine_residual_qmv(x[:1], *moved, r[:1]), one[1], f"tables {offset} elements on")
+
+
+@pytest.mark.parametrize("k,n", [(64, 5), (192, 130), (448, 257), (1024, 100)])
+@pytest.mark.parametrize("rows", [2, 70])
+def test_tcgen05_projection_with_tables_anywhere(cuda_device, rows, k, n):
+    x, r = synth.activations(1, rows, k, cuda_device), synth.activations(3, rows, n, cuda_device)
+    triple = synth.affine_weight(2, n, k, cuda_device)
+    wanted = B.mlx_affine_residual_qmv(x, *triple, r), B.mlx_affine_swiglu(x, *triple, *triple)
+    for offset in (1, 2, 3, 4):
+        moved = triple[0], at_offset(triple[1], offset), at_offset(triple[2], (offset + 2) % 4)
+        assert_bit_equal(B.mlx_affine_residual_qmv(x, *moved, r), wanted[0], f"tables {offset} elements on")
+        assert_bit_equal(B.mlx_affine_swiglu(x, *moved, *triple), wanted[1], f"gate's tables {offset} elements on")
+
+
+@pytest.mark.parametrize("batch,kv_heads,group,dim,tokens", [
+    (2, 1, 3, 64, 2100),    # 17 splits: one more than are requested at once
+    (1, 2, 8, 128, 4096),   # 32 splits: one round of the lanes
+    (3, 2, 2, 64, 4225),    # 34 splits, the last one nearly empty
+    (2, 1, 4, 128, 8192),   # 64 splits: two rounds
+])
+def test_attention_merge_edges(cuda_device, batch, kv_heads, group, dim, tokens):
+    q = synth.activations(1, batch * kv_heads * group, dim, cuda_device).view(batch, kv_heads * group, 1, dim)
+    k, v = (synth.activations(seed, batch * kv_heads * tokens, dim, cuda_device).view(batch, kv_heads, tokens, dim)
+            for seed in (2, 3))
+    k[:, :, tokens // 3] *= 4  # the maximum lies in one split
+    scale = dim ** -0.5
+    assert_within(B.mlx_attention_decode(q, k, v, scale=scale), OA.attention_decode(f32(q), f32(k), f32(v), scale))
+    for used in (1, 128, 129, 2048, 2049, tokens - 1, tokens):
+        lengths = torch.tensor([used] + [max(1, tokens // 2)] * (batch - 1), dtype=torch.int32, device=cuda_device)
+        found = B.mlx_attention_decode(q, k, v, scale=scale, lengths=lengths)
+        assert_within(found, OA.attention_decode(f32(q), f32(k), f32(v), scale, lengths=lengths.cpu().numpy()), what=f"{used} in use")
+
+
+@pytest.mark.parametrize("rows,width", [(3, 8184), (2, 8192), (2, 8200), (3, 16384), (2, 32768), (2, 32776), (3, 8193), (2, 1), (5, 31)])
+def test_norm_edges(cuda_device, rows, width):
+    x, r = synth.activations(1, rows, width, cuda_device), synth.activations(2, rows, width, cuda_device)
+    w = synth.norm_weight(3, width, cuda_device)
+    total, norm = B.mlx_add_rms_norm(x, r, w, 1e-6)
+    o_total, o_norm = A.add_rmsnorm(f32(x), f32(r), f32(w), 1e-6)
+    assert (f32(total) == o_total).all()
+    assert_within(norm, o_norm, what="add_rmsnorm")
+    assert_within(B.mlx_rms_norm(x, w, 1e-6), A.rmsnorm(f32(x), f32(w), 1e-6), what="rmsnorm")
+    # Off a 16-byte boundary: element by element, with sums in another order.
+    assert_within(B.mlx_rms_norm(at_offset(x, 1), w, 1e-6), A.rmsnorm(f32(x), f32(w), 1e-6), what="unaligned")
+
+
+def test_what_the_native_calls_do_not_take_the_general_forms_do(cuda_device):
+    rows, k, n = 6, 256, 192
+    spaced = synth.activations(1, rows, 2 * k, cuda_device)
+    x, wide = spaced[:, :k], spaced[:, :k].contiguous()  # rows apart, and dense
+    gate, up = synth.affine_weight(2, n, k, cuda_device), synth.affine_weight(3, n, k, cuda_device)
+    down = synth.affine_weight(4, k, n, cuda_device)
+    r = synth.activations(5, n, rows, cuda_device).t()
+    dense, norm = synth.dense_weight(6, n, k, cuda_device), synth.norm_weight(7, k, cuda_device)
+    execute = B.mlx_affine_mlp_executor(wide, *gate, *up, *down, None)
+    for call in (lambda v, s: B.mlx_affine_qmv(v, *gate), lambda v, s: B.mlx_affine_residual_qmv(v, *gate, s),
+                 lambda v, s: B.mlx_affine_swiglu(v, *gate, *up), lambda v, s: execute(v), lambda v, s: execute(v, v),
+                 lambda v, s: B.mlx_dense_residual_qmv(v, dense, s), lambda v, s: B.mlx_dense_swiglu(v, dense, dense),
+                 lambda v, s: B.mlx_rms_norm(v, norm, 1e-6), lambda v, s: torch.cat(B.mlx_add_rms_norm(v, v, norm, 1e-6))):
+        assert_bit_equal(call(x, r), call(wide, r.contiguous()))
+        parameter = torch.nn.Parameter(wide, requires_grad=False)  # a subclass of torch.Tensor
+        assert_bit_equal(call(parameter, r), call(wide, r.contiguous()))
+    # Attention: heads that are not the cache's order, a query of another stride, lengths that are a view.
+    q = synth.activations(8, 2 * 64, 4, cuda_device).view(2, 64, 1, 4).permute(0, 3, 2, 1)
+    kv = synth.activations(9, 2 * 300 * 2, 64, cuda_device).view(2, 300, 2, 64).transpose(1, 2)
+    lengths = torch.tensor([[7, 0], [300, 0]], dtype=torch.int32, device=cuda_device)
+    plain = B.mlx_attention_decode(q.contiguous(), kv.contiguous(), kv.contiguous(), scale=0.1, lengths=lengths[:, 0].contiguous())
+    assert_bit_equal(B.mlx_attention_decode(q, kv, kv, scale=0.1, lengths=lengths[:, 0].contiguous()), plain)
+    # Logits of another type.
+    logits, tokens = torch.randn(3, 50, device=cuda_device), torch.zeros(3, 1, dtype=torch.long, device=cuda_device)
+    assert torch.equal(B.greedy_token(logits, tokens), logits) and (tokens == logits.argmax(-1, keepdim=True)).all()
