@@ -224,8 +224,9 @@ __device__ __forceinline__ int umma_row(int n0, int r, int n_rows) {
 // past the end of the array, and is filled with zeros.  It starts with the window, which for the first row of an array
 // off an 8-byte boundary is up to six bytes in front of it.  (Word by word -- up to 24 4-byte copies per lane and
 // slot, each touching sixteen rows -- a slot took 1150 cycles at 106 rows, 6080 -> 11919.)
+template <bool kWindows>
 struct UmmaTables {
-    const uint8_t* at[2][4];   // [scales, biases][rows 32 q + lane]: first window
+    const uint8_t* at[2][4];   // [scales, biases][rows 32 q + lane]: window of the tile's first slot
     uint32_t offsets;          // two bits for each of them
 
     template <bool kSwiglu>
@@ -236,11 +237,12 @@ struct UmmaTables {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint16_t* base = (t ? p.biases : p.scales)[kSwiglu && lane >= 16];
-                const uint8_t* from = reinterpret_cast<const uint8_t*>(
-                    base + (size_t)umma_row<kSwiglu>(n0, 32 * q + lane, p.N) * w.kblocks + w.kb_begin);
-                const uint32_t offset = (uint32_t)(reinterpret_cast<uintptr_t>(from) >> 1) & 3u;
-                at[t][q] = from - 2 * offset;
-                offsets |= offset << (8 * t + 2 * q);
+                at[t][q] = reinterpret_cast<const uint8_t*>(base + (size_t)umma_row<kSwiglu>(n0, 32 * q + lane, p.N) * w.kblocks + w.kb_begin);
+                if constexpr (kWindows) {
+                    const uint32_t offset = (uint32_t)(reinterpret_cast<uintptr_t>(at[t][q]) >> 1) & 3u;
+                    at[t][q] += offset ? 8 - 2 * offset : 0;
+                    offsets |= offset << (8 * t + 2 * q);
+                }
             }
     }
     // The first windows of a tile, for rows that do not start one; a row has `left` entries.
@@ -250,34 +252,35 @@ struct UmmaTables {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
-                if (offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q], 2 * min(offset + left, 4));
+                if (offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] - 8, 2 * min(offset + left, 4));
             }
     }
     // The windows of slot `st`, of whose k-blocks `left` remain in the share.
     __device__ __forceinline__ void copy(int st, int left, uint8_t* entry, int lane) const {
-        if (left >= 7 || (left >= 4 && offsets == 0)) {  // full windows, whatever the rows' offsets
+        if (!kWindows || left >= 7) {
+            copy_full(st, entry, lane);
+        } else if constexpr (kWindows) {
 #pragma unroll
             for (int t = 0; t < 2; ++t)
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * (st + ((offsets >> (8 * t + 2 * q)) & 3u ? 1 : 0)));
-            return;
+                for (int q = 0; q < 4; ++q) {
+                    const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
+                    const int entries = offset ? left - 4 + offset : left;  // of this row from the window's start on
+                    if (entries > 0) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * st, 2 * min(entries, 4));
+                }
         }
+    }
+    __device__ __forceinline__ void copy_full(int st, uint8_t* entry, int lane) const {
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
-                const int entries = offset ? left - 4 + offset : left;  // of this row from the window's start on
-                if (entries > 0)
-                    ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * (st + (offset ? 1 : 0)), 2 * min(entries, 4));
-            }
+            for (int q = 0; q < 4; ++q) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * st);
     }
 };
 
 // Slots of the weight ring that may be in flight: with unaligned tables, short tiles leave room for fewer.
-__device__ __forceinline__ int umma_ring_in_use(const UmmaParams& p, const UmmaShare& w, int ring_slots) {
-    return p.windows ? min(ring_slots, w.nslots > 1 ? 2 * w.nslots - 2 : 1) : ring_slots;
+__device__ __forceinline__ int umma_ring_in_use(bool windows, const UmmaShare& w, int ring_slots) {
+    return windows ? min(ring_slots, w.nslots > 1 ? 2 * w.nslots - 2 : 1) : ring_slots;
 }
 
 // Sixteen accumulator columns of this warp's TMEM lanes, plus a second sixteen where there are some (eight at a
@@ -361,7 +364,10 @@ __device__ __forceinline__ void umma_finish_rows(const UmmaParams& p, const Umma
     }
 }
 
-template <bool kSwiglu, bool kCluster>
+// kWindows: see UmmaTables.  A kernel of its own, because every instruction that the dequantising warps do not issue counts
+// (with the layout as a run-time condition 512 rows 1536 -> 8960, gate|up, took 35.3 to 37.6 us, now 34.1; 2000 rows 2048 ->
+// 8192 146 to 155, now 144).
+template <bool kSwiglu, bool kCluster, bool kWindows>
 __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
     constexpr int kOut = kSwiglu ? 64 : 128;  // outputs per tile
     extern __shared__ uint8_t smem_raw[];
@@ -370,14 +376,14 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int npad = p.npad;
     const UmmaShare w = umma_share<kCluster>(p);
-    const int ring_space = umma_ring_slots(npad, p.windows, p.side_bytes);
-    const int ring_slots = umma_ring_in_use(p, w, ring_space);
-    const int table_slots = p.windows ? ring_slots + 3 : ring_slots;
-    const int x_slots = umma_x_slots(npad, p.windows, p.side_bytes), x_slot_bytes = 2 * npad * 128;
+    const int ring_space = umma_ring_slots(npad, kWindows, p.side_bytes);
+    const int ring_slots = umma_ring_in_use(kWindows, w, ring_space);
+    const int table_slots = kWindows ? ring_slots + 3 : ring_slots;
+    const int x_slots = umma_x_slots(npad, kWindows, p.side_bytes), x_slot_bytes = 2 * npad * 128;
     uint8_t* ring = smem;
     uint8_t* x_tiles = ring + ring_space * kUmmaSlotBytes;
     uint8_t* tables = x_tiles + x_slots * x_slot_bytes;
-    float* out_tile = reinterpret_cast<float*>(tables + (p.windows ? ring_space + 3 : ring_space) * kUmmaTableBytes);
+    float* out_tile = reinterpret_cast<float*>(tables + (kWindows ? ring_space + 3 : ring_space) * kUmmaTableBytes);
     float* sum_tile = out_tile + kUmmaOutBytes / 4;
     uint8_t* residual_ring = reinterpret_cast<uint8_t*>(sum_tile) + p.sum_bytes;
     uint64_t* ring_full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sum_tile) + p.side_bytes);
@@ -442,12 +448,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
             if (kSwiglu) ptx::prefetch_tensor_map(&p.w_map[1]);
         }
         __syncwarp();
-        UmmaTables copies;
+        UmmaTables<kWindows> copies;
         RingCursor at, table_at;
         bool alive = true;
         for (int tile = w.first_tile; tile < w.tiles && alive; tile += w.tile_step) {
             const int n0 = tile / p.act_tiles * kOut;
-            copies.start_tile<kSwiglu>(p, w, n0, lane);
+            copies.template start_tile<kSwiglu>(p, w, n0, lane);
             for (int st = 0; st < w.nslots; ++st, at.advance(ring_slots)) {
                 if (!ptx::mbar_wait(&ring_empty[at.slot], at.phase ^ 1u, abort_flag, kWaitRingEmpty)) { alive = false; break; }
                 __syncwarp();
@@ -459,7 +465,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                     if (kSwiglu) ptx::tma_load_2d(slot + kUmmaSlotBytes / 2, &p.w_map[1], word, n0, &ring_full[at.slot]);
                 }
                 __syncwarp();
-                if (p.windows && st == 0) {
+                if (kWindows && st == 0) {
                     copies.copy_head(tables + table_at.slot * kUmmaTableBytes, w.nkb, lane);
                     table_at.advance(table_slots);
                 }
@@ -776,7 +782,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
             // Position of this thread's first entry in the eight entries of the window before and the slot's own.
             // (kb_begin and a slot are multiples of four entries, so it is the same for all slots of a row.)
             uint32_t position[2] = {4u + 2u * half, 4u + 2u * half};
-            if (p.windows) {
+            if (kWindows) {
                 const size_t entry = (size_t)umma_row<kSwiglu>(tile / p.act_tiles * kOut, r, p.N) * w.kblocks;
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
@@ -796,7 +802,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 const uint8_t* slot = ring + at.slot * kUmmaSlotBytes + row * 128;
                 uint32_t pair[2];  // the scales and the biases of this thread's two k-blocks
                 const uint8_t* own = tables + table_at.slot * kUmmaTableBytes + r * 8;
-                if (p.windows) {
+                if (kWindows) {
                     const uint8_t* before = table_at.slot > 0 ? own - kUmmaTableBytes : own + (table_slots - 1) * kUmmaTableBytes;
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
@@ -975,11 +981,11 @@ inline bool encode_weight_map(CUtensorMap* map, const void* base, int K, int N, 
     return true;
 }
 
-template <bool kSwiglu, bool kCluster>
+template <bool kSwiglu, bool kCluster, bool kWindows>
 inline cudaError_t configure_umma_instance(int device) {
     static bool configured[64] = {};
     if (device < 64 && configured[device]) return cudaSuccess;
-    const cudaError_t rc = cudaFuncSetAttribute(affine_umma_kernel<kSwiglu, kCluster>,
+    const cudaError_t rc = cudaFuncSetAttribute(affine_umma_kernel<kSwiglu, kCluster, kWindows>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmemBytes);
     if (rc == cudaSuccess && device < 64) configured[device] = true;
     return rc;
@@ -990,7 +996,7 @@ template <bool kSwiglu>
 inline int umma_active_clusters(int size, int device) {
     static int cached[64][9] = {};
     if (device < 64 && cached[device][size]) return cached[device][size];
-    if (configure_umma_instance<kSwiglu, true>(device) != cudaSuccess) return 0;
+    if (configure_umma_instance<kSwiglu, true, false>(device) != cudaSuccess) return 0;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(size * 64, 1, 1);
     config.blockDim = dim3(kUmmaThreads, 1, 1);
@@ -1003,7 +1009,7 @@ inline int umma_active_clusters(int size, int device) {
     config.attrs = attrs;
     config.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, affine_umma_kernel<kSwiglu, true>, &config) != cudaSuccess) clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, affine_umma_kernel<kSwiglu, true, false>, &config) != cudaSuccess) clusters = 0;
     if (device < 64) cached[device][size] = clusters > 0 ? clusters : -1;
     return clusters;
 }
@@ -1093,9 +1099,9 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
     }
 }
 
-template <bool kSwiglu, bool kCluster>
+template <bool kSwiglu, bool kCluster, bool kWindows>
 inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, cudaStream_t stream) {
-    if (configure_umma_instance<kSwiglu, kCluster>(device) != cudaSuccess) return MT_ERR_LAUNCH;
+    if (configure_umma_instance<kSwiglu, kCluster, kWindows>(device) != cudaSuccess) return MT_ERR_LAUNCH;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(ctas, 1, 1);
     config.blockDim = dim3(kUmmaThreads, 1, 1);
@@ -1110,7 +1116,7 @@ inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, 
     attrs[1].val.clusterDim.z = 1;
     config.attrs = attrs;
     config.numAttrs = kCluster ? 2 : 1;
-    return cudaLaunchKernelEx(&config, affine_umma_kernel<kSwiglu, kCluster>, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&config, affine_umma_kernel<kSwiglu, kCluster, kWindows>, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
 template <bool kSwiglu>
@@ -1126,9 +1132,14 @@ inline int launch_umma_family(UmmaParams& params, cudaStream_t stream) {
     params.side_bytes = params.sum_bytes + (params.residual && params.ksplit == 1 ? kUmmaResidualBytes : 0);
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
     const int tiles = params.row_tiles * params.act_tiles;
-    if (params.ksplit > 1) return launch_umma_instance<kSwiglu, true>(params, tiles * params.ksplit, device, stream);
-    const int resident = umma_active_clusters<kSwiglu>(1, device);
-    return launch_umma_instance<kSwiglu, false>(params, tiles < resident ? tiles : resident, device, stream);
+    if (params.ksplit > 1) {
+        const int ctas = tiles * params.ksplit;
+        return params.windows ? launch_umma_instance<kSwiglu, true, true>(params, ctas, device, stream)
+                              : launch_umma_instance<kSwiglu, true, false>(params, ctas, device, stream);
+    }
+    const int resident = umma_active_clusters<kSwiglu>(1, device), ctas = tiles < resident ? tiles : resident;
+    return params.windows ? launch_umma_instance<kSwiglu, false, true>(params, ctas, device, stream)
+                          : launch_umma_instance<kSwiglu, false, false>(params, ctas, device, stream);
 }
 
 struct AffineWeights {
