@@ -43,7 +43,6 @@ from ._common import (
 )
 
 _state = threading.local()
-_dispatch_lock = threading.RLock()
 _swiglu_dispatches = {}
 _residual_dispatches = {}
 
@@ -108,8 +107,7 @@ def _record_call(table, values, weight, group_size, bits, flags):
         if len(_calls) >= _MOST_CALLS:
             _calls.clear()
         _calls[call] = row
-    with _dispatch_lock:
-        table[row[0]] = row[1]
+    table[row[0]] = row[1]  # one store; a reader takes all items in one step (_dispatch_rows)
 
 
 def _project(name, values, weight, scales, biases, residual, group_size, bits):
@@ -368,8 +366,7 @@ def repack_mlx_affine_weight(weight, scales, biases):
 
 
 def _dispatch_rows(table):
-    with _dispatch_lock:
-        items = sorted(table.items())
+    items = sorted(list(table.items()))
     return tuple(
         {
             "rows": key[0],
