@@ -16,8 +16,9 @@
  *   scales   bf16  [N, K/64]     one per group of 64 along K
  *   biases   bf16  [N, K/64]     w[n,k] = scales[n,k/64] * q[n,k] + biases[n,k/64]
  *   out      bf16  [M, N]        y = x @ w^T, fp32 accumulation, one rounding at the store
- * No array is read past its end.  One that does not start on an 8-byte boundary (scales, biases) or a 4-byte one
- * (residual) is read from that boundary on, which lies in the same allocation.
+ * The aligned 8 bytes around the first and the last element of scales and biases, and the aligned 4 bytes around
+ * those of a residual, must be readable (any allocation's granularity sees to that); what lies there beside the
+ * array is never used.
  *
  * Packed weights, scales and biases are read ahead of the stream order: a kernel may start on them while
  * the one in front of it still runs.  What writes them must be complete when the call is made, or be followed

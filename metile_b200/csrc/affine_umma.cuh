@@ -119,7 +119,6 @@ struct UmmaParams {
     int sum_bytes;         // shared memory of the running sum over a CTA's slices, or of the slices a cluster's CTA adds
     int side_bytes;        // that and the residuals in flight
     bool wide_out;         // rows of the output and the residual are 16-byte aligned
-    bool windows;          // the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables)
 };
 
 enum : unsigned int {
@@ -220,9 +219,10 @@ __device__ __forceinline__ int umma_row(int n0, int r, int n_rows) {
 // its own window and the one before, which the previous slot brought; the first slot of a tile brings window 0 in
 // an entry of its own.  So the table ring has three entries more than the weight ring: entry E is overwritten
 // ring + 3 entries later, when the slot after E's is known to be done, tile starts included while a tile has at
-// least ring / 2 + 1 slots (umma_ring_in_use).  A copy ends with the row's last entry: the rest of its window may lie
-// past the end of the array, and is filled with zeros.  It starts with the window, which for the first row of an array
-// off an 8-byte boundary is up to six bytes in front of it.  (Word by word -- up to 24 4-byte copies per lane and
+// least ring / 2 + 1 slots (umma_ring_in_use).  A window holds at least one entry of the row, so no copy
+// touches memory outside the aligned 8 bytes around an array's ends, which the header asks to be readable.  (Copies that
+// end with the array need a size each: 3 to 8 % of a launch over windows, and the same for the residuals' last word 5 to 18 %
+// of many rows of an odd width.)  (Word by word -- up to 24 4-byte copies per lane and
 // slot, each touching sixteen rows -- a slot took 1150 cycles at 106 rows, 6080 -> 11919.)
 template <bool kWindows>
 struct UmmaTables {
@@ -245,36 +245,26 @@ struct UmmaTables {
                 }
             }
     }
-    // The first windows of a tile, for rows that do not start one; a row has `left` entries.
-    __device__ __forceinline__ void copy_head(uint8_t* entry, int left, int lane) const {
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
-                if (offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] - 8, 2 * min(offset + left, 4));
-            }
+    // The first windows of a tile, for rows that do not start one.
+    __device__ __forceinline__ void copy_head(uint8_t* entry, int lane) const {
+        each([&](int t, int q, int offset) {
+            if (offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] - 8);
+        });
     }
     // The windows of slot `st`, of whose k-blocks `left` remain in the share.
     __device__ __forceinline__ void copy(int st, int left, uint8_t* entry, int lane) const {
-        if (!kWindows || left >= 7) {
-            copy_full(st, entry, lane);
-        } else if constexpr (kWindows) {
-#pragma unroll
-            for (int t = 0; t < 2; ++t)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int offset = (int)(offsets >> (8 * t + 2 * q)) & 3;
-                    const int entries = offset ? left - 4 + offset : left;  // of this row from the window's start on
-                    if (entries > 0) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * st, 2 * min(entries, 4));
-                }
-        }
+        each([&](int t, int q, int offset) {
+            if (!kWindows || offset == 0 || left >= 5 - offset) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * st);
+        });
     }
-    __device__ __forceinline__ void copy_full(int st, uint8_t* entry, int lane) const {
+
+private:
+    template <typename F>
+    __device__ __forceinline__ void each(F&& f) const {
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) ptx::cp_async_8(entry + t * 1024 + (32 * q + lane) * 8, at[t][q] + 8 * st);
+            for (int q = 0; q < 4; ++q) f(t, q, (int)(offsets >> (8 * t + 2 * q)) & 3);
     }
 };
 
@@ -364,9 +354,9 @@ __device__ __forceinline__ void umma_finish_rows(const UmmaParams& p, const Umma
     }
 }
 
-// kWindows: see UmmaTables.  A kernel of its own, because every instruction that the dequantising warps do not issue counts
-// (with the layout as a run-time condition 512 rows 1536 -> 8960, gate|up, took 35.3 to 37.6 us, now 34.1; 2000 rows 2048 ->
-// 8192 146 to 155, now 144).
+// kWindows: the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables).  A kernel of its own,
+// because every instruction that the dequantising warps do not issue counts: with the layout as a run-time condition 512
+// rows 1536 -> 8960, gate|up, took 37.6 us, now 34.0; 2000 rows 2048 -> 8192 153, now 144; 16 rows 8192 -> 2048 8.5, now 8.2.
 template <bool kSwiglu, bool kCluster, bool kWindows>
 __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
     constexpr int kOut = kSwiglu ? 64 : 128;  // outputs per tile
@@ -466,7 +456,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 }
                 __syncwarp();
                 if (kWindows && st == 0) {
-                    copies.copy_head(tables + table_at.slot * kUmmaTableBytes, w.nkb, lane);
+                    copies.copy_head(tables + table_at.slot * kUmmaTableBytes, lane);
                     table_at.advance(table_slots);
                 }
                 copies.copy(st, w.nkb - st * kUmmaKBlocksPerSlot, tables + table_at.slot * kUmmaTableBytes, lane);
@@ -619,9 +609,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                         } else if (c0 < rows) {
                             auto copy_word = [&](int j, int word) {
                                 const int n = n_tile + 2 * word - odd_start(p.residual, c0 + j);  // n, n + 1: at least one is in the row
-                                const bool inside = n + 1 < p.N || m0 + c0 + j + 1 < p.M;  // else the array ends within the word
                                 if (c0 + j < rows && n < p.N)
-                                    ptx::cp_async_4(step + j * kUmmaResidualPitch + 4 * word, p.residual + (size_t)(m0 + c0 + j) * p.N + n, inside ? 4 : 2);
+                                    ptx::cp_async_4(step + j * kUmmaResidualPitch + 4 * word, p.residual + (size_t)(m0 + c0 + j) * p.N + n);
                             };
 #pragma unroll
                             for (int i = 0; i < 8; ++i) copy_word(quadrant * 4 + (i >> 1), lane + 32 * (i & 1));
@@ -1119,6 +1108,14 @@ inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, 
     return cudaLaunchKernelEx(&config, affine_umma_kernel<kSwiglu, kCluster, kWindows>, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
+template <bool kSwiglu, bool kWindows>
+inline int launch_umma_tables(const UmmaParams& params, int device, cudaStream_t stream) {
+    const int tiles = params.row_tiles * params.act_tiles;
+    if (params.ksplit > 1) return launch_umma_instance<kSwiglu, true, kWindows>(params, tiles * params.ksplit, device, stream);
+    const int resident = umma_active_clusters<kSwiglu>(1, device);
+    return launch_umma_instance<kSwiglu, false, kWindows>(params, tiles < resident ? tiles : resident, device, stream);
+}
+
 template <bool kSwiglu>
 inline int launch_umma_family(UmmaParams& params, cudaStream_t stream) {
     int device = 0;
@@ -1131,15 +1128,9 @@ inline int launch_umma_family(UmmaParams& params, cudaStream_t stream) {
     if (params.npad == 0) return MT_ERR_LAUNCH;  // not even one CTA fits the device
     params.side_bytes = params.sum_bytes + (params.residual && params.ksplit == 1 ? kUmmaResidualBytes : 0);
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
-    const int tiles = params.row_tiles * params.act_tiles;
-    if (params.ksplit > 1) {
-        const int ctas = tiles * params.ksplit;
-        return params.windows ? launch_umma_instance<kSwiglu, true, true>(params, ctas, device, stream)
-                              : launch_umma_instance<kSwiglu, true, false>(params, ctas, device, stream);
-    }
-    const int resident = umma_active_clusters<kSwiglu>(1, device), ctas = tiles < resident ? tiles : resident;
-    return params.windows ? launch_umma_instance<kSwiglu, false, true>(params, ctas, device, stream)
-                          : launch_umma_instance<kSwiglu, false, false>(params, ctas, device, stream);
+    bool windows = kblocks % 4 != 0;
+    for (int t = 0; t < 2; ++t) windows = windows || !aligned_to(params.scales[t], 8) || !aligned_to(params.biases[t], 8);
+    return windows ? launch_umma_tables<kSwiglu, true>(params, device, stream) : launch_umma_tables<kSwiglu, false>(params, device, stream);
 }
 
 struct AffineWeights {
@@ -1167,9 +1158,6 @@ inline int launch_umma(const void* x, const AffineWeights* first, const AffineWe
     params.N = N;
     params.row_tiles = swiglu ? (N + 63) / 64 : (N + 127) / 128;
     params.wide_out = N % 8 == 0 && aligned_to(out, 16) && (!residual || aligned_to(residual, 16));
-    params.windows = (K / kUmmaBlockK) % 4 != 0;
-    for (int t = 0; t < 2; ++t)
-        params.windows = params.windows || !aligned_to(params.scales[t], 8) || !aligned_to(params.biases[t], 8);
     const int box_rows = swiglu ? 64 : 128;
     if (!encode_weight_map(&params.w_map[0], first->w, K, N, box_rows)) return MT_ERR_LAUNCH;
     if (swiglu && !encode_weight_map(&params.w_map[1], second->w, K, N, box_rows)) return MT_ERR_LAUNCH;

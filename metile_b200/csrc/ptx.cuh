@@ -148,13 +148,6 @@ __device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src) {
 __device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
-// The same, reading only the first `bytes` of the source; zeros fill the rest of what is written.
-__device__ __forceinline__ void cp_async_8(void* smem_dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }

@@ -133,37 +133,36 @@ def test_ring_tasks_store_every_row_once(k, n, dual):
 
 
 def window_copies(start, entries):
-    """(window, first byte, bytes) of a row's table copies; `start` is the byte address of its first entry.  Window 0 is
+    """(window, first byte) of a row's 8-byte table copies; `start` is the byte address of its first entry.  Window 0 is
     the one the row starts in the middle of; window st + 1 belongs to slot st, as does window st of an aligned row."""
     offset = start // 2 % 4
     base = start - 2 * offset
     if offset:
-        yield 0, base, 2 * min(offset + entries, 4)
+        yield 0, base
     for st in range(-(-entries // 4)):
         left = entries - 4 * st
         there = left - 4 + offset if offset else left
         if there > 0:
-            yield st + (offset > 0), base + 8 * (st + (offset > 0)), 2 * min(there, 4)
+            yield st + (offset > 0), base + 8 * (st + (offset > 0))
 
 
 @pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 7, 8, 21, 95])
-@pytest.mark.parametrize("rows", [1, 2, 3, 130])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 129, 130, 131])
 @pytest.mark.parametrize("shift", [0, 2, 4, 6])
-def test_window_copies_bring_every_entry_and_end_with_the_row(groups, rows, shift):
-    for row in {0, 1, rows - 1} & set(range(rows)):
+def test_window_copies_bring_every_entry_and_stay_within_the_arrays_own_windows(groups, rows, shift):
+    for row in range(rows):
         start = 1024 + shift + 2 * row * groups
         brought = set()
-        for _, at, size in window_copies(start, groups):
-            assert at % 8 == 0 and size in (2, 4, 6, 8)
-            assert at + size <= start + 2 * groups                  # nothing past the row, so nothing past the array
-            assert at >= 1024 + (0 if row * groups >= 3 or shift == 0 else shift - 6)
-            brought |= set(range(at, at + size, 2))
+        for _, at in window_copies(start, groups):
+            first, last = 1024 + shift, 1024 + shift + 2 * rows * groups - 2
+            assert at % 8 == 0 and first // 8 <= at // 8 <= last // 8
+            brought |= set(range(at, at + 8, 2))
         assert brought >= {start + 2 * entry for entry in range(groups)}
 
 
 @pytest.mark.parametrize("rows,n", [(1, 1), (1, 129), (3, 5), (16, 257), (17, 131), (4, 128)])
 @pytest.mark.parametrize("odd", [0, 1])  # the residual starts in the middle of a word
-def test_residual_words_bring_every_element_and_stay_inside_the_array(rows, n, odd):
+def test_residual_words_bring_every_element_and_stay_within_the_arrays_own_words(rows, n, odd):
     brought = set()
     for m in range(rows):
         start = (odd + m * n) % 2
@@ -171,8 +170,7 @@ def test_residual_words_bring_every_element_and_stay_inside_the_array(rows, n, o
             for word in range(65 if (odd + m * n + tile) % 2 else 64):
                 first = tile + 2 * word - start                     # elements first, first + 1
                 if first < n:
-                    size = 4 if first + 1 < n or m + 1 < rows else 2
                     at = 2 * (odd + m * n + first)
-                    assert at % 4 == 0 and at + size <= 2 * (odd + rows * n) and at >= 0
-                    brought |= {at, at + size - 2}
+                    assert at % 4 == 0 and 2 * odd // 4 <= at // 4 <= 2 * (odd + rows * n - 1) // 4
+                    brought |= {at, at + 2}
     assert brought >= {2 * (odd + i) for i in range(rows * n)}
