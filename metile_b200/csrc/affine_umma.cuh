@@ -1028,7 +1028,7 @@ inline int umma_slices(int N, int slots_total, int device) {
 }
 
 // How the work is laid over the SMs: rows per activation tile and CTAs per tile.  Nothing here changes a bit of
-// the result.  Costs in SM cycles, fitted to measurements of every split at eight shapes and 16 to 512 rows:
+// the result.  Costs in SM cycles of a B200 at its 1.965 GHz, fitted to measurements of every split at eight shapes and 16 to 512 rows:
 //   ring slot (four k-blocks)   530 + 4 per row on a nearly idle chip, 550 + 11 per row with every SM at work (the
 //                               activations of all tiles come from L2); never below the weights at 4.8 TB/s
 //   CTAs                        45 each, as far as they are resident: what they leave idle, the next kernel starts on
@@ -1041,10 +1041,11 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
     const int S = p.slices;
     const int splits[3] = {1, (S + 1) / 2, S};
     const long weights = (long)((double)p.N * p.K * (kSwiglu ? 2 : 1) * (0.5625 * 1.965e9 / 4.8e12));
-    for (int max_rows = 64; max_rows <= 128; max_rows *= 2) {
+    const int sms = umma_active_clusters<kSwiglu>(1, device);  // with room for a CTA
+    for (int max_rows = kUmmaMaxRows / 2; max_rows <= kUmmaMaxRows; max_rows *= 2) {
         const int act_tiles = (p.M + max_rows - 1) / max_rows;
         const int npad = ((p.M + act_tiles - 1) / act_tiles + 15) / 16 * 16;
-        if (max_rows == 128 && npad <= 64) continue;  // the same tiles again
+        if (max_rows == kUmmaMaxRows && npad <= kUmmaMaxRows / 2) continue;  // the same tiles again
         const bool big = npad > 64;
         const long idle_slot = 530 + 4 * npad, busy_slot = 550 + 11 * npad;
         const long tiles = (long)p.row_tiles * act_tiles;
@@ -1068,7 +1069,7 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
             if (sum && big) continue;
             const long waves = (tiles + active - 1) / active;
             const long resident = (long)active * P, ctas = tiles * P < resident ? tiles * P : resident;
-            const long slot = busy_slot > idle_slot ? idle_slot + (busy_slot - idle_slot) * ctas / 148 : idle_slot;
+            const long slot = busy_slot > idle_slot ? idle_slot + (busy_slot - idle_slot) * ctas / sms : idle_slot;
             const long stream = waves * slots * slot;
             long cost = (stream > weights ? stream : weights) + 45 * ctas;
             if (P > 1) {

@@ -208,7 +208,6 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 __device__ __forceinline__ void tc_fence_after_sync() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Waits for this thread's tcgen05.ld and names the 16 destination registers as in/out operands, so
 // that no arithmetic on them can be scheduled above the wait.
 __device__ __forceinline__ void tc_wait_ld16(uint32_t (&v)[16]) {
