@@ -804,11 +804,11 @@ def run_ours(args):
 
             bound = "tensor" if m >= 128 else "hbm"
             roofline_kernels.append(entry(
-                f"gate|up SwiGLU on tcgen05, {m}-row instance (affine_umma_kernel<2,{m}>)", rows_served,
+                f"gate|up SwiGLU on tcgen05, {m}-row instance (affine_umma_kernel<true, ...>)", rows_served,
                 per_launch_seconds(gate_up, 1), 2 * packed + m * hidden * 2 + m * inter * 2, TRAFFIC[f"swiglu_{m}"],
                 PROFILE_K2, bound, 2.0 * 2 * hidden * inter * m))
             roofline_kernels.append(entry(
-                f"down projection on tcgen05, {m}-row instance (affine_umma_kernel<1,{m}>)", rows_served,
+                f"down projection on tcgen05, {m}-row instance (affine_umma_kernel<false, ...>)", rows_served,
                 per_launch_seconds(down_projection, 1), packed + m * inter * 2 + 2 * m * hidden * 2,
                 TRAFFIC[f"down_{m}"], PROFILE_K2, bound, 2.0 * hidden * inter * m))
         if roofline_kernels:

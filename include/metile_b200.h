@@ -16,6 +16,8 @@
  *   scales   bf16  [N, K/64]     one per group of 64 along K
  *   biases   bf16  [N, K/64]     w[n,k] = scales[n,k/64] * q[n,k] + biases[n,k/64]
  *   out      bf16  [M, N]        y = x @ w^T, fp32 accumulation, one rounding at the store
+ * The tcgen05 kernel holds weights times 2^-37: scales from 2^32 on overflow there, and a weight below 2^-89
+ * loses bits.  The other kernels take every bf16 scale.
  * The aligned 8 bytes around the first and the last element of scales and biases, and the aligned 4 bytes around
  * those of a residual, must be readable (any allocation's granularity sees to that); what lies there beside the
  * array is never used.

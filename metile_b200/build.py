@@ -21,6 +21,7 @@ HEADERS = ("common.cuh", "ptx.cuh", "affine_gemv.cuh", "affine_umma.cuh", "affin
            "dense_rows.cuh", os.path.join("..", "..", "include", "metile_b200.h"))
 BINDING_SOURCE = os.path.join(CSRC, "binding.cpp")
 BINDING_OUTPUT = os.path.join(HERE, "_native.so")
+BINDING_TORCH = os.path.join(CSRC, "build", "native.torch")  # the torch version it was compiled against
 
 
 def _nvcc():
@@ -41,8 +42,20 @@ def is_stale():
     return _older(OUTPUT, [os.path.join(CSRC, name) for name in SOURCES + HEADERS])
 
 
+def _torch_version():
+    import torch
+
+    return f"{torch.__version__} {sys.version_info[:2]}"
+
+
 def binding_is_stale():
-    return _older(BINDING_OUTPUT, [BINDING_SOURCE, os.path.join(CSRC, HEADERS[-1])])
+    if _older(BINDING_OUTPUT, [BINDING_SOURCE, os.path.join(CSRC, HEADERS[-1])]):
+        return True
+    try:
+        with open(BINDING_TORCH) as file:
+            return file.read() != _torch_version()
+    except OSError:
+        return True
 
 
 def _build_binding():
@@ -60,6 +73,9 @@ def _build_binding():
     command += [BINDING_SOURCE, OUTPUT, f"-L{libraries}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
                 "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN/csrc", "-o", BINDING_OUTPUT]
     subprocess.run(command, check=True)
+    os.makedirs(os.path.dirname(BINDING_TORCH), exist_ok=True)
+    with open(BINDING_TORCH, "w") as file:
+        file.write(_torch_version())
 
 
 def build(force=False, verbose=False):

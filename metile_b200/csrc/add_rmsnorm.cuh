@@ -125,7 +125,7 @@ inline int launch_add_rmsnorm(const void* x, const void* residual, const void* w
         const int vectors = H / 8;
         threads = ((vectors + 31) / 32) * 32;
         if (threads > 1024) threads = 1024;
-        // Keep at least two vectors per thread for wide rows so fewer warps take part in the reduce.
+        // Wider rows than the registers hold are read element by element.
         if (vectors > 1024 * kNormMaxVecPerThread) vector = false;
     }
     if (!vector) threads = H >= 1024 ? 1024 : ((H + 31) / 32) * 32;

@@ -301,9 +301,10 @@ affine_gemv_kernel(const uint16_t* x, GemvWeights first, GemvWeights second, con
 
 // ---- one activation row, weights through per-warp rings --------------------------------------------
 // The same sums in the same order as affine_gemv_kernel<1, ...>; what differs is how the operands get there.
-// Weights requested into registers one iteration ahead kept about 70 KB in flight per SM at best.  Here every lane
+// Weights requested into registers one iteration ahead cost 125 registers a thread, and a warp waits for all of an
+// iteration's loads together.  Here every lane
 // copies its own 16 bytes of packed words, and a warp the words that hold its scales and biases, into a ring of the
-// warp's, two iterations ahead, by asynchronous copies (96 KB in flight per SM, no registers, and no synchronisation
+// warp's, two iterations ahead, by asynchronous copies (64 KB of words and up to 10 KB of tables in flight per SM, no registers, and no synchronisation
 // beyond the warp's).  The fp32 activations and the slot sums are made by one thread per slot with one barrier; the
 // lanes' totals of all rows are folded together (5 exchanges instead of 16); the warps' rows are dealt out SM by SM.
 // Times in a replayed graph, with registers and with rings: 1536 -> 8960 6.8 and 4.7 us, 4096 -> 4096 7.6 and 5.0, 2048 ->

@@ -59,9 +59,12 @@ constexpr int kFusedComputeWarps = MT_FUSED_WARPS;
 constexpr int kFusedComputeThreads = kFusedComputeWarps * 32;
 constexpr int kFusedThreads = kFusedComputeThreads + 32;  // + the producer warp
 constexpr int kFusedMaxRows = 4;       // activation rows (each lane keeps 32 fp32 activations per row in registers)
-constexpr int kFusedDefaultRows = 1;   // rows the FMA kernel serves by default (measured: 16.2 / 20.1 / 22.4 us at
-                                       // 1 / 2 / 3 rows against 19.3 us for the warp-MMA kernel); two to four
-                                       // rows only when asked with MT_FLAG_MLP_FUSED
+// Rows the FMA kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED (16.2 / 20.1 / 22.4 us at 1 / 2 / 3
+// rows against 19.3 us for the warp-MMA kernel).  The rule for one row is older than the GEMV's rings: in replayed graphs
+// two GEMV launches now take 5.1 / 6.2 / 8.2 / 13.0 / 21.1 us at hidden / intermediate widths of 1024 / 1024, 1024 / 4096, 2048 /
+// 4096, 2048 / 8192, 4096 / 8192, this kernel 9.2 / 8.0 / 11.1 / 15.4 / 24.6 (8192 / 8192: 37.4 and 37.5).  The order of a
+// row's sums differs between the two.
+constexpr int kFusedDefaultRows = 1;
 constexpr int kFusedMaxSlots = 12;
 constexpr int kFusedItemRows = MT_FUSED_ITEM_ROWS;  // gate/up rows per ring item
 constexpr int kFusedSmemBudget = 226 * 1024;  // one CTA per SM

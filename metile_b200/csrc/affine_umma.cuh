@@ -1042,6 +1042,7 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
     const int splits[3] = {1, (S + 1) / 2, S};
     const long weights = (long)((double)p.N * p.K * (kSwiglu ? 2 : 1) * (0.5625 * 1.965e9 / 4.8e12));
     const int sms = umma_active_clusters<kSwiglu>(1, device);  // with room for a CTA
+    if (sms <= 0) return;
     for (int max_rows = kUmmaMaxRows / 2; max_rows <= kUmmaMaxRows; max_rows *= 2) {
         const int act_tiles = (p.M + max_rows - 1) / max_rows;
         const int npad = ((p.M + act_tiles - 1) / act_tiles + 15) / 16 * 16;

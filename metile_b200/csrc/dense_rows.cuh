@@ -64,8 +64,8 @@ __device__ __forceinline__ int folded_first(int lane, bool& owner) {
     }
 }
 
-// One CTA of sixteen warps per SM.  Weights go through a private ring of each warp by asynchronous copies, 60 to 90 KB in
-// flight per SM: requested into registers some blocks ahead they arrived one block at a time, since a
+// One CTA of sixteen warps per SM.  Weights go through a private ring of each warp by asynchronous copies, 28 KB (one row of
+// weights at a time) to 80 KB in flight per SM: requested into registers some blocks ahead they arrived one block at a time, since a
 // warp's few scoreboards are shared by the blocks (1536 -> 8960, one row: 12.4 us, now 6.3).  No registers are
 // spent on it, so a warp holds 64 accumulators, and an activation is read and converted once for four outputs.
 constexpr int kDenseThreads = 512;

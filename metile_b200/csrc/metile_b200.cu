@@ -50,9 +50,11 @@ static int check_affine_ptrs(const void* x, const uint32_t* w, const void* s, co
     return MT_OK;
 }
 
-// Row-count split: the CUDA-core GEMV issues one FMA per weight per row on top of the unpack, so
-// it is instruction-bound already at one row; measured, it wins at one row only (fused MLP at the
-// Llama-3.2-1B shape: 18.7 us vs 24.6 us) and loses from two rows on (26.1 us vs 24.7 us).
+// Row-count split: the CUDA-core GEMV issues one FMA per weight per row on top of the unpack, so its time grows with
+// the rows; the tcgen05 kernel's does not.  In replayed graphs, GEMV | tcgen05, us: one row 1536 -> 1536 3.4 | 3.9,
+// 4096 -> 4096 4.5 | 7.0, 8192 -> 2048 4.9 | 8.2, 2048 -> 16384 7.0 | 8.4, 2048 -> 128256 40.0 | 36.8; two rows 5.1 | 4.0,
+// 7.5 | 7.0, 8.2 | 8.2, 10.4 | 8.4, 64.0 | 36.7.  At one row the largest outputs would gain 8 % on the tensor cores, but the
+// GEMV never rounds a weight, and one row keeps one kernel for all widths.
 static bool use_gemv(int M, unsigned int flags) {
     if (flags & MT_FLAG_FORCE_GEMV) return true;
     if (flags & MT_FLAG_FORCE_UMMA) return false;
@@ -362,7 +364,9 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         params.H = H;
         params.I = I;
         const int sms = device_sm_count();
-        // Up to kFusedDefaultRows rows: the FMA kernel.  Above, to eight rows: the warp-MMA kernel.
+        // Up to kFusedDefaultRows rows: the FMA kernel.  Above, to eight rows: the warp-MMA kernel, which does not round
+        // the weights (against the tcgen05 pair, us at 2 to 8 rows: 1024 / 1024 7.6 | 9.3, 2048 / 4096 12.1 | 15.0, 1024 / 4096
+        // 10.7 | 9.8, 2048 / 8192 18.6 | 18.1).
         const bool want_mma = (flags & MT_FLAG_MLP_FUSED_MMA) != 0;
         const bool fma = !want_mma && (flags || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
         const bool mma = !fma && (want_mma || (!flags && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);

@@ -107,3 +107,15 @@ def test_operators_refuse_cpu_tensors_and_bad_formats():
         backends.MLXAffineWeight.from_mlx(w, s, b, bits=8)
     with pytest.raises(TypeError):
         backends.mlx_rms_norm(x, torch.ones(64), 1e-5)
+
+
+def test_the_binding_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    from metile_b200 import build
+
+    monkeypatch.setattr(build, "_older", lambda output, inputs: False)
+    monkeypatch.setattr(build, "BINDING_TORCH", str(tmp_path / "native.torch"))
+    assert build.binding_is_stale()
+    (tmp_path / "native.torch").write_text(build._torch_version())
+    assert not build.binding_is_stale()
+    monkeypatch.setattr(build, "_torch_version", lambda: "another")
+    assert build.binding_is_stale()
