@@ -34,13 +34,15 @@
  * what the CUDA runtime reported for a launch.  There is no CPU fallback.
  *
  * `flags`: 0 selects the kernel by row count.  A single projection (mt_affine_qmv, mt_affine_swiglu):
- * the CUDA-core GEMV for M = 1, the tcgen05 kernel above.  mt_affine_mlp: one cooperative launch for
+ * the CUDA-core GEMV for M = 1, the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one cooperative launch for
  * the whole MLP when the shape allows it -- on CUDA cores for M = 1 (H and I in {1024, 2048, 4096,
  * 8192}), on mma.sync for M = 2 ... 8 (H in {512, 1024, 1536, 2048}, I a multiple of 512) -- else two
  * kernels (gate|up SwiGLU, then down) of the families above.
  *   MT_FLAG_FORCE_GEMV (1)   CUDA-core GEMV (M <= 8)
  *   MT_FLAG_FORCE_UMMA (2)   tcgen05 kernel for any M (one accumulation order for every M: use it
  *                            when rows must be bit-identical across batch sizes 1..128)
+ *   MT_FLAG_FIXED_ORDER (256) the tcgen05 kernel's sums in the order of MT_FLAG_FORCE_UMMA, the kernel by row
+ *                            count as with 0 (may be combined with the flags that choose a kernel)
  *   MT_FLAG_GELU (16)        mt_dense_act: x/(1+exp(-1.702x)) instead of SiLU
  *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch CUDA-core kernel (M <= 4); -1
  *                            when it does not apply.  With flags = 0 the default dispatch falls back
@@ -65,6 +67,7 @@ extern "C" {
 #define MT_FLAG_MLP_FUSED 0x20u
 #define MT_FLAG_HOST_PAIR 0x40u
 #define MT_FLAG_MLP_FUSED_MMA 0x80u
+#define MT_FLAG_FIXED_ORDER 0x100u
 
 /* Library version (major*10000 + minor*100 + patch). */
 int mt_version(void);

@@ -16,6 +16,7 @@ from .cuda_dense import (  # noqa: F401
 )
 from .cuda_quantized import (  # noqa: F401
     batch_invariant,
+    fixed_order,
     force_kernel,
     kernel_pinned,
     mlx_affine_mlp_executor,

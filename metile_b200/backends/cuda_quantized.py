@@ -42,21 +42,25 @@ from ._common import (
     rows_of,
 )
 
-_state = threading.local()
+class _State(threading.local):
+    flags = 0  # of this thread's calls: a pinned kernel family, FLAG_FIXED_ORDER within fixed_order()
+
+
+_state = _State()
 _swiglu_dispatches = {}
 _residual_dispatches = {}
 
 
 def _flags():
-    return getattr(_state, "flags", 0)
+    return _state.flags
 
 
 @contextlib.contextmanager
 def batch_invariant(enabled=True):
     """Serve every row count from the tcgen05 kernel family, so that a row's output bits do not
     depend on whether it runs alone or in a batch of up to 128 (one accumulation order)."""
-    previous = _flags()
-    _state.flags = _lib.FLAG_FORCE_UMMA if enabled else 0
+    previous = _state.flags
+    _state.flags = previous & _lib.FLAG_FIXED_ORDER | (_lib.FLAG_FORCE_UMMA if enabled else 0)
     try:
         yield
     finally:
@@ -65,7 +69,23 @@ def batch_invariant(enabled=True):
 
 def kernel_pinned():
     """Whether a kernel family is pinned in this thread (batch_invariant, force_kernel)."""
-    return _flags() != 0
+    return _state.flags & ~_lib.FLAG_FIXED_ORDER != 0
+
+
+class fixed_order:
+    """Within it, the sums of the tcgen05 kernels are cut as in batch-invariant mode, whatever the row count; the kernel
+    family follows the row count as always.  A model's modules run in it: a token's keys and values are then the same bits
+    in a prompt of any length (of two tokens and more) and beside any other sequences.  An operator called on its own
+    takes the cut that is fastest for its rows."""
+
+    __slots__ = ("previous",)
+
+    def __enter__(self):
+        self.previous = _state.flags
+        _state.flags = self.previous | _lib.FLAG_FIXED_ORDER
+
+    def __exit__(self, *exception):
+        _state.flags = self.previous
 
 
 @contextlib.contextmanager
@@ -77,8 +97,8 @@ def force_kernel(name):
              "mlp_fused": _lib.FLAG_MLP_FUSED, "mlp_fused_mma": _lib.FLAG_MLP_FUSED_MMA}
     if name not in table:
         raise ValueError(f"unknown kernel family {name!r}")
-    previous = _flags()
-    _state.flags = table[name]
+    previous = _state.flags
+    _state.flags = previous & _lib.FLAG_FIXED_ORDER | table[name]
     try:
         yield
     finally:
@@ -394,6 +414,7 @@ def mlx_affine_residual_qmv_dispatches():
 
 __all__ = [
     "batch_invariant",
+    "fixed_order",
     "force_kernel",
     "mlx_affine_mlp_host_executor",
     "mlx_affine_mlp_executor",

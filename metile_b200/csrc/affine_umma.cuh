@@ -32,10 +32,13 @@
 // the K range of a tile is shared by a thread-block cluster instead (kCluster), whose CTAs store their sums into
 // one another's shared memory.
 //
-// Determinism: an output is a sum over slices of the K range, in slice order.  A slice is one accumulator chain
-// in ascending k (gate|up) or two, of its even and its odd pairs of k-blocks, added even + odd (plain).  The
-// slices are a function of (N, K, kernel family) only, and neither the tile's rows nor who computes a slice
-// changes a bit, so a row's result does not depend on how many other rows are in the batch.
+// Determinism: an output is a sum over slices of the K range, in slice order.  In the fixed order (batch-invariant mode,
+// a model's modules) a slice is one accumulator chain in ascending k (gate|up) or two, of its even and its odd pairs of
+// k-blocks, added even + odd (plain); the slices are a function of (N, K, kernel family) only, and neither the tile's
+// rows nor who computes a slice changes a bit, so a row's result does not depend on how many other rows are in the batch.
+// A call that asks for no such thing has one chain per slice and the slices that suit its rows (umma_plan): at 2000 rows the
+// MLP 2048 / 8192 takes 174 us instead of 231 (201 and 269 in a loop long enough to meet the power limit, where the SM
+// clock settles at 1.50 and 1.66 GHz), at 128 rows 5120 / 27648 123 instead of 127.5 (such a loop).
 //
 // Measured in a replayed graph, against the kernel with two CTA-wide tiles, one hand-off per pair of k-blocks and a
 // cluster sum read over DSMEM that this replaces (us): 16 rows gate|up 2048 -> 8192 10.9 -> 8.0, 8192 -> 2048 10.1 ->
@@ -47,6 +50,8 @@
 #pragma once
 
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -113,6 +118,7 @@ struct UmmaParams {
     uint16_t* out;
     int M, K, N;
     int slices;            // parts of the K range that are summed apart (see umma_slices)
+    int chains;            // of a slice: one accumulator, or two for its even and its odd pairs of k-blocks
     int ksplit;            // CTAs of a cluster that share a tile's slices
     int row_tiles, act_tiles, npad;
     int unit_shift;        // log2 of the accumulator units in tensor memory
@@ -190,7 +196,7 @@ __device__ __forceinline__ UmmaShare umma_share(const UmmaParams& p) {
     return w;
 }
 
-// Whether slice s has a second pair of k-blocks at all (the chain of the odd pairs is otherwise never written).
+// Whether slice s has a second pair of k-blocks at all (a chain of the odd pairs is otherwise never written).
 __device__ __forceinline__ bool umma_slice_has_second(const UmmaShare& w, int s) {
     return w.nkb - w.slice_slot(s) * kUmmaKBlocksPerSlot > 2;
 }
@@ -307,7 +313,7 @@ __device__ __forceinline__ void umma_push_slices(const UmmaParams& p, const Umma
     const int rows_per_cta = umma_rows_per_cta(p);
     for (int s = w.slice_begin; s < w.slice_end; ++s) {
         const uint32_t acc = tmem + (uint32_t)(s - w.slice_begin) * unit_cols;
-        const bool second = !kSwiglu && umma_slice_has_second(w, s);
+        const bool second = !kSwiglu && p.chains == 2 && umma_slice_has_second(w, s);
         uint32_t at = staging + 4u * (uint32_t)(s * rows_per_cta * kUmmaTileRows + thread);  // row / ksplit = 0
         int owner = 0;
         for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -390,8 +396,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);  // the same for the whole warp, and known to be
     const int lane = threadIdx.x & 31;
-    // Accumulator units: one slice's sums -- gate|up one accumulator, plain two (even and odd pairs of k-blocks).
+    // Accumulator units: one slice's sums, in one chain or in two halves of the unit.
     const uint32_t unit_mask = (1u << p.unit_shift) - 1u, unit_cols = (uint32_t)kUmmaAColumn >> p.unit_shift;
+    const bool two_chains = !kSwiglu && p.chains == 2;
     const uint32_t second_col = unit_cols >> 1;
 
     if (threadIdx.x == 0) {
@@ -534,11 +541,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                             if (kb >= valid) break;
                             const int x_slot = kb < 2 ? first.slot : second.slot;
                             const uint64_t b_desc = desc0 + (uint64_t)((x_slot * x_slot_bytes + (kb & 1) * npad * 128) >> 4);
-                            const uint32_t d = kSwiglu || kb < 2 ? d_tmem : d_tmem + second_col;
+                            const uint32_t d = two_chains && kb >= 2 ? d_tmem + second_col : d_tmem;
+                            const bool starts = st == begin && (kb == 0 || (kb == 2 && two_chains));
 #pragma unroll
                             for (int ks = 0; ks < kUmmaBlockK / 16; ++ks)  // the first MMA into an accumulator overwrites it
-                                ptx::umma_ts(d, a_tmem + kb * 32 + ks * 8, b_desc + (uint64_t)(ks * 2), idesc,
-                                             (kSwiglu ? kb : kb & 1) > 0 || ks > 0 || st > begin ? 1u : 0u);
+                                ptx::umma_ts(d, a_tmem + kb * 32 + ks * 8, b_desc + (uint64_t)(ks * 2), idesc, starts && ks == 0 ? 0u : 1u);
                             if (kb == 1 || (kb == 0 && valid == 1)) ptx::umma_commit(&x_empty[first.slot]);
                         }
                         ptx::tc_fence_before_sync();
@@ -628,7 +635,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 for (int s = 0; s < my_slices - direct; ++s, ++q) {
                     if (!wait_unit(q)) break;
                     const uint32_t acc = unit_address(q);
-                    const bool second = !kSwiglu && umma_slice_has_second(w, s);
+                    const bool second = two_chains && umma_slice_has_second(w, s);
                     for (int c0 = 0; c0 < rows; c0 += 16) {
                         float v[16];
                         umma_read16(acc + c0, acc + c0 + second_col, second, v);
@@ -646,11 +653,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __gr
                 }
                 if (!alive) break;
 
-                // The final pass: the last slice (two chains of a plain projection) after the running sum of the earlier
-                // ones, or both of gate|up's two slices.
+                // The final pass: the last slice (or its two chains) after the running sum of the earlier ones, or both of
+                // gate|up's two slices.
                 if (!wait_unit(q) || (direct == 2 && !wait_unit(q + 1))) break;
                 const uint32_t acc = unit_address(q);
-                const bool second = kSwiglu ? direct == 2 : umma_slice_has_second(w, w.slice_end - 1);
+                const bool second = kSwiglu ? direct == 2 : two_chains && umma_slice_has_second(w, w.slice_end - 1);
                 const uint32_t acc2 = kSwiglu ? unit_address(q + 1) : acc + second_col;
                 const bool earlier = my_slices > direct;
                 // Sixteen activation rows at a time through shared memory, so that an output row leaves as 16-byte
@@ -1003,9 +1010,9 @@ inline int umma_active_clusters(int size, int device) {
     return clusters;
 }
 
-// Slices of the K range that are accumulated apart and added in order: part of a result's bits, and a function
-// of (N, K, kernel family, device) only -- never of the number of activation rows, nor of how the slices are
-// spread over CTAs.  The rule: the split over a thread-block cluster that finishes 128-row tiles soonest,
+// Slices of the K range that are accumulated apart and added in order: part of a result's bits.  Where those may not depend
+// on the row count they are a function of (N, K, kernel family, device) only, and how the slices are spread over CTAs
+// changes nothing.  The rule: the split over a thread-block cluster that finishes 128-row tiles soonest,
 // waves x (k-blocks per CTA + a fixed part).
 template <bool kSwiglu>
 inline int umma_slices(int N, int slots_total, int device) {
@@ -1027,8 +1034,7 @@ inline int umma_slices(int N, int slots_total, int device) {
     return best;
 }
 
-// How the work is laid over the SMs: rows per activation tile and CTAs per tile.  Nothing here changes a bit of
-// the result.  Costs in SM cycles of a B200 at its 1.965 GHz, fitted to measurements of every split at eight shapes and 16 to 512 rows:
+// How the work is then laid over the SMs: rows per activation tile and CTAs per tile.  Costs in SM cycles of a B200 at its 1.965 GHz, fitted to measurements of every split at eight shapes and 16 to 512 rows:
 //   ring slot (four k-blocks)   530 + 4 per row on a nearly idle chip, 550 + 11 per row with every SM at work (the
 //                               activations of all tiles come from L2); never below the weights at 4.8 TB/s
 //   CTAs                        45 each, as far as they are resident: what they leave idle, the next kernel starts on
@@ -1036,7 +1042,9 @@ inline int umma_slices(int N, int slots_total, int device) {
 //   running sum                 14 per row and slice
 //   cluster                     45 per row and slice of a CTA; 8000 per wave after the first (it is not persistent)
 template <bool kSwiglu>
-inline void umma_plan(UmmaParams& p, int slots_total, int device) {
+inline void umma_fixed_plan(UmmaParams& p, int slots_total, int device) {
+    p.slices = umma_slices<kSwiglu>(p.N, slots_total, device);
+    p.chains = kSwiglu ? 1 : 2;
     long best_cost = -1;
     const int S = p.slices;
     const int splits[3] = {1, (S + 1) / 2, S};
@@ -1090,6 +1098,51 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
     }
 }
 
+// Where nothing ties a row's bits to other row counts: a plain projection has one chain too, so that the accumulators of two
+// tiles of 128 rows find room and finishing one overlaps the next (in two chains 8192 -> 2048 at 2000 rows took 83 us, now
+// 57), and the K range is cut into as many slices as pay for these rows, a CTA each.  Costs in SM cycles at 1.9 GHz, fitted to
+// every such split at fourteen shapes and ten row counts from 16 to 2000 in replayed graphs (what the model picks takes 0.5 %
+// longer than the best split on average, 8 % at most):
+//   ring slot (four k-blocks)   923 + 3.2 per row on a nearly idle chip, 12.5 per row with every SM at work; never below the
+//                               weights at 4 TB/s
+//   CTAs                        3.5 each; 2165 where they are more than half of the SMs, for then the next kernel's find
+//                               no SM to start on (8192 -> 2048, 16 rows: 64 CTAs 6.6 us, 80 CTAs 7.9)
+//   finishing a tile            55 per row, 4 behind another tile
+//   cluster                     1180, 64 per row; 8800 + 35 per row for a wave after the first (it is not persistent).
+//                               More than five CTAs never paid
+template <bool kSwiglu>
+inline void umma_plan(UmmaParams& p, int slots_total, int device) {
+    constexpr int kMostSlices = 5;
+    const int sms = umma_active_clusters<kSwiglu>(1, device);  // with room for a CTA
+    if (sms <= 0) return;
+    const double weights = (double)p.N * p.K * (kSwiglu ? 2 : 1) * (0.5625 / 2120.0);
+    double best_cost = -1.0;
+    for (int max_rows = kUmmaMaxRows / 2; max_rows <= kUmmaMaxRows; max_rows *= 2) {
+        const int act_tiles = (p.M + max_rows - 1) / max_rows;
+        const int npad = ((p.M + act_tiles - 1) / act_tiles + 15) / 16 * 16;
+        if (max_rows == kUmmaMaxRows && npad <= kUmmaMaxRows / 2) continue;  // the same tiles again
+        const long tiles = (long)p.row_tiles * act_tiles;
+        const double idle = 923 + 3.2 * npad, busy = 12.5 * npad;
+        for (int P = 1; P <= kMostSlices && P <= slots_total; ++P) {
+            const int active = umma_active_clusters<kSwiglu>(P, device);
+            if (active <= 0) continue;
+            const long waves = (tiles + active - 1) / active, ctas = std::min(tiles, (long)active) * P;
+            const double slot = busy > idle ? idle + (busy - idle) * ctas / sms : idle;
+            double cost = std::max((double)waves * ((slots_total + P - 1) / P) * slot, weights) + 3.5 * ctas + (2 * ctas > sms ? 2165 : 0);
+            if (P > 1) cost += 1180 + 64.0 * npad + (waves - 1) * (8800 + 35.0 * npad);
+            else cost += 55.0 * npad + (waves - 1) * 4.4 * npad;
+            if (best_cost >= 0 && cost >= best_cost) continue;
+            best_cost = cost;
+            p.act_tiles = act_tiles;
+            p.npad = npad;
+            p.slices = p.ksplit = P;
+            p.chains = 1;
+            p.unit_shift = npad > 64 ? 1 : 2;
+            p.sum_bytes = P > 1 && npad <= 64 ? P * ((npad + P - 1) / P) * kUmmaTileRows * 4 : 0;
+        }
+    }
+}
+
 template <bool kSwiglu, bool kCluster, bool kWindows>
 inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, cudaStream_t stream) {
     if (configure_umma_instance<kSwiglu, kCluster, kWindows>(device) != cudaSuccess) return MT_ERR_LAUNCH;
@@ -1119,14 +1172,14 @@ inline int launch_umma_tables(const UmmaParams& params, int device, cudaStream_t
 }
 
 template <bool kSwiglu>
-inline int launch_umma_family(UmmaParams& params, cudaStream_t stream) {
+inline int launch_umma_family(UmmaParams& params, bool invariant, cudaStream_t stream) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return MT_ERR_DEVICE;
     const int kblocks = params.K / kUmmaBlockK;
     const int slots_total = (kblocks + kUmmaKBlocksPerSlot - 1) / kUmmaKBlocksPerSlot;
-    params.slices = umma_slices<kSwiglu>(params.N, slots_total, device);
     params.npad = 0;
-    umma_plan<kSwiglu>(params, slots_total, device);
+    if (invariant) umma_fixed_plan<kSwiglu>(params, slots_total, device);
+    else umma_plan<kSwiglu>(params, slots_total, device);
     if (params.npad == 0) return MT_ERR_LAUNCH;  // not even one CTA fits the device
     params.side_bytes = params.sum_bytes + (params.residual && params.ksplit == 1 ? kUmmaResidualBytes : 0);
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
@@ -1141,9 +1194,9 @@ struct AffineWeights {
     const uint16_t* biases;
 };
 
-// x [M,K] bf16, one weight triple (plain / residual) or two (gate, up -> SwiGLU).
+// x [M,K] bf16, one weight triple (plain / residual) or two (gate, up -> SwiGLU).  `invariant`: a row's bits do not depend on M.
 inline int launch_umma(const void* x, const AffineWeights* first, const AffineWeights* second, const void* residual,
-                       void* out, int M, int K, int N, cudaStream_t stream) {
+                       void* out, int M, int K, int N, bool invariant, cudaStream_t stream) {
     if (M < 1 || K % kUmmaBlockK || K < kUmmaBlockK || N < 1) return MT_ERR_SHAPE;
     if (!aligned_to(x, 16) || !aligned_to(first->w, 16) || (second && !aligned_to(second->w, 16))) return MT_ERR_ALIGN;
     const bool swiglu = second != nullptr;
@@ -1163,7 +1216,7 @@ inline int launch_umma(const void* x, const AffineWeights* first, const AffineWe
     const int box_rows = swiglu ? 64 : 128;
     if (!encode_weight_map(&params.w_map[0], first->w, K, N, box_rows)) return MT_ERR_LAUNCH;
     if (swiglu && !encode_weight_map(&params.w_map[1], second->w, K, N, box_rows)) return MT_ERR_LAUNCH;
-    return swiglu ? launch_umma_family<true>(params, stream) : launch_umma_family<false>(params, stream);
+    return swiglu ? launch_umma_family<true>(params, invariant, stream) : launch_umma_family<false>(params, invariant, stream);
 }
 
 }  // namespace mt

@@ -73,7 +73,7 @@ static int run_projection(const void* x, const AffineWeights& first, const Affin
         return second ? launch_gemv<true>(x, a, b, residual, out, M, K, N, sms, stream)
                       : launch_gemv<false>(x, a, b, residual, out, M, K, N, sms, stream);
     }
-    return launch_umma(x, &first, second, residual, out, M, K, N, stream);
+    return launch_umma(x, &first, second, residual, out, M, K, N, (flags & (MT_FLAG_FORCE_UMMA | MT_FLAG_FIXED_ORDER)) != 0, stream);
 }
 
 // C[M,N] = act(A[M,K] @ B[K,N]); a thread owns two adjacent output columns of kRows rows.
@@ -340,7 +340,8 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
     if (!device_is_sm100()) return MT_ERR_DEVICE;
     // A handful of rows: the whole MLP as one cooperative launch when the shape fits it.  Any flag
     // that pins a kernel family keeps the two-kernel path; MT_FLAG_MLP_FUSED insists on this one.
-    if (flags == 0 || (flags & (MT_FLAG_MLP_FUSED | MT_FLAG_MLP_FUSED_MMA))) {
+    const unsigned int family = flags & ~MT_FLAG_FIXED_ORDER;
+    if (family == 0 || (family & (MT_FLAG_MLP_FUSED | MT_FLAG_MLP_FUSED_MMA))) {
         if (!x || !gate_w || !gate_scales || !gate_biases || !up_w || !up_scales || !up_biases || !down_w ||
             !down_scales || !down_biases || !out)
             return MT_ERR_NULL;
@@ -368,17 +369,17 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         // the weights (against the tcgen05 pair, us at 2 to 8 rows: 1024 / 1024 7.6 | 9.3, 2048 / 4096 12.1 | 15.0, 1024 / 4096
         // 10.7 | 9.8, 2048 / 8192 18.6 | 18.1).
         const bool want_mma = (flags & MT_FLAG_MLP_FUSED_MMA) != 0;
-        const bool fma = !want_mma && (flags || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
-        const bool mma = !fma && (want_mma || (!flags && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
+        const bool fma = !want_mma && (family || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
+        const bool mma = !fma && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
         if (fma || mma) {
             const int fused_rc = launch_mlp_fused(params, sms, mma, static_cast<cudaStream_t>(stream));
             // A cooperative launch is refused when the whole grid cannot be resident (a GPU shared with
             // another context, a carve-out that leaves too little shared memory).  Nothing was queued:
             // the default dispatch then takes the two-kernel path; an explicit request reports it.
-            if (fused_rc != MT_ERR_LAUNCH || flags) return fused_rc;
+            if (fused_rc != MT_ERR_LAUNCH || family) return fused_rc;
             cudaGetLastError();
         }
-        if (flags) return MT_ERR_SHAPE;
+        if (family) return MT_ERR_SHAPE;
     }
     rc = mt_affine_swiglu(x, gate_w, gate_scales, gate_biases, up_w, up_scales, up_biases, workspace, M, H, I,
                           group_size, bits, flags, stream);
@@ -439,6 +440,7 @@ int mt_affine_mlp_host(const void* x_host, const void* residual_host, void* out_
 
 int mt_affine_mlp_launches(int M, int H, int I, unsigned int flags) {
     if (M <= 0) return 0;
+    flags &= ~MT_FLAG_FIXED_ORDER;
     if (flags != 0 && !(flags & (MT_FLAG_MLP_FUSED | MT_FLAG_MLP_FUSED_MMA))) return 2;
     FusedMlpParams params = {};
     params.M = M;

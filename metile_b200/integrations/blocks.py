@@ -54,8 +54,9 @@ class QuantizedLinear(nn.Module):
         return cls(*synth.affine_weight(seed, out_features, in_features, device))
 
     def forward(self, values):
-        out = backends.mlx_affine_qmv(values, self.weight, self.scales, self.biases,
-                                      group_size=self.group_size, bits=self.bits)
+        with backends.fixed_order():
+            out = backends.mlx_affine_qmv(values, self.weight, self.scales, self.biases,
+                                          group_size=self.group_size, bits=self.bits)
         return out if self.bias is None else out + self.bias
 
 

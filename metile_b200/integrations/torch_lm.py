@@ -204,7 +204,8 @@ def execute_quantized_mlp(module, values, residual=None):
             values, gate.weight, gate.scales, gate.biases, up.weight, up.scales, up.biases, down.weight,
             down.scales, down.biases, None)
         _executor_cache[module] = execute
-    return execute(values, residual)
+    with backends.fixed_order():
+        return execute(values, residual)
 
 
 _qkv_cache = weakref.WeakKeyDictionary()
@@ -259,6 +260,11 @@ def execute_attention_decode(module, values, cache, residual=None):
     """One decode step of an attention module without a framework op between its kernels:
     fused q|k|v projection, rotary embedding + cache append, attention over the cache, output
     projection (+ residual, added to the un-rounded sum).  values [B, 1, H]; returns [B, 1, H]."""
+    with backends.fixed_order():
+        return _attention_decode(module, values, cache, residual)
+
+
+def _attention_decode(module, values, cache, residual):
     batch = values.shape[0]
     heads, kv_heads, dim = module.heads, module.kv_heads, module.head_dim
     rows = values.reshape(batch, values.shape[-1])
@@ -331,8 +337,9 @@ def prompt_attention(norm, attention, values, cache):
         triples.append(triple)
     normed = backends.mlx_rms_norm(values, weight, eps)
     project = backends.mlx_affine_qmv
-    q, k, v = project(normed, *triples[0]), project(normed, *triples[1]), project(normed, *triples[2])
-    return project(attention.attend(q, k, v, cache), *triples[3])
+    with backends.fixed_order():
+        q, k, v = project(normed, *triples[0]), project(normed, *triples[1]), project(normed, *triples[2])
+        return project(attention.attend(q, k, v, cache), *triples[3])
 
 
 def _replace_forward(patch, cls, make_replacement):

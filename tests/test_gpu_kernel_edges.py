@@ -86,6 +86,37 @@ def test_tcgen05_projection_of_short_rows_over_many_tiles(cuda_device, rows, k, 
     assert _lib.device_status()[0]
 
 
+@pytest.mark.parametrize("rows,k,n", [
+    (2, 64, 5),           # one k-block
+    (16, 8192, 2048),     # four slices over clusters
+    (48, 1088, 700),      # slices of unequal length, unaligned tables
+    (65, 1536, 1003),     # two tiles of activations, odd rows
+    (128, 8960, 1536),    # five slices
+    (300, 2048, 2112),    # one slice, tiles of 112 rows
+])
+def test_tcgen05_sums_cut_for_the_rows_and_for_all(cuda_device, rows, k, n):
+    """A call on its own is cut as its rows need; within fixed_order() its bits are batch-invariant mode's."""
+    x = synth.activations(1, rows, k, cuda_device)
+    triple, other = synth.affine_weight(2, n, k, cuda_device), synth.affine_weight(4, n, k, cuda_device)
+    r = synth.activations(3, rows, n, cuda_device)
+    calls = [lambda: B.mlx_affine_qmv(x, *triple), lambda: B.mlx_affine_residual_qmv(x, *triple, r),
+             lambda: B.mlx_affine_swiglu(x, *triple, *other)]
+    own = [call() for call in calls]
+    with B.batch_invariant():
+        invariant = [call() for call in calls]
+    with B.fixed_order():
+        fixed = [call() for call in calls]
+    assert not B.kernel_pinned()
+    for a, b in zip(fixed, invariant):
+        assert_bit_equal(a, b, "fixed order")
+    weights, up = triple_np(triple), triple_np(other)
+    some = sorted({0, rows // 2, rows - 1})
+    for outputs in (own, fixed):
+        assert_within(outputs[0][some], A.qmm(f32(x[some]), *weights, weights="bf16"))
+        assert_within(outputs[1][some], A.qmm(f32(x[some]), *weights, residual=f32(r[some]), weights="bf16"))
+        assert_within(outputs[2][some], A.swiglu_fused(f32(x[some]), weights, up, weights="bf16"))
+
+
 @pytest.mark.parametrize("batch,steps,first,heads,kv_heads,dim", [
     (1, 1, 0, 1, 1, 2), (2, 7, 3, 3, 1, 20), (1, 130, 0, 6, 2, 64), (3, 33, 40, 4, 4, 128), (1, 2, 30000, 2, 1, 48),
 ])
