@@ -947,14 +947,12 @@ inline bool encode_weight_map_uncached(CUtensorMap* map, const void* base, int K
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-inline bool encode_activation_map(CUtensorMap* map, const void* base, int M, int K, int box_rows) {
-    const TensorMapKey key{base, M, K, box_rows, 1};
+template <typename Encode>
+inline bool remembered_tensor_map(CUtensorMap* map, const TensorMapKey& key, Encode&& encode) {
     TensorMapSlot& slot = tensor_map_slot(key);
     if (!(slot.valid && slot.key == key)) {
-        if (!encode_activation_map_uncached(&slot.map, base, M, K, box_rows)) {
-            slot.valid = false;
-            return false;
-        }
+        slot.valid = false;
+        if (!encode(&slot.map)) return false;
         slot.key = key;
         slot.valid = true;
     }
@@ -962,19 +960,14 @@ inline bool encode_activation_map(CUtensorMap* map, const void* base, int M, int
     return true;
 }
 
+inline bool encode_activation_map(CUtensorMap* map, const void* base, int M, int K, int box_rows) {
+    return remembered_tensor_map(map, TensorMapKey{base, M, K, box_rows, 1},
+                                 [&](CUtensorMap* to) { return encode_activation_map_uncached(to, base, M, K, box_rows); });
+}
+
 inline bool encode_weight_map(CUtensorMap* map, const void* base, int K, int N, int box_rows = kUmmaTileRows) {
-    const TensorMapKey key{base, K, N, box_rows, 2};
-    TensorMapSlot& slot = tensor_map_slot(key);
-    if (!(slot.valid && slot.key == key)) {
-        if (!encode_weight_map_uncached(&slot.map, base, K, N, box_rows)) {
-            slot.valid = false;
-            return false;
-        }
-        slot.key = key;
-        slot.valid = true;
-    }
-    *map = slot.map;
-    return true;
+    return remembered_tensor_map(map, TensorMapKey{base, K, N, box_rows, 2},
+                                 [&](CUtensorMap* to) { return encode_weight_map_uncached(to, base, K, N, box_rows); });
 }
 
 template <bool kSwiglu, bool kCluster, bool kWindows>

@@ -6,6 +6,7 @@
 #include "attention_decode.cuh"
 #include "peer_reduce.cuh"
 #include "affine_gemv.cuh"
+#include "affine_gemv_mma.cuh"
 #include "affine_umma.cuh"
 #include "affine_mlp_fused.cuh"
 #include <string.h>
@@ -70,6 +71,12 @@ static int run_projection(const void* x, const AffineWeights& first, const Affin
         if (M > 8) return MT_ERR_SHAPE;
         GemvWeights a{first.w, first.scales, first.biases};
         GemvWeights b = second ? GemvWeights{second->w, second->scales, second->biases} : a;
+        // One row of a call that asks for no order of its own.
+        OneRowPlan plan;
+        if (M == 1 && !(flags & (MT_FLAG_FORCE_GEMV | MT_FLAG_FIXED_ORDER)) && one_row_applicable(a, b, K, N, second != nullptr) &&
+            one_row_plan(plan, K, N, second != nullptr, sms))
+            return second ? launch_one_row<true>(x, a, b, residual, out, K, N, plan, stream)
+                          : launch_one_row<false>(x, a, b, residual, out, K, N, plan, stream);
         return second ? launch_gemv<true>(x, a, b, residual, out, M, K, N, sms, stream)
                       : launch_gemv<false>(x, a, b, residual, out, M, K, N, sms, stream);
     }

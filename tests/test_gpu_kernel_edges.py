@@ -117,6 +117,43 @@ def test_tcgen05_sums_cut_for_the_rows_and_for_all(cuda_device, rows, k, n):
         assert_within(outputs[2][some], A.swiglu_fused(f32(x[some]), weights, up, weights="bf16"))
 
 
+@pytest.mark.parametrize("k,n", [
+    (512, 16401),         # one item per row; a last tile of one row, whose tables end within sixteen bytes
+    (704, 16001),         # items of eight and of three groups
+    (1536, 5500),         # three items over three warps
+    (2048, 40000),        # several tiles per team
+    (2560, 6007),         # five items over four warps
+    (4096, 11100),        # eight items
+    (14336, 4840),        # a long K range, beyond the rings of the CUDA-core form
+])
+def test_one_row_on_warp_mma(cuda_device, k, n):
+    """The default form of one row against the CUDA-core form (both keep the weights exact) and the oracle."""
+    x, r = synth.activations(1, 1, k, cuda_device), synth.activations(3, 1, n, cuda_device)
+    triple, other = synth.affine_weight(2, n, k, cuda_device), synth.affine_weight(4, n, k, cuda_device)
+    odd = torch.empty(n + 1, dtype=r.dtype, device=r.device)[1:].view_as(r).copy_(r)
+    calls = [lambda: B.mlx_affine_qmv(x, *triple), lambda: B.mlx_affine_residual_qmv(x, *triple, r),
+             lambda: B.mlx_affine_swiglu(x, *triple, *other)]
+    own = [call() for call in calls]
+    for a, b in zip(own, [call() for call in calls]):
+        assert_bit_equal(a, b, "twice")
+    assert_bit_equal(B.mlx_affine_residual_qmv(x, *triple, odd), own[1], "a residual at an odd address")
+    with B.force_kernel("gemv"):
+        cores = [call() for call in calls]
+    with B.fixed_order():
+        for a, b in zip([call() for call in calls], cores):
+            assert_bit_equal(a, b, "a model's call")
+    # Tables that do not start at sixteen bytes are served by the CUDA-core form.
+    shifted = [torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view_as(t).copy_(t) for t in triple[1:]]
+    assert_bit_equal(B.mlx_affine_qmv(x, triple[0], *shifted), cores[0], "tables at odd addresses")
+    for a, b in zip(own, cores):
+        assert_within(a, f32(b), rel=1e-5)  # fp32 sums of the same products in two orders, one rounding each
+    weights = triple_np(triple)
+    assert_within(own[0], A.qmm(f32(x), *weights))
+    assert_within(own[1], A.qmm(f32(x), *weights, residual=f32(r)))
+    assert_within(own[2], A.swiglu_fused(f32(x), weights, triple_np(other)))
+    assert _lib.device_status()[0]
+
+
 @pytest.mark.parametrize("batch,steps,first,heads,kv_heads,dim", [
     (1, 1, 0, 1, 1, 2), (2, 7, 3, 3, 1, 20), (1, 130, 0, 6, 2, 64), (3, 33, 40, 4, 4, 128), (1, 2, 30000, 2, 1, 48),
 ])
