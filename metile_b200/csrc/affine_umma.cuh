@@ -1094,18 +1094,18 @@ inline void umma_fixed_plan(UmmaParams& p, int slots_total, int device) {
 // Where nothing ties a row's bits to other row counts: a plain projection has one chain too, so that the accumulators of two
 // tiles of 128 rows find room and finishing one overlaps the next (in two chains 8192 -> 2048 at 2000 rows took 83 us, now
 // 57), and the K range is cut into as many slices as pay for these rows, a CTA each.  Costs in SM cycles at 1.9 GHz, fitted to
-// every such split at fourteen shapes and ten row counts from 16 to 2000 in replayed graphs (what the model picks takes 0.5 %
-// longer than the best split on average, 8 % at most):
+// every such split at fourteen shapes and ten row counts from 16 to 2000 in replayed graphs, and to the down projection's in
+// eleven MLPs of 9 to 400 rows (what the model picks takes 0.5 and 1.2 % longer than the best split on average, 9 % at most):
 //   ring slot (four k-blocks)   923 + 3.2 per row on a nearly idle chip, 12.5 per row with every SM at work; never below the
 //                               weights at 4 TB/s
-//   CTAs                        3.5 each; 2165 where they are more than half of the SMs, for then the next kernel's find
-//                               no SM to start on (8192 -> 2048, 16 rows: 64 CTAs 6.6 us, 80 CTAs 7.9)
+//   CTAs                        3.5 each; 2165 where they find no SMs to start on beside the kernel in front, another like
+//                               this one (8192 -> 2048, 16 rows: 64 CTAs 6.6 us, 80 CTAs 7.9) or the MLP's gate|up (1088
+//                               / 4096, nine rows, 64 CTAs in front: 72 CTAs 9.6 us, 45 CTAs 10.5)
 //   finishing a tile            55 per row, 4 behind another tile
-//   cluster                     1180, 64 per row; 8800 + 35 per row for a wave after the first (it is not persistent).
-//                               More than five CTAs never paid
+//   cluster                     1180, 64 per row; 8800 + 35 per row for a wave after the first (it is not persistent)
 template <bool kSwiglu>
-inline void umma_plan(UmmaParams& p, int slots_total, int device) {
-    constexpr int kMostSlices = 5;
+inline void umma_plan(UmmaParams& p, int slots_total, int ctas_before, int device) {
+    constexpr int kMostSlices = 8;
     const int sms = umma_active_clusters<kSwiglu>(1, device);  // with room for a CTA
     if (sms <= 0) return;
     const double weights = (double)p.N * p.K * (kSwiglu ? 2 : 1) * (0.5625 / 2120.0);
@@ -1121,7 +1121,8 @@ inline void umma_plan(UmmaParams& p, int slots_total, int device) {
             if (active <= 0) continue;
             const long waves = (tiles + active - 1) / active, ctas = std::min(tiles, (long)active) * P;
             const double slot = busy > idle ? idle + (busy - idle) * ctas / sms : idle;
-            double cost = std::max((double)waves * ((slots_total + P - 1) / P) * slot, weights) + 3.5 * ctas + (2 * ctas > sms ? 2165 : 0);
+            double cost = std::max((double)waves * ((slots_total + P - 1) / P) * slot, weights) + 3.5 * ctas;
+            if (ctas_before ? ctas_before + ctas > sms : 2 * tiles > active) cost += 2165;
             if (P > 1) cost += 1180 + 64.0 * npad + (waves - 1) * (8800 + 35.0 * npad);
             else cost += 55.0 * npad + (waves - 1) * 4.4 * npad;
             if (best_cost >= 0 && cost >= best_cost) continue;
@@ -1165,15 +1166,16 @@ inline int launch_umma_tables(const UmmaParams& params, int device, cudaStream_t
 }
 
 template <bool kSwiglu>
-inline int launch_umma_family(UmmaParams& params, bool invariant, cudaStream_t stream) {
+inline int launch_umma_family(UmmaParams& params, bool invariant, int* ctas, cudaStream_t stream) {
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) return MT_ERR_DEVICE;
     const int kblocks = params.K / kUmmaBlockK;
     const int slots_total = (kblocks + kUmmaKBlocksPerSlot - 1) / kUmmaKBlocksPerSlot;
     params.npad = 0;
     if (invariant) umma_fixed_plan<kSwiglu>(params, slots_total, device);
-    else umma_plan<kSwiglu>(params, slots_total, device);
+    else umma_plan<kSwiglu>(params, slots_total, ctas ? *ctas : 0, device);
     if (params.npad == 0) return MT_ERR_LAUNCH;  // not even one CTA fits the device
+    if (ctas) *ctas = std::min(params.row_tiles * params.act_tiles, umma_active_clusters<kSwiglu>(1, device)) * params.ksplit;
     params.side_bytes = params.sum_bytes + (params.residual && params.ksplit == 1 ? kUmmaResidualBytes : 0);
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
     bool windows = kblocks % 4 != 0;
@@ -1188,8 +1190,9 @@ struct AffineWeights {
 };
 
 // x [M,K] bf16, one weight triple (plain / residual) or two (gate, up -> SwiGLU).  `invariant`: a row's bits do not depend on M.
+// `ctas`, where given: CTAs of the kernel in front (0: unknown) before, of this one after.
 inline int launch_umma(const void* x, const AffineWeights* first, const AffineWeights* second, const void* residual,
-                       void* out, int M, int K, int N, bool invariant, cudaStream_t stream) {
+                       void* out, int M, int K, int N, bool invariant, int* ctas, cudaStream_t stream) {
     if (M < 1 || K % kUmmaBlockK || K < kUmmaBlockK || N < 1) return MT_ERR_SHAPE;
     if (!aligned_to(x, 16) || !aligned_to(first->w, 16) || (second && !aligned_to(second->w, 16))) return MT_ERR_ALIGN;
     const bool swiglu = second != nullptr;
@@ -1209,7 +1212,7 @@ inline int launch_umma(const void* x, const AffineWeights* first, const AffineWe
     const int box_rows = swiglu ? 64 : 128;
     if (!encode_weight_map(&params.w_map[0], first->w, K, N, box_rows)) return MT_ERR_LAUNCH;
     if (swiglu && !encode_weight_map(&params.w_map[1], second->w, K, N, box_rows)) return MT_ERR_LAUNCH;
-    return swiglu ? launch_umma_family<true>(params, invariant, stream) : launch_umma_family<false>(params, invariant, stream);
+    return swiglu ? launch_umma_family<true>(params, invariant, ctas, stream) : launch_umma_family<false>(params, invariant, ctas, stream);
 }
 
 }  // namespace mt

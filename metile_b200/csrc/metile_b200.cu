@@ -63,7 +63,7 @@ static bool use_gemv(int M, unsigned int flags) {
 }
 
 static int run_projection(const void* x, const AffineWeights& first, const AffineWeights* second, const void* residual,
-                          void* out, int M, int K, int N, unsigned int flags, cudaStream_t stream) {
+                          void* out, int M, int K, int N, unsigned int flags, cudaStream_t stream, int* ctas = nullptr) {
     const int sms = device_sm_count();
     if (sms <= 0) return MT_ERR_DEVICE;
     if (M == 0) return MT_OK;
@@ -80,7 +80,7 @@ static int run_projection(const void* x, const AffineWeights& first, const Affin
         return second ? launch_gemv<true>(x, a, b, residual, out, M, K, N, sms, stream)
                       : launch_gemv<false>(x, a, b, residual, out, M, K, N, sms, stream);
     }
-    return launch_umma(x, &first, second, residual, out, M, K, N, (flags & (MT_FLAG_FORCE_UMMA | MT_FLAG_FIXED_ORDER)) != 0, stream);
+    return launch_umma(x, &first, second, residual, out, M, K, N, (flags & (MT_FLAG_FORCE_UMMA | MT_FLAG_FIXED_ORDER)) != 0, ctas, stream);
 }
 
 // C[M,N] = act(A[M,K] @ B[K,N]); a thread owns two adjacent output columns of kRows rows.
@@ -388,11 +388,14 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         }
         if (family) return MT_ERR_SHAPE;
     }
-    rc = mt_affine_swiglu(x, gate_w, gate_scales, gate_biases, up_w, up_scales, up_biases, workspace, M, H, I,
-                          group_size, bits, flags, stream);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const AffineWeights gate{gate_w, static_cast<const uint16_t*>(gate_scales), static_cast<const uint16_t*>(gate_biases)};
+    const AffineWeights up{up_w, static_cast<const uint16_t*>(up_scales), static_cast<const uint16_t*>(up_biases)};
+    const AffineWeights down{down_w, static_cast<const uint16_t*>(down_scales), static_cast<const uint16_t*>(down_biases)};
+    int ctas = 0;  // of gate|up, for the down projection behind it
+    rc = run_projection(x, gate, &up, nullptr, workspace, M, H, I, flags, s, &ctas);
     if (rc != MT_OK) return rc;
-    return mt_affine_qmv(workspace, down_w, down_scales, down_biases, residual, out, M, I, H, group_size, bits, flags,
-                         stream);
+    return run_projection(workspace, down, nullptr, residual, out, M, I, H, flags, s, &ctas);
 }
 
 int mt_affine_mlp_host(const void* x_host, const void* residual_host, void* out_host, void* x_device,
