@@ -79,6 +79,10 @@ constexpr int kUmmaResidualPitch = 272;              // bytes of a residual row:
 constexpr int kUmmaResidualSteps = 4;                // steps of sixteen rows whose residuals are in flight
 constexpr int kUmmaResidualBytes = kUmmaResidualSteps * 16 * kUmmaResidualPitch;
 constexpr int kUmmaSmemBytes = 227 * 1024;           // one CTA per SM, whatever the row count
+// With few rows the kernel is as long as its start and its neighbours': a norm, a rotary embedding or a merge of attention splits
+// finds room beside a CTA of 192 KB and 72 registers a thread (see the launch bounds), so that they overlap (decoding sixteen
+// sequences of a four-block model, eight tokens: 1929 us with 227 KB and 80 registers, 1875 with 192 KB, 1843 with both).
+__host__ __device__ constexpr int umma_smem_bytes(int npad) { return npad > 32 ? kUmmaSmemBytes : 192 * 1024; }
 constexpr int kUmmaTmemCols = 512;                   // 256 accumulator columns, 2 x 128 operand columns
 constexpr int kUmmaAColumn = 256;
 
@@ -90,7 +94,7 @@ __host__ __device__ constexpr int umma_x_slots(int npad, bool windows, int side_
 // three more table entries than slots (see UmmaTables).
 __host__ __device__ constexpr int umma_ring_slots(int npad, bool windows, int side_bytes) {
     const int x_bytes = umma_x_slots(npad, windows, side_bytes) * 2 * npad * 128;
-    const int left = kUmmaSmemBytes - 1024 - kUmmaBarrierBytes - kUmmaOutBytes - side_bytes - x_bytes - (windows ? 3 * kUmmaTableBytes : 0);
+    const int left = umma_smem_bytes(npad) - 1024 - kUmmaBarrierBytes - kUmmaOutBytes - side_bytes - x_bytes - (windows ? 3 * kUmmaTableBytes : 0);
     const int slots = left / (kUmmaSlotBytes + kUmmaTableBytes);
     return slots > kUmmaMaxSlots ? kUmmaMaxSlots : slots > 3 ? slots & ~1 : slots;  // even where there is a choice
 }
@@ -363,8 +367,9 @@ __device__ __forceinline__ void umma_finish_rows(const UmmaParams& p, const Umma
 // kWindows: the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables).  A kernel of its own,
 // because every instruction that the dequantising warps do not issue counts: with the layout as a run-time condition 512
 // rows 1536 -> 8960, gate|up, took 37.6 us, now 34.0; 2000 rows 2048 -> 8192 153, now 144; 16 rows 8192 -> 2048 8.5, now 8.2.
+// The bounds: 72 registers a thread instead of 80 where the kernel has no use for more; with windows it loses 2 to 3 % by it.
 template <bool kSwiglu, bool kCluster, bool kWindows>
-__global__ void __launch_bounds__(kUmmaThreads, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
+__global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
     constexpr int kOut = kSwiglu ? 64 : 128;  // outputs per tile
     extern __shared__ uint8_t smem_raw[];
     // Aligned by offsetting the array itself (not by rounding a generic address), so that the compiler
@@ -1143,7 +1148,7 @@ inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, 
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(ctas, 1, 1);
     config.blockDim = dim3(kUmmaThreads, 1, 1);
-    config.dynamicSmemBytes = kUmmaSmemBytes;
+    config.dynamicSmemBytes = umma_smem_bytes(params.npad);
     config.stream = stream;
     cudaLaunchAttribute attrs[2];
     attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
