@@ -227,6 +227,10 @@ int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long 
 #define MT_GREEDY_MAX_VOCABULARY 0x7FFFBFFF
 int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream);
 
+/* out[r] = table[index[r]]: rows of `width` bf16 (a multiple of 8), table [table_rows, width], out [rows, width], both
+ * 16-byte aligned (else -2).  An index outside the table gives a row of NaN. */
+int mt_gather_rows(const void* table, const long long* index, void* out, int rows, long long table_rows, int width, void* stream);
+
 /* The same for the `steps` tokens of a prompt, which go to rows first, first + 1, ... of every cache.
  * q: dense bf16 [batch, steps, q_heads, head_dim], k, v: [batch, steps, kv_heads, head_dim]; q_out like q;
  * inverse: fp32 [head_dim / 2] on the device, the angle of pair i is position * inverse[i] in fp32; products,

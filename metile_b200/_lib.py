@@ -49,6 +49,7 @@ SIGNATURES = {
     "mt_attention_decode": (_i, [_p, _p, _p, _p, _p, _p, _z, _i, _i, _i, _i, _i, _i, _f, _p]),
     "mt_rope_kv_append_advance": (_i, [_p, _p, _p, ctypes.c_longlong, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _p]),
     "mt_greedy_token": (_i, [_p, _p, _p, _i, _i, _p]),
+    "mt_gather_rows": (_i, [_p, _p, _p, _i, ctypes.c_longlong, _i, _p]),
     "mt_rope_kv_prefill": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p]),
     "mt_rope_kv_append": (_i, [_p, _p, _p, ctypes.c_longlong, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _p]),
     "mt_peer_group_create": (_i, [_i, _i, _z, ctypes.POINTER(ctypes.c_void_p), _p]),

@@ -4,6 +4,7 @@ from .cuda import (  # noqa: F401
     mlx_add_rms_norm,
     mlx_attention_decode,
     mlx_rms_norm,
+    embedding,
     greedy_token,
     rope_kv_append,
     rope_kv_prefill,

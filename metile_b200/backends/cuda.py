@@ -216,6 +216,13 @@ def greedy_token(logits, tokens):
     return out
 
 
+def embedding(tokens, table):
+    """table[tokens] for int64 tokens of any shape and a bfloat16 table [V, H]; None, and nothing done, unless both are dense
+    tensors on one CUDA device that no gradient is asked for.  A token outside the table gives NaN."""
+    out = native().embedding(tokens, table)
+    return None if out is None else native_result(out, "embedding")
+
+
 def rope_kv_prefill(query, key, value, inverse, positions, first, key_cache, value_cache, *, only_native=False):
     """Rotate the query and key rows of a prompt and write key and value to the caches, in place.
 

@@ -20,6 +20,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/core/GradMode.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -409,6 +410,28 @@ PyObject* greedy_token(PyObject* const* args) {
     return code_or(code, std::move(out));
 }
 
+// embedding(tokens int64 [...], table [V, H] bf16) -> [..., H]
+PyObject* embedding(PyObject* const* args) {
+    const Tensor *tokens = plain(args[0]), *table = plain(args[1]);
+    if (!tokens || !table || !table->is_cuda() || table->dim() != 2 || (table->requires_grad() && c10::GradMode::is_enabled())) Py_RETURN_NONE;
+    const auto device = table->device();
+    const int64_t rows = tokens->numel(), width = table->size(1);
+    if (!bf16_on(*table, device) || tokens->device() != device || tokens->scalar_type() != at::kLong || !tokens->is_contiguous() ||
+        rows < 1 || !fits_int(rows) || width < 8 || width % 8 || !fits_int(width) || reinterpret_cast<uintptr_t>(address(*table)) % 16)
+        Py_RETURN_NONE;
+    const Launch launch(device);
+    c10::SmallVector<int64_t, 6> sizes(tokens->sizes().begin(), tokens->sizes().end());
+    sizes.push_back(width);
+    Tensor out = new_bf16(sizes, device);
+    int code;
+    {
+        const Unlocked unlocked;
+        code = mt_gather_rows(address(*table), static_cast<const long long*>(address(*tokens)), address(out), (int)rows, table->size(0), (int)width,
+                              launch.stream());
+    }
+    return code_or(code, std::move(out));
+}
+
 template <PyObject* (*kBody)(PyObject* const*), Py_ssize_t kCount>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t count) {
     try {
@@ -424,7 +447,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t count) {
     {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(entry<name, count>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {MT_METHOD(project, 8), MT_METHOD(swiglu, 8), MT_METHOD(mlp_plan, 9), MT_METHOD(mlp, 4), MT_METHOD(norm, 4),
                          MT_METHOD(dense, 4), MT_METHOD(attention, 5), MT_METHOD(rope_kv_append, 8), MT_METHOD(rope_kv_prefill, 8),
-                         MT_METHOD(greedy_token, 2), {nullptr, nullptr, 0, nullptr}};
+                         MT_METHOD(greedy_token, 2), MT_METHOD(embedding, 2), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -9,6 +9,7 @@
 #include "affine_gemv_mma.cuh"
 #include "affine_umma.cuh"
 #include "affine_mlp_fused.cuh"
+#include "gather_rows.cuh"
 #include <string.h>
 
 #include "common.cuh"
@@ -616,6 +617,14 @@ int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows,
     const cudaError_t rc = vector ? cudaLaunchKernelEx(&config, greedy_token_kernel<true>, params)
                                   : cudaLaunchKernelEx(&config, greedy_token_kernel<false>, params);
     return rc == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+}
+
+int mt_gather_rows(const void* table, const long long* index, void* out, int rows, long long table_rows, int width, void* stream) {
+    if (rows < 0 || table_rows < 1 || width < 1) return MT_ERR_SHAPE;
+    if (rows == 0) return MT_OK;
+    if (!table || !index || !out) return MT_ERR_NULL;
+    if (!device_is_sm100()) return MT_ERR_DEVICE;
+    return launch_gather_rows(table, index, out, rows, table_rows, width, static_cast<cudaStream_t>(stream));
 }
 
 int mt_rope_kv_prefill(const void* q, const void* k, const void* v, const float* inverse, void* q_out, void* k_cache,

@@ -348,3 +348,38 @@ def test_what_the_native_calls_do_not_take_the_general_forms_do(cuda_device):
     # Logits of another type.
     logits, tokens = torch.randn(3, 50, device=cuda_device), torch.zeros(3, 1, dtype=torch.long, device=cuda_device)
     assert torch.equal(B.greedy_token(logits, tokens), logits) and (tokens == logits.argmax(-1, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("rows,width,vocab", [(1, 8, 1), (16, 1536, 1000), (17, 2056, 7), (700, 512, 300)])
+def test_embedding_rows(cuda_device, rows, width, vocab):
+    table = synth.activations(1, vocab, width, cuda_device)
+    tokens = torch.randint(0, vocab, (rows, 1), device=cuda_device)
+    assert_bit_equal(B.embedding(tokens, table), torch.nn.functional.embedding(tokens, table), "rows")
+    outside = tokens.clone()
+    outside[0], outside[-1] = -1, vocab
+    found = B.embedding(outside, table)
+    assert found[0].isnan().all() and found[-1].isnan().all()
+    for other in (tokens.int(), tokens.expand(rows, 2)[:, ::2].T, tokens.cpu()):
+        if other.dtype != torch.int64 or not other.is_contiguous() or not other.is_cuda:
+            assert B.embedding(other, table) is None
+    assert B.embedding(tokens, table.float()) is None and B.embedding(tokens[:0], table) is None
+    assert B.embedding(tokens, table.clone().requires_grad_()) is None
+
+
+@pytest.mark.parametrize("change", [
+    lambda e: None,
+    lambda e: e.register_forward_hook(lambda module, args, out: 2 * out),
+    lambda e: setattr(e, "forward", lambda tokens: 3 * torch.nn.functional.embedding(tokens, e.weight)),
+    lambda e: setattr(e, "max_norm", 0.5),
+    lambda e: e.weight.requires_grad_(),
+    lambda e: setattr(e, "weight", torch.nn.Parameter(e.weight.float(), requires_grad=False)),
+])
+def test_a_model_embeds_as_its_module_does(cuda_device, change):
+    from metile_b200.integrations import blocks
+
+    modules = [torch.nn.Embedding.from_pretrained(synth.activations(1, 50, 64, cuda_device), freeze=True) for _ in range(2)]
+    for module in modules:  # a look-up with max_norm changes the table
+        change(module)
+    tokens = torch.randint(0, 50, (3, 4), device=cuda_device)
+    found, wanted = blocks._embed(modules[0], tokens), modules[1](tokens)
+    assert found.dtype == wanted.dtype and torch.equal(found, wanted) and found.requires_grad == wanted.requires_grad
