@@ -311,13 +311,13 @@ __device__ __forceinline__ void umma_read16(uint32_t acc, uint32_t acc2, bool se
 // 15000-cycle launch at 16 rows, 8192 -> 2048.)
 __device__ __forceinline__ int umma_rows_per_cta(const UmmaParams& p) { return (p.npad + p.ksplit - 1) / p.ksplit; }
 
-template <bool kSwiglu>
+template <bool kSwiglu, bool kTwo>
 __device__ __forceinline__ void umma_push_slices(const UmmaParams& p, const UmmaShare& w, uint32_t staging, uint32_t tmem, uint32_t unit_cols,
                                                  int rows, int thread) {
     const int rows_per_cta = umma_rows_per_cta(p);
     for (int s = w.slice_begin; s < w.slice_end; ++s) {
         const uint32_t acc = tmem + (uint32_t)(s - w.slice_begin) * unit_cols;
-        const bool second = !kSwiglu && p.chains == 2 && umma_slice_has_second(w, s);
+        const bool second = kTwo && umma_slice_has_second(w, s);
         uint32_t at = staging + 4u * (uint32_t)(s * rows_per_cta * kUmmaTileRows + thread);  // row / ksplit = 0
         int owner = 0;
         for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -367,9 +367,11 @@ __device__ __forceinline__ void umma_finish_rows(const UmmaParams& p, const Umma
 // kWindows: the four scales (biases) of a slot are not one aligned 8-byte vector (see UmmaTables).  A kernel of its own,
 // because every instruction that the dequantising warps do not issue counts: with the layout as a run-time condition 512
 // rows 1536 -> 8960, gate|up, took 37.6 us, now 34.0; 2000 rows 2048 -> 8192 153, now 144; 16 rows 8192 -> 2048 8.5, now 8.2.
-// The bounds: 72 registers a thread instead of 80 where the kernel has no use for more; with windows it loses 2 to 3 % by it.
-template <bool kSwiglu, bool kCluster, bool kWindows>
-__global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
+// kFew: 72 registers a thread instead of 80, for up to 32 rows (umma_smem_bytes).  With windows a launch loses 2 to 3 % by it.
+// kTwo: two chains per slice.  As a run-time condition it cost launches at 512 rows 2 % (the 24 of a prompt through four blocks, with
+// the bounds of kFew: 3.5 us of 548).
+template <bool kSwiglu, bool kCluster, bool kWindows, bool kFew, bool kTwo>
+__global__ void __launch_bounds__(kFew ? kUmmaThreads + 128 : kUmmaThreads, 1) affine_umma_kernel(const __grid_constant__ UmmaParams p) {
     constexpr int kOut = kSwiglu ? 64 : 128;  // outputs per tile
     extern __shared__ uint8_t smem_raw[];
     // Aligned by offsetting the array itself (not by rounding a generic address), so that the compiler
@@ -403,7 +405,6 @@ __global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 
     const int lane = threadIdx.x & 31;
     // Accumulator units: one slice's sums, in one chain or in two halves of the unit.
     const uint32_t unit_mask = (1u << p.unit_shift) - 1u, unit_cols = (uint32_t)kUmmaAColumn >> p.unit_shift;
-    const bool two_chains = !kSwiglu && p.chains == 2;
     const uint32_t second_col = unit_cols >> 1;
 
     if (threadIdx.x == 0) {
@@ -546,8 +547,8 @@ __global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 
                             if (kb >= valid) break;
                             const int x_slot = kb < 2 ? first.slot : second.slot;
                             const uint64_t b_desc = desc0 + (uint64_t)((x_slot * x_slot_bytes + (kb & 1) * npad * 128) >> 4);
-                            const uint32_t d = two_chains && kb >= 2 ? d_tmem + second_col : d_tmem;
-                            const bool starts = st == begin && (kb == 0 || (kb == 2 && two_chains));
+                            const uint32_t d = kTwo && kb >= 2 ? d_tmem + second_col : d_tmem;
+                            const bool starts = st == begin && (kb == 0 || (kb == 2 && kTwo));
 #pragma unroll
                             for (int ks = 0; ks < kUmmaBlockK / 16; ++ks)  // the first MMA into an accumulator overwrites it
                                 ptx::umma_ts(d, a_tmem + kb * 32 + ks * 8, b_desc + (uint64_t)(ks * 2), idesc, starts && ks == 0 ? 0u : 1u);
@@ -640,7 +641,7 @@ __global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 
                 for (int s = 0; s < my_slices - direct; ++s, ++q) {
                     if (!wait_unit(q)) break;
                     const uint32_t acc = unit_address(q);
-                    const bool second = two_chains && umma_slice_has_second(w, s);
+                    const bool second = kTwo && umma_slice_has_second(w, s);
                     for (int c0 = 0; c0 < rows; c0 += 16) {
                         float v[16];
                         umma_read16(acc + c0, acc + c0 + second_col, second, v);
@@ -662,7 +663,7 @@ __global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 
                 // gate|up's two slices.
                 if (!wait_unit(q) || (direct == 2 && !wait_unit(q + 1))) break;
                 const uint32_t acc = unit_address(q);
-                const bool second = kSwiglu ? direct == 2 : two_chains && umma_slice_has_second(w, w.slice_end - 1);
+                const bool second = kSwiglu ? direct == 2 : kTwo && umma_slice_has_second(w, w.slice_end - 1);
                 const uint32_t acc2 = kSwiglu ? unit_address(q + 1) : acc + second_col;
                 const bool earlier = my_slices > direct;
                 // Sixteen activation rows at a time through shared memory, so that an output row leaves as 16-byte
@@ -867,7 +868,7 @@ __global__ void __launch_bounds__(kWindows ? kUmmaThreads : kUmmaThreads + 128, 
             ptx::cluster_wait();
         }
         if (warp >= kUmmaEpilogueWarp && !*abort_flag)
-            umma_push_slices<kSwiglu>(p, w, ptx::smem_u32(staging), tmem_base + ((uint32_t)((warp & 3) * 32) << 16), unit_cols, rows,
+            umma_push_slices<kSwiglu, kTwo>(p, w, ptx::smem_u32(staging), tmem_base + ((uint32_t)((warp & 3) * 32) << 16), unit_cols, rows,
                                       (warp & 3) * 32 + lane);
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -975,11 +976,11 @@ inline bool encode_weight_map(CUtensorMap* map, const void* base, int K, int N, 
                                  [&](CUtensorMap* to) { return encode_weight_map_uncached(to, base, K, N, box_rows); });
 }
 
-template <bool kSwiglu, bool kCluster, bool kWindows>
+template <bool kSwiglu, bool kCluster, bool kWindows, bool kFew, bool kTwo>
 inline cudaError_t configure_umma_instance(int device) {
     static bool configured[64] = {};
     if (device < 64 && configured[device]) return cudaSuccess;
-    const cudaError_t rc = cudaFuncSetAttribute(affine_umma_kernel<kSwiglu, kCluster, kWindows>,
+    const cudaError_t rc = cudaFuncSetAttribute(affine_umma_kernel<kSwiglu, kCluster, kWindows, kFew, kTwo>,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaSmemBytes);
     if (rc == cudaSuccess && device < 64) configured[device] = true;
     return rc;
@@ -990,7 +991,7 @@ template <bool kSwiglu>
 inline int umma_active_clusters(int size, int device) {
     static int cached[64][9] = {};
     if (device < 64 && cached[device][size]) return cached[device][size];
-    if (configure_umma_instance<kSwiglu, true, false>(device) != cudaSuccess) return 0;
+    if (configure_umma_instance<kSwiglu, true, false, false, !kSwiglu>(device) != cudaSuccess) return 0;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(size * 64, 1, 1);
     config.blockDim = dim3(kUmmaThreads, 1, 1);
@@ -1003,7 +1004,7 @@ inline int umma_active_clusters(int size, int device) {
     config.attrs = attrs;
     config.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, affine_umma_kernel<kSwiglu, true, false>, &config) != cudaSuccess) clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, affine_umma_kernel<kSwiglu, true, false, false, !kSwiglu>, &config) != cudaSuccess) clusters = 0;
     if (device < 64) cached[device][size] = clusters > 0 ? clusters : -1;
     return clusters;
 }
@@ -1142,9 +1143,9 @@ inline void umma_plan(UmmaParams& p, int slots_total, int ctas_before, int devic
     }
 }
 
-template <bool kSwiglu, bool kCluster, bool kWindows>
+template <bool kSwiglu, bool kCluster, bool kWindows, bool kFew, bool kTwo>
 inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, cudaStream_t stream) {
-    if (configure_umma_instance<kSwiglu, kCluster, kWindows>(device) != cudaSuccess) return MT_ERR_LAUNCH;
+    if (configure_umma_instance<kSwiglu, kCluster, kWindows, kFew, kTwo>(device) != cudaSuccess) return MT_ERR_LAUNCH;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(ctas, 1, 1);
     config.blockDim = dim3(kUmmaThreads, 1, 1);
@@ -1159,15 +1160,22 @@ inline int launch_umma_instance(const UmmaParams& params, int ctas, int device, 
     attrs[1].val.clusterDim.z = 1;
     config.attrs = attrs;
     config.numAttrs = kCluster ? 2 : 1;
-    return cudaLaunchKernelEx(&config, affine_umma_kernel<kSwiglu, kCluster, kWindows>, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&config, affine_umma_kernel<kSwiglu, kCluster, kWindows, kFew, kTwo>, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
-template <bool kSwiglu, bool kWindows>
+template <bool kSwiglu, bool kWindows, bool kFew, bool kTwo>
 inline int launch_umma_tables(const UmmaParams& params, int device, cudaStream_t stream) {
     const int tiles = params.row_tiles * params.act_tiles;
-    if (params.ksplit > 1) return launch_umma_instance<kSwiglu, true, kWindows>(params, tiles * params.ksplit, device, stream);
+    if (params.ksplit > 1) return launch_umma_instance<kSwiglu, true, kWindows, kFew, kTwo>(params, tiles * params.ksplit, device, stream);
     const int resident = umma_active_clusters<kSwiglu>(1, device);
-    return launch_umma_instance<kSwiglu, false, kWindows>(params, tiles < resident ? tiles : resident, device, stream);
+    return launch_umma_instance<kSwiglu, false, kWindows, kFew, kTwo>(params, tiles < resident ? tiles : resident, device, stream);
+}
+
+template <bool kSwiglu, bool kTwo>
+inline int launch_umma_chains(const UmmaParams& params, bool windows, int device, cudaStream_t stream) {
+    if (windows) return launch_umma_tables<kSwiglu, true, false, kTwo>(params, device, stream);
+    return params.npad <= 32 ? launch_umma_tables<kSwiglu, false, true, kTwo>(params, device, stream)
+                             : launch_umma_tables<kSwiglu, false, false, kTwo>(params, device, stream);
 }
 
 template <bool kSwiglu>
@@ -1185,7 +1193,8 @@ inline int launch_umma_family(UmmaParams& params, bool invariant, int* ctas, cud
     if (!encode_activation_map(&params.x_map, params.x, params.M, params.K, params.npad)) return MT_ERR_LAUNCH;
     bool windows = kblocks % 4 != 0;
     for (int t = 0; t < 2; ++t) windows = windows || !aligned_to(params.scales[t], 8) || !aligned_to(params.biases[t], 8);
-    return windows ? launch_umma_tables<kSwiglu, true>(params, device, stream) : launch_umma_tables<kSwiglu, false>(params, device, stream);
+    if (!kSwiglu && params.chains == 2) return launch_umma_chains<kSwiglu, !kSwiglu>(params, windows, device, stream);
+    return launch_umma_chains<kSwiglu, false>(params, windows, device, stream);
 }
 
 struct AffineWeights {
