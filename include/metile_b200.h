@@ -34,8 +34,8 @@
  * what the CUDA runtime reported for a launch.  There is no CPU fallback.
  *
  * `flags`: 0 selects the kernel by row count.  A single projection (mt_affine_qmv, mt_affine_swiglu):
- * the CUDA-core GEMV for M = 1, the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one cooperative launch for
- * the whole MLP when the shape allows it -- on CUDA cores for M = 1 (H and I in {1024, 2048, 4096,
+ * the CUDA-core GEMV for M = 1, the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one launch for
+ * the whole MLP when the shape allows it -- for M = 1 (H and I in {1024, 2048, 4096,
  * 8192}), on mma.sync for M = 2 ... 8 (H in {512, 1024, 1536, 2048}, I a multiple of 512) -- else two
  * kernels (gate|up SwiGLU, then down) of the families above.
  *   MT_FLAG_FORCE_GEMV (1)   CUDA-core GEMV (M <= 8)
@@ -43,8 +43,10 @@
  *                            when rows must be bit-identical across batch sizes 1..128)
  *   MT_FLAG_FIXED_ORDER (256) the tcgen05 kernel's sums in the order of MT_FLAG_FORCE_UMMA, the kernel by row
  *                            count as with 0 (may be combined with the flags that choose a kernel)
+ *   MT_FLAG_MLP_IMPATIENT (512) mt_affine_mlp in one launch at one row: a CTA does not wait for the others between the
+ *                            projections but leaves its rows to the last one (the same bits; for tests)
  *   MT_FLAG_GELU (16)        mt_dense_act: x/(1+exp(-1.702x)) instead of SiLU
- *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch CUDA-core kernel (M <= 4); -1
+ *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch one-row kernel (M <= 4); -1
  *                            when it does not apply.  With flags = 0 the default dispatch falls back
  *                            to the two-kernel path if the driver refuses the cooperative launch.
  *   MT_FLAG_HOST_PAIR (64)   mt_affine_mlp_host: see there
@@ -68,6 +70,7 @@ extern "C" {
 #define MT_FLAG_HOST_PAIR 0x40u
 #define MT_FLAG_MLP_FUSED_MMA 0x80u
 #define MT_FLAG_FIXED_ORDER 0x100u
+#define MT_FLAG_MLP_IMPATIENT 0x200u
 
 /* Library version (major*10000 + minor*100 + patch). */
 int mt_version(void);
@@ -145,7 +148,7 @@ int mt_affine_mlp_host(const void* x_host, const void* residual_host, void* out_
                        unsigned int flags, void* stream);
 
 /* How many kernels mt_affine_mlp queues for this problem on the current device with 16-byte
- * aligned operands: 1 when a single-launch kernel serves it (one row on CUDA cores, up to four with
+ * aligned operands: 1 when a single-launch kernel serves it (one row, up to four with
  * MT_FLAG_MLP_FUSED, H and I in {1024, 2048, 4096, 8192}; two to eight rows on mma.sync, H <= 2048),
  * else 2 (gate|up
  * SwiGLU, then down); 0 for M <= 0.  No counterpart in the reference project; used for launch

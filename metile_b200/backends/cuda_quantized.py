@@ -91,7 +91,7 @@ class fixed_order:
 @contextlib.contextmanager
 def force_kernel(name):
     """Pin the kernel family: "gemv" (CUDA cores, up to 8 rows), "umma" (tcgen05), "mlp_fused" /
-    "mlp_fused_mma" (the single-launch MLP on CUDA cores / on mma.sync; projections called on their
+    "mlp_fused_mma" (the single-launch MLP for one row / for up to eight; projections called on their
     own are unaffected) or None (the default dispatch by row count)."""
     table = {None: 0, "gemv": _lib.FLAG_FORCE_GEMV, "umma": _lib.FLAG_FORCE_UMMA,
              "mlp_fused": _lib.FLAG_MLP_FUSED, "mlp_fused_mma": _lib.FLAG_MLP_FUSED_MMA}

@@ -48,6 +48,44 @@ struct OneRowParams {
     int table_bytes;  // of the scales (and of the biases) of sixteen rows
 };
 
+// The weight row of lane group g (and 8 + it): neighbouring groups, whose reads go together, take rows four apart, which the
+// swizzle puts into the two halves of the banks.
+__device__ __forceinline__ int one_row_tile_row(int g) { return (g >> 1) + 4 * (g & 1); }
+
+// This lane's words of an item: of row tile_row and of the eighth row after it, of groups t / 2, 2 + t / 2, ...
+__device__ __forceinline__ void one_row_words(const uint8_t* words, int tile_row, int t, uint32_t (&row)[4][4], uint32_t (&row8)[4][4]) {
+    const uint32_t word_lane = (uint32_t)tile_row * 128u + ((uint32_t)(t ^ tile_row) << 4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint8_t* at = words + (i >> 1) * 2048 + (word_lane ^ (uint32_t)((i & 1) << 6));
+        const uint4 lo = *reinterpret_cast<const uint4*>(at), hi = *reinterpret_cast<const uint4*>(at + 1024);
+        row[i][0] = lo.x; row[i][1] = lo.y; row[i][2] = lo.z; row[i][3] = lo.w;
+        row8[i][0] = hi.x; row8[i][1] = hi.y; row8[i][2] = hi.z; row8[i][3] = hi.w;
+    }
+}
+
+// Sums of (128 + q) x over groups 2t and 2t + 1 of the item: own[0], own[1] of this lane's row, own[2], own[3] of the eighth
+// row after it.
+__device__ __forceinline__ void one_row_products(const uint32_t (&row)[4][4], const uint32_t (&row8)[4][4], const uint32_t (&xr)[16], int t,
+                                                 float (&own)[4]) {
+    float sum[4][4] = {};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)  // four chains side by side
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t a[4], b[4];
+            unpack_word_offset128(row[i][u], a);
+            unpack_word_offset128(row8[i][u], b);
+            ptx::mma_bf16_m16n8k16(sum[i], a[0], b[0], a[1], b[1], xr[4 * u], xr[4 * u + 1]);
+            ptx::mma_bf16_m16n8k16(sum[i], a[2], b[2], a[3], b[3], xr[4 * u + 2], xr[4 * u + 3]);
+        }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float low = t & 1 ? sum[1][e] : sum[0][e], high = t & 1 ? sum[3][e] : sum[2][e];
+        own[e] = t & 2 ? high : low;
+    }
+}
+
 template <bool kDual>
 __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(const __grid_constant__ OneRowParams p) {
     constexpr int kStreams = kDual ? 2 : 1;
@@ -142,10 +180,7 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
     }
     __syncthreads();
 
-    // The weight row of lane group g (and 8 + it): neighbouring groups, whose reads go together, take rows four apart, which
-    // the swizzle puts into the two halves of the banks.
-    const int tile_row = (g >> 1) + 4 * (g & 1);
-    const uint32_t word_lane = (uint32_t)tile_row * 128u + ((uint32_t)(t ^ tile_row) << 4);
+    const int tile_row = one_row_tile_row(g);
     const bool carries = (g & 1) == (t >> 1);  // whether this lane's column belongs to its half of the pairs
     const uint8_t* x_lane = x_tile + g * 128 + (t & 1) * 64;
     uint32_t xr[16];
@@ -181,30 +216,9 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
                 const uint8_t* words = ring + slot * kOneRowItemBytes;
                 if (++slot == kOneRowDepth) slot = 0;
                 uint32_t row[4][4], row8[4][4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint8_t* at = words + (i >> 1) * 2048 + (word_lane ^ (uint32_t)((i & 1) << 6));
-                    const uint4 lo = *reinterpret_cast<const uint4*>(at), hi = *reinterpret_cast<const uint4*>(at + 1024);
-                    row[i][0] = lo.x; row[i][1] = lo.y; row[i][2] = lo.z; row[i][3] = lo.w;
-                    row8[i][0] = hi.x; row8[i][1] = hi.y; row8[i][2] = hi.z; row8[i][3] = hi.w;
-                }
-                float sum[4][4] = {};
-#pragma unroll
-                for (int u = 0; u < 4; ++u)  // four chains side by side
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint32_t a[4], b[4];
-                        unpack_word_offset128(row[i][u], a);
-                        unpack_word_offset128(row8[i][u], b);
-                        ptx::mma_bf16_m16n8k16(sum[i], a[0], b[0], a[1], b[1], xr[4 * u], xr[4 * u + 1]);
-                        ptx::mma_bf16_m16n8k16(sum[i], a[2], b[2], a[3], b[3], xr[4 * u + 2], xr[4 * u + 3]);
-                    }
+                one_row_words(words, tile_row, t, row, row8);
                 float own[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float low = t & 1 ? sum[1][e] : sum[0][e], high = t & 1 ? sum[3][e] : sum[2][e];
-                    own[e] = t & 2 ? high : low;
-                }
+                one_row_products(row, row8, xr, t, own);
                 const uint16_t* scale_row = reinterpret_cast<const uint16_t*>(tile_tables + 2 * s * p.table_bytes);
                 const uint16_t* bias_row = reinterpret_cast<const uint16_t*>(tile_tables + (2 * s + 1) * p.table_bytes);
 #pragma unroll
@@ -255,20 +269,6 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
 }
 
 // ------------------------------------------------------------------------------- host side
-inline bool encode_one_row_weight_map(CUtensorMap* map, const void* base, int K, int N) {
-    return remembered_tensor_map(map, TensorMapKey{base, K, N, 16, 3}, [&](CUtensorMap* to) {
-        EncodeTiledFn fn = encode_tiled_fn();
-        if (!fn) return false;
-        cuuint64_t dims[2] = {(cuuint64_t)K / 8, (cuuint64_t)N};
-        cuuint64_t strides[1] = {(cuuint64_t)K / 2};
-        cuuint32_t box[2] = {32, 16};
-        cuuint32_t elem_strides[2] = {1, 1};
-        return fn(to, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    });
-}
-
 struct OneRowPlan {
     int parts, teams, grid, table_bytes, smem;
 };
@@ -331,8 +331,8 @@ inline int launch_one_row(const void* x, const GemvWeights& a, const GemvWeights
         if (device < 64) configured[device] = true;
     }
     OneRowParams params;
-    if (!encode_one_row_weight_map(&params.w_map[0], a.w, K, N)) return MT_ERR_LAUNCH;
-    if (kDual && !encode_one_row_weight_map(&params.w_map[1], b.w, K, N)) return MT_ERR_LAUNCH;
+    if (!encode_weight_map(&params.w_map[0], a.w, K, N, 16)) return MT_ERR_LAUNCH;
+    if (kDual && !encode_weight_map(&params.w_map[1], b.w, K, N, 16)) return MT_ERR_LAUNCH;
     params.x = static_cast<const uint16_t*>(x);
     params.scales[0] = a.scales;
     params.scales[1] = b.scales;

@@ -1,74 +1,58 @@
 // The whole INT4 affine MLP  out = down(silu(x Wg^T) * (x Wu^T)) + residual  for a handful of
-// activation rows as ONE cooperative launch, one CTA per SM.  Two kernels share the launch structure:
-// the FMA kernel described first (one to four rows, default for one) and the warp-MMA kernel
+// activation rows as ONE launch, one CTA per SM.  Two kernels share the launch structure:
+// the one-row kernel described first (one to four rows, default for one) and the eight-column kernel
 // further down (up to eight rows, default from two).
 //
 // Why one launch.  At a few rows the MLP is a pure stream of packed weights (28 MB at the
 // Llama-3.2-1B shape: 4.4 us at the measured HBM rate), and two dependent kernels spend more time
 // starting, ramping up their loads and draining than moving those bytes.  Here a CTA streams its rows
-// of gate and up, then its rows of down, through ONE ring of shared-memory slots fed by bulk copies.
-// At the Llama-3.2-1B shape the ring holds the CTA's whole share (6 items of 36 KB), so every
-// weight byte of the MLP is requested in the first microsecond and HBM stays busy while the
-// arithmetic runs behind the copies; larger shapes reuse slots.  The two projections are separated
-// by a grid-wide barrier (every hidden activation must exist before any down row can be summed);
-// the down rows are already in the ring when the barrier opens.
+// of gate and up, then its rows of down, through rings of shared memory fed by bulk copies.
+// At the Llama-3.2-1B shape they hold the CTA's whole share, so every weight byte of the MLP is
+// requested in the first microsecond and HBM stays busy while the arithmetic runs behind the copies;
+// larger shapes reuse slots.  The two projections are separated by a grid-wide barrier (every hidden
+// activation must exist before any down row can be summed); the down rows are already in the rings
+// when the barrier opens.
 //
-// Work split.  CTA c owns gate/up rows [c*I/grid, (c+1)*I/grid) and down rows [c*H/grid,
-// (c+1)*H/grid).  A weight row of K columns is cut into K/1024 sets of 1024 columns (32 lanes x 32
-// nibbles): warp w of the compute warps serves set w % sets and, in every ring item, the share-rows
-// w / sets + (warps / sets) * j.  Its activations (32 per lane and row, fp32 in registers) therefore
-// never change during a projection.  Per-set partial sums of a row meet in shared memory and are added
-// in set order, so the fp32 order depends on (H, I, grid) only.
+// Rows.  CTA c owns gate/up rows [c*I/grid, (c+1)*I/grid) and down rows [c*H/grid, (c+1)*H/grid).
 //
-// Arithmetic.  A lane turns 16 bytes of a weight row into the floats 128+q with one byte-permute
-// each (the nibble becomes mantissa bits 16..19 of 0x43000000 = 128.0f) and multiplies them with
-// its 32 activations by plain FMAs, four weight-row shares at a time so that their dependency
-// chains overlap.  Scale and bias are folded per lane:  s * dot + (b - 128 s) * (sum of the lane's
-// activations);  a butterfly adds the 32 lanes.  Weights are never rounded.
+// The one-row kernel multiplies as affine_gemv_mma.cuh does: mma.sync over units of 16 weight rows x 512
+// columns, eight quantisation groups in the product's eight columns.  A CTA's rows are cut into as few
+// tiles as sixteen rows allow, all of one height (55 gate rows: four of fourteen), a tile's K range into
+// units, and unit u of the CTA belongs to warp u % 16: the columns of a warp's units are the same ones throughout
+// a projection (the column units of a tile divide sixteen), so its activations are read once, into registers.  Every warp
+// has a ring of its own and issues its own copies; the tables of all rows of the CTA come by one copy each.  The units' sums of a
+// row meet in shared memory and are added in column order: the fp32 order depends on (H, I) only.  More rows than one
+// multiply the same words again.
 //
-// Ring items (all the same size): gate|up item = 16 rows of gate, 16 rows of up and their four
-// 16-row blocks of scales and biases (18*H bytes); down item = 32*H/I rows of down with their
-// scales and biases.
-//
-// What bounds it (measured on B200).  One weight-row share costs about 76 instructions per warp
-// (32 byte-permutes, 32 FMAs, masks, scale fold, butterfly) and the SM sub-partition sustains about
-// 0.7 of them per cycle, so the MLP's 50 M weights take about 5 us of instruction issue per SM --
-// more than the 4.4 us the bytes take.  Eight compute warps with 146 registers beat sixteen with 96.
-// Each further activation row adds 32 FMAs per share, which is why the warp-MMA kernel takes over
-// at two rows.  Also measured and dropped: the packed fma.rn.f32x2 (the compiler moves every
-// unpacked weight into a register pair first, two extra instructions per weight), a bf16-pair
-// unpack (same instruction count as the byte-permutes), and a half-SM variant meant to let two
-// launches overlap (a cooperative launch does not start before its predecessor has drained, so
-// nothing overlapped).
+// What bounds it (2048 / 8192): its start and end and the grid barrier, about 5 us, beside the bytes' 4.4.
+// With byte-permutes and FMAs on the CUDA cores, eight warps and a cooperative launch it took 16.4 us; the products on mma.sync,
+// sixteen warps 16.2; in an ordinary launch (fused_meet) 13.2.
 #pragma once
 
 #include <cuda.h>
 
+#include "affine_gemv_mma.cuh"
 #include "common.cuh"
 #include "ptx.cuh"
 
 namespace mt {
 
-#ifndef MT_FUSED_WARPS
-#define MT_FUSED_WARPS 8
-#endif
-#ifndef MT_FUSED_ITEM_ROWS
-#define MT_FUSED_ITEM_ROWS 16
-#endif
-constexpr int kFusedComputeWarps = MT_FUSED_WARPS;
+constexpr int kFusedComputeWarps = 8;
 constexpr int kFusedComputeThreads = kFusedComputeWarps * 32;
 constexpr int kFusedThreads = kFusedComputeThreads + 32;  // + the producer warp
-constexpr int kFusedMaxRows = 4;       // activation rows (each lane keeps 32 fp32 activations per row in registers)
-// Rows the FMA kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED (16.2 / 20.1 / 22.4 us at 1 / 2 / 3
-// rows against 19.3 us for the warp-MMA kernel).  The rule for one row is older than the GEMV's rings: in replayed graphs
-// two GEMV launches now take 5.1 / 6.2 / 8.2 / 13.0 / 21.1 us at hidden / intermediate widths of 1024 / 1024, 1024 / 4096, 2048 /
-// 4096, 2048 / 8192, 4096 / 8192, this kernel 9.2 / 8.0 / 11.1 / 15.4 / 24.6 (8192 / 8192: 37.4 and 37.5).  The order of a
-// row's sums differs between the two.
+constexpr int kFusedOneWarps = 16;
+constexpr int kFusedOneThreads = kFusedOneWarps * 32;
+constexpr int kFusedMaxRows = 4;
+// Rows the one-row kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED.
+// The order of a row's sums differs between the two.
 constexpr int kFusedDefaultRows = 1;
 constexpr int kFusedMaxSlots = 12;
-constexpr int kFusedItemRows = MT_FUSED_ITEM_ROWS;  // gate/up rows per ring item
+constexpr int kFusedItemRows = 16;  // gate/up rows per ring item of the eight-column kernel
 constexpr int kFusedSmemBudget = 226 * 1024;  // one CTA per SM
+constexpr int kFusedOneSmem = kFusedSmemBudget - 2048;  // beside what the one-row kernel declares
 constexpr int kFusedBarrierSlots = 64;
+constexpr int kFusedMaxGrid = 256;
+constexpr unsigned int kFusedPatienceNs = 100000;
 
 enum FusedWaitCode : unsigned int {
     kWaitFusedFull = 0x201,
@@ -81,9 +65,13 @@ enum FusedWaitCode : unsigned int {
 // unless a bounded wait gave up and left its slot short; mt_device_status(reset) zeroes the slots again.
 __device__ unsigned long long g_fused_barrier[kFusedBarrierSlots];
 
+// Down rows that their CTA has left to the last CTA of the launch, a flag per CTA (FusedMeeting); all zero between launches.
+__device__ unsigned int g_fused_left[kFusedBarrierSlots][kFusedMaxGrid];
+
 struct FusedMlpParams {
-    CUtensorMap gate_map;      // warp-MMA kernel only: gate_w / up_w as [I, H/8] uint32 tensors, boxes of
-    CUtensorMap up_map;        // 32 words x 16 rows with the 128-byte swizzle
+    CUtensorMap gate_map;      // gate_w / up_w as [I, H/8] uint32 tensors, boxes of 32 words x a tile's rows with the
+    CUtensorMap up_map;        // 128-byte swizzle
+    CUtensorMap down_map;      // down_w as [H, I/8], one-row kernel only
     const uint16_t* x;         // [1, H] bf16
     const uint32_t* gate_w;    // [I, H/8]
     const uint32_t* up_w;      // [I, H/8]
@@ -98,35 +86,66 @@ struct FusedMlpParams {
     uint16_t* hidden;          // [1, I] bf16, written then read
     uint16_t* out;             // [1, H]
     unsigned long long* barrier;
+    unsigned int* left;        // one-row kernel only: its slot of g_fused_left
+    unsigned int patience_ns;
     int M, H, I;
 };
 
-struct FusedMlpLayout {
+__host__ __device__ inline int fused_round16(int v) { return (v + 15) & ~15; }
+
+// Shared memory of the one-row kernel.
+struct FusedOneLayout {
     int rows1_max, rows2_max;  // most rows any CTA owns in each projection
-    int sets1, sets2;          // 1024-column sets per weight row
+    int tile1, tile2;          // rows of a tile
+    int chunks1, chunks2;      // 512-column units of a weight row
+    int depth;                 // units in a warp's ring
+    int tables1, tables2, scratch, bars, total;  // byte offsets; the rings come first
+};
+
+__host__ __device__ inline FusedOneLayout fused_one_layout(int M, int H, int I, int grid) {
+    FusedOneLayout l;
+    l.rows1_max = (I + grid - 1) / grid;
+    l.rows2_max = (H + grid - 1) / grid;
+    const int tiles1 = (l.rows1_max + 15) / 16, tiles2 = (l.rows2_max + 15) / 16;
+    l.tile1 = (l.rows1_max + tiles1 - 1) / tiles1;
+    l.tile2 = (l.rows2_max + tiles2 - 1) / tiles2;
+    l.chunks1 = H / 512;
+    l.chunks2 = I / 512;
+    const int tables1 = 4 * l.rows1_max * (H >> 5), tables2 = 2 * l.rows2_max * (I >> 5);
+    const int floats1 = l.rows1_max * 2 * l.chunks1 * M, floats2 = l.rows2_max * l.chunks2 * M;
+    const int scratch = fused_round16(4 * (floats1 > floats2 ? floats1 : floats2));
+    const int units = (tiles1 * 2 * l.chunks1 + kFusedOneWarps - 1) / kFusedOneWarps + (tiles2 * l.chunks2 + kFusedOneWarps - 1) / kFusedOneWarps;
+    constexpr int kBars = 8 * (kFusedOneWarps * kFusedMaxSlots + 2) + 16;
+    const int left = kFusedOneSmem - 1024 - tables1 - tables2 - scratch - kBars;
+    l.depth = left / (kFusedOneWarps * kOneRowItemBytes);
+    if (l.depth > units) l.depth = units;
+    if (l.depth > kFusedMaxSlots) l.depth = kFusedMaxSlots;
+    l.tables1 = l.depth * kFusedOneWarps * kOneRowItemBytes;
+    l.tables2 = l.tables1 + tables1;
+    l.scratch = l.tables2 + tables2;
+    l.bars = l.scratch + scratch;
+    l.total = l.bars + kBars;
+    return l;
+}
+
+// Shared memory of the eight-column kernel.
+struct FusedMlpLayout {
     int item_bytes, slots;     // ring geometry
     int down_rows;             // down rows per ring item
     int ring, scratch, bars, total;  // byte offsets
 };
 
-__host__ __device__ inline int fused_round16(int v) { return (v + 15) & ~15; }
-
-__host__ __device__ inline FusedMlpLayout fused_mlp_layout(int M, int H, int I, int grid) {
+// Ring items (all the same size): gate|up item = 16 rows of gate, 16 rows of up and their four
+// 16-row blocks of scales and biases (18*H bytes); down item = 32*H/I rows of down with their
+// scales and biases.
+__host__ __device__ inline FusedMlpLayout fused_mlp_layout(int H, int I) {
     FusedMlpLayout l;
-    l.rows1_max = (I + grid - 1) / grid;
-    l.rows2_max = (H + grid - 1) / grid;
-    l.sets1 = H / 1024;
-    l.sets2 = I / 1024;
     l.item_bytes = kFusedItemRows * (H + H / 8);  // rows x (H/2 gate + H/2 up) + rows x 4 x H/32
     int down = (2 * kFusedItemRows * H) / I;      // rows r with r * (I/2 + 2 * I/32) <= item_bytes
     if (down > 2 * kFusedItemRows) down = 2 * kFusedItemRows;
-    if (down > 8) down -= down % 8;  // whole 8-row halves of a 16-row fragment (the warp-MMA variant needs it)
+    if (down > 8) down -= down % 8;  // whole 8-row halves of a 16-row fragment
     l.down_rows = down;
-    const int floats1 = l.rows1_max * 2 * l.sets1 * M, floats2 = l.rows2_max * l.sets2 * M;
-    int scratch_floats = floats1 > floats2 ? floats1 : floats2;
-    const int mma_floats = kFusedComputeWarps * 2 * 16 * 8;  // per-item partial tiles of the warp-MMA variant
-    if (M > kFusedMaxRows && scratch_floats < mma_floats) scratch_floats = mma_floats;
-    const int scratch_bytes = fused_round16(4 * scratch_floats);
+    const int scratch_bytes = 4 * kFusedComputeWarps * 2 * 16 * 8;  // per-item partial tiles
     const int bars_bytes = 8 * (2 * kFusedMaxSlots) + 16;
     const int fixed = scratch_bytes + bars_bytes + 128;
     int slots = (kFusedSmemBudget - fixed) / l.item_bytes;
@@ -142,86 +161,6 @@ __host__ __device__ inline FusedMlpLayout fused_mlp_layout(int M, int H, int I, 
 // Barrier among the compute warps only (the producer warp keeps feeding the ring).
 __device__ __forceinline__ void fused_compute_sync() {
     asm volatile("bar.sync 1, %0;" ::"r"(kFusedComputeThreads) : "memory");
-}
-
-// The lane's 32 consecutive activations starting at column k0 of each of kM rows, as fp32 in
-// registers, and their sums.
-template <int kM>
-struct LaneActivations {
-    float value[kM][32];
-    float sum[kM];
-};
-
-template <int kM, bool kFromL2>
-__device__ __forceinline__ void load_lane_activations(const uint16_t* src, int width, int k0, LaneActivations<kM>& x) {
-#pragma unroll
-    for (int m = 0; m < kM; ++m) {
-        const uint16_t* from = src + (size_t)m * width + k0;
-        uint4 v[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) v[c] = kFromL2 ? ptx::ld_global_l2_u4(from + c * 8) : ptx::ld_global_dependent_u4(from + c * 8);
-        float total = 0.0f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const uint32_t words[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                x.value[m][8 * c + 2 * i] = bf16_lo(words[i]);
-                x.value[m][8 * c + 2 * i + 1] = bf16_hi(words[i]);
-                total += bf16_lo(words[i]);
-                total += bf16_hi(words[i]);
-            }
-        }
-        x.sum[m] = total;
-    }
-}
-
-// kN weight-row shares (32 nibbles each, same columns) against the lane's activations, interleaved so
-// that their dependency chains overlap.  out[i][m] = s_i * sum x_m (128+q_i) + (b_i - 128 s_i) * sum x_m,
-// added over the 32 lanes by a butterfly.  The unpacked weights are shared by the kM activation rows.
-template <int kN, int kM>
-__device__ __forceinline__ void fma_shares(const uint4 (&pk)[kN], const uint32_t (&scale_bits)[kN],
-                                           const uint32_t (&bias_bits)[kN], const LaneActivations<kM>& x,
-                                           float (&out)[kN][kM]) {
-    constexpr int kChains = 4;  // independent accumulators per (share, row); the same for every kM, so a
-                                // row's fp32 order does not depend on how many rows share the launch
-    float a[kN][kM][kChains];
-#pragma unroll
-    for (int i = 0; i < kN; ++i)
-#pragma unroll
-        for (int m = 0; m < kM; ++m)
-#pragma unroll
-            for (int c = 0; c < kChains; ++c) a[i][m][c] = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int i = 0; i < kN; ++i) {
-            const uint32_t word = j == 0 ? pk[i].x : j == 1 ? pk[i].y : j == 2 ? pk[i].z : pk[i].w;
-            float q[8];
-            unpack_word_f32_offset128(word, q);
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-#pragma unroll
-                for (int m = 0; m < kM; ++m)
-                    a[i][m][e % kChains] = fmaf(q[e], x.value[m][8 * j + e], a[i][m][e % kChains]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < kN; ++i) {
-        const float scale = bf16_bits_to_f32(scale_bits[i]);
-        const float offset = fmaf(-128.0f, scale, bf16_bits_to_f32(bias_bits[i]));
-#pragma unroll
-        for (int m = 0; m < kM; ++m) {
-            const float dot = (a[i][m][0] + a[i][m][1]) + (a[i][m][2] + a[i][m][3]);
-            out[i][m] = fmaf(scale, dot, offset * x.sum[m]);
-        }
-    }
-#pragma unroll
-    for (int offset = 16; offset >= 1; offset >>= 1)
-#pragma unroll
-        for (int i = 0; i < kN; ++i)
-#pragma unroll
-            for (int m = 0; m < kM; ++m) out[i][m] += __shfl_xor_sync(0xFFFFFFFFu, out[i][m], offset);
 }
 
 // The grid-wide barrier, called by the compute warps: every CTA arrives once; the slot grows by
@@ -250,13 +189,11 @@ __device__ __forceinline__ void fused_grid_barrier(unsigned long long* slot, int
     fused_compute_sync();
 }
 
-// The producer warp of both kernel variants: streams the CTA's items through the ring.  Weights do
-// not depend on the preceding kernel, so nothing here waits for it.  Lanes 0..5 each issue one copy.
-// kTiled: the gate|up rows of an item arrive as 128-byte-wide tensor-map boxes (32 words x 16 rows, 128-byte
-// swizzle; layout [matrix][H/256 column blocks][16 rows][128 B]) instead of dense rows -- what the warp-MMA
-// kernel's fragment loads need to stay free of bank conflicts.  A box is always 16 rows: rows past the
-// CTA's share (or past the tensor, zero-filled) are simply not used.
-template <bool kTiled>
+// The producer warp of the eight-column kernel: streams the CTA's items through the ring.  Weights do
+// not depend on the preceding kernel, so nothing here waits for it.  The gate|up rows of an item arrive as
+// 128-byte-wide tensor-map boxes (32 words x 16 rows, 128-byte swizzle; layout [matrix][H/256 column
+// blocks][16 rows][128 B]), which keeps the fragment loads free of bank conflicts.  A box is always 16
+// rows: rows past the CTA's share (or past the tensor, zero-filled) are simply not used.
 __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const FusedMlpLayout& lay, uint8_t* ring,
                                                uint64_t* full_bar, uint64_t* empty_bar, volatile int* abort_flag,
                                                int lane, int row1, int n1, int row2, int n2) {
@@ -273,33 +210,20 @@ __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const Fu
         if (it < items1) {
             const int rows = min(kFusedItemRows, n1 - kFusedItemRows * it);
             const size_t r0 = (size_t)(row1 + kFusedItemRows * it);
-            if constexpr (kTiled) {
-                const int blocks = H >> 8;  // 256 columns = 128 packed bytes per box
-                if (lane == 0)
-                    ptx::mbar_expect_tx(&full_bar[slot], (uint32_t)(2 * kFusedItemRows * rb1) + (uint32_t)rows * (uint32_t)(4 * sb1));
-                __syncwarp();
-                for (int box = lane; box < 2 * blocks; box += 32) {
-                    const int matrix = box / blocks, block = box - matrix * blocks;
-                    ptx::tma_load_2d(dst + (size_t)box * (kFusedItemRows * 128), matrix ? &p.up_map : &p.gate_map, block * 32,
-                                     (int)r0, &full_bar[slot]);
-                }
-                if (lane >= 28) {
-                    const int which = lane - 28;
-                    const uint16_t* base = which == 0 ? p.gate_s : which == 1 ? p.gate_b : which == 2 ? p.up_s : p.up_b;
-                    ptx::bulk_load(dst + 2 * kFusedItemRows * rb1 + which * kFusedItemRows * sb1,
-                                   base + r0 * (size_t)(H >> 6), (uint32_t)rows * sb1, &full_bar[slot]);
-                }
-            } else {
-                if (lane == 0) ptx::mbar_expect_tx(&full_bar[slot], (uint32_t)rows * (uint32_t)(2 * rb1 + 4 * sb1));
-                __syncwarp();
-                if (lane < 2) {
-                    const uint32_t* src = (lane ? p.up_w : p.gate_w) + r0 * (size_t)(H >> 3);
-                    ptx::bulk_load(dst + lane * kFusedItemRows * rb1, src, (uint32_t)rows * rb1, &full_bar[slot]);
-                } else if (lane < 6) {
-                    const uint16_t* base = lane == 2 ? p.gate_s : lane == 3 ? p.gate_b : lane == 4 ? p.up_s : p.up_b;
-                    ptx::bulk_load(dst + 2 * kFusedItemRows * rb1 + (lane - 2) * kFusedItemRows * sb1,
-                                   base + r0 * (size_t)(H >> 6), (uint32_t)rows * sb1, &full_bar[slot]);
-                }
+            const int blocks = H >> 8;  // 256 columns = 128 packed bytes per box
+            if (lane == 0)
+                ptx::mbar_expect_tx(&full_bar[slot], (uint32_t)(2 * kFusedItemRows * rb1) + (uint32_t)rows * (uint32_t)(4 * sb1));
+            __syncwarp();
+            for (int box = lane; box < 2 * blocks; box += 32) {
+                const int matrix = box / blocks, block = box - matrix * blocks;
+                ptx::tma_load_2d(dst + (size_t)box * (kFusedItemRows * 128), matrix ? &p.up_map : &p.gate_map, block * 32,
+                                 (int)r0, &full_bar[slot]);
+            }
+            if (lane >= 28) {
+                const int which = lane - 28;
+                const uint16_t* base = which == 0 ? p.gate_s : which == 1 ? p.gate_b : which == 2 ? p.up_s : p.up_b;
+                ptx::bulk_load(dst + 2 * kFusedItemRows * rb1 + which * kFusedItemRows * sb1,
+                               base + r0 * (size_t)(H >> 6), (uint32_t)rows * sb1, &full_bar[slot]);
             }
         } else {
             const int j = it - items1;
@@ -318,181 +242,261 @@ __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const Fu
     }
 }
 
-template <int kM>
-__global__ void __launch_bounds__(kFusedThreads, 1)
+// How the CTAs of the one-row kernel meet between the projections, in an ordinary launch (a cooperative one does not begin before the
+// kernel in front has left the chip: 2048 / 8192, launch after launch, 16.2 us, so 13.0).  Nothing then says that all CTAs are on
+// the chip together: beside another stream's kernel, or another such launch, some may not start before others have left.  So
+// none waits for good: a CTA whose patience ends leaves its down rows to the last CTA to arrive, and makes room.
+//
+// The slot counts arrivals and, from bit 48, CTAs that have left their rows: one word, so the last arrival and a leaving CTA see one
+// another in its order.  A flag is raised before its CTA is counted, and whoever lowers it has the rows and takes the CTA off the
+// count again.
+enum FusedMeeting : int { kMeetOpen, kMeetLast, kMeetLeft };  // kMeetLast: the last one, where some have left
+constexpr unsigned long long kMeetOneLeft = 1ull << 48;
+
+__device__ __forceinline__ int fused_meet(const FusedMlpParams& p, unsigned int grid, unsigned int cta) {
+    // Release: the hidden activations of this CTA (ordered by the caller's barrier) are visible to whoever acquires the count.
+    const unsigned long long before = ptx::atom_add_acq_rel_gpu_u64(p.barrier, 1ull), arrived = before % kMeetOneLeft;
+    const unsigned long long target = (arrived / grid + 1ull) * grid;
+    if (arrived + 1ull == target) return before >= kMeetOneLeft ? kMeetLast : kMeetOpen;
+    const unsigned long long start = ptx::global_timer_ns();
+    while (ptx::ld_acquire_gpu_u64(p.barrier) % kMeetOneLeft < target) {
+        if (ptx::global_timer_ns() - start < p.patience_ns) continue;
+        atomicExch(p.left + cta, 1u);
+        if (ptx::atom_add_acq_rel_gpu_u64(p.barrier, kMeetOneLeft) % kMeetOneLeft < target) return kMeetLeft;
+        if (atomicExch(p.left + cta, 0u) == 0u) return kMeetLeft;  // the last CTA saw the flag on its way to another's
+        ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
+        return kMeetOpen;
+    }
+    return kMeetOpen;
+}
+
+// Lane (g, t)'s activations of a 512-column unit: the B registers of one_row_products, and the sums of groups 2t and 2t + 1.
+template <bool kFromL2>
+__device__ __forceinline__ void fused_one_activations(const uint16_t* unit, int g, int t, uint32_t (&xr)[16], float2& sums) {
+    const bool carries = (g & 1) == (t >> 1);  // whether column g belongs to this lane's half of the groups
+    float total = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint16_t* from = unit + g * 64 + (t & 1) * 32 + u * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (carries) v = kFromL2 ? ptx::ld_global_l2_u4(from) : ptx::ld_global_dependent_u4(from);
+        total += ((bf16_lo(v.x) + bf16_hi(v.x)) + (bf16_lo(v.y) + bf16_hi(v.y))) + ((bf16_lo(v.z) + bf16_hi(v.z)) + (bf16_lo(v.w) + bf16_hi(v.w)));
+        xr[4 * u] = __byte_perm(v.x, v.z, 0x5410);
+        xr[4 * u + 1] = __byte_perm(v.x, v.z, 0x7632);
+        xr[4 * u + 2] = __byte_perm(v.y, v.w, 0x5410);
+        xr[4 * u + 3] = __byte_perm(v.y, v.w, 0x7632);
+    }
+    total += __shfl_xor_sync(0xFFFFFFFFu, total, 1);
+    sums.x = __shfl_sync(0xFFFFFFFFu, total, 8 * t);      // group 2t: lanes (2t, 0) and (2t, 1)
+    sums.y = __shfl_sync(0xFFFFFFFFu, total, 8 * t + 6);  // group 2t + 1: lanes (2t + 1, 2) and (2t + 1, 3)
+}
+
+__global__ void __launch_bounds__(kFusedOneThreads, 1)
 affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
-    constexpr int kShares = kM == 1 ? 4 : 2;  // weight-row shares in flight per warp
     extern __shared__ uint8_t fused_smem_raw[];
-    uint8_t* smem = fused_smem_raw + ((128u - (ptx::smem_u32(fused_smem_raw) & 127u)) & 127u);  // stays a shared-memory address
+    // 1024-byte alignment: the swizzle pattern of the tensor-map boxes repeats every 1024 bytes.
+    uint8_t* smem = fused_smem_raw + ((1024u - (ptx::smem_u32(fused_smem_raw) & 1023u)) & 1023u);  // stays a shared-memory address
     const int grid = gridDim.x, cta = blockIdx.x;
-    const int H = p.H, I = p.I;
-    const FusedMlpLayout lay = fused_mlp_layout(kM, H, I, grid);
-    uint8_t* ring = smem + lay.ring;
+    const int M = p.M, H = p.H, I = p.I;
+    const FusedOneLayout lay = fused_one_layout(M, H, I, grid);
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int depth = lay.depth;
+    uint8_t* ring = smem + warp * depth * kOneRowItemBytes;
     float* scratch = reinterpret_cast<float*>(smem + lay.scratch);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + lay.bars);
-    uint64_t* empty_bar = full_bar + kFusedMaxSlots;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(empty_bar + kFusedMaxSlots);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t* unit_full = reinterpret_cast<uint64_t*>(smem + lay.bars) + warp * depth;
+    uint64_t* table_full = reinterpret_cast<uint64_t*>(smem + lay.bars) + kFusedOneWarps * kFusedMaxSlots;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(table_full + 2);
+    __shared__ int meeting, left_count, left_ctas[kFusedMaxGrid];
 
     const int row1 = (int)((unsigned)I * (unsigned)cta / (unsigned)grid);
     const int n1 = (int)((unsigned)I * (unsigned)(cta + 1) / (unsigned)grid) - row1;
-    const int row2 = (int)((unsigned)H * (unsigned)cta / (unsigned)grid);
-    const int n2 = (int)((unsigned)H * (unsigned)(cta + 1) / (unsigned)grid) - row2;
-    const int items1 = (n1 + kFusedItemRows - 1) / kFusedItemRows;
-    const int items2 = (n2 + lay.down_rows - 1) / lay.down_rows;
-    const int rb1 = H >> 1, rb2 = I >> 1;  // bytes of a packed weight row
-    const int sb1 = H >> 5, sb2 = I >> 5;  // bytes of a row of scales (or biases)
-    const int slots = lay.slots;
+    int row2, n2, units2;
+    // Units in the order (tile, matrix, chunk); the chunks of a tile divide the warps, so a warp's chunk never changes.
+    const int per_tile1 = 2 * lay.chunks1, units1 = (n1 + lay.tile1 - 1) / lay.tile1 * per_tile1;
+    const int per_tile2 = lay.chunks2;
+    auto down_rows_of = [&](int owner) {
+        row2 = (int)((unsigned)H * (unsigned)owner / (unsigned)grid);
+        n2 = (int)((unsigned)H * (unsigned)(owner + 1) / (unsigned)grid) - row2;
+        units2 = (n2 + lay.tile2 - 1) / lay.tile2 * per_tile2;
+    };
+    down_rows_of(cta);
+    const int chunk1 = warp & (lay.chunks1 - 1), chunk2 = warp & (lay.chunks2 - 1);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kFusedMaxSlots; ++i) {
-            ptx::mbar_init(&full_bar[i], 1);
-            ptx::mbar_init(&empty_bar[i], kFusedComputeWarps);
-        }
+        for (int i = 0; i < kFusedOneWarps * depth; ++i) ptx::mbar_init(reinterpret_cast<uint64_t*>(smem + lay.bars) + i, 1);
+        ptx::mbar_init(&table_full[0], 1);
+        ptx::mbar_init(&table_full[1], 1);
         *abort_flag = 0;
+        left_count = 0;
         ptx::mbar_fence_init();
     }
     __syncthreads();
     ptx::griddep_launch_dependents();
 
-    if (warp == kFusedComputeWarps) {
-        fused_producer<false>(p, lay, ring, full_bar, empty_bar, abort_flag, lane, row1, n1, row2, n2);
-        return;
+    // ---- the copies of this warp's units: those of gate|up, then those of down
+    int copy_unit = warp;
+    bool copy_down = false;
+    auto copy_next = [&](int slot) {
+        if (!copy_down && copy_unit >= units1) {
+            copy_down = true;
+            copy_unit = warp;
+        }
+        if (copy_down && copy_unit >= units2) return;
+        if (ptx::elect_one()) {
+            uint8_t* to = ring + slot * kOneRowItemBytes;
+            const int per_tile = copy_down ? per_tile2 : per_tile1, tile = copy_unit / per_tile;
+            const int rows = copy_down ? lay.tile2 : lay.tile1, at = (copy_down ? row2 : row1) + tile * rows;
+            const bool up = !copy_down && copy_unit - tile * per_tile >= lay.chunks1;
+            const CUtensorMap* map = copy_down ? &p.down_map : up ? &p.up_map : &p.gate_map;
+            ptx::mbar_expect_tx(&unit_full[slot], 256u * (uint32_t)rows);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)  // rows past the CTA's share are not used, past the matrix filled with zeros
+                ptx::tma_load_2d(to + i * 2048, map, (copy_down ? chunk2 : chunk1) * 64 + i * 32, at, &unit_full[slot]);
+        }
+        __syncwarp();
+        copy_unit += kFusedOneWarps;
+    };
+    copy_next(0);
+    if (warp == 0 && ptx::elect_one()) {  // the tables of all rows of this CTA
+        const uint32_t bytes1 = (uint32_t)n1 * (uint32_t)(H >> 5);
+        const uint16_t* const tables1[4] = {p.gate_s, p.gate_b, p.up_s, p.up_b};
+        ptx::mbar_expect_tx(&table_full[0], 4u * bytes1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            ptx::bulk_load(smem + lay.tables1 + i * lay.rows1_max * (H >> 5), tables1[i] + (size_t)row1 * (H >> 6), bytes1, &table_full[0]);
     }
+    __syncwarp();
+    auto copy_down_tables = [&] {
+        if (warp == 0 && ptx::elect_one()) {
+            const uint32_t bytes = (uint32_t)n2 * (uint32_t)(I >> 5);
+            const uint16_t* const from[2] = {p.down_s, p.down_b};
+            ptx::mbar_expect_tx(&table_full[1], 2u * bytes);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                ptx::bulk_load(smem + lay.tables2 + i * lay.rows2_max * (I >> 5), from[i] + (size_t)row2 * (I >> 6), bytes, &table_full[1]);
+        }
+        __syncwarp();
+    };
+    copy_down_tables();
+    for (int slot = 1; slot < depth; ++slot) copy_next(slot);
 
-    // ---------------------------------------------------------------------- compute warps
     ptx::griddep_wait();  // the activations and the residual are the preceding kernel's output
-    float residual_value = 0.0f;  // fetched now, used at the very end
-    if ((int)threadIdx.x < n2 * kM && p.residual) {
-        const int row = threadIdx.x / kM, m = threadIdx.x - row * kM;
-        residual_value = bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + (size_t)m * H + row2 + row));
-    }
+    float residual_value;  // fetched now, used at the very end
+    auto fetch_residual = [&] {
+        residual_value = 0.0f;
+        if ((int)threadIdx.x < n2 * M && p.residual) {
+            const int row = threadIdx.x / M, m = threadIdx.x - row * M;
+            residual_value = bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + (size_t)m * H + row2 + row));
+        }
+    };
+    fetch_residual();
+    const int tile_row = one_row_tile_row(g);
     bool alive = true;
-    {
-        // ------------------------------------------------------------------ gate | up
-        // A step of a warp = kShares of the item's 2 * rows share-rows (share-row 2 r + matrix).
-        const int sets = lay.sets1, step = kFusedComputeWarps / sets;
-        const int set = warp % sets, first = warp / sets;
-        const int chunk = (set * 32 + lane) * 16;        // byte offset of the lane's 32 nibbles in a row
-        const int group = (set * 16 + (lane >> 1)) * 2;  // byte offset of their scale in a row of scales
-        LaneActivations<kM> x;
-        load_lane_activations<kM, false>(p.x, H, set * 1024 + lane * 32, x);
-        for (int it = 0; it < items1 && alive; ++it) {
-            const int slot = it % slots, use = it / slots;
-            if (!ptx::mbar_wait(&full_bar[slot], (uint32_t)use & 1u, abort_flag, kWaitFusedFull)) { alive = false; break; }
+    int slot = 0;
+    uint32_t phase = 0, down_tables_phase = 0;  // phase: a bit per slot
+    // Sums of this warp's units, to scratch[((row * matrices + matrix) * chunks + chunk) * M + m].
+    auto project = [&](auto down) {
+        constexpr bool kDown = decltype(down)::value;
+        const int units = kDown ? units2 : units1, per_tile = kDown ? per_tile2 : per_tile1, tile_rows = kDown ? lay.tile2 : lay.tile1;
+        const int n = kDown ? n2 : n1, chunks = kDown ? lay.chunks2 : lay.chunks1, chunk = kDown ? chunk2 : chunk1;
+        const int width = kDown ? I : H, groups = width >> 6;
+        const int table = (kDown ? lay.rows2_max : lay.rows1_max) * (width >> 5);
+        const uint8_t* tables = smem + (kDown ? lay.tables2 : lay.tables1);
+        const uint16_t* x = kDown ? p.hidden : p.x;
+        if (warp >= units) return;
+        uint32_t xr[16];
+        float2 xs;
+        fused_one_activations<kDown>(x + chunk * 512, g, t, xr, xs);
+        if (alive) alive = __all_sync(0xFFFFFFFFu, ptx::mbar_wait(&table_full[kDown], kDown ? down_tables_phase : 0u, abort_flag, kWaitFusedFull));
+        for (int unit = warp; unit < units; unit += kFusedOneWarps) {
+            if (alive) alive = __all_sync(0xFFFFFFFFu, ptx::mbar_wait(&unit_full[slot], (phase >> slot) & 1u, abort_flag, kWaitFusedFull));
+            if (!alive) return;
+            phase ^= 1u << slot;
+            uint32_t row[4][4], row8[4][4];
+            one_row_words(ring + slot * kOneRowItemBytes, tile_row, t, row, row8);
+            ptx::fence_proxy_async_smem();  // the slot is filled again
             __syncwarp();
-            const uint8_t* item = ring + (size_t)slot * lay.item_bytes;
-            const uint8_t* tables = item + 2 * kFusedItemRows * rb1;
-            const int share_rows = 2 * min(kFusedItemRows, n1 - kFusedItemRows * it);
-            for (int base = first; base < share_rows; base += kShares * step) {
-                uint4 pk[kShares];
-                uint32_t scale_bits[kShares], bias_bits[kShares];
-                int where[kShares];  // share-row, or the first one again past the end (computed, discarded)
+            copy_next(slot);
+            if (++slot == depth) slot = 0;
+            const int tile = unit / per_tile, matrix = !kDown && unit - tile * per_tile >= lay.chunks1 ? 1 : 0;
+            const int first = tile * tile_rows, last = min(first + tile_rows, n) - 1;
+            const uint8_t* scales = tables + 2 * matrix * table;
+            uint32_t scale[2], bias[2];  // of groups 2t and 2t + 1 of this lane's rows
 #pragma unroll
-                for (int i = 0; i < kShares; ++i) {
-                    where[i] = base + i * step < share_rows ? base + i * step : base;
-                    const int row = where[i] >> 1, matrix = where[i] & 1;
-                    pk[i] = *reinterpret_cast<const uint4*>(item + (matrix * kFusedItemRows + row) * rb1 + chunk);
-                    scale_bits[i] = *reinterpret_cast<const uint16_t*>(tables + ((2 * matrix) * kFusedItemRows + row) * sb1 + group);
-                    bias_bits[i] = *reinterpret_cast<const uint16_t*>(tables + ((2 * matrix + 1) * kFusedItemRows + row) * sb1 + group);
-                }
-                float part[kShares][kM];
-                fma_shares<kShares, kM>(pk, scale_bits, bias_bits, x, part);
-                if (lane == 0) {
-#pragma unroll
-                    for (int i = 0; i < kShares; ++i)
-                        if (base + i * step < share_rows) {
-#pragma unroll
-                            for (int m = 0; m < kM; ++m)
-                                scratch[((2 * kFusedItemRows * it + where[i]) * sets + set) * kM + m] = part[i][m];
-                        }
-                }
+            for (int r = 0; r < 2; ++r) {
+                const int at = (min(first + tile_row + 8 * r, last) * groups + chunk * kOneRowItemGroups + 2 * t) * 2;
+                scale[r] = *reinterpret_cast<const uint32_t*>(scales + at);
+                bias[r] = *reinterpret_cast<const uint32_t*>(scales + table + at);
             }
-            // The slot was read with ordinary loads; if the copy engine will overwrite it, order the two.
-            if (it + slots < items1 + items2) {
-                ptx::fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&empty_bar[slot]);
+            for (int m = 0; m < M; ++m) {
+                if (M > 1) fused_one_activations<kDown>(x + (size_t)m * width + chunk * 512, g, t, xr, xs);
+                float own[4], total[2];
+                one_row_products(row, row8, xr, t, own);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float s0 = bf16_lo(scale[r]), s1 = bf16_hi(scale[r]);
+                    const float b0 = fmaf(-128.0f, s0, bf16_lo(bias[r])), b1 = fmaf(-128.0f, s1, bf16_hi(bias[r]));  // undoes the 128 in 128 + q
+                    total[r] = fmaf(s0, own[2 * r], b0 * xs.x);
+                    total[r] = fmaf(s1, own[2 * r + 1], fmaf(b1, xs.y, total[r]));
+                    total[r] += __shfl_xor_sync(0xFFFFFFFFu, total[r], 1);
+                    total[r] += __shfl_xor_sync(0xFFFFFFFFu, total[r], 2);
+                }
+                const int mine = first + tile_row + 8 * (t & 1);
+                if (t < 2 && mine <= last)
+                    scratch[((mine * (kDown ? 1 : 2) + matrix) * chunks + chunk) * M + m] = t == 0 ? total[0] : total[1];
             }
         }
-        fused_compute_sync();
-        for (int idx = threadIdx.x; idx < n1 * kM; idx += kFusedComputeThreads) {
-            const int row = idx / kM, m = idx - row * kM;
-            float gate = 0.0f, up = 0.0f;
-            for (int s = 0; s < sets; ++s) {
-                gate += scratch[((2 * row + 0) * sets + s) * kM + m];
-                up += scratch[((2 * row + 1) * sets + s) * kM + m];
-            }
-            p.hidden[(size_t)m * I + row1 + row] = f32_to_bf16_bits(swiglu_f32(gate, up));
+    };
+    project(std::false_type{});
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < n1 * M; idx += kFusedOneThreads) {
+        const int row = idx / M, m = idx - row * M;
+        float gate = 0.0f, up = 0.0f;
+        for (int c = 0; c < lay.chunks1; ++c) {
+            gate += scratch[((2 * row + 0) * lay.chunks1 + c) * M + m];
+            up += scratch[((2 * row + 1) * lay.chunks1 + c) * M + m];
         }
+        p.hidden[(size_t)m * I + row1 + row] = f32_to_bf16_bits(swiglu_f32(gate, up));
     }
-    fused_grid_barrier(p.barrier, grid, abort_flag);
-    {
-        // ------------------------------------------------------------------ down
-        const int sets = lay.sets2, step = kFusedComputeWarps / sets;
-        const int set = warp % sets, first = warp / sets;
-        const int chunk = (set * 32 + lane) * 16;
-        const int group = (set * 16 + (lane >> 1)) * 2;
-        LaneActivations<kM> x;
-        load_lane_activations<kM, true>(p.hidden, I, set * 1024 + lane * 32, x);
-        for (int j = 0; j < items2 && alive; ++j) {
-            const int it = items1 + j;
-            const int slot = it % slots, use = it / slots;
-            if (!ptx::mbar_wait(&full_bar[slot], (uint32_t)use & 1u, abort_flag, kWaitFusedFull)) { alive = false; break; }
-            __syncwarp();
-            const uint8_t* item = ring + (size_t)slot * lay.item_bytes;
-            const uint8_t* tables = item + lay.down_rows * rb2;
-            const int rows_here = min(lay.down_rows, n2 - lay.down_rows * j);
-            for (int base = first; base < rows_here; base += kShares * step) {
-                uint4 pk[kShares];
-                uint32_t scale_bits[kShares], bias_bits[kShares];
-                int rows[kShares];
-#pragma unroll
-                for (int i = 0; i < kShares; ++i) {
-                    rows[i] = base + i * step < rows_here ? base + i * step : base;  // past the end: recompute, discard
-                    pk[i] = *reinterpret_cast<const uint4*>(item + rows[i] * rb2 + chunk);
-                    scale_bits[i] = *reinterpret_cast<const uint16_t*>(tables + rows[i] * sb2 + group);
-                    bias_bits[i] = *reinterpret_cast<const uint16_t*>(tables + (lay.down_rows + rows[i]) * sb2 + group);
-                }
-                float part[kShares][kM];
-                fma_shares<kShares, kM>(pk, scale_bits, bias_bits, x, part);
-                if (lane == 0) {
-#pragma unroll
-                    for (int i = 0; i < kShares; ++i)
-                        if (base + i * step < rows_here) {
-#pragma unroll
-                            for (int m = 0; m < kM; ++m)
-                                scratch[((lay.down_rows * j + rows[i]) * sets + set) * kM + m] = part[i][m];
-                        }
-                }
-            }
-            if (it + slots < items1 + items2) {
-                ptx::fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&empty_bar[slot]);
-            }
-        }
-        fused_compute_sync();
-        if ((int)threadIdx.x < n2 * kM) {
-            const int row = threadIdx.x / kM, m = threadIdx.x - row * kM;
+    __syncthreads();
+    if (threadIdx.x == 0) meeting = fused_meet(p, (unsigned)grid, (unsigned)cta);
+    __syncthreads();
+    const int met = meeting;
+    for (int next = 0;; ++next) {
+        project(std::true_type{});  // of a CTA that has left its rows, too: its copies have then landed
+        __syncthreads();
+        if (met != kMeetLeft && (int)threadIdx.x < n2 * M) {
+            const int row = threadIdx.x / M, m = threadIdx.x - row * M;
             float v = 0.0f;
-            for (int s = 0; s < sets; ++s) v += scratch[(row * sets + s) * kM + m];
+            for (int c = 0; c < lay.chunks2; ++c) v += scratch[(row * lay.chunks2 + c) * M + m];
             p.out[(size_t)m * H + row2 + row] = f32_to_bf16_bits(v + residual_value);
         }
+        if (met != kMeetLast) break;
+        if (next == 0 && (int)threadIdx.x < grid && atomicExch(p.left + threadIdx.x, 0u) == 1u) {
+            left_ctas[atomicAdd(&left_count, 1)] = threadIdx.x;
+            ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
+        }
+        ptx::fence_proxy_async_smem();  // the tables are filled again
+        __syncthreads();
+        if (next == left_count || *abort_flag) break;
+        down_rows_of(left_ctas[next]);
+        copy_unit = warp;
+        copy_down_tables();
+        for (int i = 0; i < depth; ++i) copy_next(slot + i < depth ? slot + i : slot + i - depth);
+        fetch_residual();
+        down_tables_phase ^= 1u;
     }
+    if (*abort_flag) ptx::drain_copies();
 }
 
 // ===================================================================================================
-// Warp-MMA variant for four to eight activation rows.
+// Eight-column kernel for two to eight activation rows.
 //
-// The FMA kernel above costs one FMA per weight per row, so it loses to the tensor-core path from four
-// rows on.  Here the multiply runs on mma.sync (m16n8k16, bf16 in, fp32 out): the A fragment is exactly
+// The multiply runs on mma.sync (m16n8k16, bf16 in, fp32 out): the A fragment is exactly
 // what the nibble unpack produces -- bf16 pairs (128+q_i, 128+q_{i+4}), 7 integer instructions per
 // packed word -- and up to eight activation rows ride in the B fragment for free.  Four MMAs cover one
 // quantisation group (64 k) of 16 weight rows; the group's partial sums P are folded as
-// acc += s * P + (b - 128 s) * X, X = the group's activation sum, so weights stay exact.  mma.sync issues
-// about once per 32 cycles per SM sub-partition on this part, which bounds the kernel near the FMA
-// kernel's one-row time, independent of the row count.  The four MMAs of a group are a dependent chain,
+// acc += s * P + (b - 128 s) * X, X = the group's activation sum, so weights stay exact.  The four MMAs of a group are a dependent chain,
 // so four (block, group) pairs are issued round-robin; with one chain at a time the kernel took 25 us.
 // The fragment loads are 64 bits per lane from four weight rows at a time; in a dense row layout those
 // rows share their banks (4-way conflicts, 1.5 M extra wavefronts per launch), so the gate|up rows arrive
@@ -620,7 +624,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
     uint8_t* smem = fused_smem_raw + ((1024u - (ptx::smem_u32(fused_smem_raw) & 1023u)) & 1023u);  // stays a shared-memory address
     const int grid = gridDim.x, cta = blockIdx.x;
     const int M = p.M, H = p.H, I = p.I;
-    const FusedMlpLayout lay = fused_mlp_layout(kFusedMmaMaxRows, H, I, grid);
+    const FusedMlpLayout lay = fused_mlp_layout(H, I);
     uint8_t* ring = smem + lay.ring;
     float* scratch = reinterpret_cast<float*>(smem + lay.scratch);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + lay.bars);
@@ -653,7 +657,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             ptx::prefetch_tensor_map(&p.gate_map);
             ptx::prefetch_tensor_map(&p.up_map);
         }
-        fused_producer<true>(p, lay, ring, full_bar, empty_bar, abort_flag, lane, row1, n1, row2, n2);
+        fused_producer(p, lay, ring, full_bar, empty_bar, abort_flag, lane, row1, n1, row2, n2);
         return;
     }
 
@@ -884,12 +888,12 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
     }
 }
 
-// Whether the warp-MMA variant serves this problem.
+// Whether the eight-column kernel serves this problem.
 inline bool fused_mlp_mma_applicable(const FusedMlpParams& p, int sm_count) {
     if (p.M < 1 || p.M > kFusedMmaMaxRows || sm_count < 1) return false;
     if (p.H < 512 || p.H % (64 * kFusedComputeWarps) || (p.H >> 6) / kFusedComputeWarps > kFusedMmaMaxGroups1) return false;
     if (p.I < 512 || p.I % (64 * kFusedComputeWarps)) return false;
-    const FusedMlpLayout lay = fused_mlp_layout(kFusedMmaMaxRows, p.H, p.I, sm_count);
+    const FusedMlpLayout lay = fused_mlp_layout(p.H, p.I);
     if (lay.slots < 2 || lay.down_rows < 8 || lay.down_rows % 8) return false;
     if (16 * p.M > kFusedComputeThreads) return false;
     if (p.H % 256 || lay.item_bytes % 1024) return false;  // whole tensor-map boxes, swizzle-aligned items
@@ -903,15 +907,13 @@ inline bool fused_mlp_mma_applicable(const FusedMlpParams& p, int sm_count) {
 
 // Whether the fused kernel serves this problem on a device with `sm_count` SMs.
 inline bool fused_mlp_applicable(const FusedMlpParams& p, int sm_count) {
-    if (p.M < 1 || p.M > kFusedMaxRows || sm_count < 1) return false;
-    auto supported = [](int v) {  // a whole number of 1024-column sets that divides the compute warps
-        return v >= 1024 && v % 1024 == 0 && kFusedComputeWarps % (v / 1024) == 0;
+    if (p.M < 1 || p.M > kFusedMaxRows || sm_count < 1 || sm_count > kFusedMaxGrid) return false;
+    auto supported = [](int v) {  // a whole number of 512-column units that divides the warps
+        return v >= 1024 && v % 512 == 0 && kFusedOneWarps % (v / 512) == 0;
     };
-    if (!supported(p.H) || !supported(p.I)) return false;
-    const FusedMlpLayout lay = fused_mlp_layout(p.M, p.H, p.I, sm_count);
-    if (lay.slots < 2 || lay.down_rows < 1) return false;
-    if (lay.rows2_max * p.M > kFusedComputeThreads) return false;
-    if (lay.total + 128 > kFusedSmemBudget) return false;
+    if (!supported(p.H) || !supported(p.I) || p.H > 4096) return false;  // 8192 / 8192: two GEMV launches are as fast
+    const FusedOneLayout lay = fused_one_layout(p.M, p.H, p.I, sm_count);
+    if (lay.depth < 2 || lay.rows2_max * p.M > kFusedOneThreads) return false;
     const void* pointers[] = {p.x, p.gate_w, p.up_w, p.down_w, p.gate_s, p.gate_b, p.up_s, p.up_b, p.down_s, p.down_b,
                               p.hidden};
     for (const void* ptr : pointers)
@@ -922,8 +924,7 @@ inline bool fused_mlp_applicable(const FusedMlpParams& p, int sm_count) {
 // 0 = untried, 1 = programmatic dependent launch accepted together with a cooperative launch, -1 = refused.
 static int g_fused_pdl_state[64] = {};
 
-// `kKind` only separates the per-kernel static state (1..4 = FMA kernel rows, 0 = warp-MMA kernel).
-template <int kKind>
+template <int kThreads>  // of a CTA, which also separates the kernels' static state
 inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int smem, const FusedMlpParams& params,
                                    int sm_count, int device, cudaStream_t stream) {
     static bool configured[64] = {};
@@ -932,13 +933,13 @@ inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int sme
             return MT_ERR_LAUNCH;
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         int resident = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kFusedThreads, smem) != cudaSuccess || resident < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, smem) != cudaSuccess || resident < 1)
             return MT_ERR_LAUNCH;
         configured[device] = true;
     }
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(sm_count, 1, 1);
-    config.blockDim = dim3(kFusedThreads, 1, 1);
+    config.blockDim = dim3(kThreads, 1, 1);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attrs[2];
@@ -964,24 +965,23 @@ inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int sme
     return cudaLaunchKernelEx(&config, kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
-template <int kM>
-inline int launch_mlp_fused_rows(const FusedMlpParams& params, int sm_count, int device, cudaStream_t stream) {
-    const int smem = fused_mlp_layout(kM, params.H, params.I, sm_count).total + 128;
-    return launch_mlp_fused_kernel<kM>(affine_mlp_fused_kernel<kM>, smem, params, sm_count, device, stream);
-}
-
-// The barrier slot of the next launch on the current device (slots rotate, one per launch in flight).
-inline unsigned long long* next_fused_barrier_slot() {
+// The barrier slot of the next launch on the current device (slots rotate, one per launch in flight), and its flags.
+inline bool next_fused_barrier_slot(unsigned long long*& barrier, unsigned int*& left) {
     static unsigned long long* slots[64] = {};
+    static unsigned int* flags[64] = {};
     static unsigned int launches = 0;
     int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return nullptr;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
     if (!slots[device]) {
-        void* address = nullptr;
-        if (cudaGetSymbolAddress(&address, g_fused_barrier) != cudaSuccess) return nullptr;
-        slots[device] = static_cast<unsigned long long*>(address);
+        void *first = nullptr, *second = nullptr;
+        if (cudaGetSymbolAddress(&first, g_fused_barrier) != cudaSuccess || cudaGetSymbolAddress(&second, g_fused_left) != cudaSuccess) return false;
+        flags[device] = static_cast<unsigned int*>(second);
+        __atomic_store_n(&slots[device], static_cast<unsigned long long*>(first), __ATOMIC_RELEASE);
     }
-    return slots[device] + (__atomic_fetch_add(&launches, 1u, __ATOMIC_RELAXED) % kFusedBarrierSlots);
+    const unsigned int slot = __atomic_fetch_add(&launches, 1u, __ATOMIC_RELAXED) % kFusedBarrierSlots;
+    barrier = slots[device] + slot;
+    left = flags[device] + slot * kFusedMaxGrid;
+    return true;
 }
 
 // Caller has checked fused_mlp_applicable(), or fused_mlp_mma_applicable() when `mma` is set.
@@ -989,22 +989,36 @@ inline int launch_mlp_fused(FusedMlpParams params, int sm_count, bool mma, cudaS
     int device = 0;
     cudaGetDevice(&device);
     if (device >= 64) return MT_ERR_DEVICE;
-    params.barrier = next_fused_barrier_slot();
-    if (!params.barrier) return MT_ERR_LAUNCH;
+    if (!next_fused_barrier_slot(params.barrier, params.left)) return MT_ERR_LAUNCH;
     if (mma) {
         if (!encode_weight_map(&params.gate_map, params.gate_w, params.H, params.I, kFusedItemRows) ||
             !encode_weight_map(&params.up_map, params.up_w, params.H, params.I, kFusedItemRows))
             return MT_ERR_LAUNCH;
-        const int smem = fused_mlp_layout(kFusedMmaMaxRows, params.H, params.I, sm_count).total + 1024;
-        return launch_mlp_fused_kernel<0>(affine_mlp_fused_mma_kernel, smem, params, sm_count, device, stream);
+        const int smem = fused_mlp_layout(params.H, params.I).total + 1024;
+        return launch_mlp_fused_kernel<kFusedThreads>(affine_mlp_fused_mma_kernel, smem, params, sm_count, device, stream);
     }
-    switch (params.M) {
-        case 1: return launch_mlp_fused_rows<1>(params, sm_count, device, stream);
-        case 2: return launch_mlp_fused_rows<2>(params, sm_count, device, stream);
-        case 3: return launch_mlp_fused_rows<3>(params, sm_count, device, stream);
-        case 4: return launch_mlp_fused_rows<4>(params, sm_count, device, stream);
-        default: return MT_ERR_SHAPE;
+    const FusedOneLayout lay = fused_one_layout(params.M, params.H, params.I, sm_count);
+    if (!encode_weight_map(&params.gate_map, params.gate_w, params.H, params.I, lay.tile1) ||
+        !encode_weight_map(&params.up_map, params.up_w, params.H, params.I, lay.tile1) ||
+        !encode_weight_map(&params.down_map, params.down_w, params.I, params.H, lay.tile2))
+        return MT_ERR_LAUNCH;
+    static bool configured[64] = {};
+    if (!configured[device]) {
+        if (cudaFuncSetAttribute(affine_mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedOneSmem) != cudaSuccess)
+            return MT_ERR_LAUNCH;
+        configured[device] = true;
     }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(sm_count, 1, 1);
+    config.blockDim = dim3(kFusedOneThreads, 1, 1);
+    config.dynamicSmemBytes = lay.total + 1024;
+    config.stream = stream;
+    cudaLaunchAttribute attrs[1];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attrs;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, affine_mlp_fused_kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
 }  // namespace mt

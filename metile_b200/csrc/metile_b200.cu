@@ -280,8 +280,9 @@ int mt_selftest_bounded_wait(int which, unsigned int limit_us, void* stream) {
     if (which == 0) {
         selftest_mbarrier_wait_kernel<<<1, 64, 0, s>>>(limit_ns);
     } else if (which == 1) {
-        unsigned long long* slot = next_fused_barrier_slot();
-        if (!slot) return MT_ERR_LAUNCH;
+        unsigned long long* slot = nullptr;
+        unsigned int* left = nullptr;
+        if (!next_fused_barrier_slot(slot, left)) return MT_ERR_LAUNCH;
         selftest_grid_barrier_kernel<<<2, kFusedComputeThreads, 0, s>>>(slot, limit_ns);
     } else {
         return MT_ERR_SHAPE;
@@ -346,9 +347,9 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
     if (rc != MT_OK) return rc;
     if ((flags & MT_FLAG_FORCE_GEMV) && M > 8) return MT_ERR_SHAPE;
     if (!device_is_sm100()) return MT_ERR_DEVICE;
-    // A handful of rows: the whole MLP as one cooperative launch when the shape fits it.  Any flag
+    // A handful of rows: the whole MLP as one launch when the shape fits it.  Any flag
     // that pins a kernel family keeps the two-kernel path; MT_FLAG_MLP_FUSED insists on this one.
-    const unsigned int family = flags & ~MT_FLAG_FIXED_ORDER;
+    const unsigned int family = flags & ~(MT_FLAG_FIXED_ORDER | MT_FLAG_MLP_IMPATIENT);
     if (family == 0 || (family & (MT_FLAG_MLP_FUSED | MT_FLAG_MLP_FUSED_MMA))) {
         if (!x || !gate_w || !gate_scales || !gate_biases || !up_w || !up_scales || !up_biases || !down_w ||
             !down_scales || !down_biases || !out)
@@ -369,17 +370,19 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         params.hidden = static_cast<uint16_t*>(workspace);
         params.out = static_cast<uint16_t*>(out);
         params.barrier = nullptr;
+        params.left = nullptr;
+        params.patience_ns = flags & MT_FLAG_MLP_IMPATIENT ? 0u : kFusedPatienceNs;
         params.M = M;
         params.H = H;
         params.I = I;
         const int sms = device_sm_count();
-        // Up to kFusedDefaultRows rows: the FMA kernel.  Above, to eight rows: the warp-MMA kernel, which does not round
+        // Up to kFusedDefaultRows rows: the one-row kernel.  Above, to eight rows: the eight-column kernel, which does not round
         // the weights (against the tcgen05 pair, us at 2 to 8 rows: 1024 / 1024 7.6 | 9.3, 2048 / 4096 12.1 | 15.0, 1024 / 4096
         // 10.7 | 9.8, 2048 / 8192 18.6 | 18.1).
         const bool want_mma = (flags & MT_FLAG_MLP_FUSED_MMA) != 0;
-        const bool fma = !want_mma && (family || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
-        const bool mma = !fma && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
-        if (fma || mma) {
+        const bool one_row = !want_mma && (family || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
+        const bool mma = !one_row && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
+        if (one_row || mma) {
             const int fused_rc = launch_mlp_fused(params, sms, mma, static_cast<cudaStream_t>(stream));
             // A cooperative launch is refused when the whole grid cannot be resident (a GPU shared with
             // another context, a carve-out that leaves too little shared memory).  Nothing was queued:
@@ -451,7 +454,7 @@ int mt_affine_mlp_host(const void* x_host, const void* residual_host, void* out_
 
 int mt_affine_mlp_launches(int M, int H, int I, unsigned int flags) {
     if (M <= 0) return 0;
-    flags &= ~MT_FLAG_FIXED_ORDER;
+    flags &= ~(MT_FLAG_FIXED_ORDER | MT_FLAG_MLP_IMPATIENT);
     if (flags != 0 && !(flags & (MT_FLAG_MLP_FUSED | MT_FLAG_MLP_FUSED_MMA))) return 2;
     FusedMlpParams params = {};
     params.M = M;

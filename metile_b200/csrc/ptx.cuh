@@ -344,6 +344,12 @@ __device__ __forceinline__ unsigned long long atom_add_release_gpu_u64(unsigned 
     return old;
 }
 
+__device__ __forceinline__ unsigned long long atom_add_acq_rel_gpu_u64(unsigned long long* p, unsigned long long v) {
+    unsigned long long old;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], %2;" : "=l"(old) : "l"(p), "l"(v) : "memory");
+    return old;
+}
+
 // ---- warp-level MMA: D[16x8] += A[16x16] * B[16x8], bf16 inputs, fp32 accumulate --------------
 // Fragments (g = lane / 4, t = lane % 4): a0 = A[g][2t, 2t+1], a1 = A[g+8][2t, 2t+1],
 // a2 = A[g][2t+8, 2t+9], a3 = A[g+8][2t+8, 2t+9]; b0 = B[2t, 2t+1][g], b1 = B[2t+8, 2t+9][g];

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from metile_b200 import _lib, backends as B, synth
+from metile_b200.backends import cuda_quantized
 from metile_b200.integrations import blocks
 from oracle import affine as A
 from oracle import attention as OA
@@ -383,3 +384,33 @@ def test_a_model_embeds_as_its_module_does(cuda_device, change):
     tokens = torch.randint(0, 50, (3, 4), device=cuda_device)
     found, wanted = blocks._embed(modules[0], tokens), modules[1](tokens)
     assert found.dtype == wanted.dtype and torch.equal(found, wanted) and found.requires_grad == wanted.requires_grad
+
+
+@pytest.mark.parametrize("rows,hidden,inter", [(1, 1024, 1024), (1, 2048, 8192), (1, 4096, 2048), (1, 1024, 8192), (3, 4096, 8192)])
+def test_single_launch_mlp_whose_ctas_do_not_wait(cuda_device, rows, hidden, inter):
+    """Between the projections a CTA may leave its down rows to the last CTA to arrive, as it does when others are kept off
+    the chip.  Without patience nearly all do; whoever sums a row, its bits are the same."""
+    gate, up, down = synth.mlp_weights(330, hidden, inter, cuda_device)
+    x, res = synth.activations(5, rows, hidden, cuda_device), synth.activations(6, rows, hidden, cuda_device)
+    execute = B.mlx_affine_mlp_executor(x, *gate, *up, *down, res)
+    state = cuda_quantized._state
+    with B.force_kernel("mlp_fused"):
+        want = execute(x, res)
+        state.flags |= _lib.FLAG_MLP_IMPATIENT
+        for _ in range(100):  # more launches than barrier slots
+            assert_bit_equal(execute(x, res), want, "rows left to the last CTA")
+    assert_within(want, A.mlp(f32(x), *[triple_np(t) for t in (gate, up, down)], f32(res)), rel=3e-3, what="single-launch MLP")
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    outs = [[] for _ in streams]
+    for stream in streams:
+        stream.wait_stream(torch.cuda.current_stream())
+    executors = [B.mlx_affine_mlp_executor(x, *gate, *up, *down, res) for _ in streams]
+    with B.force_kernel("mlp_fused"):
+        for _ in range(10):  # side by side: some CTAs find no room while others wait
+            for out, stream, run in zip(outs, streams, executors):
+                with torch.cuda.stream(stream):
+                    out.append(run(x, res))
+    torch.cuda.synchronize()
+    for out in outs:
+        for y in out:
+            assert_bit_equal(y, want, "side by side")
