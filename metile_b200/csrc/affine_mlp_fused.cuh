@@ -7,10 +7,8 @@
 // Llama-3.2-1B shape: 4.4 us at the measured HBM rate), and two dependent kernels spend more time
 // starting, ramping up their loads and draining than moving those bytes.  Here a CTA streams its rows
 // of gate and up, then its rows of down, through rings of shared memory fed by bulk copies.
-// At the Llama-3.2-1B shape they hold the CTA's whole share, so every weight byte of the MLP is
-// requested in the first microsecond and HBM stays busy while the arithmetic runs behind the copies;
-// larger shapes reuse slots.  The two projections are separated by a grid-wide barrier (every hidden
-// activation must exist before any down row can be summed); the down rows are already in the rings
+// HBM stays busy while the arithmetic runs behind the copies.  The two projections are separated by a grid-wide barrier (every hidden
+// activation must exist before any down row can be summed); down rows are already in the rings
 // when the barrier opens.
 //
 // Rows.  CTA c owns gate/up rows [c*I/grid, (c+1)*I/grid) and down rows [c*H/grid, (c+1)*H/grid).
@@ -18,15 +16,17 @@
 // The one-row kernel multiplies as affine_gemv_mma.cuh does: mma.sync over units of 16 weight rows x 512
 // columns, eight quantisation groups in the product's eight columns.  A CTA's rows are cut into as few
 // tiles as sixteen rows allow, all of one height (55 gate rows: four of fourteen), a tile's K range into
-// units, and unit u of the CTA belongs to warp u % 16: the columns of a warp's units are the same ones throughout
-// a projection (the column units of a tile divide sixteen), so its activations are read once, into registers.  Every warp
+// units, and unit u of the CTA belongs to warp u % 8: where a tile has no more than eight column units, a warp's are of the
+// same columns throughout a projection, and its activations are read once, into registers.  Every warp
 // has a ring of its own and issues its own copies; the tables of all rows of the CTA come by one copy each.  The units' sums of a
 // row meet in shared memory and are added in column order: the fp32 order depends on (H, I) only.  More rows than one
 // multiply the same words again.
 //
-// What bounds it (2048 / 8192): its start and end and the grid barrier, about 5 us, beside the bytes' 4.4.
-// With byte-permutes and FMAs on the CUDA cores, eight warps and a cooperative launch it took 16.4 us; the products on mma.sync,
-// sixteen warps 16.2; in an ordinary launch (fused_meet) 13.2.
+// What bounds it (2048 / 8192): its start and end and the meeting of the CTAs, about 5 us, beside the bytes' 4.4.  Launch after
+// launch, us, called from Python and in a replayed graph: byte-permutes and FMAs on the CUDA cores in a cooperative
+// launch 16.4 and 15.1, products on mma.sync 16.2, an ordinary launch (fused_meet) of sixteen warps with all weights of a
+// CTA on their way at once 13.2 and 15.3, eight warps and room for two CTAs per SM, so that the next launch begins its
+// copies behind the meeting, 13.2 and 12.6.
 #pragma once
 
 #include <cuda.h>
@@ -40,16 +40,20 @@ namespace mt {
 constexpr int kFusedComputeWarps = 8;
 constexpr int kFusedComputeThreads = kFusedComputeWarps * 32;
 constexpr int kFusedThreads = kFusedComputeThreads + 32;  // + the producer warp
-constexpr int kFusedOneWarps = 16;
+constexpr int kFusedOneWarps = 8;
 constexpr int kFusedOneThreads = kFusedOneWarps * 32;
 constexpr int kFusedMaxRows = 4;
-// Rows the one-row kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED.
-// The order of a row's sums differs between the two.
+// Rows the one-row kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED.  The rule
+// for one row is older than affine_gemv_mma.cuh: at hidden / intermediate widths of 1024 / 1024, 1024 / 4096, 2048 / 4096, 2048 / 8192, 4096 /
+// 4096, 4096 / 8192 this kernel takes 6.1 / 6.8 / 8.2 / 12.6 / 12.1 / 21.4 us in a replayed graph (before: 9.2 / 8.1 / 10.9 / 15.1 / 15.9 /
+// 23.6), two projections called one after the other, which overlap more, 4.9 / 6.3 / 8.2 / 10.9 / 11.2 / 17.7.  The order of a
+// row's sums differs between the two.
 constexpr int kFusedDefaultRows = 1;
 constexpr int kFusedMaxSlots = 12;
 constexpr int kFusedItemRows = 16;  // gate/up rows per ring item of the eight-column kernel
 constexpr int kFusedSmemBudget = 226 * 1024;  // one CTA per SM
 constexpr int kFusedOneSmem = kFusedSmemBudget - 2048;  // beside what the one-row kernel declares
+constexpr int kFusedOnePairSmem = 223 * 512;               // two CTAs per SM
 constexpr int kFusedBarrierSlots = 64;
 constexpr int kFusedMaxGrid = 256;
 constexpr unsigned int kFusedPatienceNs = 100000;
@@ -116,7 +120,9 @@ __host__ __device__ inline FusedOneLayout fused_one_layout(int M, int H, int I, 
     const int scratch = fused_round16(4 * (floats1 > floats2 ? floats1 : floats2));
     const int units = (tiles1 * 2 * l.chunks1 + kFusedOneWarps - 1) / kFusedOneWarps + (tiles2 * l.chunks2 + kFusedOneWarps - 1) / kFusedOneWarps;
     constexpr int kBars = 8 * (kFusedOneWarps * kFusedMaxSlots + 2) + 16;
-    const int left = kFusedOneSmem - 1024 - tables1 - tables2 - scratch - kBars;
+    const int fixed = 1024 + tables1 + tables2 + scratch + kBars;
+    const bool pair = kFusedOnePairSmem - fixed >= 2 * kFusedOneWarps * kOneRowItemBytes;
+    const int left = (pair ? kFusedOnePairSmem : kFusedOneSmem) - fixed;
     l.depth = left / (kFusedOneWarps * kOneRowItemBytes);
     if (l.depth > units) l.depth = units;
     if (l.depth > kFusedMaxSlots) l.depth = kFusedMaxSlots;
@@ -291,7 +297,7 @@ __device__ __forceinline__ void fused_one_activations(const uint16_t* unit, int 
     sums.y = __shfl_sync(0xFFFFFFFFu, total, 8 * t + 6);  // group 2t + 1: lanes (2t + 1, 2) and (2t + 1, 3)
 }
 
-__global__ void __launch_bounds__(kFusedOneThreads, 1)
+__global__ void __launch_bounds__(kFusedOneThreads, 2)
 affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
     extern __shared__ uint8_t fused_smem_raw[];
     // 1024-byte alignment: the swizzle pattern of the tensor-map boxes repeats every 1024 bytes.
@@ -311,7 +317,8 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
     const int row1 = (int)((unsigned)I * (unsigned)cta / (unsigned)grid);
     const int n1 = (int)((unsigned)I * (unsigned)(cta + 1) / (unsigned)grid) - row1;
     int row2, n2, units2;
-    // Units in the order (tile, matrix, chunk); the chunks of a tile divide the warps, so a warp's chunk never changes.
+    // Units in the order (tile, matrix, chunk); where the chunks of a tile divide the warps a warp's chunk never changes (always in
+    // gate|up).
     const int per_tile1 = 2 * lay.chunks1, units1 = (n1 + lay.tile1 - 1) / lay.tile1 * per_tile1;
     const int per_tile2 = lay.chunks2;
     auto down_rows_of = [&](int owner) {
@@ -320,7 +327,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
         units2 = (n2 + lay.tile2 - 1) / lay.tile2 * per_tile2;
     };
     down_rows_of(cta);
-    const int chunk1 = warp & (lay.chunks1 - 1), chunk2 = warp & (lay.chunks2 - 1);
+    const int chunk1 = warp & (lay.chunks1 - 1);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kFusedOneWarps * depth; ++i) ptx::mbar_init(reinterpret_cast<uint64_t*>(smem + lay.bars) + i, 1);
@@ -351,7 +358,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
             ptx::mbar_expect_tx(&unit_full[slot], 256u * (uint32_t)rows);
 #pragma unroll
             for (int i = 0; i < 2; ++i)  // rows past the CTA's share are not used, past the matrix filled with zeros
-                ptx::tma_load_2d(to + i * 2048, map, (copy_down ? chunk2 : chunk1) * 64 + i * 32, at, &unit_full[slot]);
+                ptx::tma_load_2d(to + i * 2048, map, (copy_down ? copy_unit & (lay.chunks2 - 1) : chunk1) * 64 + i * 32, at, &unit_full[slot]);
         }
         __syncwarp();
         copy_unit += kFusedOneWarps;
@@ -398,7 +405,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
     auto project = [&](auto down) {
         constexpr bool kDown = decltype(down)::value;
         const int units = kDown ? units2 : units1, per_tile = kDown ? per_tile2 : per_tile1, tile_rows = kDown ? lay.tile2 : lay.tile1;
-        const int n = kDown ? n2 : n1, chunks = kDown ? lay.chunks2 : lay.chunks1, chunk = kDown ? chunk2 : chunk1;
+        const int n = kDown ? n2 : n1, chunks = kDown ? lay.chunks2 : lay.chunks1, chunk0 = kDown ? warp & (lay.chunks2 - 1) : chunk1;
         const int width = kDown ? I : H, groups = width >> 6;
         const int table = (kDown ? lay.rows2_max : lay.rows1_max) * (width >> 5);
         const uint8_t* tables = smem + (kDown ? lay.tables2 : lay.tables1);
@@ -406,7 +413,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
         if (warp >= units) return;
         uint32_t xr[16];
         float2 xs;
-        fused_one_activations<kDown>(x + chunk * 512, g, t, xr, xs);
+        fused_one_activations<kDown>(x + chunk0 * 512, g, t, xr, xs);
         if (alive) alive = __all_sync(0xFFFFFFFFu, ptx::mbar_wait(&table_full[kDown], kDown ? down_tables_phase : 0u, abort_flag, kWaitFusedFull));
         for (int unit = warp; unit < units; unit += kFusedOneWarps) {
             if (alive) alive = __all_sync(0xFFFFFFFFu, ptx::mbar_wait(&unit_full[slot], (phase >> slot) & 1u, abort_flag, kWaitFusedFull));
@@ -418,6 +425,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
             __syncwarp();
             copy_next(slot);
             if (++slot == depth) slot = 0;
+            const int chunk = kDown ? unit & (lay.chunks2 - 1) : chunk0;
             const int tile = unit / per_tile, matrix = !kDown && unit - tile * per_tile >= lay.chunks1 ? 1 : 0;
             const int first = tile * tile_rows, last = min(first + tile_rows, n) - 1;
             const uint8_t* scales = tables + 2 * matrix * table;
@@ -429,7 +437,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
                 bias[r] = *reinterpret_cast<const uint32_t*>(scales + table + at);
             }
             for (int m = 0; m < M; ++m) {
-                if (M > 1) fused_one_activations<kDown>(x + (size_t)m * width + chunk * 512, g, t, xr, xs);
+                if (M > 1 || (kDown && lay.chunks2 > kFusedOneWarps && unit != warp)) fused_one_activations<kDown>(x + (size_t)m * width + chunk * 512, g, t, xr, xs);
                 float own[4], total[2];
                 one_row_products(row, row8, xr, t, own);
 #pragma unroll
@@ -908,8 +916,8 @@ inline bool fused_mlp_mma_applicable(const FusedMlpParams& p, int sm_count) {
 // Whether the fused kernel serves this problem on a device with `sm_count` SMs.
 inline bool fused_mlp_applicable(const FusedMlpParams& p, int sm_count) {
     if (p.M < 1 || p.M > kFusedMaxRows || sm_count < 1 || sm_count > kFusedMaxGrid) return false;
-    auto supported = [](int v) {  // a whole number of 512-column units that divides the warps
-        return v >= 1024 && v % 512 == 0 && kFusedOneWarps % (v / 512) == 0;
+    auto supported = [](int v) {  // two, four, eight or sixteen 512-column units
+        return v >= 1024 && v <= 8192 && (v & (v - 1)) == 0;
     };
     if (!supported(p.H) || !supported(p.I) || p.H > 4096) return false;  // 8192 / 8192: two GEMV launches are as fast
     const FusedOneLayout lay = fused_one_layout(p.M, p.H, p.I, sm_count);
@@ -1006,6 +1014,7 @@ inline int launch_mlp_fused(FusedMlpParams params, int sm_count, bool mma, cudaS
     if (!configured[device]) {
         if (cudaFuncSetAttribute(affine_mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedOneSmem) != cudaSuccess)
             return MT_ERR_LAUNCH;
+        cudaFuncSetAttribute(affine_mlp_fused_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         configured[device] = true;
     }
     cudaLaunchConfig_t config = {};
