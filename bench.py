@@ -769,8 +769,8 @@ def run_ours(args):
         packed = hidden * inter * (0.5 + 4 / 64)  # one projection: nibbles + bf16 scales and biases
         single_rows = [m for m in sweep if library.mt_affine_mlp_launches(m, hidden, inter, 0) == 1]
         for rows_served, label, traffic, profile in (
-                ([m for m in single_rows if m <= 1], "single-launch MLP on CUDA cores (affine_mlp_fused_kernel)", 28378368,
-                 "profiles/affine_mlp_fused_m1_llama1b.md"),
+                ([m for m in single_rows if m <= 1], "single-launch MLP of one row (affine_mlp_fused_kernel)", 28384256,
+                 "profiles/affine_gemv_mma_m1.md"),
                 ([m for m in single_rows if m > 1], "single-launch MLP on mma.sync (affine_mlp_fused_mma_kernel)", 28456192,
                  "profiles/affine_mlp_fused_mma_m8_llama1b.md")):
             if not rows_served:

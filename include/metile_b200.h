@@ -34,7 +34,8 @@
  * what the CUDA runtime reported for a launch.  There is no CPU fallback.
  *
  * `flags`: 0 selects the kernel by row count.  A single projection (mt_affine_qmv, mt_affine_swiglu):
- * the CUDA-core GEMV for M = 1, the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one launch for
+ * for M = 1 the CUDA-core GEMV, or mma.sync where there are weights enough (from 8 to 45 million) and MT_FLAG_FIXED_ORDER
+ * is not given; the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one launch for
  * the whole MLP when the shape allows it -- for M = 1 (H and I in {1024, 2048, 4096,
  * 8192}), on mma.sync for M = 2 ... 8 (H in {512, 1024, 1536, 2048}, I a multiple of 512) -- else two
  * kernels (gate|up SwiGLU, then down) of the families above.
@@ -48,7 +49,7 @@
  *   MT_FLAG_GELU (16)        mt_dense_act: x/(1+exp(-1.702x)) instead of SiLU
  *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch one-row kernel (M <= 4); -1
  *                            when it does not apply.  With flags = 0 the default dispatch falls back
- *                            to the two-kernel path if the driver refuses the cooperative launch.
+ *                            to the two-kernel path if the driver refuses the launch.
  *   MT_FLAG_HOST_PAIR (64)   mt_affine_mlp_host: see there
  *   MT_FLAG_MLP_FUSED_MMA (128) mt_affine_mlp: insist on the mma.sync single-launch kernel (M <= 8);
  *                            -1 when it does not apply.

@@ -11,8 +11,8 @@ Reference surface reproduced (names, argument order, defaults, error behaviour):
 
 Differences that are deliberate:
   * activations are bfloat16 torch CUDA tensors; packed weights keep the MLX layout unchanged;
-  * there is no timing tournament: the kernel is chosen by row count (CUDA-core GEMV for one
-    row, tcgen05 MMA above), so `autotune`, `block`, `outputs_per_simdgroup` and
+  * there is no timing tournament: the kernel is chosen by row count (CUDA-core GEMV or
+    mma.sync for one row, tcgen05 MMA above), so `autotune`, `block`, `outputs_per_simdgroup` and
     `decode_dtype` are accepted for call-site compatibility and ignored;
   * any number of rows is served from one read of the weights (the reference's scalar kernels
     re-read them per row and its tuned residual path hands multi-row inputs to native MLX,

@@ -7,9 +7,9 @@
 // Llama-3.2-1B shape: 4.4 us at the measured HBM rate), and two dependent kernels spend more time
 // starting, ramping up their loads and draining than moving those bytes.  Here a CTA streams its rows
 // of gate and up, then its rows of down, through rings of shared memory fed by bulk copies.
-// HBM stays busy while the arithmetic runs behind the copies.  The two projections are separated by a grid-wide barrier (every hidden
+// HBM stays busy while the arithmetic runs behind the copies.  The two projections are separated by a meeting of all CTAs (every hidden
 // activation must exist before any down row can be summed); down rows are already in the rings
-// when the barrier opens.
+// when it is over.
 //
 // Rows.  CTA c owns gate/up rows [c*I/grid, (c+1)*I/grid) and down rows [c*H/grid, (c+1)*H/grid).
 //
@@ -51,8 +51,7 @@ constexpr int kFusedMaxRows = 4;
 constexpr int kFusedDefaultRows = 1;
 constexpr int kFusedMaxSlots = 12;
 constexpr int kFusedItemRows = 16;  // gate/up rows per ring item of the eight-column kernel
-constexpr int kFusedSmemBudget = 226 * 1024;  // one CTA per SM
-constexpr int kFusedOneSmem = kFusedSmemBudget - 2048;  // beside what the one-row kernel declares
+constexpr int kFusedSmem = 227 * 1024 - 1040;              // one CTA per SM, beside what the kernels declare
 constexpr int kFusedOnePairSmem = 223 * 512;               // two CTAs per SM
 constexpr int kFusedBarrierSlots = 64;
 constexpr int kFusedMaxGrid = 256;
@@ -64,9 +63,9 @@ enum FusedWaitCode : unsigned int {
     kWaitFusedGrid = 0x203,
 };
 
-// Grid-barrier counters, one slot per launch in flight (launch n uses slot n % 64).  Every launch
+// Counters of the meetings, one slot per launch in flight (launch n uses slot n % 64).  Every launch
 // adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses --
-// unless a bounded wait gave up and left its slot short; mt_device_status(reset) zeroes the slots again.
+// but for the self test of a bounded wait, which leaves one short; mt_device_status(reset) zeroes the slots again.
 __device__ unsigned long long g_fused_barrier[kFusedBarrierSlots];
 
 // Down rows that their CTA has left to the last CTA of the launch, a flag per CTA (FusedMeeting); all zero between launches.
@@ -90,7 +89,7 @@ struct FusedMlpParams {
     uint16_t* hidden;          // [1, I] bf16, written then read
     uint16_t* out;             // [1, H]
     unsigned long long* barrier;
-    unsigned int* left;        // one-row kernel only: its slot of g_fused_left
+    unsigned int* left;        // its slot of g_fused_left
     unsigned int patience_ns;
     int M, H, I;
 };
@@ -122,7 +121,7 @@ __host__ __device__ inline FusedOneLayout fused_one_layout(int M, int H, int I, 
     constexpr int kBars = 8 * (kFusedOneWarps * kFusedMaxSlots + 2) + 16;
     const int fixed = 1024 + tables1 + tables2 + scratch + kBars;
     const bool pair = kFusedOnePairSmem - fixed >= 2 * kFusedOneWarps * kOneRowItemBytes;
-    const int left = (pair ? kFusedOnePairSmem : kFusedOneSmem) - fixed;
+    const int left = (pair ? kFusedOnePairSmem : kFusedSmem) - fixed;
     l.depth = left / (kFusedOneWarps * kOneRowItemBytes);
     if (l.depth > units) l.depth = units;
     if (l.depth > kFusedMaxSlots) l.depth = kFusedMaxSlots;
@@ -154,7 +153,7 @@ __host__ __device__ inline FusedMlpLayout fused_mlp_layout(int H, int I) {
     const int scratch_bytes = 4 * kFusedComputeWarps * 2 * 16 * 8;  // per-item partial tiles
     const int bars_bytes = 8 * (2 * kFusedMaxSlots) + 16;
     const int fixed = scratch_bytes + bars_bytes + 128;
-    int slots = (kFusedSmemBudget - fixed) / l.item_bytes;
+    int slots = (kFusedSmem - fixed) / l.item_bytes;
     if (slots > kFusedMaxSlots) slots = kFusedMaxSlots;
     l.slots = slots;
     l.ring = 0;
@@ -169,48 +168,23 @@ __device__ __forceinline__ void fused_compute_sync() {
     asm volatile("bar.sync 1, %0;" ::"r"(kFusedComputeThreads) : "memory");
 }
 
-// The grid-wide barrier, called by the compute warps: every CTA arrives once; the slot grows by
-// gridDim.x per launch.
-__device__ __forceinline__ void fused_grid_barrier(unsigned long long* slot, int grid, volatile int* abort_flag,
-                                                   unsigned long long limit_ns = ptx::kWaitLimitNs) {
-    fused_compute_sync();  // orders this CTA's stores before thread 0's release
-    if (threadIdx.x == 0) {
-        // Release: this CTA's stores are visible to whoever acquires the counter afterwards; the
-        // acquire loads below pair with the other CTAs' releases.
-        const unsigned long long arrived = ptx::atom_add_release_gpu_u64(slot, 1ull);
-        const unsigned long long target = (arrived / (unsigned long long)grid + 1ull) * (unsigned long long)grid;
-        const unsigned long long start = ptx::global_timer_ns();
-        while (ptx::ld_acquire_gpu_u64(slot) < target) {
-            if (ptx::global_timer_ns() - start > limit_ns) {
-                if (atomicCAS(&g_device_status[0], 0u, (unsigned int)kWaitFusedGrid) == 0u) {
-                    g_device_status[1] = blockIdx.x;
-                    g_device_status[2] = threadIdx.x;
-                    g_device_status[3] = 0;
-                }
-                *abort_flag = 1;
-                break;
-            }
-        }
-    }
-    fused_compute_sync();
-}
-
 // The producer warp of the eight-column kernel: streams the CTA's items through the ring.  Weights do
 // not depend on the preceding kernel, so nothing here waits for it.  The gate|up rows of an item arrive as
 // 128-byte-wide tensor-map boxes (32 words x 16 rows, 128-byte swizzle; layout [matrix][H/256 column
 // blocks][16 rows][128 B]), which keeps the fragment loads free of bank conflicts.  A box is always 16
-// rows: rows past the CTA's share (or past the tensor, zero-filled) are simply not used.
+// rows: rows past the CTA's share (or past the tensor, zero-filled) are simply not used.  `first`: items before these, 0 or
+// (other CTAs' down rows, which fit the ring) all of them read.
 __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const FusedMlpLayout& lay, uint8_t* ring,
                                                uint64_t* full_bar, uint64_t* empty_bar, volatile int* abort_flag,
-                                               int lane, int row1, int n1, int row2, int n2) {
+                                               int lane, int first, int row1, int n1, int row2, int n2) {
     const int H = p.H, I = p.I;
     const int items1 = (n1 + kFusedItemRows - 1) / kFusedItemRows;
     const int items2 = (n2 + lay.down_rows - 1) / lay.down_rows;
     const int rb1 = H >> 1, rb2 = I >> 1, sb1 = H >> 5, sb2 = I >> 5;
     const int slots = lay.slots;
     for (int it = 0; it < items1 + items2; ++it) {
-        const int slot = it % slots, use = it / slots;
-        if (use > 0 && !ptx::mbar_wait(&empty_bar[slot], (uint32_t)(use - 1) & 1u, abort_flag, kWaitFusedEmpty)) break;
+        const int slot = (first + it) % slots, use = (first + it) / slots;
+        if (use > 0 && first == 0 && !ptx::mbar_wait(&empty_bar[slot], (uint32_t)(use - 1) & 1u, abort_flag, kWaitFusedEmpty)) break;
         __syncwarp();
         uint8_t* dst = ring + (size_t)slot * lay.item_bytes;
         if (it < items1) {
@@ -248,7 +222,7 @@ __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const Fu
     }
 }
 
-// How the CTAs of the one-row kernel meet between the projections, in an ordinary launch (a cooperative one does not begin before the
+// How the CTAs of both kernels meet between the projections, in an ordinary launch (a cooperative one does not begin before the
 // kernel in front has left the chip: 2048 / 8192, launch after launch, 16.2 us, so 13.0).  Nothing then says that all CTAs are on
 // the chip together: beside another stream's kernel, or another such launch, some may not start before others have left.  So
 // none waits for good: a CTA whose patience ends leaves its down rows to the last CTA to arrive, and makes room.
@@ -514,7 +488,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
 // 1-8 rows (22 us with dense rows, 20.3 us before the wide table loads) against 25.4-25.9 us on the
 // two-kernel tensor-core path, so it is the default for two to eight rows.
 //
-// Same producer, ring and grid barrier.  The K range is cut into one slice per compute warp; every
+// A producer warp feeds one ring; the CTAs meet as above.  The K range is cut into one slice per compute warp; every
 // warp walks all rows of an item for its slice; the warps' partial 16 x 8 tiles meet in shared memory
 // and are added in warp order.  Activation fragments hold element pairs in the order the unpack emits
 // them: (e0,e4), (e1,e5), (e2,e6), (e3,e7).
@@ -643,14 +617,22 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
 
     const int row1 = (int)((unsigned)I * (unsigned)cta / (unsigned)grid);
     const int n1 = (int)((unsigned)I * (unsigned)(cta + 1) / (unsigned)grid) - row1;
-    const int row2 = (int)((unsigned)H * (unsigned)cta / (unsigned)grid);
-    const int n2 = (int)((unsigned)H * (unsigned)(cta + 1) / (unsigned)grid) - row2;
+    int row2, n2, items2;
+    auto down_rows_of = [&](int owner) {
+        row2 = (int)((unsigned)H * (unsigned)owner / (unsigned)grid);
+        n2 = (int)((unsigned)H * (unsigned)(owner + 1) / (unsigned)grid) - row2;
+        items2 = (n2 + lay.down_rows - 1) / lay.down_rows;
+    };
+    down_rows_of(cta);
     const int items1 = (n1 + kFusedItemRows - 1) / kFusedItemRows;
-    const int items2 = (n2 + lay.down_rows - 1) / lay.down_rows;
+    const int own_items = items1 + items2;
+    int first_down = items1;  // items before the present down rows
     const int rb1 = H >> 1, rb2 = I >> 1, sb1 = H >> 5, sb2 = I >> 5;
     const int slots = lay.slots;
 
+    __shared__ int meeting, left_count, left_ctas[kFusedMaxGrid], next_owner[2];
     if (threadIdx.x == 0) {
+        left_count = 0;
         for (int i = 0; i < kFusedMaxSlots; ++i) {
             ptx::mbar_init(&full_bar[i], 1);
             ptx::mbar_init(&empty_bar[i], kFusedComputeWarps);
@@ -665,17 +647,28 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             ptx::prefetch_tensor_map(&p.gate_map);
             ptx::prefetch_tensor_map(&p.up_map);
         }
-        fused_producer(p, lay, ring, full_bar, empty_bar, abort_flag, lane, row1, n1, row2, n2);
-        return;
+        fused_producer(p, lay, ring, full_bar, empty_bar, abort_flag, lane, 0, row1, n1, row2, n2);
+        for (int next = 0;; ++next) {  // down rows that others have left
+            ptx::named_barrier_sync(2, kFusedThreads);
+            const int owner = next_owner[next & 1];
+            if (owner < 0) return;
+            first_down += items2;
+            down_rows_of(owner);
+            fused_producer(p, lay, ring, full_bar, empty_bar, abort_flag, lane, first_down, 0, 0, row2, n2);
+        }
     }
 
     // ---------------------------------------------------------------------- compute warps
     ptx::griddep_wait();  // the activations and the residual are the preceding kernel's output
-    float residual_value = 0.0f;
-    if ((int)threadIdx.x < n2 * M && p.residual) {
-        const int row = threadIdx.x / M, m = threadIdx.x - row * M;
-        residual_value = bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + (size_t)m * H + row2 + row));
-    }
+    float residual_value;
+    auto fetch_residual = [&] {
+        residual_value = 0.0f;
+        if ((int)threadIdx.x < n2 * M && p.residual) {
+            const int row = threadIdx.x / M, m = threadIdx.x - row * M;
+            residual_value = bf16_bits_to_f32(ptx::ld_global_dependent_u16(p.residual + (size_t)m * H + row2 + row));
+        }
+    };
+    fetch_residual();
     const bool active = g < M;  // fragment column g carries activation row g
     bool alive = true;
     {
@@ -760,7 +753,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
                     }
                 }
             }
-            if (it + slots < items1 + items2) {
+            if (it + slots < own_items) {
                 ptx::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&empty_bar[slot]);
@@ -785,8 +778,11 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             fused_compute_sync();
         }
     }
-    fused_grid_barrier(p.barrier, grid, abort_flag);
-    {
+    fused_compute_sync();
+    if (threadIdx.x == 0) meeting = fused_meet(p, (unsigned)grid, (unsigned)cta);
+    fused_compute_sync();
+    const int met = meeting;
+    for (int next = 0;; ++next) {
         // ------------------------------------------------------------------ down
         const int groups = (I >> 6) / kFusedComputeWarps;
         const int group0 = warp * groups;
@@ -800,13 +796,13 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             const bool upper = r_hi < n2;
             const int j_lo = r_lo / lay.down_rows, j_hi = upper ? r_hi / lay.down_rows : j_lo;
             for (int j = j_lo; j <= j_hi; ++j) {
-                const int it = items1 + j;
+                const int it = first_down + j;
                 if (alive && !ptx::mbar_wait(&full_bar[it % slots], (uint32_t)(it / slots) & 1u, abort_flag, kWaitFusedFull))
                     alive = false;
             }
             alive = __all_sync(0xFFFFFFFFu, alive);
-            const uint8_t* item_lo = ring + (size_t)((items1 + j_lo) % slots) * lay.item_bytes;
-            const uint8_t* item_hi = ring + (size_t)((items1 + j_hi) % slots) * lay.item_bytes;
+            const uint8_t* item_lo = ring + (size_t)((first_down + j_lo) % slots) * lay.item_bytes;
+            const uint8_t* item_hi = ring + (size_t)((first_down + j_hi) % slots) * lay.item_bytes;
             const int local_lo = r_lo - j_lo * lay.down_rows + g, local_hi = r_hi - j_hi * lay.down_rows + g;
             const uint8_t* lower = item_lo + local_lo * rb2 + t * 8;
             const uint8_t* upper_row = item_hi + local_hi * rb2 + t * 8;
@@ -867,8 +863,8 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             }
             // Hand back the items that end inside this tile.
             while (released < items2 && (released + 1) * lay.down_rows <= 16 * (tile + 1)) {
-                const int it = items1 + released;
-                if (it + slots < items1 + items2) {
+                const int it = first_down + released;
+                if (it + slots < own_items) {
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(&empty_bar[it % slots]);
@@ -880,7 +876,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             *reinterpret_cast<float2*>(part + (g + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
             fused_compute_sync();
             const int rows_here = min(16, n2 - 16 * tile);
-            for (int idx = threadIdx.x; idx < rows_here * M; idx += kFusedComputeThreads) {
+            for (int idx = threadIdx.x; idx < rows_here * M && met != kMeetLeft; idx += kFusedComputeThreads) {
                 const int row = idx / M, m = idx - row * M;
                 float v = 0.0f;
                 for (int w = 0; w < kFusedComputeWarps; ++w) v += scratch[(w * 16 + row) * 8 + m];
@@ -893,7 +889,21 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             }
             fused_compute_sync();
         }
+        if (met == kMeetLast && next == 0 && (int)threadIdx.x < grid && atomicExch(p.left + threadIdx.x, 0u) == 1u) {
+            left_ctas[atomicAdd(&left_count, 1)] = threadIdx.x;
+            ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
+        }
+        ptx::fence_proxy_async_smem();  // the ring is filled again
+        fused_compute_sync();
+        if (threadIdx.x == 0) next_owner[next & 1] = next < left_count && !*abort_flag ? left_ctas[next] : -1;
+        ptx::named_barrier_sync(2, kFusedThreads);  // the producer, too
+        const int owner = next_owner[next & 1];
+        if (owner < 0) break;
+        first_down += items2;
+        down_rows_of(owner);
+        fetch_residual();
     }
+    if (*abort_flag) ptx::drain_copies();
 }
 
 // Whether the eight-column kernel serves this problem.
@@ -903,9 +913,10 @@ inline bool fused_mlp_mma_applicable(const FusedMlpParams& p, int sm_count) {
     if (p.I < 512 || p.I % (64 * kFusedComputeWarps)) return false;
     const FusedMlpLayout lay = fused_mlp_layout(p.H, p.I);
     if (lay.slots < 2 || lay.down_rows < 8 || lay.down_rows % 8) return false;
+    if (((p.H + sm_count - 1) / sm_count + lay.down_rows - 1) / lay.down_rows > lay.slots) return false;
     if (16 * p.M > kFusedComputeThreads) return false;
     if (p.H % 256 || lay.item_bytes % 1024) return false;  // whole tensor-map boxes, swizzle-aligned items
-    if (lay.total + 1024 > kFusedSmemBudget) return false;
+    if (lay.total + 1024 > kFusedSmem || sm_count > kFusedMaxGrid) return false;
     const void* pointers[] = {p.x, p.gate_w, p.up_w, p.down_w, p.gate_s, p.gate_b, p.up_s, p.up_b, p.down_s, p.down_b,
                               p.hidden};
     for (const void* ptr : pointers)
@@ -929,20 +940,14 @@ inline bool fused_mlp_applicable(const FusedMlpParams& p, int sm_count) {
     return true;
 }
 
-// 0 = untried, 1 = programmatic dependent launch accepted together with a cooperative launch, -1 = refused.
-static int g_fused_pdl_state[64] = {};
-
 template <int kThreads>  // of a CTA, which also separates the kernels' static state
 inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int smem, const FusedMlpParams& params,
                                    int sm_count, int device, cudaStream_t stream) {
     static bool configured[64] = {};
     if (!configured[device]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmemBudget) != cudaSuccess)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmem) != cudaSuccess)
             return MT_ERR_LAUNCH;
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        int resident = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, smem) != cudaSuccess || resident < 1)
-            return MT_ERR_LAUNCH;
         configured[device] = true;
     }
     cudaLaunchConfig_t config = {};
@@ -950,26 +955,11 @@ inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int sme
     config.blockDim = dim3(kThreads, 1, 1);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
-    cudaLaunchAttribute attrs[2];
-    attrs[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident together: they meet at a grid barrier
-    attrs[0].val.cooperative = 1;
-    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attrs[1];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attrs;
-    // Whether the two attributes combine is decided by one trial launch outside stream capture (a
-    // refused launch would invalidate a capture); until then captures use the cooperative attribute alone.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(stream, &capturing);
-    if (g_fused_pdl_state[device] == 0 && capturing == cudaStreamCaptureStatusNone) {
-        config.numAttrs = 2;
-        if (cudaLaunchKernelEx(&config, kernel, params) == cudaSuccess) {
-            g_fused_pdl_state[device] = 1;
-            return MT_OK;
-        }
-        cudaGetLastError();
-        g_fused_pdl_state[device] = -1;
-    }
-    config.numAttrs = g_fused_pdl_state[device] == 1 ? 2 : 1;
+    config.numAttrs = 1;
     return cudaLaunchKernelEx(&config, kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
@@ -1010,24 +1000,7 @@ inline int launch_mlp_fused(FusedMlpParams params, int sm_count, bool mma, cudaS
         !encode_weight_map(&params.up_map, params.up_w, params.H, params.I, lay.tile1) ||
         !encode_weight_map(&params.down_map, params.down_w, params.I, params.H, lay.tile2))
         return MT_ERR_LAUNCH;
-    static bool configured[64] = {};
-    if (!configured[device]) {
-        if (cudaFuncSetAttribute(affine_mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedOneSmem) != cudaSuccess)
-            return MT_ERR_LAUNCH;
-        cudaFuncSetAttribute(affine_mlp_fused_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        configured[device] = true;
-    }
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(sm_count, 1, 1);
-    config.blockDim = dim3(kFusedOneThreads, 1, 1);
-    config.dynamicSmemBytes = lay.total + 1024;
-    config.stream = stream;
-    cudaLaunchAttribute attrs[1];
-    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attrs;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, affine_mlp_fused_kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
+    return launch_mlp_fused_kernel<kFusedOneThreads>(affine_mlp_fused_kernel, lay.total + 1024, params, sm_count, device, stream);
 }
 
 }  // namespace mt

@@ -222,13 +222,38 @@ __global__ void selftest_mbarrier_wait_kernel(unsigned long long limit_ns) {
     ptx::mbar_wait(&bar, 0, &abort_flag, kWaitSelfTest, limit_ns);
 }
 
+// A wait for all CTAs of a grid to arrive at a slot, with a limit.
+__device__ __forceinline__ void selftest_grid_barrier(unsigned long long* slot, int grid, volatile int* abort_flag,
+                                                   unsigned long long limit_ns = ptx::kWaitLimitNs) {
+    __syncthreads();  // orders this CTA's stores before thread 0's release
+    if (threadIdx.x == 0) {
+        // Release: this CTA's stores are visible to whoever acquires the counter afterwards; the
+        // acquire loads below pair with the other CTAs' releases.
+        const unsigned long long arrived = ptx::atom_add_release_gpu_u64(slot, 1ull);
+        const unsigned long long target = (arrived / (unsigned long long)grid + 1ull) * (unsigned long long)grid;
+        const unsigned long long start = ptx::global_timer_ns();
+        while (ptx::ld_acquire_gpu_u64(slot) < target) {
+            if (ptx::global_timer_ns() - start > limit_ns) {
+                if (atomicCAS(&g_device_status[0], 0u, (unsigned int)kWaitFusedGrid) == 0u) {
+                    g_device_status[1] = blockIdx.x;
+                    g_device_status[2] = threadIdx.x;
+                    g_device_status[3] = 0;
+                }
+                *abort_flag = 1;
+                break;
+            }
+        }
+    }
+    __syncthreads();
+}
+
 // Two CTAs meet at the single-launch MLP's grid barrier with a target no arrival count can reach.
 __global__ void __launch_bounds__(kFusedComputeThreads)
 selftest_grid_barrier_kernel(unsigned long long* slot, unsigned long long limit_ns) {
     __shared__ int abort_flag;
     if (threadIdx.x == 0) abort_flag = 0;
     __syncthreads();
-    fused_grid_barrier(slot, (int)gridDim.x + 1, &abort_flag, limit_ns);
+    selftest_grid_barrier(slot, (int)gridDim.x + 1, &abort_flag, limit_ns);
 }
 
 }  // namespace mt
@@ -384,8 +409,7 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         const bool mma = !one_row && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
         if (one_row || mma) {
             const int fused_rc = launch_mlp_fused(params, sms, mma, static_cast<cudaStream_t>(stream));
-            // A cooperative launch is refused when the whole grid cannot be resident (a GPU shared with
-            // another context, a carve-out that leaves too little shared memory).  Nothing was queued:
+            // A launch may be refused (a GPU shared with another context that leaves too little shared memory).  Nothing was queued:
             // the default dispatch then takes the two-kernel path; an explicit request reports it.
             if (fused_rc != MT_ERR_LAUNCH || family) return fused_rc;
             cudaGetLastError();

@@ -386,15 +386,18 @@ def test_a_model_embeds_as_its_module_does(cuda_device, change):
     assert found.dtype == wanted.dtype and torch.equal(found, wanted) and found.requires_grad == wanted.requires_grad
 
 
-@pytest.mark.parametrize("rows,hidden,inter", [(1, 1024, 1024), (1, 2048, 8192), (1, 4096, 2048), (1, 1024, 8192), (3, 4096, 8192)])
-def test_single_launch_mlp_whose_ctas_do_not_wait(cuda_device, rows, hidden, inter):
+@pytest.mark.parametrize("family,rows,hidden,inter", [
+    ("mlp_fused", 1, 1024, 1024), ("mlp_fused", 1, 2048, 8192), ("mlp_fused", 1, 4096, 2048), ("mlp_fused", 1, 1024, 8192),
+    ("mlp_fused", 3, 4096, 8192), ("mlp_fused_mma", 8, 2048, 8192), ("mlp_fused_mma", 2, 512, 1536), ("mlp_fused_mma", 5, 2048, 1024),
+])
+def test_single_launch_mlp_whose_ctas_do_not_wait(cuda_device, family, rows, hidden, inter):
     """Between the projections a CTA may leave its down rows to the last CTA to arrive, as it does when others are kept off
     the chip.  Without patience nearly all do; whoever sums a row, its bits are the same."""
     gate, up, down = synth.mlp_weights(330, hidden, inter, cuda_device)
     x, res = synth.activations(5, rows, hidden, cuda_device), synth.activations(6, rows, hidden, cuda_device)
     execute = B.mlx_affine_mlp_executor(x, *gate, *up, *down, res)
     state = cuda_quantized._state
-    with B.force_kernel("mlp_fused"):
+    with B.force_kernel(family):
         want = execute(x, res)
         state.flags |= _lib.FLAG_MLP_IMPATIENT
         for _ in range(100):  # more launches than barrier slots
@@ -405,7 +408,7 @@ def test_single_launch_mlp_whose_ctas_do_not_wait(cuda_device, rows, hidden, int
     for stream in streams:
         stream.wait_stream(torch.cuda.current_stream())
     executors = [B.mlx_affine_mlp_executor(x, *gate, *up, *down, res) for _ in streams]
-    with B.force_kernel("mlp_fused"):
+    with B.force_kernel(family):
         for _ in range(10):  # side by side: some CTAs find no room while others wait
             for out, stream, run in zip(outs, streams, executors):
                 with torch.cuda.stream(stream):
