@@ -49,7 +49,8 @@
  *   MT_FLAG_GELU (16)        mt_dense_act: x/(1+exp(-1.702x)) instead of SiLU
  *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch one-row kernel (M <= 4); -1
  *                            when it does not apply.  With flags = 0 the default dispatch falls back
- *                            to the two-kernel path if the driver refuses the launch.
+ *                            to the two-kernel path if the driver refuses the launch, or if a
+ *                            captured launch finds no slot for the meeting of its CTAs.
  *   MT_FLAG_HOST_PAIR (64)   mt_affine_mlp_host: see there
  *   MT_FLAG_MLP_FUSED_MMA (128) mt_affine_mlp: insist on the mma.sync single-launch kernel (M <= 8);
  *                            -1 when it does not apply.

@@ -17,7 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUTPUT = os.path.join(CSRC, "libmetile_b200.so")
 SOURCES = ("metile_b200.cu",)
-HEADERS = ("common.cuh", "ptx.cuh", "affine_gemv.cuh", "affine_gemv_mma.cuh", "affine_umma.cuh", "affine_mlp_fused.cuh", "add_rmsnorm.cuh", "gather_rows.cuh", "attention_decode.cuh", "peer_reduce.cuh",
+HEADERS = ("common.cuh", "ptx.cuh", "affine_gemv.cuh", "affine_gemv_mma.cuh", "affine_umma.cuh", "affine_mlp_fused.cuh", "meeting_slots.h", "add_rmsnorm.cuh", "gather_rows.cuh", "attention_decode.cuh", "peer_reduce.cuh",
            "dense_rows.cuh", os.path.join("..", "..", "include", "metile_b200.h"))
 BINDING_SOURCE = os.path.join(CSRC, "binding.cpp")
 BINDING_OUTPUT = os.path.join(HERE, "_native.so")

@@ -33,6 +33,7 @@
 
 #include "affine_gemv_mma.cuh"
 #include "common.cuh"
+#include "meeting_slots.h"
 #include "ptx.cuh"
 
 namespace mt {
@@ -53,7 +54,6 @@ constexpr int kFusedMaxSlots = 12;
 constexpr int kFusedItemRows = 16;  // gate/up rows per ring item of the eight-column kernel
 constexpr int kFusedSmem = 227 * 1024 - 1040;              // one CTA per SM, beside what the kernels declare
 constexpr int kFusedOnePairSmem = 223 * 512;               // two CTAs per SM
-constexpr int kFusedBarrierSlots = 64;
 constexpr int kFusedMaxGrid = 256;
 constexpr unsigned int kFusedPatienceNs = 100000;
 
@@ -63,13 +63,13 @@ enum FusedWaitCode : unsigned int {
     kWaitFusedGrid = 0x203,
 };
 
-// Counters of the meetings, one slot per launch in flight (launch n uses slot n % 64).  Every launch
-// adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses --
+// Counters of the meetings, one per slot; launches that may run at the same time have different slots (meeting_slots.h).
+// Every launch adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses --
 // but for the self test of a bounded wait, which leaves one short; mt_device_status(reset) zeroes the slots again.
-__device__ unsigned long long g_fused_barrier[kFusedBarrierSlots];
+__device__ unsigned long long g_fused_barrier[kMeetingSlotsInAll];
 
 // Down rows that their CTA has left to the last CTA of the launch, a flag per CTA (FusedMeeting); all zero between launches.
-__device__ unsigned int g_fused_left[kFusedBarrierSlots][kFusedMaxGrid];
+__device__ unsigned int g_fused_left[kMeetingSlotsInAll][kFusedMaxGrid];
 
 struct FusedMlpParams {
     CUtensorMap gate_map;      // gate_w / up_w as [I, H/8] uint32 tensors, boxes of 32 words x a tile's rows with the
@@ -963,23 +963,69 @@ inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int sme
     return cudaLaunchKernelEx(&config, kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
-// The barrier slot of the next launch on the current device (slots rotate, one per launch in flight), and its flags.
-inline bool next_fused_barrier_slot(unsigned long long*& barrier, unsigned int*& left) {
+inline MeetingSlots& meeting_slots() {
+    static MeetingSlots* const slots = new MeetingSlots;  // never destroyed: graphs may outlive everything else
+    return *slots;
+}
+
+inline void CUDART_CB give_back_meeting_slot(void* slot) { meeting_slots().give_back((int)reinterpret_cast<intptr_t>(slot)); }
+
+// The slot of a launch into `stream`; -1 when there is none.  The graph that is being captured keeps the slot of its launches,
+// and so does whatever is instantiated from it, until the last of them is destroyed.
+inline int meeting_slot_of(cudaStream_t stream) {
+    cudaStreamCaptureStatus status;
+    unsigned long long capture = 0, id = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(stream, &status, &capture, &graph) != cudaSuccess) return -1;
+    if (status == cudaStreamCaptureStatusNone) return cudaStreamGetId(stream, &id) == cudaSuccess ? meeting_slots().of_stream(id) : -1;
+    if (status != cudaStreamCaptureStatusActive) return -1;
+    static thread_local char thread;  // a capturing stream does not tell its id (and asking ends the capture)
+    bool fresh = false;
+    const int slot = meeting_slots().of_capture(capture, reinterpret_cast<uintptr_t>(stream == cudaStreamPerThread ? (void*)&thread : (void*)stream), fresh);
+    if (slot < 0 || !fresh) return slot;
+    cudaUserObject_t keeper;
+    if (cudaUserObjectCreate(&keeper, reinterpret_cast<void*>((intptr_t)slot), give_back_meeting_slot, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        meeting_slots().give_back(slot);
+        return -1;
+    }
+    if (cudaGraphRetainUserObject(graph, keeper, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaUserObjectRelease(keeper, 1);  // gives the slot back
+        return -1;
+    }
+    return slot;
+}
+
+// The counter and the flags of a slot on the current device.
+inline bool meeting_slot_memory(int slot, unsigned long long*& barrier, unsigned int*& left) {
     static unsigned long long* slots[64] = {};
     static unsigned int* flags[64] = {};
-    static unsigned int launches = 0;
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
-    if (!slots[device]) {
+    if (!__atomic_load_n(&slots[device], __ATOMIC_ACQUIRE)) {
         void *first = nullptr, *second = nullptr;
         if (cudaGetSymbolAddress(&first, g_fused_barrier) != cudaSuccess || cudaGetSymbolAddress(&second, g_fused_left) != cudaSuccess) return false;
-        flags[device] = static_cast<unsigned int*>(second);
+        __atomic_store_n(&flags[device], static_cast<unsigned int*>(second), __ATOMIC_RELAXED);
         __atomic_store_n(&slots[device], static_cast<unsigned long long*>(first), __ATOMIC_RELEASE);
     }
-    const unsigned int slot = __atomic_fetch_add(&launches, 1u, __ATOMIC_RELAXED) % kFusedBarrierSlots;
     barrier = slots[device] + slot;
-    left = flags[device] + slot * kFusedMaxGrid;
+    left = __atomic_load_n(&flags[device], __ATOMIC_RELAXED) + slot * kFusedMaxGrid;
     return true;
+}
+
+// `launch` in its turn among the launches that share a slot although their streams do not: each begins behind the one before it.
+template <typename Launch>
+inline int launch_in_turn(int device, cudaStream_t stream, Launch&& launch) {
+    static std::mutex mutex;
+    static cudaEvent_t last[64] = {};
+    const std::lock_guard<std::mutex> lock(mutex);
+    if (!last[device] && cudaEventCreateWithFlags(&last[device], cudaEventDisableTiming) != cudaSuccess) {
+        last[device] = nullptr;
+        return MT_ERR_LAUNCH;
+    }
+    if (cudaStreamWaitEvent(stream, last[device], 0) != cudaSuccess) return MT_ERR_LAUNCH;  // an event not yet recorded holds nothing up
+    const int rc = launch();
+    if (rc == MT_OK && cudaEventRecord(last[device], stream) != cudaSuccess) cudaStreamSynchronize(stream);
+    return rc;
 }
 
 // Caller has checked fused_mlp_applicable(), or fused_mlp_mma_applicable() when `mma` is set.
@@ -987,20 +1033,22 @@ inline int launch_mlp_fused(FusedMlpParams params, int sm_count, bool mma, cudaS
     int device = 0;
     cudaGetDevice(&device);
     if (device >= 64) return MT_ERR_DEVICE;
-    if (!next_fused_barrier_slot(params.barrier, params.left)) return MT_ERR_LAUNCH;
+    const int slot = meeting_slot_of(stream);
+    if (slot < 0 || !meeting_slot_memory(slot, params.barrier, params.left)) return MT_ERR_LAUNCH;
+    auto start = [&](auto&& launch) { return slot == kMeetingShared ? launch_in_turn(device, stream, launch) : launch(); };
     if (mma) {
         if (!encode_weight_map(&params.gate_map, params.gate_w, params.H, params.I, kFusedItemRows) ||
             !encode_weight_map(&params.up_map, params.up_w, params.H, params.I, kFusedItemRows))
             return MT_ERR_LAUNCH;
         const int smem = fused_mlp_layout(params.H, params.I).total + 1024;
-        return launch_mlp_fused_kernel<kFusedThreads>(affine_mlp_fused_mma_kernel, smem, params, sm_count, device, stream);
+        return start([&] { return launch_mlp_fused_kernel<kFusedThreads>(affine_mlp_fused_mma_kernel, smem, params, sm_count, device, stream); });
     }
     const FusedOneLayout lay = fused_one_layout(params.M, params.H, params.I, sm_count);
     if (!encode_weight_map(&params.gate_map, params.gate_w, params.H, params.I, lay.tile1) ||
         !encode_weight_map(&params.up_map, params.up_w, params.H, params.I, lay.tile1) ||
         !encode_weight_map(&params.down_map, params.down_w, params.I, params.H, lay.tile2))
         return MT_ERR_LAUNCH;
-    return launch_mlp_fused_kernel<kFusedOneThreads>(affine_mlp_fused_kernel, lay.total + 1024, params, sm_count, device, stream);
+    return start([&] { return launch_mlp_fused_kernel<kFusedOneThreads>(affine_mlp_fused_kernel, lay.total + 1024, params, sm_count, device, stream); });
 }
 
 }  // namespace mt

@@ -290,7 +290,7 @@ int mt_device_status(unsigned int words[4], int reset) {
         if (cudaMemcpyToSymbol(g_device_status, zeros, sizeof(zeros)) != cudaSuccess) return MT_ERR_LAUNCH;
         // A wait that gave up at the single-launch MLP's grid barrier leaves its counter short of a
         // multiple of the grid size; the device is idle here, so every counter can start over.
-        static const unsigned long long no_arrivals[kFusedBarrierSlots] = {};
+        static const unsigned long long no_arrivals[kMeetingSlotsInAll] = {};
         if (words[0] && cudaMemcpyToSymbol(g_fused_barrier, no_arrivals, sizeof(no_arrivals)) != cudaSuccess)
             return MT_ERR_LAUNCH;
     }
@@ -307,7 +307,7 @@ int mt_selftest_bounded_wait(int which, unsigned int limit_us, void* stream) {
     } else if (which == 1) {
         unsigned long long* slot = nullptr;
         unsigned int* left = nullptr;
-        if (!next_fused_barrier_slot(slot, left)) return MT_ERR_LAUNCH;
+        if (!meeting_slot_memory(kMeetingSelfTest, slot, left)) return MT_ERR_LAUNCH;
         selftest_grid_barrier_kernel<<<2, kFusedComputeThreads, 0, s>>>(slot, limit_ns);
     } else {
         return MT_ERR_SHAPE;
@@ -409,7 +409,8 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         const bool mma = !one_row && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
         if (one_row || mma) {
             const int fused_rc = launch_mlp_fused(params, sms, mma, static_cast<cudaStream_t>(stream));
-            // A launch may be refused (a GPU shared with another context that leaves too little shared memory).  Nothing was queued:
+            // A launch may be refused (a GPU shared with another context that leaves too little shared memory, no slot left for
+            // the meeting of a captured launch).  Nothing was queued:
             // the default dispatch then takes the two-kernel path; an explicit request reports it.
             if (fused_rc != MT_ERR_LAUNCH || family) return fused_rc;
             cudaGetLastError();

@@ -417,3 +417,77 @@ def test_single_launch_mlp_whose_ctas_do_not_wait(cuda_device, family, rows, hid
     for out in outs:
         for y in out:
             assert_bit_equal(y, want, "side by side")
+
+
+@pytest.mark.parametrize("family,rows,hidden,inter", [("mlp_fused", 1, 1024, 1024), ("mlp_fused_mma", 8, 512, 512)])
+def test_single_launch_mlps_of_many_streams_meet_apart(cuda_device, family, rows, hidden, inter):
+    """Queues of three streams that reach any two launches at once, and more streams than there are meeting slots."""
+    gate, up, down = synth.mlp_weights(331, hidden, inter, cuda_device)
+    count = 200
+    xs = [synth.activations(seed, rows, hidden, cuda_device) for seed in range(count)]
+    execute = B.mlx_affine_mlp_executor(xs[0], *gate, *up, *down, None)
+    with B.force_kernel(family):
+        wanted = [execute(x) for x in xs]
+        streams = [torch.cuda.Stream() for _ in range(3)]
+        outs = [[] for _ in streams]
+        for stream in streams:
+            stream.wait_stream(torch.cuda.current_stream())
+        for out, stream in zip(outs, streams):
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(4_000_000)  # the queues fill up before they begin
+                out.extend(execute(x) for x in xs)
+        torch.cuda.synchronize()
+        for out in outs:
+            assert_bit_equal(torch.cat(out), torch.cat(wanted), "side by side")
+        # Streams without end: beyond 512 they share a slot, in turn.
+        runtime = torch.cuda.cudart()
+        handles = (ctypes.c_void_p * 700)()
+        outs = []
+        for i in range(len(handles)):
+            assert int(runtime.cudaStreamCreate(ctypes.addressof(handles) + 8 * i)) == 0
+            with torch.cuda.stream(torch.cuda.ExternalStream(handles[i])):
+                outs.append(execute(xs[i % count]))
+        torch.cuda.synchronize()
+        for handle in handles:
+            assert int(runtime.cudaStreamDestroy(handle)) == 0
+        for i, out in enumerate(outs):
+            assert torch.equal(out, wanted[i % count]), i
+    assert _lib.device_status()[0]
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_graphs_of_single_launch_mlps_side_by_side(cuda_device, batch):
+    """Two decoders of 32 blocks whose captures follow one another launch for launch, replayed on their own streams."""
+    from metile_b200.integrations.graphed import GraphedDecoder
+    from metile_b200.integrations.torch_lm import apply_metile_to_torch_lm
+
+    model = blocks.random_model(5, hidden=1024, intermediate=1024, heads=4, kv_heads=1, head_dim=64, layers=32, vocab=128,
+                                device=cuda_device)
+    with apply_metile_to_torch_lm(model, attention=True):
+        assert _lib.load().mt_affine_mlp_launches(batch, 1024, 1024, 0) == 1
+        prompts = [torch.randint(0, 128, (batch, 9), device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(seed))
+                   for seed in (1, 2)]
+        tokens = torch.randint(0, 128, (150, batch), device=cuda_device, generator=torch.Generator(cuda_device).manual_seed(3))
+        decoders = [GraphedDecoder(model, batch=batch, capacity=200) for _ in prompts]
+        wanted = []
+        for decoder, prompt in zip(decoders, prompts):
+            decoder.prefill(prompt)
+            wanted.append([decoder.step(token).clone() for token in tokens])
+        torch.cuda.synchronize()
+        found = [[], []]
+        for decoder in decoders:
+            for cache in decoder.cache:
+                cache.reset(9)
+            decoder.stream.wait_stream(torch.cuda.current_stream())
+        for decoder, logits in zip(decoders, found):  # each a queue of its own
+            with torch.cuda.stream(decoder.stream):
+                torch.cuda._sleep(10_000_000)
+        for token in tokens:
+            for decoder, logits in zip(decoders, found):
+                with torch.cuda.stream(decoder.stream):
+                    logits.append(decoder.step(token).clone())
+        torch.cuda.synchronize()
+    for a, b in zip(found, wanted):
+        for x, y in zip(a, b):
+            assert torch.equal(x, y)
+    assert _lib.device_status()[0]
