@@ -89,11 +89,13 @@ int mt_device_check(void);
 int mt_device_status(unsigned int words[4], int reset);
 
 /* Self-test of the bounded device-side waits: queues a tiny kernel whose wait can never be satisfied
- * (which = 0: an mbarrier nobody arrives at; which = 1: the single-launch MLP's grid barrier with an
- * unreachable target) and gives up after limit_us microseconds (1 ... 100000).  Nothing faults or
+ * (which = 0: an mbarrier nobody arrives at; which = 1: two of three CTAs at the meeting of the single-launch MLP)
+ * and gives up after limit_us microseconds (1 ... 100000).  Nothing faults or
  * hangs: the kernel records the wait code and returns, the next mt_device_status() reports -8 and,
- * with reset != 0, clears the record and the grid-barrier counters.  Production kernels run the same
- * wait code with a 2 s limit.  No counterpart in the reference project. */
+ * with reset != 0, clears the record and every meeting's counter and flags.  With which = 1 the third CTA comes afterwards
+ * and takes over what the two have left, as in an MLP, where nothing is then reported: the code is 0x203, or 0x2FF if the
+ * meeting did not go as it should; with which = 2 it never comes, and the meeting's slot stays as a launch that gave up leaves
+ * it.  The MLP's own patience is 100 us; an mbarrier is waited for 2 s.  No counterpart in the reference project. */
 int mt_selftest_bounded_wait(int which, unsigned int limit_us, void* stream);
 
 /* y = x @ dequant(w)^T (+ residual, added to the un-rounded sum).

@@ -60,16 +60,23 @@ constexpr unsigned int kFusedPatienceNs = 100000;
 enum FusedWaitCode : unsigned int {
     kWaitFusedFull = 0x201,
     kWaitFusedEmpty = 0x202,
-    kWaitFusedGrid = 0x203,
+    kWaitFusedMeeting = 0x203,       // reported by the self test alone: a CTA of an MLP that waits in vain leaves its rows
+    kWaitFusedMeetingWrong = 0x2FF,  // ... whose meeting did not go as it should
 };
 
 // Counters of the meetings, one per slot; launches that may run at the same time have different slots (meeting_slots.h).
-// Every launch adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses --
-// but for the self test of a bounded wait, which leaves one short; mt_device_status(reset) zeroes the slots again.
+// Every launch adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses, but behind a
+// launch that gave up (a copy that never landed); mt_device_status(reset) then zeroes counters and flags.
 __device__ unsigned long long g_fused_barrier[kMeetingSlotsInAll];
 
 // Down rows that their CTA has left to the last CTA of the launch, a flag per CTA (FusedMeeting); all zero between launches.
 __device__ unsigned int g_fused_left[kMeetingSlotsInAll][kFusedMaxGrid];
+
+struct FusedMeetingPlace {
+    unsigned long long* count;
+    unsigned int* left;        // a flag per CTA
+    unsigned int patience_ns;
+};
 
 struct FusedMlpParams {
     CUtensorMap gate_map;      // gate_w / up_w as [I, H/8] uint32 tensors, boxes of 32 words x a tile's rows with the
@@ -88,9 +95,7 @@ struct FusedMlpParams {
     const uint16_t* residual;  // [1, H] or null
     uint16_t* hidden;          // [1, I] bf16, written then read
     uint16_t* out;             // [1, H]
-    unsigned long long* barrier;
-    unsigned int* left;        // its slot of g_fused_left
-    unsigned int patience_ns;
+    FusedMeetingPlace meeting;
     int M, H, I;
 };
 
@@ -233,21 +238,28 @@ __device__ __forceinline__ void fused_producer(const FusedMlpParams& p, const Fu
 enum FusedMeeting : int { kMeetOpen, kMeetLast, kMeetLeft };  // kMeetLast: the last one, where some have left
 constexpr unsigned long long kMeetOneLeft = 1ull << 48;
 
-__device__ __forceinline__ int fused_meet(const FusedMlpParams& p, unsigned int grid, unsigned int cta) {
+__device__ __forceinline__ int fused_meet(const FusedMeetingPlace& at, unsigned int grid, unsigned int cta) {
     // Release: the hidden activations of this CTA (ordered by the caller's barrier) are visible to whoever acquires the count.
-    const unsigned long long before = ptx::atom_add_acq_rel_gpu_u64(p.barrier, 1ull), arrived = before % kMeetOneLeft;
+    const unsigned long long before = ptx::atom_add_acq_rel_gpu_u64(at.count, 1ull), arrived = before % kMeetOneLeft;
     const unsigned long long target = (arrived / grid + 1ull) * grid;
     if (arrived + 1ull == target) return before >= kMeetOneLeft ? kMeetLast : kMeetOpen;
     const unsigned long long start = ptx::global_timer_ns();
-    while (ptx::ld_acquire_gpu_u64(p.barrier) % kMeetOneLeft < target) {
-        if (ptx::global_timer_ns() - start < p.patience_ns) continue;
-        atomicExch(p.left + cta, 1u);
-        if (ptx::atom_add_acq_rel_gpu_u64(p.barrier, kMeetOneLeft) % kMeetOneLeft < target) return kMeetLeft;
-        if (atomicExch(p.left + cta, 0u) == 0u) return kMeetLeft;  // the last CTA saw the flag on its way to another's
-        ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
+    while (ptx::ld_acquire_gpu_u64(at.count) % kMeetOneLeft < target) {
+        if (ptx::global_timer_ns() - start < at.patience_ns) continue;
+        atomicExch(at.left + cta, 1u);
+        if (ptx::atom_add_acq_rel_gpu_u64(at.count, kMeetOneLeft) % kMeetOneLeft < target) return kMeetLeft;
+        if (atomicExch(at.left + cta, 0u) == 0u) return kMeetLeft;  // the last CTA saw the flag on its way to another's
+        ptx::atom_add_acq_rel_gpu_u64(at.count, 0ull - kMeetOneLeft);
         return kMeetOpen;
     }
     return kMeetOpen;
+}
+
+// Takes over the rows of `cta` if it has left them.
+__device__ __forceinline__ void fused_take_over(const FusedMeetingPlace& at, int cta, int* taken, int* count) {
+    if (atomicExch(at.left + cta, 0u) != 1u) return;
+    taken[atomicAdd(count, 1)] = cta;
+    ptx::atom_add_acq_rel_gpu_u64(at.count, 0ull - kMeetOneLeft);
 }
 
 // Lane (g, t)'s activations of a 512-column unit: the B registers of one_row_products, and the sums of groups 2t and 2t + 1.
@@ -441,7 +453,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
         p.hidden[(size_t)m * I + row1 + row] = f32_to_bf16_bits(swiglu_f32(gate, up));
     }
     __syncthreads();
-    if (threadIdx.x == 0) meeting = fused_meet(p, (unsigned)grid, (unsigned)cta);
+    if (threadIdx.x == 0) meeting = fused_meet(p.meeting, (unsigned)grid, (unsigned)cta);
     __syncthreads();
     const int met = meeting;
     for (int next = 0;; ++next) {
@@ -454,10 +466,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
             p.out[(size_t)m * H + row2 + row] = f32_to_bf16_bits(v + residual_value);
         }
         if (met != kMeetLast) break;
-        if (next == 0 && (int)threadIdx.x < grid && atomicExch(p.left + threadIdx.x, 0u) == 1u) {
-            left_ctas[atomicAdd(&left_count, 1)] = threadIdx.x;
-            ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
-        }
+        if (next == 0 && (int)threadIdx.x < grid) fused_take_over(p.meeting, threadIdx.x, left_ctas, &left_count);
         ptx::fence_proxy_async_smem();  // the tables are filled again
         __syncthreads();
         if (next == left_count || *abort_flag) break;
@@ -779,7 +788,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
         }
     }
     fused_compute_sync();
-    if (threadIdx.x == 0) meeting = fused_meet(p, (unsigned)grid, (unsigned)cta);
+    if (threadIdx.x == 0) meeting = fused_meet(p.meeting, (unsigned)grid, (unsigned)cta);
     fused_compute_sync();
     const int met = meeting;
     for (int next = 0;; ++next) {
@@ -889,10 +898,7 @@ affine_mlp_fused_mma_kernel(const __grid_constant__ FusedMlpParams p) {
             }
             fused_compute_sync();
         }
-        if (met == kMeetLast && next == 0 && (int)threadIdx.x < grid && atomicExch(p.left + threadIdx.x, 0u) == 1u) {
-            left_ctas[atomicAdd(&left_count, 1)] = threadIdx.x;
-            ptx::atom_add_acq_rel_gpu_u64(p.barrier, 0ull - kMeetOneLeft);
-        }
+        if (met == kMeetLast && next == 0 && (int)threadIdx.x < grid) fused_take_over(p.meeting, threadIdx.x, left_ctas, &left_count);
         ptx::fence_proxy_async_smem();  // the ring is filled again
         fused_compute_sync();
         if (threadIdx.x == 0) next_owner[next & 1] = next < left_count && !*abort_flag ? left_ctas[next] : -1;
@@ -996,20 +1002,27 @@ inline int meeting_slot_of(cudaStream_t stream) {
 }
 
 // The counter and the flags of a slot on the current device.
-inline bool meeting_slot_memory(int slot, unsigned long long*& barrier, unsigned int*& left) {
-    static unsigned long long* slots[64] = {};
+inline bool meeting_place_of(int slot, FusedMeetingPlace& place) {
+    static unsigned long long* counters[64] = {};
     static unsigned int* flags[64] = {};
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
-    if (!__atomic_load_n(&slots[device], __ATOMIC_ACQUIRE)) {
+    if (!__atomic_load_n(&counters[device], __ATOMIC_ACQUIRE)) {
         void *first = nullptr, *second = nullptr;
         if (cudaGetSymbolAddress(&first, g_fused_barrier) != cudaSuccess || cudaGetSymbolAddress(&second, g_fused_left) != cudaSuccess) return false;
         __atomic_store_n(&flags[device], static_cast<unsigned int*>(second), __ATOMIC_RELAXED);
-        __atomic_store_n(&slots[device], static_cast<unsigned long long*>(first), __ATOMIC_RELEASE);
+        __atomic_store_n(&counters[device], static_cast<unsigned long long*>(first), __ATOMIC_RELEASE);
     }
-    barrier = slots[device] + slot;
-    left = __atomic_load_n(&flags[device], __ATOMIC_RELAXED) + slot * kFusedMaxGrid;
+    place.count = __atomic_load_n(&counters[device], __ATOMIC_RELAXED) + slot;
+    place.left = __atomic_load_n(&flags[device], __ATOMIC_RELAXED) + slot * kFusedMaxGrid;
     return true;
+}
+
+// Every slot of the current device, which is idle, as it was in the beginning.
+inline bool clear_meeting_places() {
+    FusedMeetingPlace first;
+    return meeting_place_of(0, first) && cudaMemset(first.count, 0, sizeof(g_fused_barrier)) == cudaSuccess &&
+           cudaMemset(first.left, 0, sizeof(g_fused_left)) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
 }
 
 // `launch` in its turn among the launches that share a slot although their streams do not: each begins behind the one before it.
@@ -1034,7 +1047,7 @@ inline int launch_mlp_fused(FusedMlpParams params, int sm_count, bool mma, cudaS
     cudaGetDevice(&device);
     if (device >= 64) return MT_ERR_DEVICE;
     const int slot = meeting_slot_of(stream);
-    if (slot < 0 || !meeting_slot_memory(slot, params.barrier, params.left)) return MT_ERR_LAUNCH;
+    if (slot < 0 || !meeting_place_of(slot, params.meeting)) return MT_ERR_LAUNCH;
     auto start = [&](auto&& launch) { return slot == kMeetingShared ? launch_in_turn(device, stream, launch) : launch(); };
     if (mma) {
         if (!encode_weight_map(&params.gate_map, params.gate_w, params.H, params.I, kFusedItemRows) ||

@@ -222,38 +222,28 @@ __global__ void selftest_mbarrier_wait_kernel(unsigned long long limit_ns) {
     ptx::mbar_wait(&bar, 0, &abort_flag, kWaitSelfTest, limit_ns);
 }
 
-// A wait for all CTAs of a grid to arrive at a slot, with a limit.
-__device__ __forceinline__ void selftest_grid_barrier(unsigned long long* slot, int grid, volatile int* abort_flag,
-                                                   unsigned long long limit_ns = ptx::kWaitLimitNs) {
-    __syncthreads();  // orders this CTA's stores before thread 0's release
-    if (threadIdx.x == 0) {
-        // Release: this CTA's stores are visible to whoever acquires the counter afterwards; the
-        // acquire loads below pair with the other CTAs' releases.
-        const unsigned long long arrived = ptx::atom_add_release_gpu_u64(slot, 1ull);
-        const unsigned long long target = (arrived / (unsigned long long)grid + 1ull) * (unsigned long long)grid;
-        const unsigned long long start = ptx::global_timer_ns();
-        while (ptx::ld_acquire_gpu_u64(slot) < target) {
-            if (ptx::global_timer_ns() - start > limit_ns) {
-                if (atomicCAS(&g_device_status[0], 0u, (unsigned int)kWaitFusedGrid) == 0u) {
-                    g_device_status[1] = blockIdx.x;
-                    g_device_status[2] = threadIdx.x;
-                    g_device_status[3] = 0;
-                }
-                *abort_flag = 1;
-                break;
-            }
-        }
-    }
-    __syncthreads();
+__device__ __forceinline__ void selftest_record(unsigned int code) {
+    if (atomicCAS(&g_device_status[0], 0u, code) != 0u) return;
+    g_device_status[1] = blockIdx.x;
+    g_device_status[2] = threadIdx.x;
+    g_device_status[3] = 0;
 }
 
-// Two CTAs meet at the single-launch MLP's grid barrier with a target no arrival count can reach.
-__global__ void __launch_bounds__(kFusedComputeThreads)
-selftest_grid_barrier_kernel(unsigned long long* slot, unsigned long long limit_ns) {
-    __shared__ int abort_flag;
-    if (threadIdx.x == 0) abort_flag = 0;
-    __syncthreads();
-    selftest_grid_barrier(slot, (int)gridDim.x + 1, &abort_flag, limit_ns);
+// CTAs 0 and 1 of three come to a meeting of the single-launch MLP; the third comes in the next launch, or not at all.
+__global__ void selftest_meeting_left_kernel(FusedMeetingPlace at) {
+    selftest_record(fused_meet(at, 3, blockIdx.x) == kMeetLeft ? kWaitFusedMeeting : kWaitFusedMeetingWrong);
+}
+
+__global__ void selftest_meeting_last_kernel(FusedMeetingPlace at) {
+    __shared__ int taken[3], count;  // atomics do not reach local memory
+    count = 0;
+    const int met = fused_meet(at, 3, 2);
+    for (int cta = 0; cta < 3; ++cta) fused_take_over(at, cta, taken, &count);
+    // Both have left their rows, and the slot is as it was but for the three arrivals.
+    bool right = met == kMeetLast && count == 2 && taken[0] == 0 && taken[1] == 1 && ptx::ld_acquire_gpu_u64(at.count) % 3 == 0 &&
+                 ptx::ld_acquire_gpu_u64(at.count) < kMeetOneLeft;
+    for (int cta = 0; cta < 3; ++cta) right = right && atomicAdd(at.left + cta, 0u) == 0u;
+    if (!right) g_device_status[0] = kWaitFusedMeetingWrong;
 }
 
 }  // namespace mt
@@ -288,11 +278,8 @@ int mt_device_status(unsigned int words[4], int reset) {
     if (reset) {
         const unsigned int zeros[4] = {0, 0, 0, 0};
         if (cudaMemcpyToSymbol(g_device_status, zeros, sizeof(zeros)) != cudaSuccess) return MT_ERR_LAUNCH;
-        // A wait that gave up at the single-launch MLP's grid barrier leaves its counter short of a
-        // multiple of the grid size; the device is idle here, so every counter can start over.
-        static const unsigned long long no_arrivals[kMeetingSlotsInAll] = {};
-        if (words[0] && cudaMemcpyToSymbol(g_fused_barrier, no_arrivals, sizeof(no_arrivals)) != cudaSuccess)
-            return MT_ERR_LAUNCH;
+        // A single-launch MLP that gave up may have left its slot's counter and flags as no other launch expects them.
+        if (words[0] && !clear_meeting_places()) return MT_ERR_LAUNCH;
     }
     return words[0] ? MT_ERR_DEVICE_WAIT : MT_OK;
 }
@@ -304,11 +291,12 @@ int mt_selftest_bounded_wait(int which, unsigned int limit_us, void* stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (which == 0) {
         selftest_mbarrier_wait_kernel<<<1, 64, 0, s>>>(limit_ns);
-    } else if (which == 1) {
-        unsigned long long* slot = nullptr;
-        unsigned int* left = nullptr;
-        if (!meeting_slot_memory(kMeetingSelfTest, slot, left)) return MT_ERR_LAUNCH;
-        selftest_grid_barrier_kernel<<<2, kFusedComputeThreads, 0, s>>>(slot, limit_ns);
+    } else if (which == 1 || which == 2) {
+        FusedMeetingPlace place;
+        if (!meeting_place_of(kMeetingSelfTest, place)) return MT_ERR_LAUNCH;
+        place.patience_ns = (unsigned int)limit_ns;
+        selftest_meeting_left_kernel<<<2, 1, 0, s>>>(place);
+        if (which == 1) selftest_meeting_last_kernel<<<1, 1, 0, s>>>(place);
     } else {
         return MT_ERR_SHAPE;
     }
@@ -394,9 +382,7 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         params.residual = static_cast<const uint16_t*>(residual);
         params.hidden = static_cast<uint16_t*>(workspace);
         params.out = static_cast<uint16_t*>(out);
-        params.barrier = nullptr;
-        params.left = nullptr;
-        params.patience_ns = flags & MT_FLAG_MLP_IMPATIENT ? 0u : kFusedPatienceNs;
+        params.meeting = {nullptr, nullptr, flags & MT_FLAG_MLP_IMPATIENT ? 0u : kFusedPatienceNs};
         params.M = M;
         params.H = H;
         params.I = I;

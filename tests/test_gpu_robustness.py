@@ -16,7 +16,7 @@ from tests.helpers import assert_bit_equal, assert_within, f32, triple_np
 pytestmark = pytest.mark.gpu
 
 WAIT_SELFTEST = 0x7E1
-WAIT_GRID_BARRIER = 0x203
+WAIT_MEETING = 0x203
 
 
 def _stream(device):
@@ -42,9 +42,9 @@ def test_a_wait_nothing_satisfies_gives_up_with_a_status(cuda_device):
     assert lib.mt_selftest_bounded_wait(0, 0, None) == -1 and lib.mt_selftest_bounded_wait(7, 10, None) == -1
 
 
-def test_grid_barrier_that_gives_up_is_repaired_by_the_reset(cuda_device):
-    """A grid barrier whose wait runs out leaves its counter short.  The reset zeroes the counters,
-    so every later single-launch MLP -- whichever of the 64 rotating counters it draws -- is right."""
+def test_meeting_some_never_come_to_is_left_and_repaired_by_the_reset(cuda_device):
+    """CTAs that wait in vain at the single-launch MLP's meeting leave their rows to the last to arrive.  What a launch
+    that gave up leaves behind, counter and flags, is cleared by the reset."""
     lib = _lib.load()
     hidden, inter = 1024, 2048
     gate, up, down = synth.mlp_weights(77, hidden, inter, cuda_device)
@@ -54,11 +54,13 @@ def test_grid_barrier_that_gives_up_is_repaired_by_the_reset(cuda_device):
     assert lib.mt_affine_mlp_launches(1, hidden, inter, 0) == 1
     before = execute(x, res)
     torch.cuda.synchronize()
-    assert lib.mt_selftest_bounded_wait(1, 2000, _stream(cuda_device)) == 0
     words = (ctypes.c_uint * 4)()
-    assert lib.mt_device_status(words, 1) == -8 and words[0] == WAIT_GRID_BARRIER
-    for _ in range(70):  # more launches than counters
-        assert_bit_equal(execute(x, res), before, "single-launch MLP after a barrier time-out and reset")
+    for which in (1, 1, 2, 1, 2, 1):  # after 2 without the reset, the next meeting would go wrong
+        assert lib.mt_selftest_bounded_wait(which, 2000, _stream(cuda_device)) == 0
+        assert_bit_equal(execute(x, res), before, "beside a meeting that fails")
+        assert lib.mt_device_status(words, 0) == -8 and words[0] == WAIT_MEETING
+        assert lib.mt_device_status(words, 1) == -8 and words[0] == WAIT_MEETING
+        assert_bit_equal(execute(x, res), before, "single-launch MLP after a meeting that failed and the reset")
     ok, words = _lib.device_status()
     assert ok, [hex(w) for w in words]
 
