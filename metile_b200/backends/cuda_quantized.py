@@ -74,9 +74,12 @@ def kernel_pinned():
 
 class fixed_order:
     """Within it, the sums of the tcgen05 kernels are cut as in batch-invariant mode, whatever the row count; the kernel
-    family follows the row count as always.  A model's modules run in it: a token's keys and values are then the same bits
-    in a prompt of any length (of two tokens and more) and beside any other sequences.  An operator called on its own
-    takes the cut that is fastest for its rows."""
+    family follows the row count as always.  A row's bits then depend on the family alone: one row, more rows, and for an
+    MLP that the single launch serves (mt_affine_mlp_launches) also two to eight rows.  A model's modules run in it, so a
+    token's norms and projections do not depend on the length of a prompt of two tokens and more, nor its MLP on that of a
+    prompt of more than eight.  (The attention of a prompt is torch's, whose sums may follow the length.)  Bits that no row
+    count changes take batch_invariant().  An operator called on its own takes the cut
+    that is fastest for its rows."""
 
     __slots__ = ("previous",)
 

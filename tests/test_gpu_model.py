@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import metile_b200
-from metile_b200 import backends, synth
+from metile_b200 import _lib, backends, synth
 from metile_b200.integrations import blocks, torch_lm
 from metile_b200.integrations.graphed import GraphedDecoder
 from tests.helpers import assert_bit_equal
@@ -129,6 +129,33 @@ def test_cache_methods_replaced_on_the_instance_are_called(cuda_device):
         assert_bit_equal(model(tokens[:, :1], cache=replaced), model(tokens[:, :1], cache=plain), "decode step")
         assert called[2:] == ["advance"] and replaced[0].length == 10 and (replaced[0].positions == 10).all()
         assert_bit_equal(replaced[0].keys, plain[0].keys, "keys")
+
+
+@pytest.mark.parametrize("hidden,inter,single_launch", [(1024, 1024, True), (2048, 2048, True), (256, 512, False)])
+def test_a_tokens_projections_in_prompts_of_other_lengths(cuda_device, hidden, inter, single_launch):
+    """The same bits in every prompt of two tokens and more; an MLP that the single launch serves at two to eight rows has
+    other bits there.  (Of a block; the attention between the projections is torch's.)"""
+    assert (_lib.load().mt_affine_mlp_launches(5, hidden, inter, 0) == 1) == single_launch
+    model = blocks.random_model(8, device=cuda_device, hidden=hidden, intermediate=inter, layers=1, head_dim=64)
+    block = model.layers[0]
+    attention, rows = block.self_attn, synth.activations(1, 140, hidden, cuda_device).view(1, 140, hidden)
+    attended = synth.activations(2, 140, attention.heads * 64, cuda_device).view(1, 140, -1)
+
+    def parts(length):
+        values = rows[:, :length].contiguous()
+        normed = block.input_layernorm(values)
+        out = [normed, attention.q_proj(normed), attention.k_proj(normed), attention.v_proj(normed),
+               attention.o_proj(attended[:, :length].contiguous())]
+        return out, torch_lm.execute_quantized_mlp(block.mlp, normed, values)
+
+    with torch_lm.apply_metile_to_torch_lm(model, attention=True), torch.no_grad():
+        (wanted, mlp), (_, eight) = parts(140), parts(8)
+        for length in (2, 5, 8, 9, 20, 64, 65, 129):
+            found, mlp_found = parts(length)
+            for name, a, b in zip(("norm", "q", "k", "v", "o"), found, wanted):
+                assert_bit_equal(a, b[:, :length], f"{name}, {length} of 140")
+            assert_bit_equal(mlp_found, (eight if single_launch and length <= 8 else mlp)[:, :length], f"MLP, {length} tokens")
+        assert bool((eight != mlp[:, :8]).any()) == single_launch
 
 
 def test_a_captured_step_keeps_its_scratch_when_a_longer_prompt_follows(cuda_device):
