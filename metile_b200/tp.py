@@ -16,8 +16,8 @@ GPU's bandwidth budget:
 The sum is the library's own one-shot exchange (`PeerAllReduce`, mt_peer_all_reduce): one kernel per
 rank stores the bf16 partial into every peer's memory over NVLink, waits for the peers' stores and
 adds the partials in RANK ORDER in fp32.  Every rank gets the same bits and the order does not change
-with the message size, so a row's result does not depend on the batch it arrives in as long as the
-shard kernels are batch-invariant themselves (`batch_invariant()`).  `all_reduce="nccl"` selects
+with the message size.  The shards run in `fixed_order()`, so a row's result depends on the batch it
+arrives in only by the kernel that serves its row count, and not at all in `batch_invariant()`.  `all_reduce="nccl"` selects
 torch.distributed's all-reduce instead, whose summation order is NCCL's choice.  Either way the
 partials are rounded to bf16 before they are added, so the sharded result agrees with the single-GPU
 MLP to the tolerance of two bf16 roundings more, not bit for bit.
@@ -218,7 +218,10 @@ class TensorParallelMLP:
         residual on rank 0."""
         mine = residual if self.rank == 0 else None
         if self._swiglu is None and self._down is None:
-            return self._bound_executor(values)(values, mine)
+            from .backends.cuda_quantized import fixed_order
+
+            with fixed_order():
+                return self._bound_executor(values)(values, mine)
         hidden = self._swiglu(values, *self.gate, *self.up)
         return self._down(hidden, *self.down, mine)
 

@@ -12,6 +12,9 @@ import socket
 import pytest
 import torch
 
+from metile_b200 import synth, tp
+from tests.helpers import assert_bit_equal
+
 pytestmark = pytest.mark.gpu
 
 
@@ -190,3 +193,15 @@ def test_late_peer_makes_the_wait_run_out_and_the_next_call_recovers():
 def test_exchange_inside_a_replayed_cuda_graph():
     results = _run("graph")
     assert results == {0: True, 1: True}
+
+
+@pytest.mark.parametrize("hidden,inter", [(1024, 4096), (1536, 8960)])
+def test_a_row_of_a_shard_does_not_depend_on_the_rows_beside_it(cuda_device, hidden, inter):
+    """The partial sums of both ranks, computed here one after the other: the exchange adds no order of its own."""
+    gate, up, down = synth.mlp_weights(21, hidden, inter, cuda_device)
+    x, res = synth.activations(5, 300, hidden, cuda_device), synth.activations(6, 300, hidden, cuda_device)
+    for rank in range(2):
+        shard = tp.TensorParallelMLP.from_full(gate, up, down, cuda_device, rank, 2)
+        whole = shard.partial(x, res)
+        for rows in (9, 16, 37, 64, 128):
+            assert_bit_equal(shard.partial(x[:rows], res[:rows]), whole[:rows], f"rank {rank}, {rows} of 300 rows")
