@@ -29,7 +29,8 @@
  *
  * Return value: 0 (MT_OK) or a negative code; mt_status_string() names it.  Codes:
  *   -1 shape, -2 alignment, -3 quantisation format, -4 CUDA launch error, -5 wrong device,
- *   -6 null pointer, -7 workspace, -8 a bounded device-side wait gave up.
+ *   -6 null pointer, -7 workspace, -8 a bounded device-side wait gave up, -9 a kernel met an index outside its table
+ *   (-8 and -9: from mt_device_status).
  * Argument errors (codes -1, -2, -3, -5, -6, -7) are detected before any GPU work is queued; -4 is
  * what the CUDA runtime reported for a launch.  There is no CPU fallback.
  *
@@ -85,7 +86,8 @@ int mt_device_check(void);
 
 /* Reads (and with reset != 0 clears) the device-side record of a bounded wait that gave up:
  * words[0] = wait code (0 = none), [1] = block, [2] = thread, [3] = parity.  Synchronises the
- * device.  Returns 0, or -8 when words[0] != 0. */
+ * device.  Returns 0, or -8 when words[0] != 0.  Code 0x301, with -9: mt_gather_rows met an index outside its table,
+ * [1] = output row, [2] and [3] = the index, low and high half. */
 int mt_device_status(unsigned int words[4], int reset);
 
 /* Self-test of the bounded device-side waits: queues a tiny kernel whose wait can never be satisfied
@@ -235,7 +237,7 @@ int mt_rope_kv_append_advance(const void* q, const void* k, const void* v, long 
 int mt_greedy_token(const void* logits, float* out, long long* tokens, int rows, int vocabulary, void* stream);
 
 /* out[r] = table[index[r]]: rows of `width` bf16 (a multiple of 8), table [table_rows, width], out [rows, width], both
- * 16-byte aligned (else -2).  An index outside the table gives a row of NaN. */
+ * 16-byte aligned (else -2).  An index outside the table gives a row of NaN and is recorded (mt_device_status, -9). */
 int mt_gather_rows(const void* table, const long long* index, void* out, int rows, long long table_rows, int width, void* stream);
 
 /* The same for the `steps` tokens of a prompt, which go to rows first, first + 1, ... of every cache.

@@ -115,7 +115,8 @@ def check(code, what):
 
 
 def device_status(reset=True):
-    """(ok, words) -- words[0] != 0 means a bounded device-side wait gave up."""
+    """(ok, words) -- words[0] != 0 means a bounded device-side wait gave up, or (0x301) that an embedding met a token
+    outside its table: words[1] is the output row, words[2] the token."""
     words = (ctypes.c_uint * 4)()
     code = load().mt_device_status(words, 1 if reset else 0)
     return code == 0, tuple(int(v) for v in words)

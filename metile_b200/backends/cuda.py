@@ -218,7 +218,7 @@ def greedy_token(logits, tokens):
 
 def embedding(tokens, table):
     """table[tokens] for int64 tokens of any shape and a bfloat16 table [V, H]; None, and nothing done, unless both are dense
-    tensors on one CUDA device that no gradient is asked for.  A token outside the table gives NaN."""
+    tensors on one CUDA device that no gradient is asked for.  A token outside the table gives a row of NaN, and _lib.device_status() tells of the first."""
     out = native().embedding(tokens, table)
     return None if out is None else native_result(out, "embedding")
 

@@ -15,6 +15,7 @@
 #define MT_ERR_NULL (-6)         // required pointer is null
 #define MT_ERR_WORKSPACE (-7)    // workspace missing or too small
 #define MT_ERR_DEVICE_WAIT (-8)  // a bounded device-side wait gave up (see mt_device_status)
+#define MT_ERR_INDEX (-9)        // a kernel met an index outside its table (see mt_device_status)
 
 // ---- flags word ---------------------------------------------------------------------------
 #define MT_FLAG_FORCE_GEMV 0x1u   // CUDA-core GEMV regardless of row count (rows <= 8 only)
@@ -27,8 +28,8 @@
 
 namespace mt {
 
-// Device-side record of a bounded wait that gave up: word 0 = code, 1 = block, 2 = detail.
-// Written with atomicCAS so the first failure wins; zero means every wait completed.
+// Device-side record of a bounded wait that gave up, or of an index outside its table: word 0 = code, 1 = block, 2 = detail.
+// Written with atomicCAS so the first failure wins; zero means that there was none.
 // The library is one translation unit, so the definition lives here.
 __device__ unsigned int g_device_status[4] = {0, 0, 0, 0};
 

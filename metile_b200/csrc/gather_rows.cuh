@@ -11,14 +11,20 @@
 namespace mt {
 
 constexpr int kGatherThreads = 256;
+constexpr unsigned int kGatherIndexOutside = 0x301;
 
-// out[r] = table[index[r]], rows of `vectors` 16-byte vectors; an index outside the table gives a row of NaN.
+// out[r] = table[index[r]], rows of `vectors` 16-byte vectors; an index outside the table gives a row of NaN and is recorded.
 __global__ void __launch_bounds__(kGatherThreads) gather_rows_kernel(const uint4* table, const long long* index, uint4* out, long long table_rows, int vectors) {
     ptx::griddep_launch_dependents();
     ptx::griddep_wait();  // the indices are, and the output may still be read by, a preceding kernel
     long long row;
     asm volatile("ld.global.s64 %0, [%1];" : "=l"(row) : "l"(index + blockIdx.x));
     const bool inside = row >= 0 && row < table_rows;
+    if (!inside && threadIdx.x == 0 && atomicCAS(&g_device_status[0], 0u, kGatherIndexOutside) == 0u) {
+        g_device_status[1] = blockIdx.x;
+        g_device_status[2] = (unsigned int)row;
+        g_device_status[3] = (unsigned int)(row >> 32);
+    }
     const uint4* from = table + (inside ? row : 0) * (long long)vectors;
     uint4* to = out + (long long)blockIdx.x * vectors;
     for (int i = threadIdx.x; i < vectors; i += blockDim.x) {

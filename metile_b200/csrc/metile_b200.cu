@@ -265,6 +265,7 @@ const char* mt_status_string(int status) {
         case MT_ERR_NULL: return "null pointer";
         case MT_ERR_WORKSPACE: return "workspace missing, misaligned or too small";
         case MT_ERR_DEVICE_WAIT: return "a bounded device-side wait gave up";
+        case MT_ERR_INDEX: return "a kernel met an index outside its table";
         default: return "unknown status";
     }
 }
@@ -281,7 +282,7 @@ int mt_device_status(unsigned int words[4], int reset) {
         // A single-launch MLP that gave up may have left its slot's counter and flags as no other launch expects them.
         if (words[0] && !clear_meeting_places()) return MT_ERR_LAUNCH;
     }
-    return words[0] ? MT_ERR_DEVICE_WAIT : MT_OK;
+    return words[0] == kGatherIndexOutside ? MT_ERR_INDEX : words[0] ? MT_ERR_DEVICE_WAIT : MT_OK;
 }
 
 int mt_selftest_bounded_wait(int which, unsigned int limit_us, void* stream) {

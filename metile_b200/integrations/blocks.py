@@ -277,7 +277,9 @@ _EMBEDDING_FORWARD, _EMBEDDING_CALL = nn.Embedding.forward, nn.Embedding.__call_
 
 
 def _embed(module, tokens):
-    """module(tokens), by the gather kernel where the module is torch's embedding and looks rows up and nothing else."""
+    """module(tokens), by the gather kernel where the module is torch's embedding and looks rows up and nothing else.
+    (Of a token outside the table torch's kernel makes an assertion that ends the context; this one a row of NaN, recorded in
+    the status word.)"""
     state = module.__dict__
     if type(module) is nn.Embedding and state["max_norm"] is None and nn.Embedding.forward is _EMBEDDING_FORWARD \
             and nn.Embedding.__call__ is _EMBEDDING_CALL and not (

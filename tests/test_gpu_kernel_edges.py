@@ -358,11 +358,19 @@ def test_embedding_rows(cuda_device, rows, width, vocab):
     assert_bit_equal(B.embedding(tokens, table), torch.nn.functional.embedding(tokens, table), "rows")
     outside = tokens.clone()
     outside[0], outside[-1] = -1, vocab
+    assert _lib.device_status()[0]
     found = B.embedding(outside, table)
     assert found[0].isnan().all() and found[-1].isnan().all()
-    for other in (tokens.int(), tokens.expand(rows, 2)[:, ::2].T, tokens.cpu()):
-        if other.dtype != torch.int64 or not other.is_contiguous() or not other.is_cuda:
-            assert B.embedding(other, table) is None
+    if rows > 2:
+        assert_bit_equal(found[1:-1], table[tokens[1:-1]], "rows beside one that is not there")
+    ok, words = _lib.device_status()
+    row, token = words[1], words[2] | words[3] << 32
+    assert not ok and words[0] == 0x301 and (row, token) in ((0, 2**64 - 1), (rows - 1, vocab))
+    assert _lib.device_status()[0]
+    apart = torch.zeros(rows + 1, 4, dtype=torch.int64, device=cuda_device)[:, ::2]
+    assert not apart.is_contiguous()
+    for other in (tokens.int(), apart, tokens.cpu()):
+        assert B.embedding(other, table) is None
     assert B.embedding(tokens, table.float()) is None and B.embedding(tokens[:0], table) is None
     assert B.embedding(tokens, table.clone().requires_grad_()) is None
 
