@@ -2,16 +2,19 @@
 //
 // Computes what affine_gemv.cuh computes (kernels/affine_qmv.py:4-54, SwiGLU :204-208, residual :124-131).  On the CUDA cores
 // a weight costs one byte-permute and one FMA, and a warp issues 117 instructions per 1024 weights: at 2048 -> 128256 that is
-// 27 of the 38 us, with the bytes needing 23.  Here a nibble q becomes the exact bf16 number 128 + q (seven instructions
-// per word of eight), m16n8k16 products with fp32 accumulators add (128 + q) x over a quantisation group of 64 columns,
-// and a group is folded into the fp32 sum as fma(scale, P, fma(bias - 128 * scale, X, acc)), X = sum of the group's x.
+// 27 of the 38 us, with the bytes needing 23.  Here a nibble q becomes the exact bf16 number (q - 8) / 64 (nine instructions
+// per word of eight), m16n8k16 products with fp32 accumulators add (q - 8) x / 64 over a quantisation group of 64 columns,
+// and a group is folded into the fp32 sum as fma(scale, P, fma(bias + 8 scale, X / 64, acc)), X = sum of the group's x.
+//
+// The codes are centred for the accumulators' sake, which cut off what lies 2^23 below the largest product: with 128 + q (seven
+// instructions) sums that cancel were off by 2.4e-5 of their size in an MLP's down projection at 2048 / 8192, all to one
+// side, on the CUDA cores by 9e-7; with centred codes by 5e-8.  2048 -> 128256 33.2 us (33.5 with 128 + q), MLP 2048 / 8192 13.2 (13.0).
 //
 // One activation row leaves seven of the product's eight columns over.  They hold eight GROUPS: column n of the B operand is
 // x of group n of an item of eight.  Of an A operand, lanes t = 0, 1 of a row carry the two halves of group 2i and lanes t =
 // 2, 3 those of group 2i + 1 (so a lane reads four words with one 16-byte load), and B is zero where the column's parity is
 // not the lanes'.  Eight products make the sums of both groups, in columns 2i and 2i + 1, which are lane t = i's: it
-// reads the scales of just those two groups, and nothing is multiplied, read or exchanged twice.  41 instructions per 1024
-// weights.
+// reads the scales of just those two groups, and nothing is multiplied, read or exchanged twice.
 //
 // A tile of 16 outputs belongs to a team of `parts` warps that share its K range; teams and CTAs take the tiles in turn.
 // Items (16 rows x 512 columns, 4 KB) come by TMA into a ring of the warp's, two ahead and the first ones before the wait
@@ -31,6 +34,7 @@ constexpr int kOneRowDepth = 2;        // ring items of a warp: one being read, 
 constexpr int kOneRowTables = 2;       // tiles whose tables a team holds
 constexpr int kOneRowItemGroups = 8;
 constexpr int kOneRowItemBytes = 16 * kOneRowItemGroups * 32;
+constexpr float kOneRowUnit = 1.0f / 64.0f;  // of the sums, which are of w / 64 (see unpack_word_centred64)
 constexpr int kOneRowSmemLimit = 224 * 1024;
 constexpr int kOneRowSmemTwo = 110 * 1024;  // two CTAs per SM
 
@@ -64,7 +68,7 @@ __device__ __forceinline__ void one_row_words(const uint8_t* words, int tile_row
     }
 }
 
-// Sums of (128 + q) x over groups 2t and 2t + 1 of the item: own[0], own[1] of this lane's row, own[2], own[3] of the eighth
+// Sums of (q - 8) / 64 x over groups 2t and 2t + 1 of the item: own[0], own[1] of this lane's row, own[2], own[3] of the eighth
 // row after it.
 __device__ __forceinline__ void one_row_products(const uint32_t (&row)[4][4], const uint32_t (&row8)[4][4], const uint32_t (&xr)[16], int t,
                                                  float (&own)[4]) {
@@ -74,8 +78,8 @@ __device__ __forceinline__ void one_row_products(const uint32_t (&row)[4][4], co
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             uint32_t a[4], b[4];
-            unpack_word_offset128(row[i][u], a);
-            unpack_word_offset128(row8[i][u], b);
+            unpack_word_centred64(row[i][u], a);
+            unpack_word_centred64(row8[i][u], b);
             ptx::mma_bf16_m16n8k16(sum[i], a[0], b[0], a[1], b[1], xr[4 * u], xr[4 * u + 1]);
             ptx::mma_bf16_m16n8k16(sum[i], a[2], b[2], a[3], b[3], xr[4 * u + 2], xr[4 * u + 3]);
         }
@@ -176,7 +180,7 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
                     ((bf16_lo(raw.z) + bf16_hi(raw.z)) + (bf16_lo(raw.w) + bf16_hi(raw.w)));
 #pragma unroll
         for (int offset = 1; offset < 8; offset <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, offset);
-        if ((v & 7) == 0) x_sums[v >> 3] = sum;
+        if ((v & 7) == 0) x_sums[v >> 3] = kOneRowUnit * sum;
     }
     __syncthreads();
 
@@ -227,8 +231,8 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
                     for (int e = 0; e < 2; ++e) {
                         if (group + e >= groups) continue;
                         const int at = (tile_row + 8 * r) * groups + group + e;
-                        const float scale = bf16_bits_to_f32(scale_row[at]), shifted = fmaf(-128.0f, scale, bf16_bits_to_f32(bias_row[at]));
-                        acc[s][r] = fmaf(scale, own[2 * r + e], fmaf(shifted, e ? xs.y : xs.x, acc[s][r]));
+                        const float scale = bf16_bits_to_f32(scale_row[at]), centre = fmaf(8.0f, scale, bf16_bits_to_f32(bias_row[at]));
+                        acc[s][r] = fmaf(scale, own[2 * r + e], fmaf(centre, e ? xs.y : xs.x, acc[s][r]));
                     }
             }
         }
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(kOneRowWarps * 32, 2) affine_gemv_mma_kernel(c
                 acc[s][r] += __shfl_xor_sync(0xFFFFFFFFu, acc[s][r], 1);
                 acc[s][r] += __shfl_xor_sync(0xFFFFFFFFu, acc[s][r], 2);
             }
-            total[s] = t == 0 ? acc[s][0] : acc[s][1];
+            total[s] = (t == 0 ? acc[s][0] : acc[s][1]) / kOneRowUnit;
         }
         const int row = tile_row + 8 * (t & 1), n = n0 + row;
         const bool finishes = part == 0 && t < 2 && n < p.N;

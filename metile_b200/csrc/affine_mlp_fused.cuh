@@ -262,7 +262,7 @@ __device__ __forceinline__ void fused_take_over(const FusedMeetingPlace& at, int
     ptx::atom_add_acq_rel_gpu_u64(at.count, 0ull - kMeetOneLeft);
 }
 
-// Lane (g, t)'s activations of a 512-column unit: the B registers of one_row_products, and the sums of groups 2t and 2t + 1.
+// Lane (g, t)'s activations of a 512-column unit: the B registers of one_row_products, and the sums of groups 2t and 2t + 1 in kOneRowUnit.
 template <bool kFromL2>
 __device__ __forceinline__ void fused_one_activations(const uint16_t* unit, int g, int t, uint32_t (&xr)[16], float2& sums) {
     const bool carries = (g & 1) == (t >> 1);  // whether column g belongs to this lane's half of the groups
@@ -278,7 +278,7 @@ __device__ __forceinline__ void fused_one_activations(const uint16_t* unit, int 
         xr[4 * u + 2] = __byte_perm(v.y, v.w, 0x5410);
         xr[4 * u + 3] = __byte_perm(v.y, v.w, 0x7632);
     }
-    total += __shfl_xor_sync(0xFFFFFFFFu, total, 1);
+    total = kOneRowUnit * (total + __shfl_xor_sync(0xFFFFFFFFu, total, 1));
     sums.x = __shfl_sync(0xFFFFFFFFu, total, 8 * t);      // group 2t: lanes (2t, 0) and (2t, 1)
     sums.y = __shfl_sync(0xFFFFFFFFu, total, 8 * t + 6);  // group 2t + 1: lanes (2t + 1, 2) and (2t + 1, 3)
 }
@@ -429,7 +429,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float s0 = bf16_lo(scale[r]), s1 = bf16_hi(scale[r]);
-                    const float b0 = fmaf(-128.0f, s0, bf16_lo(bias[r])), b1 = fmaf(-128.0f, s1, bf16_hi(bias[r]));  // undoes the 128 in 128 + q
+                    const float b0 = fmaf(8.0f, s0, bf16_lo(bias[r])), b1 = fmaf(8.0f, s1, bf16_hi(bias[r]));  // the products are of (q - 8) / 64, xs is X / 64
                     total[r] = fmaf(s0, own[2 * r], b0 * xs.x);
                     total[r] = fmaf(s1, own[2 * r + 1], fmaf(b1, xs.y, total[r]));
                     total[r] += __shfl_xor_sync(0xFFFFFFFFu, total[r], 1);
@@ -437,7 +437,7 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
                 }
                 const int mine = first + tile_row + 8 * (t & 1);
                 if (t < 2 && mine <= last)
-                    scratch[((mine * (kDown ? 1 : 2) + matrix) * chunks + chunk) * M + m] = t == 0 ? total[0] : total[1];
+                    scratch[((mine * (kDown ? 1 : 2) + matrix) * chunks + chunk) * M + m] = (t == 0 ? total[0] : total[1]) / kOneRowUnit;
             }
         }
     };

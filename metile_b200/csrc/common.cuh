@@ -54,6 +54,18 @@ __device__ __forceinline__ void unpack_word_offset128(uint32_t w, uint32_t* out)
         asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(out[i]) : "r"(w >> (4 * i)), "r"(0x000F000Fu), "r"(0x43004300u));
 }
 
+// One packed word -> four bf16 pairs ((e_i - 8) / 64, (e_{i+4} - 8) / 64), i = 0..3, exact.  Masked out, a nibble is the
+// subnormal bf16 number e 2^-133 (or 16 e 2^-133), which one fma.rn.bf16x2 brings up and centres: nine instructions.
+__device__ __forceinline__ void unpack_word_centred64(uint32_t w, uint32_t* out) {
+    const uint32_t upper = w >> 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        asm("{\n\t.reg .b32 t;\n\tand.b32 t, %1, %2;\n\tfma.rn.bf16x2 %0, t, %3, %4;\n\t}"
+            : "=r"(out[i]) : "r"(i < 2 ? w : upper), "r"(i & 1 ? 0x00F000F0u : 0x000F000Fu),
+              "r"(i & 1 ? 0x7D007D00u : 0x7F007F00u),  // 2^123, 2^127
+              "r"(0xBE00BE00u));                       // -1/8
+}
+
 // The eight nibbles of a word as the floats 128+e0 .. 128+e7 (natural order).
 __device__ __forceinline__ void unpack_word_f32_offset128(uint32_t w, float (&q)[8]) {
     const uint32_t even = w & 0x0F0F0F0Fu, odd = (w >> 4) & 0x0F0F0F0Fu;

@@ -1,4 +1,5 @@
 """The edges of the kernels' tiles, chunks and rings, against the CPU oracle or rows run alone."""
+import contextlib
 import ctypes
 
 import pytest
@@ -499,3 +500,57 @@ def test_graphs_of_single_launch_mlps_side_by_side(cuda_device, batch):
         for x, y in zip(a, b):
             assert torch.equal(x, y)
     assert _lib.device_status()[0]
+
+
+def opposites(seed, n, k, device):
+    """Weights [w, -w], exact in bf16: (q - 8) / 64 with q from 1 to 15, in a triple, and the rms of w."""
+    q = torch.randint(1, 16, (n, k // 2), generator=torch.Generator().manual_seed(seed))
+    tables = torch.full((n, k // 64), 2.0 ** -6, dtype=torch.bfloat16, device=device)
+    return (synth.pack_nibbles(torch.cat([q, 16 - q], dim=1)).to(device), tables, -8 * tables), (q - 8).double().pow(2).mean().sqrt().item() / 64
+
+
+def error_of_sums(k, codes_from_128=False, peak=1.0):
+    """What is left of a sum that is zero is the error of its accumulation, here a share of the sum's size (rms).  A step of a
+    tensor-core accumulator (16 products) loses at most 2^-22 of what it holds, sqrt(K / 16) 2^-22 in all.  Where the codes
+    are 128 + q, a group's sum is 28 times that of the weights', more where one activation stands out (`peak` times the rms),
+    and eight steps lose 28 sqrt(8) 2^-23.  A partial sum of 16 bits would lose 2e-3."""
+    return 28 * peak * 8 ** 0.5 * 2 ** -23 if codes_from_128 else (k / 16) ** 0.5 * 2 ** -22
+
+
+@pytest.mark.parametrize("rows,k,n", [
+    (1, 1536, 1536),      # CUDA cores
+    (1, 2048, 8192), (1, 4096, 11264),  # warp-level tensor cores
+    (2, 1536, 1536), (16, 8192, 2048),  # tcgen05, slices over a cluster
+    (128, 8960, 1536), (300, 2048, 2112),
+    (2000, 8192, 2048),   # one chain over the whole range
+    (100, 27648, 1280),
+])
+def test_sums_of_projections_are_of_32_bits(cuda_device, rows, k, n):
+    weight, size = opposites(1, n, k, cuda_device)
+    half = synth.activations(2, rows, k // 2, cuda_device)
+    x = torch.cat([half, half], dim=1)
+    for order in (contextlib.nullcontext, B.fixed_order, B.batch_invariant):
+        with order():
+            left = B.mlx_affine_qmv(x, *weight).double()
+        cores = rows == 1 and (order is B.fixed_order or (order is contextlib.nullcontext and n * k < 8e6))
+        allowed = error_of_sums(k, cores) * size * k ** 0.5
+        assert left.pow(2).mean().sqrt().item() <= allowed and left.abs().max().item() <= 8 * allowed, order.__name__
+
+
+@pytest.mark.parametrize("rows,hidden,inter,codes_from_128", [
+    (1, 2048, 8192, False), (1, 1024, 1024, False),  # the single launch of one row
+    (8, 2048, 8192, True),                           # and of more
+    (1, 4096, 14336, False),                         # two launches on the warp-level tensor cores
+    (1, 1536, 8960, True),                           # on the CUDA cores
+    (16, 2048, 8192, False), (300, 1536, 8960, False),
+])
+def test_sums_of_mlps_are_of_32_bits(cuda_device, rows, hidden, inter, codes_from_128):
+    """The two halves of the hidden row are the same, those of the down weights opposites."""
+    gate, up = ([torch.cat([t, t]) for t in synth.affine_weight(seed, inter // 2, hidden, cuda_device)] for seed in (1, 2))
+    down, size = opposites(3, hidden, inter, cuda_device)
+    x = synth.activations(4, rows, hidden, cuda_device)
+    left = B.mlx_affine_mlp_executor(x, *gate, *up, *down, None)(x).double()
+    activations = B.mlx_affine_swiglu(x, *gate, *up).double()
+    rms = activations.pow(2).mean().sqrt().item()
+    allowed = error_of_sums(inter, codes_from_128, activations.abs().max().item() / rms) * size * rms * inter ** 0.5
+    assert left.pow(2).mean().sqrt().item() <= allowed and left.abs().max().item() <= 8 * allowed
