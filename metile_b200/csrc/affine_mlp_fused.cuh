@@ -64,17 +64,17 @@ enum FusedWaitCode : unsigned int {
     kWaitFusedMeetingWrong = 0x2FF,  // ... whose meeting did not go as it should
 };
 
-// Counters of the meetings, one per slot; launches that may run at the same time have different slots (meeting_slots.h).
-// Every launch adds exactly gridDim.x to its slot, so a slot is always a multiple of the grid size between uses, but behind a
-// launch that gave up (a copy that never landed); mt_device_status(reset) then zeroes counters and flags.
-__device__ unsigned long long g_fused_barrier[kMeetingSlotsInAll];
-
-// Down rows that their CTA has left to the last CTA of the launch, a flag per CTA (FusedMeeting); all zero between launches.
-__device__ unsigned int g_fused_left[kMeetingSlotsInAll][kFusedMaxGrid];
+// Where the CTAs of a launch meet.  Launches that may run at the same time have different slots (meeting_slots.h).  Every launch
+// adds exactly gridDim.x to its count, so a count is always a multiple of the grid size between uses, and every flag down, but
+// behind a launch that gave up (a copy that never landed); mt_device_status(reset) then zeroes them all.
+struct __align__(64) FusedMeetingSlot {
+    unsigned long long count;
+    unsigned int left[kFusedMaxGrid / 32];  // down rows that their CTA has left to the last CTA of the launch, a bit per CTA
+};
+__device__ FusedMeetingSlot g_fused_meetings[kMeetingSlotsInAll];
 
 struct FusedMeetingPlace {
-    unsigned long long* count;
-    unsigned int* left;        // a flag per CTA
+    FusedMeetingSlot* slot;
     unsigned int patience_ns;
 };
 
@@ -239,27 +239,31 @@ enum FusedMeeting : int { kMeetOpen, kMeetLast, kMeetLeft };  // kMeetLast: the 
 constexpr unsigned long long kMeetOneLeft = 1ull << 48;
 
 __device__ __forceinline__ int fused_meet(const FusedMeetingPlace& at, unsigned int grid, unsigned int cta) {
+    unsigned long long* const count = &at.slot->count;
     // Release: the hidden activations of this CTA (ordered by the caller's barrier) are visible to whoever acquires the count.
-    const unsigned long long before = ptx::atom_add_acq_rel_gpu_u64(at.count, 1ull), arrived = before % kMeetOneLeft;
+    const unsigned long long before = ptx::atom_add_acq_rel_gpu_u64(count, 1ull), arrived = before % kMeetOneLeft;
     const unsigned long long target = (arrived / grid + 1ull) * grid;
     if (arrived + 1ull == target) return before >= kMeetOneLeft ? kMeetLast : kMeetOpen;
     const unsigned long long start = ptx::global_timer_ns();
-    while (ptx::ld_acquire_gpu_u64(at.count) % kMeetOneLeft < target) {
+    while (ptx::ld_acquire_gpu_u64(count) % kMeetOneLeft < target) {
         if (ptx::global_timer_ns() - start < at.patience_ns) continue;
-        atomicExch(at.left + cta, 1u);
-        if (ptx::atom_add_acq_rel_gpu_u64(at.count, kMeetOneLeft) % kMeetOneLeft < target) return kMeetLeft;
-        if (atomicExch(at.left + cta, 0u) == 0u) return kMeetLeft;  // the last CTA saw the flag on its way to another's
-        ptx::atom_add_acq_rel_gpu_u64(at.count, 0ull - kMeetOneLeft);
+        unsigned int* const flags = at.slot->left + (cta >> 5);
+        const unsigned int mine = 1u << (cta & 31u);
+        atomicOr(flags, mine);
+        if (ptx::atom_add_acq_rel_gpu_u64(count, kMeetOneLeft) % kMeetOneLeft < target) return kMeetLeft;
+        if (!(atomicAnd(flags, ~mine) & mine)) return kMeetLeft;  // the last CTA saw the flag on its way to another's
+        ptx::atom_add_acq_rel_gpu_u64(count, 0ull - kMeetOneLeft);
         return kMeetOpen;
     }
     return kMeetOpen;
 }
 
 // Takes over the rows of `cta` if it has left them.
-__device__ __forceinline__ void fused_take_over(const FusedMeetingPlace& at, int cta, int* taken, int* count) {
-    if (atomicExch(at.left + cta, 0u) != 1u) return;
-    taken[atomicAdd(count, 1)] = cta;
-    ptx::atom_add_acq_rel_gpu_u64(at.count, 0ull - kMeetOneLeft);
+__device__ __forceinline__ void fused_take_over(const FusedMeetingPlace& at, unsigned int cta, int* taken, int* count) {
+    const unsigned int its = 1u << (cta & 31u);
+    if (!(atomicAnd(at.slot->left + (cta >> 5), ~its) & its)) return;
+    taken[atomicAdd(count, 1)] = (int)cta;
+    ptx::atom_add_acq_rel_gpu_u64(&at.slot->count, 0ull - kMeetOneLeft);
 }
 
 // Lane (g, t)'s activations of a 512-column unit: the B registers of one_row_products, and the sums of groups 2t and 2t + 1 in kOneRowUnit.
@@ -969,60 +973,39 @@ inline int launch_mlp_fused_kernel(void (*kernel)(const FusedMlpParams), int sme
     return cudaLaunchKernelEx(&config, kernel, params) == cudaSuccess ? MT_OK : MT_ERR_LAUNCH;
 }
 
-inline MeetingSlots& meeting_slots() {
-    static MeetingSlots* const slots = new MeetingSlots;  // never destroyed: graphs may outlive everything else
-    return *slots;
-}
-
-inline void CUDART_CB give_back_meeting_slot(void* slot) { meeting_slots().give_back((int)reinterpret_cast<intptr_t>(slot)); }
-
-// The slot of a launch into `stream`; -1 when there is none.  The graph that is being captured keeps the slot of its launches,
-// and so does whatever is instantiated from it, until the last of them is destroyed.
+// The slot of a launch into `stream`; -1 when there is none.
 inline int meeting_slot_of(cudaStream_t stream) {
+    static MeetingSlots* const slots = new MeetingSlots;  // never destroyed: launches may come late
     cudaStreamCaptureStatus status;
     unsigned long long capture = 0, id = 0;
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamGetCaptureInfo(stream, &status, &capture, &graph) != cudaSuccess) return -1;
-    if (status == cudaStreamCaptureStatusNone) return cudaStreamGetId(stream, &id) == cudaSuccess ? meeting_slots().of_stream(id) : -1;
+    if (cudaStreamGetCaptureInfo(stream, &status, &capture) != cudaSuccess) return -1;
+    if (status == cudaStreamCaptureStatusNone) return cudaStreamGetId(stream, &id) == cudaSuccess ? slots->of_stream(id) : -1;
     if (status != cudaStreamCaptureStatusActive) return -1;
     static thread_local char thread;  // a capturing stream does not tell its id (and asking ends the capture)
-    bool fresh = false;
-    const int slot = meeting_slots().of_capture(capture, reinterpret_cast<uintptr_t>(stream == cudaStreamPerThread ? (void*)&thread : (void*)stream), fresh);
-    if (slot < 0 || !fresh) return slot;
-    cudaUserObject_t keeper;
-    if (cudaUserObjectCreate(&keeper, reinterpret_cast<void*>((intptr_t)slot), give_back_meeting_slot, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
-        meeting_slots().give_back(slot);
-        return -1;
-    }
-    if (cudaGraphRetainUserObject(graph, keeper, 1, cudaGraphUserObjectMove) != cudaSuccess) {
-        cudaUserObjectRelease(keeper, 1);  // gives the slot back
-        return -1;
-    }
-    return slot;
+    return slots->of_capture(capture, reinterpret_cast<uintptr_t>(stream == cudaStreamPerThread ? (void*)&thread : (void*)stream));
 }
 
-// The counter and the flags of a slot on the current device.
+// A slot on the current device.
 inline bool meeting_place_of(int slot, FusedMeetingPlace& place) {
-    static unsigned long long* counters[64] = {};
-    static unsigned int* flags[64] = {};
+    static FusedMeetingSlot* first[64] = {};
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
-    if (!__atomic_load_n(&counters[device], __ATOMIC_ACQUIRE)) {
-        void *first = nullptr, *second = nullptr;
-        if (cudaGetSymbolAddress(&first, g_fused_barrier) != cudaSuccess || cudaGetSymbolAddress(&second, g_fused_left) != cudaSuccess) return false;
-        __atomic_store_n(&flags[device], static_cast<unsigned int*>(second), __ATOMIC_RELAXED);
-        __atomic_store_n(&counters[device], static_cast<unsigned long long*>(first), __ATOMIC_RELEASE);
+    place.slot = __atomic_load_n(&first[device], __ATOMIC_ACQUIRE);
+    if (!place.slot) {
+        void* address = nullptr;
+        if (cudaGetSymbolAddress(&address, g_fused_meetings) != cudaSuccess) return false;
+        place.slot = static_cast<FusedMeetingSlot*>(address);
+        __atomic_store_n(&first[device], place.slot, __ATOMIC_RELEASE);
     }
-    place.count = __atomic_load_n(&counters[device], __ATOMIC_RELAXED) + slot;
-    place.left = __atomic_load_n(&flags[device], __ATOMIC_RELAXED) + slot * kFusedMaxGrid;
+    place.slot += slot;
     return true;
 }
 
 // Every slot of the current device, which is idle, as it was in the beginning.
 inline bool clear_meeting_places() {
     FusedMeetingPlace first;
-    return meeting_place_of(0, first) && cudaMemset(first.count, 0, sizeof(g_fused_barrier)) == cudaSuccess &&
-           cudaMemset(first.left, 0, sizeof(g_fused_left)) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+    return meeting_place_of(0, first) && cudaMemset(first.slot, 0, sizeof(g_fused_meetings)) == cudaSuccess &&
+           cudaDeviceSynchronize() == cudaSuccess;
 }
 
 // `launch` in its turn among the launches that share a slot although their streams do not: each begins behind the one before it.

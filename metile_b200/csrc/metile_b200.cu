@@ -238,11 +238,11 @@ __global__ void selftest_meeting_last_kernel(FusedMeetingPlace at) {
     __shared__ int taken[3], count;  // atomics do not reach local memory
     count = 0;
     const int met = fused_meet(at, 3, 2);
-    for (int cta = 0; cta < 3; ++cta) fused_take_over(at, cta, taken, &count);
+    for (unsigned int cta = 0; cta < 3; ++cta) fused_take_over(at, cta, taken, &count);
     // Both have left their rows, and the slot is as it was but for the three arrivals.
-    bool right = met == kMeetLast && count == 2 && taken[0] == 0 && taken[1] == 1 && ptx::ld_acquire_gpu_u64(at.count) % 3 == 0 &&
-                 ptx::ld_acquire_gpu_u64(at.count) < kMeetOneLeft;
-    for (int cta = 0; cta < 3; ++cta) right = right && atomicAdd(at.left + cta, 0u) == 0u;
+    const unsigned long long arrivals = ptx::ld_acquire_gpu_u64(&at.slot->count);
+    const bool right = met == kMeetLast && count == 2 && taken[0] == 0 && taken[1] == 1 && arrivals % 3 == 0 && arrivals < kMeetOneLeft &&
+                       atomicOr(at.slot->left, 0u) == 0u;
     if (!right) g_device_status[0] = kWaitFusedMeetingWrong;
 }
 
@@ -383,7 +383,7 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         params.residual = static_cast<const uint16_t*>(residual);
         params.hidden = static_cast<uint16_t*>(workspace);
         params.out = static_cast<uint16_t*>(out);
-        params.meeting = {nullptr, nullptr, flags & MT_FLAG_MLP_IMPATIENT ? 0u : kFusedPatienceNs};
+        params.meeting = {nullptr, flags & MT_FLAG_MLP_IMPATIENT ? 0u : kFusedPatienceNs};
         params.M = M;
         params.H = H;
         params.I = I;

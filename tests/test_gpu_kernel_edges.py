@@ -502,30 +502,6 @@ def test_graphs_of_single_launch_mlps_side_by_side(cuda_device, batch):
     assert _lib.device_status()[0]
 
 
-def test_graphs_that_are_gone_give_their_meeting_slots_back(cuda_device):
-    hidden = inter = 1024
-    gate, up, down = synth.mlp_weights(332, hidden, inter, cuda_device)
-    x = synth.activations(5, 1, hidden, cuda_device)
-    execute = B.mlx_affine_mlp_executor(x, *gate, *up, *down, None)
-    pool, stream = torch.cuda.graph_pool_handle(), torch.cuda.Stream()
-    with B.force_kernel("mlp_fused"):  # raises where a capture finds no slot
-        want = execute(x)
-        torch.cuda.synchronize()
-        keeper = torch.cuda.CUDAGraph()  # holds the pool between the others, and a slot throughout
-        for i in range(1500):  # more than there are slots
-            graph = torch.cuda.CUDAGraph() if i else keeper
-            with torch.cuda.stream(stream):
-                graph.capture_begin(pool=pool)
-                out = execute(x)
-                graph.capture_end()
-                if i % 250 == 0:
-                    graph.replay()
-                    keeper.replay()
-                    stream.synchronize()
-                    assert_bit_equal(out, want, f"graph {i}")
-    assert _lib.device_status()[0]
-
-
 def opposites(seed, n, k, device):
     """Weights [w, -w], exact in bf16: (q - 8) / 64 with q from 1 to 15, in a triple, and the rms of w."""
     q = torch.randint(1, 16, (n, k // 2), generator=torch.Generator().manual_seed(seed))
