@@ -311,7 +311,7 @@ inline bool one_row_plan(OneRowPlan& best, int K, int N, bool dual, int sm_count
 }
 
 // Where it is used: tables that bulk copies take, items that are not mostly empty, and weights enough: below, both forms take a
-// few us (here | with the rings of affine_gemv.cuh: 1024 -> 6544 3.5 | 2.9, 2048 -> 157 2.5 | 2.0; gate|up in an MLP 1088 / 4096
+// few us (with codes of 128 + q, here | with the rings of affine_gemv.cuh: 1024 -> 6544 3.5 | 2.9, 2048 -> 157 2.5 | 2.0; gate|up in an MLP 1088 / 4096
 // 9.4 | 7.4, 1536 / 5248 10.8 | 10.7, 1920 / 5056 10.5 | 11.0).  A long K range with few tiles takes more of them to pay (4096
 // -> 4096 4.5 | 4.4, 8192 -> 2048 5.7 | 4.9; down in an MLP 3584 / 12288 24.1 | 24.2, 3008 / 17024 30.0 | 32.7).
 inline bool one_row_applicable(const GemvWeights& a, const GemvWeights& b, int K, int N, bool dual) {
@@ -320,7 +320,24 @@ inline bool one_row_applicable(const GemvWeights& a, const GemvWeights& b, int K
         if (!aligned_to(w->scales, 16) || !aligned_to(w->biases, 16)) return false;
     if (10 * kOneRowItemGroups * chunks > 18 * groups) return false;
     const double weights = (double)N * K * (dual ? 2 : 1);
-    return weights >= (dual ? 18e6 : chunks <= 5 ? 8e6 : 45e6);
+    return weights >= (dual ? 18e6 : chunks <= 3 ? 8e6 : chunks <= 5 ? 11e6 : 45e6);
+}
+
+// And where the plan leaves too much of the chip idle, the rings are faster (here | there, us, in replayed graphs; of 1090 random
+// shapes of one row above the sizes above 66 took more than 2 % longer here, to 33 %, and with these rules 8, to 13 %):
+//   two matrices and few tiles                          7104 -> 1312 8.3 | 6.4, 12928 -> 775 11.2 | 8.4
+//   a second step that few of a team's warps have, on a part of the SMs    3520 -> 2688 7.8 | 6.3, 7232 -> 1920 9.0 | 8.5
+//   tiles for just more than one turn of six-warp teams, along a long row  10240 -> 5120 20.2 | 17.4, 13632 -> 5056 16.7 | 15.6
+//   several turns of small teams, six warps to a CTA    832 -> 19255 8.9 | 8.3, 768 -> 24293 10.2 | 9.5
+inline bool one_row_pays(const OneRowPlan& plan, int K, int N, bool dual, int sm_count) {
+    const int chunks = (K / 64 + kOneRowItemGroups - 1) / kOneRowItemGroups, tiles = (N + 15) / 16, warps = plan.parts * plan.teams;
+    const double turns = (double)tiles / (plan.teams * plan.grid);
+    if (K > 13824) return true;  // the rings do not serve it
+    if (plan.parts == 6 && turns > 1.0 && turns < 1.12) return false;
+    if (!dual) return true;
+    if (tiles < 0.7 * sm_count) return false;
+    if (warps == 8 && plan.parts < chunks && chunks < 2 * plan.parts && plan.grid < 0.945 * sm_count) return false;
+    return !(warps == 6 && plan.parts == chunks && chunks > 1 && turns > 1.3);
 }
 
 template <bool kDual>

@@ -55,8 +55,8 @@ static int check_affine_ptrs(const void* x, const uint32_t* w, const void* s, co
 // Row-count split: the CUDA-core GEMV issues one FMA per weight per row on top of the unpack, so its time grows with
 // the rows; the tcgen05 kernel's does not.  In replayed graphs, GEMV | tcgen05, us: one row 1536 -> 1536 3.4 | 3.9,
 // 4096 -> 4096 4.5 | 7.0, 8192 -> 2048 4.9 | 8.2, 2048 -> 16384 7.0 | 8.4, 2048 -> 128256 40.0 | 36.8; two rows 5.1 | 4.0,
-// 7.5 | 7.0, 8.2 | 8.2, 10.4 | 8.4, 64.0 | 36.7.  At one row the largest outputs would gain 8 % on the tensor cores, but the
-// GEMV never rounds a weight, and one row keeps one kernel for all widths.
+// 7.5 | 7.0, 8.2 | 8.2, 10.4 | 8.4, 64.0 | 36.7.  Neither the GEMV nor the one-row form on mma.sync, which takes its place
+// where that is faster (affine_gemv_mma.cuh), ever rounds a weight.
 static bool use_gemv(int M, unsigned int flags) {
     if (flags & MT_FLAG_FORCE_GEMV) return true;
     if (flags & MT_FLAG_FORCE_UMMA) return false;
@@ -75,7 +75,7 @@ static int run_projection(const void* x, const AffineWeights& first, const Affin
         // One row of a call that asks for no order of its own.
         OneRowPlan plan;
         if (M == 1 && !(flags & (MT_FLAG_FORCE_GEMV | MT_FLAG_FIXED_ORDER)) && one_row_applicable(a, b, K, N, second != nullptr) &&
-            one_row_plan(plan, K, N, second != nullptr, sms))
+            one_row_plan(plan, K, N, second != nullptr, sms) && one_row_pays(plan, K, N, second != nullptr, sms))
             return second ? launch_one_row<true>(x, a, b, residual, out, K, N, plan, stream)
                           : launch_one_row<false>(x, a, b, residual, out, K, N, plan, stream);
         return second ? launch_gemv<true>(x, a, b, residual, out, M, K, N, sms, stream)

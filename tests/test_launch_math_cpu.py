@@ -7,6 +7,8 @@ construction; these checks pin both halves for the shapes the library is used wi
 
 import pytest
 
+from tests.helpers import host_program
+
 SM_COUNT = 148
 WARPS = 8
 
@@ -174,3 +176,33 @@ def test_residual_words_bring_every_element_and_stay_within_the_arrays_own_words
                     assert at % 4 == 0 and 2 * odd // 4 <= at // 4 <= 2 * (odd + rows * n - 1) // 4
                     brought |= {at, at + 2}
     assert brought >= {2 * (odd + i) for i in range(rows * n)}
+
+
+ONE_ROW_FORM = """
+#include <cstdio>
+#include "affine_gemv_mma.cuh"
+using namespace mt;
+int main() {
+    const int shapes[][3] = {SHAPES};
+    uint16_t* const table = reinterpret_cast<uint16_t*>(64);
+    const GemvWeights w{nullptr, table, table}, odd{nullptr, table, table + 1};
+    for (const auto& s : shapes) {
+        OneRowPlan plan = {};
+        const bool serves = one_row_applicable(w, w, s[0], s[1], s[2]) && one_row_plan(plan, s[0], s[1], s[2], 148);
+        printf("%d %d\\n", serves && one_row_pays(plan, s[0], s[1], s[2], 148), one_row_applicable(w, odd, s[0], s[1], s[2]));
+    }
+    return 0;
+}
+"""
+
+
+def test_one_row_takes_the_tensor_cores_only_where_the_rings_are_slower(tmp_path):
+    """Shapes measured on both sides: (K, N, two matrices) and whether the warp-level tensor cores were faster."""
+    faster = {(2048, 128256, 0): 1, (1536, 32768, 0): 1, (1536, 5500, 0): 1, (4096, 14336, 0): 1, (1088, 7424, 0): 1,
+              (2048, 8192, 1): 1, (5120, 27648, 1): 1, (4096, 14336, 1): 1, (1536, 8960, 1): 1, (4288, 3959, 1): 1,
+              (2048, 4096, 0): 0, (2048, 4805, 0): 0, (13632, 5056, 0): 0, (2048, 157, 0): 0, (4096, 4096, 0): 0,
+              (7104, 1312, 1): 0, (12928, 775, 1): 0, (3520, 2688, 1): 0, (3136, 4032, 1): 0, (7232, 1920, 1): 0,
+              (10240, 5120, 1): 0, (9344, 4829, 1): 0, (832, 19255, 1): 0, (768, 24293, 1): 0, (1152, 21002, 1): 0}
+    rows = host_program(tmp_path, ONE_ROW_FORM.replace("SHAPES", ", ".join("{%d, %d, %d}" % shape for shape in faster)))
+    assert dict(zip(faster, (row[0] for row in rows))) == faster
+    assert not any(row[1] for row in rows)  # tables that bulk copies do not take
