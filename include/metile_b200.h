@@ -37,15 +37,15 @@
  * `flags`: 0 selects the kernel by row count.  A single projection (mt_affine_qmv, mt_affine_swiglu):
  * for M = 1 the CUDA-core GEMV, or mma.sync where there are weights enough (from 8 to 45 million) and MT_FLAG_FIXED_ORDER
  * is not given; the tcgen05 kernel above (its K range cut as M asks).  mt_affine_mlp: one launch for
- * the whole MLP when the shape allows it -- for M = 1 (H and I in {1024, 2048, 4096,
- * 8192}), on mma.sync for M = 2 ... 8 (H in {512, 1024, 1536, 2048}, I a multiple of 512) -- else two
+ * the whole MLP on mma.sync when the shape allows it -- for M = 1 (H and I in {1024, 2048, 4096,
+ * 8192}, H up to 4096), for M = 2 ... 8 (H in {512, 1024, 1536, 2048}, I a multiple of 512) -- else two
  * kernels (gate|up SwiGLU, then down) of the families above.
  *   MT_FLAG_FORCE_GEMV (1)   CUDA-core GEMV (M <= 8)
  *   MT_FLAG_FORCE_UMMA (2)   tcgen05 kernel for any M (one accumulation order for every M: use it
  *                            when rows must be bit-identical across batch sizes 1..128)
  *   MT_FLAG_FIXED_ORDER (256) the tcgen05 kernel's sums in the order of MT_FLAG_FORCE_UMMA, the kernel by row
  *                            count as with 0 (may be combined with the flags that choose a kernel)
- *   MT_FLAG_MLP_IMPATIENT (512) mt_affine_mlp in one launch at one row: a CTA does not wait for the others between the
+ *   MT_FLAG_MLP_IMPATIENT (512) mt_affine_mlp in one launch: a CTA does not wait for the others between the
  *                            projections but leaves its rows to the last one (the same bits; for tests)
  *   MT_FLAG_GELU (16)        mt_dense_act: x/(1+exp(-1.702x)) instead of SiLU
  *   MT_FLAG_MLP_FUSED (32)   mt_affine_mlp: insist on the single-launch one-row kernel (M <= 4); -1

@@ -17,8 +17,8 @@
 // reads the scales of just those two groups, and nothing is multiplied, read or exchanged twice.
 //
 // A tile of 16 outputs belongs to a team of `parts` warps that share its K range; teams and CTAs take the tiles in turn.
-// Items (16 rows x 512 columns, 4 KB) come by TMA into a ring of the warp's, two ahead and the first ones before the wait
-// for the preceding kernel; the tables of a tile's rows are one piece of memory and come by bulk copies.  The order of
+// Items (16 rows x 512 columns, 4 KB) come by TMA into a ring of the warp's, one ahead of the one being read and the first before
+// the wait for the preceding kernel; the tables of a tile's rows are one piece of memory and come by bulk copies.  The order of
 // the sums is a function of (K, N, device).
 #pragma once
 

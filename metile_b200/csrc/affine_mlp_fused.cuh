@@ -26,7 +26,7 @@
 // launch, us, called from Python and in a replayed graph: byte-permutes and FMAs on the CUDA cores in a cooperative
 // launch 16.4 and 15.1, products on mma.sync 16.2, an ordinary launch (fused_meet) of sixteen warps with all weights of a
 // CTA on their way at once 13.2 and 15.3, eight warps and room for two CTAs per SM, so that the next launch begins its
-// copies behind the meeting, 13.2 and 12.6.
+// copies behind the meeting, 13.2 and 12.6 (with centred codes and small meeting slots, as now, 12.8 and 12.7).
 #pragma once
 
 #include <cuda.h>
@@ -45,10 +45,11 @@ constexpr int kFusedOneWarps = 8;
 constexpr int kFusedOneThreads = kFusedOneWarps * 32;
 constexpr int kFusedMaxRows = 4;
 // Rows the one-row kernel serves by default; two to four only when asked with MT_FLAG_MLP_FUSED.  The rule
-// for one row is older than affine_gemv_mma.cuh: at hidden / intermediate widths of 1024 / 1024, 1024 / 4096, 2048 / 4096, 2048 / 8192, 4096 /
-// 4096, 4096 / 8192 this kernel takes 6.1 / 6.8 / 8.2 / 12.6 / 12.1 / 21.4 us in a replayed graph (before: 9.2 / 8.1 / 10.9 / 15.1 / 15.9 /
-// 23.6), two projections called one after the other, which overlap more, 4.9 / 6.3 / 8.2 / 10.9 / 11.2 / 17.7.  The order of a
-// row's sums differs between the two.
+// for one row is older than affine_gemv_mma.cuh and no longer the faster one everywhere: at hidden / intermediate widths of 1024 / 1024, 1024 /
+// 4096, 2048 / 4096, 2048 / 8192, 4096 / 4096, 4096 / 8192 this kernel takes 6.2 / 7.0 / 8.3 / 13.2 / 12.8 / 22.2 us in a replayed graph
+// (on the CUDA cores 9.2 / 8.1 / 10.9 / 15.1 / 15.9 / 23.6), two projections called one after the other, which overlap more, 5.4 / 6.6 /
+// 8.6 / 11.4 / 11.8 / 18.5 (launch after launch: 6.5 / 7.6 / 9.3 / 13.8 / 13.4 / 22.8 and 8.5 / 8.0 / 9.2 / 12.2 / 12.7 / 19.5).  A row
+// keeps the order of its sums by it, which differs between the two.
 constexpr int kFusedDefaultRows = 1;
 constexpr int kFusedMaxSlots = 12;
 constexpr int kFusedItemRows = 16;  // gate/up rows per ring item of the eight-column kernel
@@ -497,9 +498,9 @@ affine_mlp_fused_kernel(const __grid_constant__ FusedMlpParams p) {
 // rows share their banks (4-way conflicts, 1.5 M extra wavefronts per launch), so the gate|up rows arrive
 // as 128-byte-swizzled tensor-map boxes and fragment row g is given weight row 2 (g % 4) + g / 4, which
 // makes the four rows' swizzles differ; scales and biases are read four groups per load (their rows lie
-// 64 or 256 bytes apart, again in the same banks).  Measured at the Llama-3.2-1B shape: 19.2-19.5 us for
-// 1-8 rows (22 us with dense rows, 20.3 us before the wide table loads) against 25.4-25.9 us on the
-// two-kernel tensor-core path, so it is the default for two to eight rows.
+// 64 or 256 bytes apart, again in the same banks).  Steps of its making at 2048 / 8192, eight rows, in a cooperative launch: one
+// chain 25.6 us, four 22.5, swizzled boxes 20.1, wide table loads 19.5; in the ordinary launch of now 18.5 in a
+// replayed graph and 18.3 called from Python (20.5 before).  Why two to eight rows take it: see mt_affine_mlp.
 //
 // A producer warp feeds one ring; the CTAs meet as above.  The K range is cut into one slice per compute warp; every
 // warp walks all rows of an item for its slice; the warps' partial 16 x 8 tiles meet in shared memory

@@ -389,8 +389,8 @@ int mt_affine_mlp(const void* x, const uint32_t* gate_w, const void* gate_scales
         params.I = I;
         const int sms = device_sm_count();
         // Up to kFusedDefaultRows rows: the one-row kernel.  Above, to eight rows: the eight-column kernel, which does not round
-        // the weights (against the tcgen05 pair, us at 2 to 8 rows: 1024 / 1024 7.6 | 9.3, 2048 / 4096 12.1 | 15.0, 1024 / 4096
-        // 10.7 | 9.8, 2048 / 8192 18.6 | 18.1).
+        // the weights (against the tcgen05 pair, us at 2 and at 8 rows in a replayed graph: 1024 / 1024 7.7, 7.9 | 9.6, 9.9; 2048 / 4096 12.7, 13.3 |
+        // 15.0, 15.1; 1024 / 4096 10.4, 10.9 | 10.1, 10.3; 2048 / 8192 18.9, 19.7 | 17.5, 17.7).
         const bool want_mma = (flags & MT_FLAG_MLP_FUSED_MMA) != 0;
         const bool one_row = !want_mma && (family || M <= kFusedDefaultRows) && fused_mlp_applicable(params, sms);
         const bool mma = !one_row && (want_mma || (!family && M > kFusedDefaultRows)) && fused_mlp_mma_applicable(params, sms);
